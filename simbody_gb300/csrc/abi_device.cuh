@@ -41,6 +41,7 @@
 #include "engine.h"
 #include "spatial.cuh"
 #include "kernels.h"
+#include "steps_device.cuh"
 
 namespace sbg {
 
@@ -1346,34 +1347,6 @@ __global__ void __launch_bounds__(BS, MINB) realizeKernel(DevTables T, int first
     if (s.gl == 0) status[s.inst] = st;
 }
 
-// Mixed form: the instances of a segment (order positions [first, first +
-// count)) whose refinement reported an ill-conditioned M are recomputed in
-// FP64 on the FP64 mirror of their records, one thread per instance (the
-// level-parallel layout with a single lane). The other threads return at
-// once. T.fallbacks counts the recomputed instances.
-template <int NM, bool GROUP>
-__global__ void __launch_bounds__(128) realizeFallbackKernel(DevTables T, int first, int count,
-                                                             const double* __restrict__ y, double* __restrict__ ydot,
-                                                             int32_t* __restrict__ status) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int inst = T.order[first + t];
-    if (!(status[inst] & SBG_INST_ILL_CONDITIONED)) return;
-    YSrc src{y, T.ybase[inst], T.ystride[inst], T.inq[inst]};
-    YdOut out{ydot, T.ybase[inst], T.ystride[inst], T.inq[inst]};
-    int st;
-    if constexpr (GROUP) {
-        const ScrRows<double> S{T.scratch64 + T.sbase[inst], T.inb[inst]};
-        st = rhsGroup<double, NM, false>(T, inst, S, src, out, 0, 1, 1u << (threadIdx.x & 31));
-    } else {
-        const ScrTiled<double> S{T.scratch64 + T.sbase[inst]};
-        st = rhsChain<double, NM, false>(T, inst, S, src, out);
-    }
-    if (!out.finite) st |= SBG_INST_NONFINITE;
-    status[inst] = st;
-    atomicAdd(T.fallbacks, 1ULL);
-}
-
 template <class R, int NM, bool GROUP>
 __global__ void __launch_bounds__(128) minvKernel(DevTables T, int first, int count, const double* __restrict__ y,
                                                   const double* __restrict__ f, double* __restrict__ out,
@@ -1431,45 +1404,18 @@ __device__ __noinline__ int stageRhsMixedGroup(const DevTables& T, const Slot& s
     return r;
 }
 
-// Group g of G lanes of the FP64 list kernel: the g-th instance in FP64
-// mode at this launch.
-template <int G> __device__ __forceinline__ Slot listSlot(const DevTables& T, int launch) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = t / G, lane = threadIdx.x & 31;
-    const int* list = T.fbList + (int64_t)(launch & 1) * T.ninst;
-    const unsigned mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane & ~(G - 1));
-    return Slot{g < T.fbCount[launch & 1] ? list[g] : -1, t % G, G, mask};
-}
-
-// One-step launches of a mixed batch integration: the instance's mode at the
-// next launch (written by this launch's owner of the instance only); FP64
-// puts it on the next list.
-__device__ __forceinline__ void fbNext(const DevTables& T, int launch, int inst, bool fp64) {
-    const int k = (launch + 1) & 1;
-    T.fbMode[(int64_t)k * T.ninst + inst] = fp64 ? 1 : 0;
-    if (fp64) T.fbList[(int64_t)k * T.ninst + atomicAdd(T.fbCount + k, 1)] = inst;
-}
-
-// LIST: the FP64 steps of the instances in FP64 mode during the one-step
-// launches of a mixed batch integration (R = double, fbuf = the FP64 stage
-// planes, scratch = FP64 records at T.sbase per instance). With GROUP,
-// kFbLanes lanes per instance through the level-parallel driver on the
-// field-major layout; without, one thread per instance through the one-thread
-// driver on contiguous records.
-template <class R, int NM, bool REF, bool GROUP, int MINB = 1, bool LOOPS = false, int BS = 128, bool LIST = false>
+template <class R, int NM, bool REF, bool GROUP, int MINB = 1, bool LOOPS = false, int BS = 128>
 __global__ void __launch_bounds__(BS, MINB) rkMersonKernel(DevTables T, int first, int count, double* __restrict__ y,
                                                             double* __restrict__ time, R* __restrict__ fbuf,
                                                             int64_t fplane, R* __restrict__ scratch,
                                                             int32_t* __restrict__ status, double h, StepCtl sc,
                                                             double accuracy, double consTol, int projectEveryStep) {
-    static_assert(!LIST || (std::is_same<R, double>::value && !REF && !LOOPS), "the FP64 list is FP64");
-    const Slot s = LIST ? (GROUP ? listSlot<kFbLanes>(T, sc.launch) : listSlot<1>(T, sc.launch))
-                        : GROUP ? groupSlot(T, first) : chainSlot(T, first, count);
+    const Slot s = GROUP ? groupSlot(T, first) : chainSlot(T, first, count);
     if (s.inst < 0) return;
     const int inst = s.inst;
     // One-step launches of a mixed batch integration: an instance in FP64 mode
     // is the list kernel's at this launch.
-    const bool split = !LIST && REF && T.fbList != nullptr;
+    const bool split = REF && T.fbList != nullptr;
     if (split && T.fbMode[(int64_t)(sc.launch & 1) * T.ninst + inst]) return;
     bool toFp64 = false;  // split: this launch's mixed step met an ill-conditioned M
     const int64_t base = T.ybase[inst], stride = T.ystride[inst];
@@ -1518,9 +1464,7 @@ __global__ void __launch_bounds__(BS, MINB) rkMersonKernel(DevTables T, int firs
     auto stage = [&](int stg, double c, const R* a, const R* b, R* dst) {
         StageSrc<R> src{y, f0, a, b, base, stride, nq, stg, c};
         FOut<R> o{dst, base, stride, nq};
-        if constexpr (LIST && !GROUP) {
-            st |= rhsChain<R, NM, false>(T, inst, ScrStrided<R>{scratch + T.sbase[inst], 1}, src, o);
-        } else if constexpr (REF && GROUP) {
+        if constexpr (REF && GROUP) {
             bool fin = true;
             const bool was64 = rhs64;
             st |= stageRhsMixedGroup<NM, R>(T, s, scratch, fallback, &rhs64, y, f0, a, b, base, stride, nq, stg, c,
@@ -1702,17 +1646,10 @@ __global__ void __launch_bounds__(BS, MINB) rkMersonKernel(DevTables T, int firs
         --left;
         if (s.gl == 0) {
             if (T.stepsLeft) T.stepsLeft[inst] = left;
-            if constexpr (LIST) {
-                --T.fbLeft[inst];
-                atomicAdd(T.fbSteps, 1ULL);
-            }
         }
     }
     if (s.gl == 0) {
-        if constexpr (LIST) fbNext(T, sc.launch, inst, T.fbLeft[inst] > 0);
-        else if (split) fbNext(T, sc.launch, inst, toFp64);
-    }
-    if (s.gl == 0) {
+        if (split) fbNext(T, sc.launch, inst, toFp64);
         time[inst] = tc;
         status[inst] = st;
     }

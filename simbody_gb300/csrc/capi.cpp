@@ -61,6 +61,7 @@ bool isIdentityR(const double* X) {
 }  // namespace
 
 #include "topology_internal.h"
+#include "tile_program.h"
 
 namespace sbg {
 int setError(int code, const std::string& msg) {
@@ -130,8 +131,15 @@ struct sbg_batch_s {
     cudaEvent_t evT0 = nullptr, evT1 = nullptr;
     bool tuned = false;
     cudaGraphExec_t realizeGraph = nullptr;  // captured after tuning
-    // tree operators (allocated on first use): FP64 scratch for a batch whose
-    // own scratch is FP32, device operands and results in the host packing,
+    // FP64 on the tile driver: the tiles of the chain and group segments (FP64
+    // batches; mixed ones once an integration has switched to FP64), and one
+    // tile per instance (mixed batches)
+    std::vector<sbg_topology_s*> topos;      // the topologies used, held
+    std::vector<int32_t> topoOf;             // per instance, its index in topos
+    std::vector<int32_t> order;              // order position -> instance
+    TileSet tiles{}, ones{};
+    int tileWidth = kTile;                   // instances per tile of `tiles`
+    // tree operators (allocated on first use): FP64 scratch, device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
     void* opsScratch = nullptr;
     double* opsDev = nullptr;
@@ -140,7 +148,6 @@ struct sbg_batch_s {
     int64_t* dHostBOff = nullptr;
     cudaEvent_t evOp0 = nullptr, evOp1 = nullptr;  // bracket the last tree operator's kernels
     // one-step launches of a mixed batch integration (allocated on first use)
-    std::vector<int64_t> rowsElems;   // FP64 level-parallel record elements per instance (0: loop closures)
     int32_t* fbList = nullptr;        // 2 x ninst
     int32_t* fbCount = nullptr;       // 2, then the unfinished count
     int32_t* fbMode = nullptr;        // 2 x ninst
@@ -152,19 +159,21 @@ struct sbg_batch_s {
     double* fbuf64 = nullptr;
     unsigned long long* fbSteps = nullptr;
     long long* adaptStats = nullptr;  // accepted / rejected steps of the error-controlled integrator
-    int64_t* rowsBase = nullptr;
-    double* rows = nullptr;
     cudaStream_t fbStream = nullptr;
     cudaEvent_t fbFork = nullptr, fbJoin = nullptr;
 
     Streams streams() const { return Streams{stream, stream2, evFork, evJoin}; }
     LaunchPlan plan() const { return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop}; }
-    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems}; }
-    int segments() const { return (nChain > 0) + (nLoop > 0) + (nGroupBlocks > 0); }
+    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones}; }
+    // kernels of one pass over the batch
+    int segments() const {
+        if (precision == SBG_PRECISION_FP64) return (tiles.ntiles > 0) + (nLoop > 0);
+        return (nChain > 0) + (nLoop > 0) + (nGroupBlocks > 0);
+    }
     // kernels of one realize: the segments, and in the mixed form the FP64
     // recomputation pass after the chain and the level-parallel segment
     int realizeLaunches() const {
-        return segments() + (T.scratch64 ? (nChain > 0) + (nGroupBlocks > 0) : 0);
+        return segments() + (precision == SBG_PRECISION_MIXED ? (nChain > 0) + (nGroupBlocks > 0) : 0);
     }
 
     // Lanes per instance of the group segment: blocks of 128 threads hold
@@ -199,6 +208,7 @@ struct sbg_batch_s {
     ~sbg_batch_s() {
         if (device >= 0) cudaSetDevice(device);
         for (auto& b : bufs) cudaFree(b.p);
+        for (sbg_topology_s* t : topos) releaseTopology(t);
         if (hostPinned) cudaFreeHost(hostPinned);
         if (opsHost) cudaFreeHost(opsHost);
         if (realizeGraph) cudaGraphExecDestroy(realizeGraph);
@@ -447,7 +457,7 @@ int sbg_topology_create(const sbg_system_desc* d, sbg_topology* out) {
 }
 
 int sbg_topology_destroy(sbg_topology t) {
-    delete t;
+    releaseTopology(t);  // batches that use it keep theirs
     return SBG_OK;
 }
 
@@ -470,6 +480,105 @@ int sbg_topology_default_state(sbg_topology t, double* y) {
 }
 
 // --------------------------------------------------------------------- batch
+}  // extern "C"
+
+// The tile set of a batch's FP64 work: the chain and group segments' tiles, or
+// (single) one tile per instance that isn't in the loop-closure segment, with
+// records for every block of a launch that fills the GPU.
+static int buildTiles(sbg_batch b, bool single, TileSet* out) {
+    using namespace tile;
+    int sms = 0;
+    SBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "device attribute");
+    std::vector<TileRows> store;
+    std::vector<const TileRows*> rows(b->topos.size(), nullptr);
+    std::vector<int64_t> rowBase(b->topos.size(), 0);
+    std::vector<double> par;
+    store.reserve(b->topos.size());
+    TileProgram P;
+    bool gen = false;
+    for (size_t k = 0; k < b->topos.size(); ++k) {
+        if (b->topos[k]->ncons > 0) continue;  // the loop-closure segment's
+        store.emplace_back(*b->topos[k]);
+        rows[k] = &store.back();
+        rowBase[k] = (int64_t)par.size() / PR_COUNT;
+        par.insert(par.end(), rows[k]->par.begin(), rows[k]->par.end());
+        gen |= rows[k]->gen;
+        P.pose |= rows[k]->pose;
+    }
+    P.rs = gen ? RC_GEN : RC_SMALL;
+    P.rsTotal = P.rs + (P.pose ? RC_POSE : 0);
+    std::vector<int> at;  // topologies of the segments' positions
+    for (int p = 0; p < b->ninst; ++p)
+        if (p < b->nChain || p >= b->nChain + b->nLoop) at.push_back(b->topoOf[b->order[p]]);
+    *out = TileSet{};
+    if (at.empty()) return SBG_OK;
+    if (single) {
+        P.W = 4;  // one warp per sub-partition
+        std::vector<TileDesc> per(b->ninst, TileDesc{});
+        for (int i = 0; i < b->ninst; ++i) {
+            if (b->topos[b->topoOf[i]]->ncons > 0) continue;
+            P.add(0, {b->topoOf[i]}, 1, rows, rowBase);
+            per[i] = P.desc.back();
+            per[i].rec0 = 0;
+        }
+        P.desc.swap(per);
+    } else {
+        int TW = 32;
+        TileProgram::shape(at, rows, 4 * sms, TW, P.W);
+        b->tileWidth = TW;
+        for (const auto& seg : {std::make_pair(0, b->nChain), std::make_pair(b->nChain + b->nLoop, b->ninst)})
+            for (int p = seg.first; p < seg.second; p += TW) {
+                std::vector<int> lanes;
+                for (int k = p; k < std::min(seg.second, p + TW); ++k) lanes.push_back(b->topoOf[b->order[k]]);
+                P.add(p, lanes, TW, rows, rowBase);
+            }
+    }
+    out->ntiles = (int)P.desc.size();
+    out->tt.W = P.W;
+    out->tt.rs = P.rs;
+    out->tt.rsTotal = P.rsTotal;
+    out->tt.pose = P.pose;
+    int rc;
+    if ((rc = b->upload(&out->tt.desc, P.desc, "tile table"))) return rc;
+    if ((rc = b->upload(&out->tt.cls, P.cls, "tile table"))) return rc;
+    if ((rc = b->upload(&out->tt.slots, P.slots, "tile table"))) return rc;
+    void* p = nullptr;
+    const int64_t nPar = (int64_t)P.parRow.size() * PR_COUNT;
+    if ((rc = b->alloc(&p, std::max<int64_t>(nPar, 1) * sizeof(double), "tile parameters"))) return rc;
+    out->tt.par = static_cast<double*>(p);
+    if (single) {  // tables without lanes: the rows in slot order
+        std::vector<double> v(std::max<int64_t>(nPar, 1));
+        for (size_t k = 0; k < P.parRow.size(); ++k)
+            if (P.parRow[k] >= 0) std::copy_n(&par[(size_t)P.parRow[k] * PR_COUNT], PR_COUNT, &v[k * PR_COUNT]);
+        SBG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice), "tile parameters");
+        out->blocks = 4 * sms;
+        out->recStride = P.maxTile;
+        if ((rc = b->alloc(&p, (int64_t)out->blocks * out->recStride * sizeof(double), "FP64 records"))) return rc;
+    } else {
+        void *dRow = nullptr, *dPar = nullptr;
+        cudaError_t e = cudaMalloc(&dRow, std::max<size_t>(P.parRow.size(), 1) * sizeof(int32_t));
+        if (e == cudaSuccess) e = cudaMalloc(&dPar, par.size() * sizeof(double));
+        if (e == cudaSuccess)
+            e = cudaMemcpy(dRow, P.parRow.data(), P.parRow.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(dPar, par.data(), par.size() * sizeof(double), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = launchTilePar(out->tt.desc, out->ntiles, P.W, static_cast<int32_t*>(dRow), static_cast<double*>(dPar),
+                              PR_COUNT, static_cast<double*>(p), b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+        cudaFree(dRow);
+        cudaFree(dPar);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return cudaFail(e, "tile parameters");
+        }
+        if ((rc = b->alloc(&p, std::max<int64_t>(P.recElems, 1) * sizeof(double), "FP64 records"))) return rc;
+    }
+    out->recs = static_cast<double*>(p);
+    return SBG_OK;
+}
+
+extern "C" {
+
 int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
                      const sbg_batch_config* cfg, sbg_batch* out) {
     if (!topos || ntopo < 1 || !instTopo || ninst < 0 || !out) return fail(SBG_ERR_INVALID, "bad batch arguments");
@@ -499,6 +608,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     b->budget = cfg ? cfg->device_budget_bytes : 0;
     b->ninst = ninst;
     b->instTopo.assign(instTopo, instTopo + ninst);
+    b->topoOf.resize(ninst);
     auto bail = [&](int rc) { delete b; return rc; };
     {
         cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -521,7 +631,9 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     for (int i = 0; i < ninst; ++i) {
         const int k = instTopo[i];
         if (used[k] >= 0) continue;
-        used[k] = 1;
+        used[k] = (int)b->topos.size();
+        topos[k]->refs.fetch_add(1);
+        b->topos.push_back(topos[k]);
         const sbg_topology_s* t = topos[k];
         rowBase[k] = (int32_t)parent.size();
         const int32_t fOff = (int32_t)fkw.size();
@@ -584,19 +696,22 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         inb[i] = t->nb;
         inq[i] = t->nq;
         inu[i] = t->nu;
+        b->topoOf[i] = used[instTopo[i]];
         ilev[i] = levBase[instTopo[i]];
         inlev[i] = t->nlevels;
         for (int k = 0; k < 3; ++k) grav[3 * i + k] = t->gravity[k];
         b->hostYOff[i + 1] = b->hostYOff[i] + t->nq + t->nu;
         b->hostUOff[i + 1] = b->hostUOff[i] + t->nu;
         b->hostBOff[i + 1] = b->hostBOff[i] + t->nb;
-        b->rowsElems.push_back(t->ncons > 0 ? 0 : (int64_t)t->nb * rowsRecordWidth(*t, 3));
         if (t->ncons > 0) loopPos.push_back(i);
         else if (t->chain || t->maxLevelWidth <= 2 || t->nb < groupMinBodies) chainPos.push_back(i);
         else groupPos.push_back(i);
     }
     if (!uniform) {
-        std::stable_sort(chainPos.begin(), chainPos.end(), [&](int a, int c) { return inb[a] > inb[c]; });
+        // largest first; instances of one topology side by side
+        std::stable_sort(chainPos.begin(), chainPos.end(), [&](int a, int c) {
+            return inb[a] != inb[c] ? inb[a] > inb[c] : instTopo[a] < instTopo[c];
+        });
         std::stable_sort(loopPos.begin(), loopPos.end(), [&](int a, int c) { return inb[a] > inb[c]; });
         auto wkey = [&](int i) { int w = 1; while (w < topos[instTopo[i]]->maxLevelWidth) w <<= 1; return w; };
         std::stable_sort(groupPos.begin(), groupPos.end(), [&](int a, int c) {
@@ -611,6 +726,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     std::copy(chainPos.begin(), chainPos.end(), order.begin());
     std::copy(loopPos.begin(), loopPos.end(), order.begin() + b->nChain);
     std::copy(groupPos.begin(), groupPos.end(), order.begin() + b->nChain + b->nLoop);
+    b->order = order;
     // slot records of the loop-closure topologies follow their body records
     std::vector<int32_t> lrec(parent.size(), -1), lslot(parent.size(), -1);
     for (int k = 0; k < ntopo; ++k) {
@@ -775,16 +891,19 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     b->status = static_cast<int32_t*>(p);
     if ((rc = b->alloc(&p, std::max<int64_t>(b->nyTotal, 1) * sizeof(double), "staging"))) return bail(rc);
     b->staging = static_cast<double*>(p);
-    if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
-    if (precision == SBG_PRECISION_MIXED && b->scratchElems > 0) {
-        // FP64 mirror of the scratch for the instances whose refinement
-        // reports an ill-conditioned M, and the count of those recomputed
-        if ((rc = b->alloc(&p, b->scratchElems * sizeof(double), "FP64 scratch mirror"))) return bail(rc);
-        T.scratch64 = static_cast<double*>(p);
-        if ((rc = b->alloc(&p, sizeof(unsigned long long), "fallback counter"))) return bail(rc);
-        T.fallbacks = static_cast<unsigned long long*>(p);
-        const cudaError_t ez = cudaMemset(p, 0, sizeof(unsigned long long));
-        if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counter"));
+    if (precision == SBG_PRECISION_FP64) {
+        if ((rc = buildTiles(b, false, &b->tiles))) return bail(rc);
+    } else {
+        if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
+        if (precision == SBG_PRECISION_MIXED) {
+            // FP64 tiles for the instances whose refinement reports an
+            // ill-conditioned M, and the count of those recomputed
+            if ((rc = buildTiles(b, true, &b->ones))) return bail(rc);
+            if ((rc = b->alloc(&p, sizeof(unsigned long long), "fallback counter"))) return bail(rc);
+            T.fallbacks = static_cast<unsigned long long*>(p);
+            const cudaError_t ez = cudaMemset(p, 0, sizeof(unsigned long long));
+            if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counter"));
+        }
     }
     if ((rc = b->alloc(&b->fbuf, 4 * std::max<int64_t>(b->colElems, 1) * rsz, "stage derivatives"))) return bail(rc);
     if (b->nLoop > 0) {
@@ -891,6 +1010,10 @@ static int timePlan(sbg_batch b, float* ms) {
 
 static int tuneVariant(sbg_batch b) {
     if (b->tuned) return SBG_OK;
+    if (b->precision == SBG_PRECISION_FP64) {  // the tiles' shape is chosen when they are built
+        b->tuned = true;
+        return SBG_OK;
+    }
     if (!b->evT0) {
         SBG_CUDA(cudaEventCreate(&b->evT0), "tuner");
         SBG_CUDA(cudaEventCreate(&b->evT1), "tuner");
@@ -990,7 +1113,8 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     int nchunks = 4;
     if (const char* v = std::getenv("SBG_PIPE_CHUNKS")) nchunks = std::max(1, std::atoi(v));  // tuning override
     nchunks = std::min(nchunks, 16);
-    const bool pipelined = b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 && b->tuned && nchunks > 1 &&
+    const bool pipelined = b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 &&
+                           (b->tuned || b->precision == SBG_PRECISION_FP64) && nchunks > 1 &&
                            b->ninst >= nchunks * kTile;
     if (!pipelined) {
         if (int rc = sbg_batch_set_state(b, nullptr, y)) return rc;
@@ -1043,8 +1167,16 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
         P.chainFirst = i0;
         P.nChain = i1 - i0;
         a.P = &P;
-        if (b->precision == SBG_PRECISION_FP64) realize64Chain(a, st);
-        else realize32Chain(a, b->precision == SBG_PRECISION_MIXED, st);
+        if (b->precision == SBG_PRECISION_FP64) {  // chunks start at multiples of 32, so of the tile width
+            const int t0 = i0 / b->tileWidth, t1 = (i1 + b->tileWidth - 1) / b->tileWidth;
+            realizeTiles(a, b->tiles, t0, t1 - t0, st);
+        } else {
+            realize32Chain(a, b->precision == SBG_PRECISION_MIXED, st);
+            if (b->precision == SBG_PRECISION_MIXED) {
+                const int share = b->ones.blocks / 3;  // three streams' chunks at a time
+                realizeFallbackTiles(a, b->ones, i0, i1 - i0, (c % 3) * share, share, st);
+            }
+        }
         SBG_CUDA(cudaGetLastError(), "realize launch");
         SBG_CUDA(launchGather(b->T, b->dHostYOff, b->ydot, b->staging, 0, st, i0, i1 - i0), "derivative gather");
         SBG_CUDA(cudaEventRecord(b->pipeEv[1][c], st), "pipeline");
@@ -1054,7 +1186,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
         if (stPinned)
             SBG_CUDA(cudaMemcpyAsync(status + i0, b->status + i0, (i1 - i0) * sizeof(int32_t), cudaMemcpyDeviceToHost,
                                      down), "status download");
-        b->launches += 3 + (b->T.scratch64 ? 1 : 0);
+        b->launches += 3 + (b->precision == SBG_PRECISION_MIXED ? 1 : 0);
     }
     if (status && !stPinned)
         SBG_CUDA(cudaMemcpyAsync(status, b->status, b->ninst * sizeof(int32_t), cudaMemcpyDeviceToHost, down),
@@ -1098,10 +1230,8 @@ static int ensureTreeOps(sbg_batch b) {
     if (b->opsDev && b->opsElems >= need) return SBG_OK;
     int rc;
     void* p = nullptr;
-    if (b->precision != SBG_PRECISION_FP64 && !b->opsScratch && b->scratchElems > 0) {
-        if (b->T.scratch64) b->opsScratch = b->T.scratch64;  // the mixed form's FP64 mirror has the layout
-        else if ((rc = b->alloc(&b->opsScratch, b->scratchElems * sizeof(double), "tree-operator scratch"))) return rc;
-    }
+    if (!b->opsScratch && b->scratchElems > 0)
+        if ((rc = b->alloc(&b->opsScratch, b->scratchElems * sizeof(double), "tree-operator scratch"))) return rc;
     if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
     b->opsDev = static_cast<double*>(p);
     const int64_t* dOff = nullptr;
@@ -1144,8 +1274,7 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     if (int rc = up(fmob, dF, nu, "mobility force upload")) return rc;
     if (int rc = up(fbody, dB, 6 * nbT, "body force upload")) return rc;
     OpIO io{kind, x ? dX : nullptr, fmob ? dF : nullptr, fbody ? dB : nullptr, dOut, b->dHostUOff, b->dHostBOff};
-    double* sc = b->precision == SBG_PRECISION_FP64 ? static_cast<double*>(b->scratch)
-                                                     : static_cast<double*>(b->opsScratch);
+    double* sc = static_cast<double*>(b->opsScratch);
     SBG_CUDA(cudaEventRecord(b->evOp0, b->stream), "event");
     SBG_CUDA(launchTreeOp(b->T, b->plan(), io, b->y, sc, static_cast<double*>(b->scratchLoop), b->status, b->stream),
              "tree-operator kernel launch");
@@ -1234,8 +1363,8 @@ static int64_t stepsToReach(double t0, double tStop, double h) {
 
 // Buffers of the one-step launches of a mixed batch integration (allocated
 // on first use): the two FP64-mode lists and their lengths, the per-instance
-// FP64 modes and step counters, the FP64 stage planes, FP64 records of the
-// level-parallel layout for the list kernel, its stream and events.
+// FP64 modes and step counters, the FP64 stage planes, the list kernel's
+// stream and events.
 static int ensureFallbackSteps(sbg_batch b) {
     if (b->fbList) return SBG_OK;
     void* p = nullptr;
@@ -1257,13 +1386,6 @@ static int ensureFallbackSteps(sbg_batch b) {
     if ((rc = b->alloc(&p, sizeof(unsigned long long), "FP64 step counter"))) return rc;
     b->fbSteps = static_cast<unsigned long long*>(p);
     SBG_CUDA(cudaMemsetAsync(b->fbSteps, 0, sizeof(unsigned long long), b->stream), "FP64 step counter");
-    std::vector<int64_t> base(n + 1, 0);
-    for (int64_t i = 0; i < n; ++i) base[i + 1] = base[i] + b->rowsElems[i];
-    if ((rc = b->alloc(&p, std::max<int64_t>(base[n], 1) * sizeof(double), "FP64 level-parallel records"))) return rc;
-    b->rows = static_cast<double*>(p);
-    const int64_t* dBase = nullptr;
-    if ((rc = b->upload(&dBase, base, "FP64 record offsets"))) return rc;
-    b->rowsBase = const_cast<int64_t*>(dBase);
     SBG_CUDA(cudaStreamCreateWithFlags(&b->fbStream, cudaStreamNonBlocking), "stream");
     SBG_CUDA(cudaEventCreateWithFlags(&b->fbFork, cudaEventDisableTiming), "event");
     SBG_CUDA(cudaEventCreateWithFlags(&b->fbJoin, cudaEventDisableTiming), "event");
@@ -1318,22 +1440,19 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
         target = stepsToReach(*std::min_element(t0.begin(), t0.end()), tStop, h);
     }
     const LaunchPlan P = b->plan();
-    // FP64 steps: kFbLanes level-parallel lanes per instance (measured faster
-    // than one thread per instance: 2.4x on the uneven trees, 6 % on the
-    // random trees)
-    int fbLanes = kFbLanes;
-    if (const char* v = std::getenv("SBG_FB_LANES")) fbLanes = std::atoi(v) > 1 ? kFbLanes : 1;  // tuning override
     const int64_t limit = 2 * target + 64;
-    // The FP64 persistent kernels, on the FP64 mirror of the records, take
-    // every instance's remaining steps once the integration has switched.
+    // The FP64 persistent kernels take every instance's remaining steps once
+    // the integration has switched.
     auto allFp64 = [&]() -> int {
-        const BatchBufs B64{b->T.scratch64, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64,
-                            b->colElems};
+        if (!b->tiles.ntiles)
+            if (int rc = buildTiles(b, false, &b->tiles)) return rc;
+        const BatchBufs B64{nullptr, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64, b->colElems,
+                            &b->tiles, &b->ones};
         const StepCtl step{nsteps >= 0 ? nsteps : -1, 0, tStop, 0, 0};
         SBG_CUDA(launchRKMerson(Tk, P, SBG_PRECISION_FP64, b->y, b->time, B64, b->status, h, step, acc, ctol, pes,
                                 b->streams()),
                  "RK-Merson kernel launch");
-        b->launches += b->segments();
+        b->launches += (b->tiles.ntiles > 0) + (b->nLoop > 0);
         return SBG_OK;
     };
     if (b->fbAllFp64) return allFp64();
@@ -1363,8 +1482,8 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
             SBG_CUDA(launchRKMerson(Tk, P, b->precision, b->y, b->time, b->bufsArg(), b->status, h, step, acc, ctol, pes,
                                     b->streams()),
                      "RK-Merson kernel launch");
-            SBG_CUDA(launchRKFp64List(Tk, P, b->y, b->time, b->status, h, step, acc, ctol, pes, b->colElems, b->rowsBase,
-                                      b->rows, fbLanes, b->fbStream),
+            SBG_CUDA(launchRKFp64List(Tk, b->ones, b->y, b->time, b->status, h, step, acc, ctol, pes, b->colElems,
+                                      b->fbStream),
                      "FP64 list kernel launch");
             SBG_CUDA(cudaEventRecord(b->fbJoin, b->fbStream), "join");
             SBG_CUDA(cudaStreamWaitEvent(b->stream, b->fbJoin, 0), "join");
@@ -1508,21 +1627,9 @@ int sbg_rk_merson_adaptive(sbg_batch b, double t_final, const sbg_adaptive_opts*
     a.time = b->time;
     a.fbuf = b->fbuf;
     a.fplane = b->colElems;
-    a.scratch = b->scratch;
     a.status = b->status;
-    const Streams ss = b->streams();
-    const bool both = P.nChain > 0 && P.nGroupBlocks > 0;
-    if (both) {
-        SBG_CUDA(cudaEventRecord(ss.fork, ss.main), "fork");
-        SBG_CUDA(cudaStreamWaitEvent(ss.side, ss.fork, 0), "fork");
-    }
-    rkAdaptiveChain(a, ac, ss.main);
-    rkAdaptiveGroup(a, ac, both ? ss.side : ss.main);
+    rkAdaptiveTiles(a, b->tiles, ac, b->stream);
     SBG_CUDA(cudaGetLastError(), "error-controlled RK-Merson launch");
-    if (both) {
-        SBG_CUDA(cudaEventRecord(ss.join, ss.side), "join");
-        SBG_CUDA(cudaStreamWaitEvent(ss.main, ss.join, 0), "join");
-    }
     b->launches += 1 + b->segments();
     b->integrating = false;  // the fixed-step integrator has nothing to continue
     b->realized = false;

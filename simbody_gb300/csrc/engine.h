@@ -168,8 +168,6 @@ constexpr int kContactStride = 20;
 // FP64 steps an instance takes, from the step whose mixed RHS met an
 // ill-conditioned M, before it tries the mixed form again.
 constexpr int kFp64Steps = 16;
-// Lanes per instance of the FP64 list kernel (level-parallel driver).
-constexpr int kFbLanes = 8;
 constexpr int kCtlSteps = (1 << 24) - 1;
 constexpr int kCtlInit = 1 << 30;                // first launch: Integrator::initialize projections
 constexpr int kCtlProjectEveryStep = 1 << 29;    // Integrator::setProjectEveryStep(true)
@@ -203,6 +201,33 @@ struct LaunchPlan {
     int groupFirst;  // first block of the level-parallel launch in the block table
     int nLoopGroupBlocks;  // blocks [loopGroupFirst, +n): loop-closure instances on the level-parallel driver (FP64)
     int loopGroupFirst;
+};
+
+// Tile driver (FP64, tile_device.cuh). A tile is up to 32 instances, one per
+// lane, swept by the W warps of a block in the steps of its schedule.
+struct TileDesc {
+    int32_t pos0, lanes;   // order positions [pos0, pos0 + lanes)
+    int32_t nsteps, cls0;  // classes at cls0 + step * W + warp
+    int32_t ls, shared;    // lane stride of the records; 1: one topology, tables without lanes
+    int64_t slot0, par0, rec0;
+};
+struct TileTables {
+    const TileDesc* desc;
+    const int32_t* cls;
+    const int32_t* slots;  // integers per (step, warp) slot and lane
+    const double* par;     // parameters per slot and lane
+    int32_t W;
+    int32_t rs, rsTotal;   // doubles of a body's record without and with the Ground pose
+    int32_t pose;          // some body carries contact spheres
+};
+// A batch's tiles with their records; or one tile per instance, swept one at a
+// time by each of `blocks` blocks on records of its own (recStride doubles).
+struct TileSet {
+    TileTables tt;
+    int32_t ntiles;
+    double* recs;
+    int32_t blocks;
+    int64_t recStride;
 };
 
 }  // namespace sbg

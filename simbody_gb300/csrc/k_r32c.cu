@@ -1,6 +1,6 @@
 // k_r32c.cu -- realize(Acceleration) kernel instantiations, FP32 recursions,
-// chain driver: the dispatch and the unrefined form (the refined form, with
-// its FP64 recomputation pass, is in k_r32cr.cu; variant 8, the staged chain
+// chain driver: the dispatch and the unrefined form (the refined form is in
+// k_r32cr.cu; variant 8, the staged chain
 // driver of one shared chain topology, in k_r32s.cu).
 #include "r32c_launch.cuh"
 

@@ -242,7 +242,6 @@ void realize32ChainStaged(const KArgs& a, bool refine, cudaStream_t s) {
     } else {
         if (refine) goStaged<3, true>(a, s); else goStaged<3, false>(a, s);
     }
-    if (refine) realizeFallback(a, false, s);
 }
 
 }  // namespace sbg

@@ -1,0 +1,90 @@
+// k_tile.cu -- FP64 realize(Acceleration) and M^-1 f on the tile driver, and
+// the FP64 recomputation of a mixed realize's ill-conditioned instances.
+#include "tile_device.cuh"
+
+namespace sbg {
+
+namespace {
+
+__global__ void __launch_bounds__(32 * kTileMaxWarps)
+    realizeTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int tile0,
+                      const double* __restrict__ y, double* __restrict__ ydot, double* __restrict__ recs,
+                      int32_t* __restrict__ status) {
+    __shared__ TileShare<0> sh;
+    const TileCtx c = tileCtx(T, TT, tile0 + blockIdx.x, recs);
+    const TileYSrc src{y, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
+    TileOut out{ydot, src.base, src.stride, src.nq};
+    int st = tileRhs<false>(T, TT, c, src, out, true);
+    if (!out.finite) st |= SBG_INST_NONFINITE;
+    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    if (c.on && c.w == 0) status[c.inst] = st;
+}
+
+__global__ void __launch_bounds__(32 * kTileMaxWarps)
+    minvTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, const double* __restrict__ y,
+                   const double* __restrict__ f, double* __restrict__ o, double* __restrict__ recs,
+                   int32_t* __restrict__ status) {
+    __shared__ TileShare<0> sh;
+    const TileCtx c = tileCtx(T, TT, blockIdx.x, recs);
+    const TileFSrc src{y, f, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
+    TileUOut out{o, src.base, src.stride, src.nq};
+    int st = tileRhs<true>(T, TT, c, src, out, true);
+    if (!out.finite) st |= SBG_INST_NONFINITE;
+    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    if (c.on && c.w == 0) status[c.inst] = st;
+}
+
+// The instances at order positions [first, first + count) whose mixed realize
+// reported an ill-conditioned M, one at a time per block on the block's own
+// records (TT: one tile per instance). T.fallbacks counts them.
+__global__ void __launch_bounds__(32 * kTileMaxWarps)
+    realizeFallbackTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int first,
+                              int count, const double* __restrict__ y, double* __restrict__ ydot,
+                              double* __restrict__ recs, int64_t recStride, int32_t* __restrict__ status) {
+    __shared__ TileShare<0> sh;
+    __shared__ int list[32 * kTileMaxWarps], n;
+    // each block takes every gridDim-th run of blockDim positions
+    for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x; p0 < count; p0 += (int64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x == 0) n = 0;
+        __syncthreads();
+        const int64_t p = p0 + threadIdx.x;
+        if (p < count) {
+            const int inst = T.order[first + p];
+            if (status[inst] & SBG_INST_ILL_CONDITIONED) list[atomicAdd(&n, 1)] = inst;
+        }
+        __syncthreads();
+        for (int k = 0; k < n; ++k) {
+            const TileCtx c = tileCtxOne(TT, list[k], recs + recStride * blockIdx.x);
+            const TileYSrc src{y, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
+            TileOut out{ydot, src.base, src.stride, src.nq};
+            int st = tileRhs<false>(T, TT, c, src, out, true);
+            if (!out.finite) st |= SBG_INST_NONFINITE;
+            st = tileReduce<0>(TT, c, sh, nullptr, st);
+            if (c.on && c.w == 0) {
+                status[c.inst] = st;
+                atomicAdd(T.fallbacks, 1ULL);
+            }
+        }
+        __syncthreads();  // the list is written again
+    }
+}
+
+}  // namespace
+
+void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s) {
+    if (ntiles <= 0) return;
+    realizeTileKernel<<<ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, tile0, a.y, a.ydot, S.recs, a.status);
+}
+void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s) {
+    if (S.ntiles <= 0) return;
+    minvTileKernel<<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, a.y, a.f, a.ydot, S.recs, a.status);
+}
+void realizeFallbackTiles(const KArgs& a, const TileSet& S, int first, int count, int block0, int blocks, cudaStream_t s) {
+    if (count <= 0) return;
+    const int bs = 32 * S.tt.W, need = (count + bs - 1) / bs;
+    realizeFallbackTileKernel<<<need < blocks ? need : blocks, bs, 0, s>>>(*a.T, S.tt, first, count, a.y, a.ydot,
+                                                                           S.recs + S.recStride * block0, S.recStride,
+                                                                           a.status);
+}
+
+}  // namespace sbg

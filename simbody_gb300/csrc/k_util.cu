@@ -144,6 +144,13 @@ static KArgs baseArgs(const DevTables& T, const LaunchPlan& P, const BatchBufs& 
     a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status;
     return a;
 }
+// FP64: the tiles, then the loop-closure segment, on the main stream.
+template <class FT, class FL>
+static cudaError_t tilesThenLoops(const LaunchPlan& P, const Streams& s, FT tiles, FL loops) {
+    tiles(s.main);
+    if (P.nLoop > 0) loops(s.main);
+    return cudaGetLastError();
+}
 
 cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision, const double* y, double* ydot,
                           const BatchBufs& B, int32_t* status, const Streams& s) {
@@ -151,11 +158,15 @@ cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision
     a.y = y; a.ydot = ydot;
     auto loops = [&](cudaStream_t st) { realizeLoop(a, st); };
     if (precision == SBG_PRECISION_FP64)
-        return forkJoin(P, s, [&](cudaStream_t st) { realize64Chain(a, st); }, loops,
-                        [&](cudaStream_t st) { realize64Group(a, st); });
+        return tilesThenLoops(P, s, [&](cudaStream_t st) { realizeTiles(a, *B.tiles, 0, B.tiles->ntiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
-    return forkJoin(P, s, [&](cudaStream_t st) { realize32Chain(a, ref, st); }, loops,
-                    [&](cudaStream_t st) { realize32Group(a, ref, st); });
+    const cudaError_t e = forkJoin(P, s, [&](cudaStream_t st) { realize32Chain(a, ref, st); }, loops,
+                                   [&](cudaStream_t st) { realize32Group(a, ref, st); });
+    if (e != cudaSuccess || !ref) return e;
+    if (P.nChain > 0) realizeFallbackTiles(a, *B.ones, 0, P.nChain, 0, B.ones->blocks, s.main);
+    const int group0 = P.nChain + P.nLoop;
+    if (P.nGroupBlocks > 0) realizeFallbackTiles(a, *B.ones, group0, T.ninst - group0, 0, B.ones->blocks, s.main);
+    return cudaGetLastError();
 }
 
 cudaError_t launchMInv(const DevTables& T, const LaunchPlan& P, int precision, const double* y, const double* f,
@@ -164,8 +175,7 @@ cudaError_t launchMInv(const DevTables& T, const LaunchPlan& P, int precision, c
     a.y = y; a.f = f; a.ydot = out;
     auto loops = [&](cudaStream_t st) { minvLoop(a, st); };
     if (precision == SBG_PRECISION_FP64)
-        return forkJoin(P, s, [&](cudaStream_t st) { minv64Chain(a, st); }, loops,
-                        [&](cudaStream_t st) { minv64Group(a, st); });
+        return tilesThenLoops(P, s, [&](cudaStream_t st) { minvTiles(a, *B.tiles, st); }, loops);
     return forkJoin(P, s, [&](cudaStream_t st) { minv32Chain(a, st); }, loops,
                     [&](cudaStream_t st) { minv32Group(a, st); });
 }
@@ -178,20 +188,41 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
     a.projectEveryStep = projectEveryStep;
     auto loops = [&](cudaStream_t st) { rkLoop(a, st); };
     if (precision == SBG_PRECISION_FP64)
-        return forkJoin(P, s, [&](cudaStream_t st) { rk64Chain(a, st); }, loops,
-                        [&](cudaStream_t st) { rk64Group(a, st); });
+        return tilesThenLoops(P, s, [&](cudaStream_t st) { rkTiles(a, *B.tiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
     return forkJoin(P, s, [&](cudaStream_t st) { rk32Chain(a, ref, st); }, loops,
                     [&](cudaStream_t st) { rk32Group(a, ref, st); });
 }
 
-cudaError_t launchRKFp64List(const DevTables& T, const LaunchPlan& P, double* y, double* time, int32_t* status,
-                             double h, StepCtl step, double accuracy, double consTol, int projectEveryStep,
-                             int64_t fplane, const int64_t* rowsBase, double* rows, int lanes, cudaStream_t s) {
+cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
+                             StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
+                             cudaStream_t s) {
     KArgs a{};
-    a.T = &T; a.P = &P; a.ystate = y; a.time = time; a.status = status; a.h = h; a.step = step;
+    a.T = &T; a.ystate = y; a.time = time; a.status = status; a.h = h; a.step = step;
     a.accuracy = accuracy; a.consTol = consTol; a.projectEveryStep = projectEveryStep; a.fplane = fplane;
-    rkFp64List(a, rowsBase, rows, lanes, s);
+    rkTilesList(a, S, s);
+    return cudaGetLastError();
+}
+
+// Parameters of the tiles' slots from the topologies' rows, across the lanes.
+__global__ void tileParKernel(const TileDesc* __restrict__ desc, int ntiles, int W, const int32_t* __restrict__ parRow,
+                              const double* __restrict__ rows, int count, double* __restrict__ par) {
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const TileDesc d = desc[t];
+        const int ls = d.shared ? 1 : d.ls;
+        const int64_t n = (int64_t)d.nsteps * W * ls, p0 = d.par0 / count;
+        for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
+            const int row = parRow[p0 + k];
+            if (row < 0) continue;
+            double* o = par + d.par0 + (k / ls) * count * ls + k % ls;
+            for (int f = 0; f < count; ++f) o[(int64_t)f * ls] = rows[(int64_t)row * count + f];
+        }
+    }
+}
+cudaError_t launchTilePar(const TileDesc* desc, int ntiles, int W, const int32_t* parRow, const double* rows, int count,
+                          double* par, cudaStream_t s) {
+    if (ntiles <= 0) return cudaSuccess;
+    tileParKernel<<<ntiles < 4096 ? ntiles : 4096, 256, 0, s>>>(desc, ntiles, W, parRow, rows, count, par);
     return cudaGetLastError();
 }
 

@@ -48,6 +48,8 @@ struct BatchBufs {
     void* fbuf;          // RK stage derivatives (R), 4 planes of fplane elements
     void* fbufLoop;      // FP64 stage derivatives of the loop-closure segment, 4 planes
     int64_t fplane;
+    const TileSet* tiles;  // FP64: the chain and group segments' tiles
+    const TileSet* ones;   // mixed form: one FP64 tile per instance
 };
 cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision, const double* y, double* ydot,
                           const BatchBufs& B, int32_t* status, const Streams& s);
@@ -137,10 +139,18 @@ struct KArgs {
     StepCtl step;
     int projectEveryStep;
 };
-void realize64Chain(const KArgs& a, cudaStream_t s);
-void realize64Group(const KArgs& a, cudaStream_t s);
-void minv64Chain(const KArgs& a, cudaStream_t s);
-void minv64Group(const KArgs& a, cudaStream_t s);
+// Tile driver, FP64 (k_tile.cu, k_tilerk.cu, k_tileadapt.cu).
+void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s);
+void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s);
+void rkTiles(const KArgs& a, const TileSet& S, cudaStream_t s);
+void rkAdaptiveTiles(const KArgs& a, const TileSet& S, const AdaptCtl& ac, cudaStream_t s);
+// FP64 recomputation of the instances at order positions [first, first +
+// count) that a mixed realize flagged SBG_INST_ILL_CONDITIONED, on the records
+// of the set's blocks [block0, block0 + blocks).
+void realizeFallbackTiles(const KArgs& a, const TileSet& S, int first, int count, int block0, int blocks, cudaStream_t s);
+// One FP64 RK-Merson step for each instance in FP64 mode at this launch
+// (T.fbList[launch & 1]).
+void rkTilesList(const KArgs& a, const TileSet& S, cudaStream_t s);
 void realize32Chain(const KArgs& a, bool refine, cudaStream_t s);
 // Variant 8: the chain driver with record fields staged through shared
 // memory (one shared chain topology, no Free bodies, segment start a
@@ -149,27 +159,19 @@ void realize32ChainStaged(const KArgs& a, bool refine, cudaStream_t s);
 void realize32Group(const KArgs& a, bool refine, cudaStream_t s);
 void minv32Chain(const KArgs& a, cudaStream_t s);
 void minv32Group(const KArgs& a, cudaStream_t s);
-void rk64Chain(const KArgs& a, cudaStream_t s);
 void rk64Group(const KArgs& a, cudaStream_t s);
 void rk32Chain(const KArgs& a, bool refine, cudaStream_t s);
 void rk32Group(const KArgs& a, bool refine, cudaStream_t s);
-// FP64 recomputation of the instances the mixed realize flagged
-// SBG_INST_ILL_CONDITIONED (k_fallback.cu); a no-op without T.scratch64.
-void realizeFallback(const KArgs& a, bool group, cudaStream_t s);
 void realizeLoop(const KArgs& a, cudaStream_t s);  // k_loops.cu
 void minvLoop(const KArgs& a, cudaStream_t s);
 void rkLoop(const KArgs& a, cudaStream_t s);
 void rkLoopWidth1(const KArgs& a, cudaStream_t s);  // k_rkloops1.cu: rkLoop for batch width 1
 void rkLoopGroup(const KArgs& a, cudaStream_t s);      // loop closures, level-parallel driver
-void rkAdaptiveChain(const KArgs& a, const AdaptCtl& ac, cudaStream_t s);  // k_rkadapt.cu (FP64)
-void rkAdaptiveGroup(const KArgs& a, const AdaptCtl& ac, cudaStream_t s);
-// One FP64 RK-Merson step for each instance in FP64 mode at this launch
-// (T.fbList[launch & 1]) on FP64 records at rowsBase: one thread (lanes 1) or
-// kFbLanes lanes of the level-parallel driver per instance (k_fallback.cu).
-void rkFp64List(const KArgs& a, const int64_t* rowsBase, double* rows, int lanes, cudaStream_t s);
-cudaError_t launchRKFp64List(const DevTables& T, const LaunchPlan& P, double* y, double* time, int32_t* status,
-                             double h, StepCtl step, double accuracy, double consTol, int projectEveryStep,
-                             int64_t fplane, const int64_t* rowsBase, double* rows, int lanes, cudaStream_t s);
+cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
+                             StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
+                             cudaStream_t s);
+cudaError_t launchTilePar(const TileDesc* desc, int ntiles, int W, const int32_t* parRow, const double* rows, int count,
+                          double* par, cudaStream_t s);
 cudaError_t launchFillInt(int32_t* p, int n, int v, cudaStream_t s);
 // *out = instances with steps left in a one-step integration call
 cudaError_t launchCountUnfinished(int n, const int32_t* stepsLeft, const double* time, const int32_t* status,

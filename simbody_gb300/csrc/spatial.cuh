@@ -7,40 +7,40 @@
 namespace sbg {
 
 template <class R> struct V3 { R x, y, z; };
-template <class R> __device__ __forceinline__ V3<R> mk3(R a, R b, R c) { return V3<R>{a, b, c}; }
-template <class R> __device__ __forceinline__ V3<R> z3() { return V3<R>{R(0), R(0), R(0)}; }
-template <class R> __device__ __forceinline__ V3<R> operator+(V3<R> a, V3<R> b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-template <class R> __device__ __forceinline__ V3<R> operator-(V3<R> a, V3<R> b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-template <class R> __device__ __forceinline__ V3<R> operator-(V3<R> a) { return {-a.x, -a.y, -a.z}; }
-template <class R> __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) { return {s * a.x, s * a.y, s * a.z}; }
-template <class R> __device__ __forceinline__ R dot(V3<R> a, V3<R> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-template <class R> __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b) {
+template <class R> __host__ __device__ __forceinline__ V3<R> mk3(R a, R b, R c) { return V3<R>{a, b, c}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> z3() { return V3<R>{R(0), R(0), R(0)}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> operator+(V3<R> a, V3<R> b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> operator-(V3<R> a, V3<R> b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> operator-(V3<R> a) { return {-a.x, -a.y, -a.z}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) { return {s * a.x, s * a.y, s * a.z}; }
+template <class R> __host__ __device__ __forceinline__ R dot(V3<R> a, V3<R> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+template <class R> __host__ __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b) {
     return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 // a + s*b
-template <class R> __device__ __forceinline__ V3<R> axpy(V3<R> a, R s, V3<R> b) {
+template <class R> __host__ __device__ __forceinline__ V3<R> axpy(V3<R> a, R s, V3<R> b) {
     return {a.x + s * b.x, a.y + s * b.y, a.z + s * b.z};
 }
 
 // Rotation / general 3x3, row-major.
 template <class R> struct M3 { R a[9]; };
-template <class R> __device__ __forceinline__ M3<R> ident3() {
+template <class R> __host__ __device__ __forceinline__ M3<R> ident3() {
     M3<R> m;
 #pragma unroll
     for (int i = 0; i < 9; ++i) m.a[i] = R((i % 4) == 0 ? 1 : 0);
     return m;
 }
-template <class R> __device__ __forceinline__ V3<R> mul(const M3<R>& m, V3<R> v) {
+template <class R> __host__ __device__ __forceinline__ V3<R> mul(const M3<R>& m, V3<R> v) {
     return {m.a[0] * v.x + m.a[1] * v.y + m.a[2] * v.z,
             m.a[3] * v.x + m.a[4] * v.y + m.a[5] * v.z,
             m.a[6] * v.x + m.a[7] * v.y + m.a[8] * v.z};
 }
-template <class R> __device__ __forceinline__ V3<R> mulT(const M3<R>& m, V3<R> v) {
+template <class R> __host__ __device__ __forceinline__ V3<R> mulT(const M3<R>& m, V3<R> v) {
     return {m.a[0] * v.x + m.a[3] * v.y + m.a[6] * v.z,
             m.a[1] * v.x + m.a[4] * v.y + m.a[7] * v.z,
             m.a[2] * v.x + m.a[5] * v.y + m.a[8] * v.z};
 }
-template <class R> __device__ __forceinline__ M3<R> mul(const M3<R>& A, const M3<R>& B) {
+template <class R> __host__ __device__ __forceinline__ M3<R> mul(const M3<R>& A, const M3<R>& B) {
     M3<R> C;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -49,17 +49,17 @@ template <class R> __device__ __forceinline__ M3<R> mul(const M3<R>& A, const M3
             C.a[3 * i + j] = A.a[3 * i] * B.a[j] + A.a[3 * i + 1] * B.a[3 + j] + A.a[3 * i + 2] * B.a[6 + j];
     return C;
 }
-template <class R> __device__ __forceinline__ V3<R> col(const M3<R>& m, int j) { return {m.a[j], m.a[3 + j], m.a[6 + j]}; }
+template <class R> __host__ __device__ __forceinline__ V3<R> col(const M3<R>& m, int j) { return {m.a[j], m.a[3 + j], m.a[6 + j]}; }
 
 // Symmetric 3x3: xx yy zz xy xz yz
 template <class R> struct S3 { R xx, yy, zz, xy, xz, yz; };
-template <class R> __device__ __forceinline__ V3<R> mul(const S3<R>& s, V3<R> v) {
+template <class R> __host__ __device__ __forceinline__ V3<R> mul(const S3<R>& s, V3<R> v) {
     return {s.xx * v.x + s.xy * v.y + s.xz * v.z,
             s.xy * v.x + s.yy * v.y + s.yz * v.z,
             s.xz * v.x + s.yz * v.y + s.zz * v.z};
 }
 // R * S * R^T
-template <class R> __device__ __forceinline__ S3<R> reexpress(const M3<R>& Rm, const S3<R>& S) {
+template <class R> __host__ __device__ __forceinline__ S3<R> reexpress(const M3<R>& Rm, const S3<R>& S) {
     // rows of R*S
     V3<R> r0 = mul(S, mk3(Rm.a[0], Rm.a[1], Rm.a[2]));
     V3<R> r1 = mul(S, mk3(Rm.a[3], Rm.a[4], Rm.a[5]));
@@ -72,14 +72,14 @@ template <class R> __device__ __forceinline__ S3<R> reexpress(const M3<R>& Rm, c
 template <class R> struct AB { S3<R> M, J; M3<R> F; };
 
 // (J*w + F*v, ~F*w + M*v)
-template <class R> __device__ __forceinline__ void abmul(const AB<R>& P, V3<R> w, V3<R> v, V3<R>& ow, V3<R>& ov) {
+template <class R> __host__ __device__ __forceinline__ void abmul(const AB<R>& P, V3<R> w, V3<R> v, V3<R>& ow, V3<R>& ov) {
     ow = mul(P.J, w) + mul(P.F, v);
     ov = mulT(P.F, w) + mul(P.M, v);
 }
 
 // P shifted by -s (rigid shift of an articulated inertia toward the parent
 // origin): F' = F + s_x*M, J' = J + sym(s_x*~F - F'*s_x).
-template <class R> __device__ __forceinline__ AB<R> abshift(const AB<R>& P, V3<R> s) {
+template <class R> __host__ __device__ __forceinline__ AB<R> abshift(const AB<R>& P, V3<R> s) {
     AB<R> o;
     o.M = P.M;
     const R x = s.x, y = s.y, z = s.z;

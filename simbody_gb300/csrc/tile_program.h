@@ -1,0 +1,307 @@
+// tile_program.h -- host side of the tile driver (tile_device.cuh): the bodies'
+// parameters in joint frames and the order in which a tile of instances takes
+// them.
+//
+// A tile is up to 32 instances, one per lane, swept by W warps in lockstep
+// steps: at a step each warp takes one body of each instance, and all of them
+// are of one class (mobilizer), so lanes never diverge over mobilizers. Which
+// bodies depends on the tile: a list schedule over its instances' trees, base
+// to tip (run backwards it is the tip-to-base order). A body follows its
+// parent, and follows the sibling before it, by at least one step: children
+// add to their parent's record, and two of them at one step would race. The
+// order among siblings is fixed by the topology alone, so an instance's sums,
+// and with them its results, do not depend on which tile it is in.
+#pragma once
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+#include <map>
+#include <vector>
+
+#include "tile_core.cuh"
+#include "topology_internal.h"
+
+namespace sbg {
+
+// A body's FP64 instructions per RHS by class: what a step costs its sub-partition.
+inline int tileCost(int cls, int n) {
+    static const int c[tile::CL_COUNT] = {300, 205, 500, 390, 600, 400};
+    return c[cls] + (cls == tile::CL_GEN ? 150 * n : 0);
+}
+constexpr int kTileStepCost = 60;  // a step's own latency (loads, barrier) in FP64 instructions
+
+// The rows of one topology for the tile driver.
+struct TileRows {
+    int nb = 0;
+    bool pose = false, gen = false;
+    std::vector<int> cls, parent, prevSib, height, cost;
+    std::vector<double> par;       // PR_COUNT per row
+    std::vector<int32_t> ints;     // SI_COUNT per row, the parent's row in SI_PARENT
+
+    explicit TileRows(const sbg_topology_s& t) : nb(t.nb) {
+        using namespace tile;
+        cls.resize(nb); parent.resize(nb); prevSib.assign(nb, -1); height.assign(nb, 0); cost.resize(nb);
+        par.assign((size_t)nb * PR_COUNT, 0.0);
+        ints.assign((size_t)nb * SI_COUNT, 0);
+        for (int r = 0; r < nb; ++r) {
+            const double* b = &t.par[(size_t)r * kParamStride];
+            const int type = t.info[r] & 15, n = (t.info[r] >> 4) & 15;
+            const bool quat = (t.info[r] & F_QUAT) != 0;
+            cls[r] = type == SBG_PIN ? CL_PIN : type == SBG_SLIDER ? CL_SLIDER : type == SBG_UNIVERSAL ? CL_UNIV
+                     : type == SBG_BALL && quat ? CL_BALL : type == SBG_FREE && quat ? CL_FREE : CL_GEN;
+            gen |= cls[r] == CL_GEN;
+            cost[r] = tileCost(cls[r], n);
+            parent[r] = t.parent[r];
+            double* o = &par[(size_t)r * PR_COUNT];
+            const double m = b[0], *RMB = b + 22, *pMB = b + 31;
+            double c[3], Gm[9], T[9];
+            for (int i = 0; i < 3; ++i) c[i] = RMB[3 * i] * b[1] + RMB[3 * i + 1] * b[2] + RMB[3 * i + 2] * b[3] + pMB[i];
+            // about the mass centre in body axes, turned to M axes, then about M's origin
+            const double com2 = b[1] * b[1] + b[2] * b[2] + b[3] * b[3];
+            const double G[9] = {b[4], b[7], b[8], b[7], b[5], b[9], b[8], b[9], b[6]};
+            for (int i = 0; i < 3; ++i)
+                for (int j = 0; j < 3; ++j) Gm[3 * i + j] = G[3 * i + j] - ((i == j ? com2 : 0.0) - b[1 + i] * b[1 + j]);
+            for (int i = 0; i < 3; ++i)
+                for (int j = 0; j < 3; ++j)
+                    T[3 * i + j] = RMB[3 * i] * Gm[j] + RMB[3 * i + 1] * Gm[3 + j] + RMB[3 * i + 2] * Gm[6 + j];
+            const double c2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2];
+            auto J = [&](int i, int j) {
+                const double g = T[3 * i] * RMB[3 * j] + T[3 * i + 1] * RMB[3 * j + 1] + T[3 * i + 2] * RMB[3 * j + 2];
+                return m * (g + ((i == j ? c2 : 0.0) - c[i] * c[j]));
+            };
+            o[PR_M] = m;
+            for (int i = 0; i < 3; ++i) o[PR_MC + i] = m * c[i];
+            o[PR_J] = J(0, 0); o[PR_J + 1] = J(1, 1); o[PR_J + 2] = J(2, 2);
+            o[PR_J + 3] = J(0, 1); o[PR_J + 4] = J(0, 2); o[PR_J + 5] = J(1, 2);
+            static const double eye[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, nil[3] = {0, 0, 0};
+            const double* PR = parent[r] < 0 ? eye : &t.par[(size_t)parent[r] * kParamStride + 22];
+            const double* Pp = parent[r] < 0 ? nil : &t.par[(size_t)parent[r] * kParamStride + 31];
+            const double *RPF = b + 10, *pPF = b + 19;
+            bool ci = true;
+            for (int i = 0; i < 3; ++i) {
+                for (int j = 0; j < 3; ++j) {
+                    const double v = PR[3 * i] * RPF[j] + PR[3 * i + 1] * RPF[3 + j] + PR[3 * i + 2] * RPF[6 + j];
+                    o[PR_C + 3 * i + j] = v;
+                    ci &= v == (i == j ? 1.0 : 0.0);
+                }
+                o[PR_D + i] = PR[3 * i] * pPF[0] + PR[3 * i + 1] * pPF[1] + PR[3 * i + 2] * pPF[2] + Pp[i];
+            }
+            o[PR_PITCH] = b[34];
+            for (int k = t.fbeg[r]; k < t.fbeg[r] + t.fcnt[r]; ++k) {
+                const int j = t.fkw[k] & 255;
+                if ((t.fkw[k] >> 8) == 0) { o[PR_K + j] += t.fcoef[k]; o[PR_S + j] += t.fcoef[k] * t.fq0[k]; }
+                else o[PR_B + j] += t.fcoef[k];
+            }
+            int32_t* s = &ints[(size_t)r * SI_COUNT];
+            s[SI_Q] = t.qoff[r]; s[SI_U] = t.uoff[r]; s[SI_PARENT] = parent[r];
+            s[SI_INFO] = t.info[r] | (ci ? F_CI : 0);
+            s[SI_ROW] = r; s[SI_KBEG] = t.kbeg[r]; s[SI_KCNT] = t.kcnt[r];
+            pose |= t.kcnt[r] > 0;
+        }
+        for (int r = nb - 1; r >= 0; --r) {
+            height[r] += cost[r] + kTileStepCost;
+            if (parent[r] >= 0) height[parent[r]] = std::max(height[parent[r]], height[r]);
+        }
+        // siblings in the order of falling height
+        for (int r = 0; r < nb; ++r) {
+            std::vector<int> kids(t.clist.begin() + t.cbeg[r], t.clist.begin() + t.cbeg[r] + t.ccnt[r]);
+            std::stable_sort(kids.begin(), kids.end(), [&](int a, int b) { return height[a] > height[b]; });
+            for (size_t k = 1; k < kids.size(); ++k) prevSib[kids[k]] = kids[k - 1];
+        }
+    }
+};
+
+// Schedule of one tile: classes of (step, warp), and the row each lane takes
+// there (-1: none).
+struct TileSchedule {
+    int nsteps = 0;
+    std::vector<int32_t> cls;              // nsteps * W
+    std::vector<std::vector<int>> row;     // per slot, per lane
+    int64_t length = 0, load = 0;          // FP64 instructions: of the longest warp step by step, of all warps
+
+    TileSchedule(const std::vector<const TileRows*>& lanes, int W) {
+        using namespace tile;
+        const int nl = (int)lanes.size();
+        struct Lane {
+            std::vector<int> ready;            // ready rows, in falling height
+            std::vector<int> waits;            // parent and sibling still to come, per row
+            std::vector<std::vector<int>> next;
+            int left;
+        };
+        std::vector<Lane> L(nl);
+        for (int l = 0; l < nl; ++l) {
+            const TileRows& t = *lanes[l];
+            L[l].waits.assign(t.nb, 0);
+            L[l].next.resize(t.nb);
+            L[l].left = t.nb;
+            for (int r = 0; r < t.nb; ++r) {
+                if (t.parent[r] >= 0) { ++L[l].waits[r]; L[l].next[t.parent[r]].push_back(r); }
+                if (t.prevSib[r] >= 0) { ++L[l].waits[r]; L[l].next[t.prevSib[r]].push_back(r); }
+            }
+            for (int r = 0; r < t.nb; ++r)
+                if (!L[l].waits[r]) L[l].ready.push_back(r);
+        }
+        int remaining = 0;
+        for (int l = 0; l < nl; ++l) remaining += L[l].left;
+        std::vector<std::vector<int>> done(nl);
+        while (remaining > 0) {
+            int64_t longest = 0;
+            for (auto& d : done) d.clear();
+            for (int w = 0; w < W; ++w) {
+                // the class with the most work ready, weighted by how critical it is
+                double score[CL_COUNT] = {};
+                for (int l = 0; l < nl; ++l) {
+                    if (L[l].ready.empty()) continue;
+                    bool seen[CL_COUNT] = {};
+                    int top = 0;
+                    for (int r : L[l].ready) top = std::max(top, lanes[l]->height[r]);
+                    for (int r : L[l].ready) {
+                        const int c = lanes[l]->cls[r];
+                        if (seen[c]) continue;
+                        seen[c] = true;
+                        score[c] += 1.0 + kCritical * lanes[l]->height[r] / top;
+                    }
+                }
+                int best = -1;
+                for (int c = 0; c < CL_COUNT; ++c)
+                    if (score[c] > 0 && (best < 0 || score[c] > score[best])) best = c;
+                cls.push_back(best);
+                row.emplace_back(nl, -1);
+                if (best < 0) continue;
+                int stepCost = 0;
+                for (int l = 0; l < nl; ++l) {
+                    auto& rd = L[l].ready;
+                    int at = -1;
+                    for (int k = 0; k < (int)rd.size(); ++k)
+                        if (lanes[l]->cls[rd[k]] == best &&
+                            (at < 0 || lanes[l]->height[rd[k]] > lanes[l]->height[rd[at]])) at = k;
+                    if (at < 0) continue;
+                    const int r = rd[at];
+                    rd.erase(rd.begin() + at);
+                    row.back()[l] = r;
+                    done[l].push_back(r);
+                    --remaining;
+                    stepCost = std::max(stepCost, lanes[l]->cost[r]);
+                }
+                load += stepCost + kTileStepCost;
+                longest = std::max<int64_t>(longest, stepCost + kTileStepCost);
+            }
+            for (int l = 0; l < nl; ++l)
+                for (int r : done[l])
+                    for (int k : L[l].next[r])
+                        if (--L[l].waits[k] == 0) L[l].ready.push_back(k);
+            length += longest;
+            ++nsteps;
+        }
+    }
+    static constexpr double kCritical = 3.0;
+};
+
+// The tables of a batch's tiles on the host. Parameters are gathered on the
+// device from the topologies' rows (parRow: row per slot and lane, -1: none).
+struct TileProgram {
+    int W = 1, rs = 0, rsTotal = 0;
+    bool pose = false;
+    std::vector<TileDesc> desc;
+    std::vector<int32_t> cls, slots, parRow;
+    int64_t recElems = 0, maxTile = 0;  // record doubles of all tiles, of the largest
+
+    // One tile over `topo` (topology per lane). rows: per topology, rowBase:
+    // its first row in the parameter rows.
+    void add(int pos0, const std::vector<int>& topo, int ls, const std::vector<const TileRows*>& rows,
+             const std::vector<int64_t>& rowBase) {
+        using namespace tile;
+        const bool same = std::all_of(topo.begin(), topo.end(), [&](int k) { return k == topo[0]; });
+        TileDesc d{};
+        d.pos0 = pos0;
+        d.lanes = (int)topo.size();
+        d.ls = ls;
+        d.shared = same;
+        d.rec0 = recElems;
+        const auto it = same ? known.find(topo[0]) : known.end();
+        if (it != known.end()) {
+            d.cls0 = it->second.cls0; d.nsteps = it->second.nsteps;
+            d.slot0 = it->second.slot0; d.par0 = it->second.par0;
+        } else {
+            std::vector<const TileRows*> lanes;
+            for (int l = 0; l < (same ? 1 : d.lanes); ++l) lanes.push_back(rows[topo[l]]);
+            const TileSchedule s(lanes, W);
+            const int st = same ? 1 : ls, nl = (int)lanes.size();
+            const int64_t nslots = (int64_t)s.nsteps * W;
+            d.nsteps = s.nsteps;
+            d.cls0 = (int32_t)cls.size();
+            d.slot0 = (int64_t)slots.size();
+            d.par0 = (int64_t)parRow.size() * PR_COUNT;
+            cls.insert(cls.end(), s.cls.begin(), s.cls.end());
+            slots.resize(slots.size() + nslots * SI_COUNT * st, -1);
+            parRow.resize(parRow.size() + nslots * st, -1);
+            std::vector<int> slotOf;
+            for (int l = 0; l < nl; ++l) {
+                const TileRows& t = *lanes[l];
+                slotOf.assign(t.nb, -1);
+                for (int64_t k = 0; k < nslots; ++k)
+                    if (s.row[k][l] >= 0) slotOf[s.row[k][l]] = (int)k;
+                for (int r = 0; r < t.nb; ++r) {
+                    int32_t* o = &slots[d.slot0 + (int64_t)slotOf[r] * SI_COUNT * st + l];
+                    for (int k = 0; k < SI_COUNT; ++k) o[(int64_t)k * st] = t.ints[(size_t)r * SI_COUNT + k];
+                    o[(int64_t)SI_PARENT * st] = t.parent[r] < 0 ? -1 : slotOf[t.parent[r]];
+                    parRow[d.par0 / PR_COUNT + (int64_t)slotOf[r] * st + l] = (int32_t)(rowBase[topo[l]] + r);
+                }
+            }
+            // the lanes of a step agree on whether C is the identity
+            for (int64_t k = 0; k < nslots; ++k) {
+                int32_t* o = &slots[d.slot0 + (k * SI_COUNT + SI_INFO) * st];
+                bool ci = true;
+                for (int l = 0; l < nl; ++l) ci &= s.row[k][l] < 0 || (o[l] & F_CI);
+                if (!ci)
+                    for (int l = 0; l < nl; ++l)
+                        if (s.row[k][l] >= 0) o[l] &= ~F_CI;
+            }
+            if (same) known[topo[0]] = d;
+        }
+        const int64_t n = (int64_t)d.nsteps * W * rsTotal * ls;
+        recElems += n;
+        maxTile = std::max(maxTile, n);
+        desc.push_back(d);
+    }
+
+    // Instances per tile and warps per tile for `n` instances on `nsub` SM
+    // sub-partitions, topoAt[p] the topology at order position p: the shape
+    // with the least time by the schedule's FP64 instructions, on a sample of
+    // its tiles. A tile's warps wait for one another at each step (length);
+    // past one warp per sub-partition the warps' instructions add up (load).
+    // Fewer lanes per tile follow a lane's own tree better and more warps
+    // shorten the steps; both cost warps. Measured on 8,192 random trees.
+    static void shape(const std::vector<int>& topoAt, const std::vector<const TileRows*>& rows, int nsub, int& TW, int& W) {
+        const int n = (int)topoAt.size();
+        double best = 0;
+        TW = 32; W = 1;
+        const bool same = std::all_of(topoAt.begin(), topoAt.end(), [&](int k) { return k == topoAt[0]; });
+        for (int tw : {32, 16, 8, 4, 2, 1}) {
+            if (same && tw < 32) break;  // alignment is perfect at any width
+            const int tiles = (n + tw - 1) / tw;
+            if (tw < 32 && tiles > 4 * nsub) break;
+            for (int w : {1, 2, 4, 8}) {
+                double length = 0, load = 0;
+                const int samples = std::min(tiles, same ? 1 : 4);
+                for (int s = 0; s < samples; ++s) {
+                    const int p0 = (int)((int64_t)tiles * s / samples) * tw;
+                    std::vector<const TileRows*> lanes;
+                    for (int p = p0; p < std::min(n, p0 + (same ? 1 : tw)); ++p) lanes.push_back(rows[topoAt[p]]);
+                    const TileSchedule sc(lanes, w);
+                    length += double(sc.length) / samples;
+                    load += double(sc.load) / samples;
+                }
+                const double waves = std::ceil(double(tiles) * w / nsub);
+                const double t = std::max(length, waves * load / w);
+                if (best == 0 || t < 0.97 * best) { best = t; TW = tw; W = w; }
+            }
+        }
+    }
+
+private:
+    std::map<int, TileDesc> known;
+};
+
+}  // namespace sbg

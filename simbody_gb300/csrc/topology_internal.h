@@ -1,6 +1,7 @@
 // topology_internal.h -- the host-side flattened topology behind the opaque
 // sbg_topology handle (shared by capi.cpp and k_noalloc.cu).
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -10,6 +11,7 @@
 
 // A flattened topology: bodies in level order (the reference's rbNodeLevels).
 struct sbg_topology_s {
+    std::atomic<int> refs{1};            // the handle's and one per batch that uses it
     int nb = 0, nq = 0, nu = 0, nlevels = 0, nquat = 0, ncons = 0;
     int maxNonFreeDof = 0;
     int64_t recSize = 0;                 // scratch elements per instance
@@ -34,6 +36,9 @@ struct sbg_topology_s {
     std::vector<double> lst;
     int nslots = 0;
 };
+inline void releaseTopology(sbg_topology_s* t) {
+    if (t && t->refs.fetch_sub(1) == 1) delete t;
+}
 
 namespace sbg {
 // Records msg as the calling thread's sbg_last_error() message; returns code.
