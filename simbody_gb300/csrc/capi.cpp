@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -79,6 +80,7 @@ struct sbg_batch_s {
     int precision = 0, device = 0;
     int64_t budget = 0;
     int ninst = 0;
+    int sms = 1;
     int nm = 3;
     bool tiled = false;
     int variant = 0;  // kernel variant: 0 = not tuned yet, else 1, 4, 7 or 8 (see LaunchPlan)
@@ -487,8 +489,7 @@ int sbg_topology_default_state(sbg_topology t, double* y) {
 // records for every block of a launch that fills the GPU.
 static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     using namespace tile;
-    int sms = 0;
-    SBG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "device attribute");
+    const int sms = b->sms;
     std::vector<TileRows> store;
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
     std::vector<int64_t> rowBase(b->topos.size(), 0);
@@ -514,27 +515,35 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     if (at.empty()) return SBG_OK;
     if (single) {
         P.W = 4;  // one warp per sub-partition
+        P.ls = 1;
+        P.shared = true;
         std::vector<TileDesc> per(b->ninst, TileDesc{});
         for (int i = 0; i < b->ninst; ++i) {
             if (b->topos[b->topoOf[i]]->ncons > 0) continue;
-            P.add(0, {b->topoOf[i]}, 1, rows, rowBase);
+            P.add(0, {b->topoOf[i]}, rows, rowBase);
             per[i] = P.desc.back();
             per[i].rec0 = 0;
         }
         P.desc.swap(per);
     } else {
         int TW = 32;
-        TileProgram::shape(at, rows, 4 * sms, TW, P.W);
+        TileProgram::shape(at, rows, sms, TW, P.W);
+        if (const char* v = std::getenv("SBG_TILE")) std::sscanf(v, "%d,%d", &TW, &P.W);  // tuning override
         b->tileWidth = TW;
+        P.ls = TW;
+        P.shared = TW == 1 || std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
         for (const auto& seg : {std::make_pair(0, b->nChain), std::make_pair(b->nChain + b->nLoop, b->ninst)})
             for (int p = seg.first; p < seg.second; p += TW) {
                 std::vector<int> lanes;
                 for (int k = p; k < std::min(seg.second, p + TW); ++k) lanes.push_back(b->topoOf[b->order[k]]);
-                P.add(p, lanes, TW, rows, rowBase);
+                P.add(p, lanes, rows, rowBase);
             }
     }
     out->ntiles = (int)P.desc.size();
     out->tt.W = P.W;
+    out->tt.ls = P.ls;
+    out->tt.shared = P.shared;
+    out->tt.ys = b->precision == SBG_PRECISION_FP64 ? kTile : 0;
     out->tt.rs = P.rs;
     out->tt.rsTotal = P.rsTotal;
     out->tt.pose = P.pose;
@@ -546,14 +555,11 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     const int64_t nPar = (int64_t)P.parRow.size() * PR_COUNT;
     if ((rc = b->alloc(&p, std::max<int64_t>(nPar, 1) * sizeof(double), "tile parameters"))) return rc;
     out->tt.par = static_cast<double*>(p);
-    if (single) {  // tables without lanes: the rows in slot order
+    if (P.shared) {  // tables without lanes: the rows in slot order
         std::vector<double> v(std::max<int64_t>(nPar, 1));
         for (size_t k = 0; k < P.parRow.size(); ++k)
             if (P.parRow[k] >= 0) std::copy_n(&par[(size_t)P.parRow[k] * PR_COUNT], PR_COUNT, &v[k * PR_COUNT]);
         SBG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice), "tile parameters");
-        out->blocks = 4 * sms;
-        out->recStride = P.maxTile;
-        if ((rc = b->alloc(&p, (int64_t)out->blocks * out->recStride * sizeof(double), "FP64 records"))) return rc;
     } else {
         void *dRow = nullptr, *dPar = nullptr;
         cudaError_t e = cudaMalloc(&dRow, std::max<size_t>(P.parRow.size(), 1) * sizeof(int32_t));
@@ -562,7 +568,7 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
             e = cudaMemcpy(dRow, P.parRow.data(), P.parRow.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(dPar, par.data(), par.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (e == cudaSuccess)
-            e = launchTilePar(out->tt.desc, out->ntiles, P.W, static_cast<int32_t*>(dRow), static_cast<double*>(dPar),
+            e = launchTilePar(out->tt, out->ntiles, static_cast<int32_t*>(dRow), static_cast<double*>(dPar),
                               PR_COUNT, static_cast<double*>(p), b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         cudaFree(dRow);
@@ -571,8 +577,14 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
             cudaGetLastError();
             return cudaFail(e, "tile parameters");
         }
-        if ((rc = b->alloc(&p, std::max<int64_t>(P.recElems, 1) * sizeof(double), "FP64 records"))) return rc;
     }
+    int64_t recElems = P.recElems;
+    if (single) {
+        out->blocks = 4 * sms;
+        out->recStride = P.maxTile;
+        recElems = (int64_t)out->blocks * out->recStride;
+    }
+    if ((rc = b->alloc(&p, std::max<int64_t>(recElems, 1) * sizeof(double), "FP64 records"))) return rc;
     out->recs = static_cast<double*>(p);
     return SBG_OK;
 }
@@ -615,6 +627,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return bail(cudaFail(e, "stream/event creation"));
     }
 
@@ -713,6 +726,16 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
             return inb[a] != inb[c] ? inb[a] > inb[c] : instTopo[a] < instTopo[c];
         });
         std::stable_sort(loopPos.begin(), loopPos.end(), [&](int a, int c) { return inb[a] > inb[c]; });
+        if (precision == SBG_PRECISION_FP64) {
+            std::vector<std::array<float, tile::CL_COUNT>> per(b->topos.size()), work(ninst);
+            for (size_t k = 0; k < per.size(); ++k) {
+                per[k].fill(0);
+                for (int32_t info : b->topos[k]->info)
+                    per[k][tileClassOf(info)] += (float)tileCost(tileClassOf(info), (info >> 4) & 15);
+            }
+            for (int i = 0; i < ninst; ++i) work[i] = per[b->topoOf[i]];
+            tileOrder(chainPos, work);
+        }
         auto wkey = [&](int i) { int w = 1; while (w < topos[instTopo[i]]->maxLevelWidth) w <<= 1; return w; };
         std::stable_sort(groupPos.begin(), groupPos.end(), [&](int a, int c) {
             const int wa = wkey(a), wc = wkey(c);
@@ -779,12 +802,25 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     for (int p = b->nChain + b->nLoop; p < ninst; ++p) {
         const int i = order[p];
         const sbg_topology_s* t = topos[instTopo[i]];
-        ybase[i] = yOff; ystride[i] = 1;
-        yOff += t->nq + t->nu;
+        if (precision != SBG_PRECISION_FP64) {
+            ybase[i] = yOff; ystride[i] = 1;
+            yOff += t->nq + t->nu;
+        }
         sbase[i] = sOff; sstride[i] = 1;
         sOff += (int64_t)t->nb * rowsRecordWidth(*t, 3);
         b->groupWidthKey.push_back(t->maxLevelWidth);
     }
+    if (precision == SBG_PRECISION_FP64)  // the tile driver takes every state column at stride 32
+        for (int t0 = b->nChain + b->nLoop; t0 < ninst; t0 += kTile) {
+            const int t1 = std::min(ninst, t0 + kTile);
+            int64_t yw = 0;
+            for (int p = t0; p < t1; ++p) {
+                yw = std::max<int64_t>(yw, inq[order[p]] + inu[order[p]]);
+                ybase[order[p]] = yOff + (p - t0);
+                ystride[order[p]] = kTile;
+            }
+            yOff += yw * kTile;
+        }
     b->nyTotal = b->hostYOff[ninst];
     b->nuTotal = b->hostUOff[ninst];
     b->colElems = yOff;
@@ -905,7 +941,9 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
             if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counter"));
         }
     }
-    if ((rc = b->alloc(&b->fbuf, 4 * std::max<int64_t>(b->colElems, 1) * rsz, "stage derivatives"))) return bail(rc);
+    // FP64: and the stage input
+    const int planes = precision == SBG_PRECISION_FP64 ? 5 : 4;
+    if ((rc = b->alloc(&b->fbuf, planes * std::max<int64_t>(b->colElems, 1) * rsz, "stage derivatives"))) return bail(rc);
     if (b->nLoop > 0) {
         if ((rc = b->alloc(&b->scratchLoop, scratchLoopElems * sizeof(double), "loop scratch"))) return bail(rc);
         if (precision == SBG_PRECISION_FP64) b->fbufLoop = b->fbuf;
@@ -1113,6 +1151,10 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     int nchunks = 4;
     if (const char* v = std::getenv("SBG_PIPE_CHUNKS")) nchunks = std::max(1, std::atoi(v));  // tuning override
     nchunks = std::min(nchunks, 16);
+    // FP64 tiles take the same time whether few or many run beside them, up to
+    // one per SM sub-partition: chunks of half as many still run side by side
+    if (b->precision == SBG_PRECISION_FP64)
+        nchunks = std::min<int64_t>(nchunks, b->tiles.ntiles / (2 * b->sms));
     const bool pipelined = b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 &&
                            (b->tuned || b->precision == SBG_PRECISION_FP64) && nchunks > 1 &&
                            b->ninst >= nchunks * kTile;
@@ -1380,7 +1422,7 @@ static int ensureFallbackSteps(sbg_batch b) {
     b->fbLeft = static_cast<int32_t*>(p);
     if ((rc = b->alloc(&p, n * sizeof(int32_t), "step counters"))) return rc;
     b->stepsLeft = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, 4 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
+    if ((rc = b->alloc(&p, 5 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
         return rc;
     b->fbuf64 = static_cast<double*>(p);
     if ((rc = b->alloc(&p, sizeof(unsigned long long), "FP64 step counter"))) return rc;

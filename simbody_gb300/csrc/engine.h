@@ -208,7 +208,6 @@ struct LaunchPlan {
 struct TileDesc {
     int32_t pos0, lanes;   // order positions [pos0, pos0 + lanes)
     int32_t nsteps, cls0;  // classes at cls0 + step * W + warp
-    int32_t ls, shared;    // lane stride of the records; 1: one topology, tables without lanes
     int64_t slot0, par0, rec0;
 };
 struct TileTables {
@@ -217,6 +216,9 @@ struct TileTables {
     const int32_t* slots;  // integers per (step, warp) slot and lane
     const double* par;     // parameters per slot and lane
     int32_t W;
+    int32_t ls, shared;    // lanes per tile (32, 8 or 1); tables without lanes: every tile has one topology
+    int32_t ys;            // stride of the state columns; 0: the instance's own (mixed batches, whose
+                           // level-parallel segment keeps contiguous columns)
     int32_t rs, rsTotal;   // doubles of a body's record without and with the Ground pose
     int32_t pose;          // some body carries contact spheres
 };

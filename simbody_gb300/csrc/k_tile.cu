@@ -6,29 +6,31 @@ namespace sbg {
 
 namespace {
 
+template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     realizeTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int tile0,
                       const double* __restrict__ y, double* __restrict__ ydot, double* __restrict__ recs,
                       int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
-    const TileCtx c = tileCtx(T, TT, tile0 + blockIdx.x, recs);
-    const TileYSrc src{y, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
-    TileOut out{ydot, src.base, src.stride, src.nq};
-    int st = tileRhs<false>(T, TT, c, src, out, true);
+    const TileCtx c = tileCtx<CF>(T, TT, tile0 + blockIdx.x, recs);
+    const TileYSrc<CF::YS> src{{T, c.inst}, y};
+    TileOut<CF::YS> out(src.c, ydot);
+    int st = tileRhs<CF, false>(T, TT, c, src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
     st = tileReduce<0>(TT, c, sh, nullptr, st);
     if (c.on && c.w == 0) status[c.inst] = st;
 }
 
+template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     minvTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, const double* __restrict__ y,
                    const double* __restrict__ f, double* __restrict__ o, double* __restrict__ recs,
                    int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
-    const TileCtx c = tileCtx(T, TT, blockIdx.x, recs);
-    const TileFSrc src{y, f, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
-    TileUOut out{o, src.base, src.stride, src.nq};
-    int st = tileRhs<true>(T, TT, c, src, out, true);
+    const TileCtx c = tileCtx<CF>(T, TT, blockIdx.x, recs);
+    const TileFSrc<CF::YS> src{{T, c.inst}, y, f};
+    TileUOut<CF::YS> out(src.c, o);
+    int st = tileRhs<CF, true>(T, TT, c, src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
     st = tileReduce<0>(TT, c, sh, nullptr, st);
     if (c.on && c.w == 0) status[c.inst] = st;
@@ -54,10 +56,10 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
         }
         __syncthreads();
         for (int k = 0; k < n; ++k) {
-            const TileCtx c = tileCtxOne(TT, list[k], recs + recStride * blockIdx.x);
-            const TileYSrc src{y, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
-            TileOut out{ydot, src.base, src.stride, src.nq};
-            int st = tileRhs<false>(T, TT, c, src, out, true);
+            const TileCtx c = tileCtxOne<TileOne>(TT, list[k], recs + recStride * blockIdx.x);
+            const TileYSrc<0> src{{T, c.inst}, y};
+            TileOut<0> out(src.c, ydot);
+            int st = tileRhs<TileOne, false>(T, TT, c, src, out, true);
             if (!out.finite) st |= SBG_INST_NONFINITE;
             st = tileReduce<0>(TT, c, sh, nullptr, st);
             if (c.on && c.w == 0) {
@@ -73,11 +75,15 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s) {
     if (ntiles <= 0) return;
-    realizeTileKernel<<<ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, tile0, a.y, a.ydot, S.recs, a.status);
+    tileDispatch<kTile>(S, [&](auto cf) {
+        realizeTileKernel<decltype(cf)><<<ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, tile0, a.y, a.ydot, S.recs, a.status);
+    });
 }
 void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s) {
     if (S.ntiles <= 0) return;
-    minvTileKernel<<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, a.y, a.f, a.ydot, S.recs, a.status);
+    tileDispatch<kTile>(S, [&](auto cf) {
+        minvTileKernel<decltype(cf)><<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, a.y, a.f, a.ydot, S.recs, a.status);
+    });
 }
 void realizeFallbackTiles(const KArgs& a, const TileSet& S, int first, int count, int block0, int blocks, cudaStream_t s) {
     if (count <= 0) return;

@@ -54,15 +54,16 @@ __device__ __forceinline__ bool adjustStepSizeDev(double err, int errOrder, bool
 
 namespace {
 
+template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     rkAdaptiveTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT,
                          double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
                          int32_t* __restrict__ status, const __grid_constant__ AdaptCtl ac) {
     __shared__ TileShare<5> sh;
-    const TileCtx c = tileCtx(T, TT, blockIdx.x, recs);
-    const int64_t base = T.ybase[c.inst], stride = T.ystride[c.inst];
-    const int nq = T.inq[c.inst], nu = T.inu[c.inst];
-    double *f0 = fbuf, *fA = fbuf + fplane, *fB = fbuf + 2 * fplane, *fC = fbuf + 3 * fplane;
+    const TileCtx c = tileCtx<CF>(T, TT, blockIdx.x, recs);
+    const TileCol<CF::YS> col(T, c.inst);
+    const int nq = col.nq, nu = T.inu[c.inst];
+    double *f0 = fbuf, *fA = fbuf + fplane, *fB = fbuf + 2 * fplane, *fC = fbuf + 3 * fplane, *yt = fbuf + 4 * fplane;
     int st = 0;
     double tc = c.on ? time[c.inst] : 0.0;
     const double tFinal = ac.tFinal;
@@ -99,9 +100,10 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 #pragma unroll 1
         for (int stg = __any_sync(0xffffffffu, needF0) ? 0 : 1; stg < 5; ++stg) {
             const double cc = stg == 0 ? 0.0 : stg == 1 ? hs / 3 : stg == 2 ? hs / 6 : stg == 3 ? hs / 8 : hs / 2;
-            const TileStageSrc src{y, f0, stg >= 3 ? fB : fA, fC, base, stride, nq, stg, cc};
-            TileOut out{stg == 0 ? f0 : stg == 2 ? fB : stg == 3 ? fC : fA, base, stride, nq};
-            bits |= tileRhs<false>(T, TT, c, src, out, stg == 0 ? needF0 : going);
+            tileStageInput<CF>(TT, c, col, nq + nu, stg == 0 ? needF0 : going, stg, cc, y, f0, stg >= 3 ? fB : fA, fC, yt);
+            const TileYSrc<CF::YS> src{col, yt};
+            TileOut<CF::YS> out(col, stg == 0 ? f0 : stg == 2 ? fB : stg == 3 ? fC : fA);
+            bits |= tileRhs<CF, false>(T, TT, c, src, out, stg == 0 ? needF0 : going);
             if (!out.finite) bits |= SBG_INST_NONFINITE;
         }
         const double h6 = hs / 6, h2 = hs / 2;
@@ -113,15 +115,14 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
         };
         // error norm and quaternion errors of y1, y untouched
         double v[5] = {0, 0, 0, 0, 0};  // sq, su, squat, nquat, sq after the projection
-        if (going)
-            tileBodies(TT, c, [&](const tile::SlotRow& r) {
+        tileBodies<CF>(TT, c, going, [&](const tile::SlotRow& r) {
                 const int nqb = slotQ(r.info), n = (r.info >> 4) & 15;
                 double q1[4], dq[4], extra = 0;
 #pragma unroll
                 for (int j = 0; j < 7; ++j)
                     if (j < nqb) {
                         double ysv;
-                        const double y1v = y1At(base + (int64_t)(r.qo + j) * stride, &ysv);
+                        const double y1v = y1At(col.at(r.qo + j), &ysv);
                         const double dj = 0.2 * fabs(y1v - ysv);
                         if (j < 4) { q1[j] = y1v; dq[j] = dj; }
                         if (j >= 4 || !(r.info & F_QUAT)) extra += dj * dj;
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                 v[0] += extra;
                 v[4] += extra;
                 for (int j = 0; j < n; ++j) {
-                    const int64_t e = base + (int64_t)(nq + r.uo + j) * stride;
+                    const int64_t e = col.atU(r.uo + j);
                     double ysv;
                     const double y1v = y1At(e, &ysv);
                     const double vi = fabs(y[e]);
@@ -182,15 +183,14 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
             st |= needF0 ? bits : 0;
         }
         int fin = 0;
-        if (take)
-            tileBodies(TT, c, [&](const tile::SlotRow& r) {
+        tileBodies<CF>(TT, c, take, [&](const tile::SlotRow& r) {
                 const int nqb = slotQ(r.info), n = (r.info >> 4) & 15;
                 double q1[4];
 #pragma unroll
                 for (int j = 0; j < 7; ++j)
                     if (j < nqb) {
                         double ysv;
-                        const int64_t e = base + (int64_t)(r.qo + j) * stride;
+                        const int64_t e = col.at(r.qo + j);
                         const double y1v = y1At(e, &ysv);
                         if (j < 4) q1[j] = y1v;
                         if (j >= 4 || !(proj && (r.info & F_QUAT))) {
@@ -203,13 +203,13 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const double qk = q1[k] / len;
-                        y[base + (int64_t)(r.qo + k) * stride] = qk;
+                        y[col.at(r.qo + k)] = qk;
                         if (!tile::finiteBits(qk)) fin |= SBG_INST_NONFINITE;
                     }
                 }
                 for (int j = 0; j < n; ++j) {
                     double ysv;
-                    const int64_t e = base + (int64_t)(nq + r.uo + j) * stride;
+                    const int64_t e = col.atU(r.uo + j);
                     const double y1v = y1At(e, &ysv);
                     y[e] = y1v;
                     if (!tile::finiteBits(y1v)) fin |= SBG_INST_NONFINITE;
@@ -238,8 +238,11 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 void rkAdaptiveTiles(const KArgs& a, const TileSet& S, const AdaptCtl& ac, cudaStream_t s) {
     if (S.ntiles <= 0) return;
-    rkAdaptiveTileKernel<<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, S.recs, a.ystate, a.time, static_cast<double*>(a.fbuf),
-                                                          a.fplane, a.status, ac);
+    tileDispatch<kTile>(S, [&](auto cf) {
+        rkAdaptiveTileKernel<decltype(cf)><<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, S.recs, a.ystate, a.time,
+                                                                            static_cast<double*>(a.fbuf), a.fplane,
+                                                                            a.status, ac);
+    });
 }
 
 }  // namespace sbg

@@ -170,7 +170,7 @@ void rkLoopGroup(const KArgs& a, cudaStream_t s);      // loop closures, level-p
 cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
                              StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
                              cudaStream_t s);
-cudaError_t launchTilePar(const TileDesc* desc, int ntiles, int W, const int32_t* parRow, const double* rows, int count,
+cudaError_t launchTilePar(const TileTables& tt, int ntiles, const int32_t* parRow, const double* rows, int count,
                           double* par, cudaStream_t s);
 cudaError_t launchFillInt(int32_t* p, int n, int v, cudaStream_t s);
 // *out = instances with steps left in a one-step integration call

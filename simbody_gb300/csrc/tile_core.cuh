@@ -40,30 +40,32 @@ enum : int { PR_M = 0, PR_MC = 1, PR_J = 4, PR_C = 10, PR_D = 19, PR_PITCH = 22,
              PR_COUNT = 41 };
 // Integers of a body: q and u slots, slot of the parent (-1 = Ground), info
 // word (body table), body row, contacts.
-enum : int { SI_Q = 0, SI_U, SI_PARENT, SI_INFO, SI_ROW, SI_KBEG, SI_KCNT, SI_COUNT };
-constexpr int F_CI = 1 << 20;  // info word of a slot: C is the identity on every lane
+enum : int { SI_Q = 0, SI_U, SI_PARENT, SI_INFO, SI_ROW, SI_KBEG, SI_KCNT, SI_COUNT = 8 };
+// Info word of a slot, on every lane alike: C is the identity; no mobility
+// force acts on the body.
+constexpr int F_CI = 1 << 20, F_FREELY = 1 << 21;
 
 // Record of a body (doubles).
 //   P (J F M) and z: own inertia and force, then the children's on top
-//   w, then A = (alpha, a of the origin of M)
+//   w and w.w, then A = (alpha, a of the origin of M)
 //   l: parent's M origin to this one's, parent axes; E = R_FM (or c s c s)
 //   gamma: velocity part of the acceleration; X: f, then the factorisation
 // In a batch with contact spheres the Ground pose and velocity follow.
-enum : int { RC_J = 0, RC_F = 6, RC_M = 15, RC_Z = 21, RC_W = 27, RC_L = 33, RC_E = 36, RC_GAM = 45, RC_X = 51,
+enum : int { RC_J = 0, RC_F = 6, RC_M = 15, RC_Z = 21, RC_W = 27, RC_W2 = 30, RC_L = 33, RC_E = 36, RC_GAM = 45, RC_X = 51,
              RC_SMALL = 63, RC_H = 63, RC_G = 99, RC_GEN = 135, RC_POSE = 15 };
 
 typedef double D;
 typedef V3<double> Vec;
 
-struct Rec {
+// A body's record and parameters, field by field across LS lanes: LS is known
+// at compile time, so a field is an offset in its load or store.
+template <int LS> struct Rec {
     D* p;
-    int64_t ls;
-    __host__ __device__ __forceinline__ D& operator[](int f) const { return p[f * ls]; }
+    __host__ __device__ __forceinline__ D& operator[](int f) const { return p[f * LS]; }
 };
-struct Par {
+template <int LS> struct Par {
     const D* p;
-    int64_t ls;
-    __host__ __device__ __forceinline__ D operator[](int f) const { return p[f * ls]; }
+    __host__ __device__ __forceinline__ D operator[](int f) const { return p[f * LS]; }
 };
 
 #define TILE_FN __host__ __device__ __forceinline__
@@ -74,8 +76,8 @@ struct Par {
 #endif
 
 template <class A> TILE_FN Vec get3(const A& a, int f) { return Vec{a[f], a[f + 1], a[f + 2]}; }
-TILE_FN void put3(const Rec& r, int f, Vec v) { r[f] = v.x; r[f + 1] = v.y; r[f + 2] = v.z; }
-TILE_FN S3<D> get6(const Rec& r, int f) { return S3<D>{r[f], r[f + 1], r[f + 2], r[f + 3], r[f + 4], r[f + 5]}; }
+template <class A> TILE_FN void put3(const A& r, int f, Vec v) { r[f] = v.x; r[f + 1] = v.y; r[f + 2] = v.z; }
+template <class A> TILE_FN S3<D> get6(const A& r, int f) { return S3<D>{r[f], r[f + 1], r[f + 2], r[f + 3], r[f + 4], r[f + 5]}; }
 template <class A> TILE_FN M3<D> get9(const A& a, int f) {
     M3<D> m;
 #pragma unroll
@@ -163,25 +165,36 @@ template <int AX> TILE_FN void rotSym2(D c, D s, S3<D>& m) {
 // A zero that adding leaves out at compile time: x + (-0.0) is x.
 #define TILE_NIL (-0.0)
 
+TILE_FN D rsqrtD(D x) {
+#ifdef __CUDA_ARCH__
+    return rsqrt(x);
+#else
+    return D(1) / sqrt(x);
+#endif
+}
 // Quaternion (normalised here) -> R_FM (RigidBodyNodeSpec_Ball.h:134-214).
 TILE_FN M3<D> quatMatrix(const D* q) {
-    const D oo = D(1) / sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+    const D oo = rsqrtD(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
     const D e0 = q[0] * oo, e1 = q[1] * oo, e2 = q[2] * oo, e3 = q[3] * oo;
     const D f1 = e1 + e1, f2 = e2 + e2, f3 = e3 + e3;
     const D p01 = e0 * f1, p02 = e0 * f2, p03 = e0 * f3;
+    const D t1 = D(1) - e1 * f1;
     M3<D> R;
+    R.a[0] = (D(1) - e2 * f2) - e3 * f3;
+    R.a[4] = t1 - e3 * f3;
+    R.a[8] = t1 - e2 * f2;
     R.a[1] = e1 * f2 - p03;
     R.a[3] = e1 * f2 + p03;
     R.a[2] = e1 * f3 + p02;
     R.a[6] = e1 * f3 - p02;
     R.a[5] = e2 * f3 - p01;
     R.a[7] = e2 * f3 + p01;
-    const D q00 = e0 * e0, q11 = e1 * e1, q22 = e2 * e2, q33 = e3 * e3;
-    const D a = q00 - q11, b = q22 - q33;
-    R.a[0] = (q00 + q11) - (q22 + q33);
-    R.a[4] = a + b;
-    R.a[8] = a - b;
     return R;
+}
+// w x (w x v), w2 = w . w
+TILE_FN Vec cross2(Vec w, D w2, Vec v) {
+    const D t = dot(w, v);
+    return Vec{t * w.x - w2 * v.x, t * w.y - w2 * v.y, t * w.z - w2 * v.z};
 }
 
 // Inverse of a symmetric 3x3; false when its determinant is zero.
@@ -257,8 +270,8 @@ struct GenJoint {
     int n;
 };
 
-template <bool MINV, class Src, class Out>
-TILE_FN void pass1Gen(const SlotRow& r, const Par& par, const Rec& rec, const Src& src, Out& out, GenJoint& j) {
+template <bool MINV, class PA, class RC, class Src, class Out>
+TILE_FN void pass1Gen(const SlotRow& r, const PA& par, const RC& rec, const Src& src, Out& out, GenJoint& j) {
     const int type = r.info & 15, n = (r.info >> 4) & 15;
     D q[6], u[6];
 #pragma unroll
@@ -340,12 +353,13 @@ TILE_FN void pass1Gen(const SlotRow& r, const Par& par, const Rec& rec, const Sr
     }
 }
 
-template <int CL, bool MINV, class Src, class Out>
-TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec& rec, const Rec& recP, const Src& src,
+template <int CL, bool MINV, class PA, class RC, class Src, class Out>
+TILE_FN void pass1(const Model& md, const SlotRow& r, const PA& par, const RC& rec, const RC& recP, const Src& src,
                    Out& out) {
-    const bool hasP = r.parent >= 0, ci = (r.info & F_CI) != 0;
+    const bool hasP = r.parent >= 0, ci = (r.info & F_CI) != 0, freely = !MINV && (r.info & F_FREELY) != 0;
     const Vec d = get3(par, PR_D);
     const Vec wP = (!MINV && hasP) ? get3(recP, RC_W) : zero();
+    const D wP2 = (!MINV && hasP) ? recP[RC_W2] : D(0);
     Vec l = d, w = zero(), gw = zero(), gv = zero();
     // rotates by C^T (into F) where C is not the identity
     auto toF = [&](Vec v) { return ci ? v : mulT(get9(par, PR_C), v); };
@@ -361,11 +375,14 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
         out.qdot(r.qo, u0);
         if (MINV) rec[RC_X] = src.fext(r.uo);
         else {
-            rec[RC_X] = (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
-            const Vec t = rotT<2>(c1, s1, wF);
-            w = Vec{t.x, t.y, t.z + u0};
-            gw = Vec{u0 * t.y, -(u0 * t.x), 0};
-            gv = rotT<2>(c1, s1, toF(cross(wP, cross(wP, l))));
+            rec[RC_X] = freely ? D(0) : (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
+            w.z = u0;
+            if (hasP) {
+                const Vec t = rotT<2>(c1, s1, wF);
+                w = Vec{t.x, t.y, t.z + u0};
+                gw = Vec{u0 * t.y, -(u0 * t.x), 0};
+                gv = rotT<2>(c1, s1, toF(cross2(wP, wP2, l)));
+            }
         }
     } else if (CL == CL_SLIDER) {
         const D q0 = src.q(r.qo), u0 = MINV ? D(0) : src.u(r.uo);
@@ -374,12 +391,14 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
         out.qdot(r.qo, u0);
         if (MINV) rec[RC_X] = src.fext(r.uo);
         else {
-            rec[RC_X] = (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
+            rec[RC_X] = freely ? D(0) : (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
             w = wF;
-            gv = toF(cross(wP, cross(wP, l)));
-            const D t = u0 + u0;
-            gv.y = gv.y + t * wF.z;
-            gv.z = gv.z - t * wF.y;
+            if (hasP) {
+                gv = toF(cross2(wP, wP2, l));
+                const D t = u0 + u0;
+                gv.y = gv.y + t * wF.z;
+                gv.z = gv.z - t * wF.y;
+            }
             vrelL.x = u0;
         }
     } else if (CL == CL_UNIV) {
@@ -392,11 +411,11 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
         out.qdot(r.qo + 1, u1);
         if (MINV) { rec[RC_X] = src.fext(r.uo); rec[RC_X + 1] = src.fext(r.uo + 1); }
         else {
-            rec[RC_X] = (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
-            rec[RC_X + 1] = (par[PR_S + 1] - par[PR_K + 1] * q1) - par[PR_B + 1] * u1;
+            rec[RC_X] = freely ? D(0) : (par[PR_S] - par[PR_K] * q0) - par[PR_B] * u0;
+            rec[RC_X + 1] = freely ? D(0) : (par[PR_S + 1] - par[PR_K + 1] * q1) - par[PR_B + 1] * u1;
             const Vec t = rotT<0>(c1, s1, wF);  // between the axes
             gw = Vec{-(t.z * u1), t.z * u0, (t.x * u1 - t.y * u0) + u0 * u1};
-            gv = rotT<0>(c1, s1, toF(cross(wP, cross(wP, l))));
+            if (hasP) gv = rotT<0>(c1, s1, toF(cross2(wP, wP2, l)));
             w = rotT<1>(c2, s2, Vec{t.x + u0, t.y + u1, t.z});
         }
     } else if (CL == CL_BALL || CL == CL_FREE) {
@@ -419,11 +438,11 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
             const Vec uw = Vec{src.u(r.uo), src.u(r.uo + 1), src.u(r.uo + 2)};
             if (CL == CL_FREE) uv = Vec{src.u(r.uo + 3), src.u(r.uo + 4), src.u(r.uo + 5)};
             // qdot = N(q) w with e = q/2 (Rotation.h:712-719, 990-992)
-            const D h0 = q[0] * D(0.5), h1 = q[1] * D(0.5), h2 = q[2] * D(0.5), h3 = q[3] * D(0.5);
-            out.qdot(r.qo + 0, -h1 * uw.x - h2 * uw.y - h3 * uw.z);
-            out.qdot(r.qo + 1, h0 * uw.x + h3 * uw.y - h2 * uw.z);
-            out.qdot(r.qo + 2, -h3 * uw.x + h0 * uw.y + h1 * uw.z);
-            out.qdot(r.qo + 3, h2 * uw.x - h1 * uw.y + h0 * uw.z);
+            const Vec hu = D(0.5) * uw;
+            out.qdot(r.qo + 0, -q[1] * hu.x - q[2] * hu.y - q[3] * hu.z);
+            out.qdot(r.qo + 1, q[0] * hu.x + q[3] * hu.y - q[2] * hu.z);
+            out.qdot(r.qo + 2, -q[3] * hu.x + q[0] * hu.y + q[1] * hu.z);
+            out.qdot(r.qo + 3, q[2] * hu.x - q[1] * hu.y + q[0] * hu.z);
             if (CL == CL_FREE) {
                 out.qdot(r.qo + 4, uv.x);
                 out.qdot(r.qo + 5, uv.y);
@@ -434,11 +453,11 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
             const D qq[6] = {q[0], q[1], q[2], q[3], pf.x, pf.y};
 #pragma unroll
             for (int k = 0; k < n; ++k)
-                rec[RC_X + k] = (par[PR_S + k] - par[PR_K + k] * qq[k]) - par[PR_B + k] * uu[k];
+                rec[RC_X + k] = freely ? D(0) : (par[PR_S + k] - par[PR_K + k] * qq[k]) - par[PR_B + k] * uu[k];
             w = mulT(E, wF + uw);
             if (hasP) {
                 gw = mulT(E, cross(wF, uw));
-                Vec t = toF(cross(wP, cross(wP, l)));
+                Vec t = toF(cross2(wP, wP2, l));
                 if (CL == CL_FREE) t = t + cross(wF + wF, uv);
                 gv = mulT(E, t);
             }
@@ -454,7 +473,7 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
         if (!MINV) {
             w = mulT(E, wF + j.wrel);
             gw = mulT(E, cross(wF, j.wrel) + j.hd);
-            gv = mulT(E, toF(cross(wP, cross(wP, l))) + cross(wF + wF, j.vrel));
+            gv = mulT(E, toF(cross2(wP, wP2, l)) + cross(wF + wF, j.vrel));
             vrelL = mulT(E, j.vrel);
         }
     }
@@ -465,11 +484,13 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
     S3<D> J{par[PR_J], par[PR_J + 1], par[PR_J + 2], par[PR_J + 3], par[PR_J + 4], par[PR_J + 5]};
     Vec zw = zero(), zv = zero();
     if (!MINV) {
+        const D w2 = dot(w, w);
         put3(rec, RC_W, w);
+        rec[RC_W2] = w2;
         put3(rec, RC_GAM, gw);
         put3(rec, RC_GAM + 3, gv);
         zw = cross(w, mul(J, w));
-        zv = cross(w, cross(w, mc));
+        zv = cross2(w, w2, mc);
         if (md.pose) {
             // Ground pose, velocity of M's origin (M axes) and contacts
             M3<D> RP = ident3<D>();
@@ -516,7 +537,7 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const Par& par, const Rec&
 // ------------------------------------------------------------------ pass 2
 // Adds P+ (in F axes about the origin of M, rotated here by C) and z+ to the
 // parent's record: P+ shifted by l, z+ by l.
-TILE_FN void pushShift(const Rec& recP, Vec l, const S3<D>& J, const M3<D>& F, const S3<D>& M, Vec zw, Vec zv) {
+template <class RC> TILE_FN void pushShift(const RC& recP, Vec l, const S3<D>& J, const M3<D>& F, const S3<D>& M, Vec zw, Vec zv) {
     const D x = l.x, y = l.y, z = l.z;
     const D* f = F.a;
     D g[9];
@@ -546,7 +567,7 @@ TILE_FN void pushShift(const Rec& recP, Vec l, const S3<D>& J, const M3<D>& F, c
     put3(recP, RC_Z, (get3(recP, RC_Z) + zw) + cross(l, zv));
     put3(recP, RC_Z + 3, get3(recP, RC_Z + 3) + zv);
 }
-TILE_FN void pushFull(const SlotRow& r, const Par& par, const Rec& recP, Vec l, const S3<D>& J, const M3<D>& F,
+template <class PA, class RC> TILE_FN void pushFull(const SlotRow& r, const PA& par, const RC& recP, Vec l, const S3<D>& J, const M3<D>& F,
                       const S3<D>& M, Vec zw, Vec zv) {
     if (r.info & F_CI) {
         pushShift(recP, l, J, F, M, zw, zv);
@@ -555,12 +576,14 @@ TILE_FN void pushFull(const SlotRow& r, const Par& par, const Rec& recP, Vec l, 
         pushShift(recP, l, reexpress(C, J), mulABt(mul(C, F), C), reexpress(C, M), mul(C, zw), mul(C, zv));
     }
 }
-// The same for P+ = (0, 0, M): what a rotational joint with three axes passes on.
-TILE_FN void pushMass(const SlotRow& r, const Par& par, const Rec& recP, Vec l, S3<D> M, Vec zw, Vec zv) {
+// The same for P+ = (0, 0, M): what a rotational joint with three axes passes
+// on. force: zw (the joint's own torque) is not zero.
+template <class PA, class RC> TILE_FN void pushMass(const SlotRow& r, const PA& par, const RC& recP, Vec l, S3<D> M, Vec zw, bool force,
+                                                   Vec zv) {
     if (!(r.info & F_CI)) {
         const M3<D> C = get9(par, PR_C);
         M = reexpress(C, M);
-        zw = mul(C, zw);
+        if (force) zw = mul(C, zw);
         zv = mul(C, zv);
     }
     const D x = l.x, y = l.y, z = l.z;
@@ -588,7 +611,9 @@ TILE_FN void pushMass(const SlotRow& r, const Par& par, const Rec& recP, Vec l, 
     recP[RC_M + 3] = recP[RC_M + 3] + M.xy;
     recP[RC_M + 4] = recP[RC_M + 4] + M.xz;
     recP[RC_M + 5] = recP[RC_M + 5] + M.yz;
-    put3(recP, RC_Z, (get3(recP, RC_Z) + zw) + cross(l, zv));
+    Vec t = get3(recP, RC_Z) + cross(l, zv);
+    if (force) t = t + zw;
+    put3(recP, RC_Z, t);
     put3(recP, RC_Z + 3, get3(recP, RC_Z + 3) + zv);
 }
 
@@ -623,8 +648,8 @@ template <int AX> TILE_FN D eliminate(S3<D>& J, M3<D>& F, S3<D>& M, Vec& zw, Vec
     return d;
 }
 
-template <int CL, bool MINV>
-TILE_FN bool pass2(const SlotRow& r, const Par& par, const Rec& rec, const Rec& recP) {
+template <int CL, bool MINV, class PA, class RC>
+TILE_FN bool pass2(const SlotRow& r, const PA& par, const RC& rec, const RC& recP) {
     const bool hasP = r.parent >= 0;
     S3<D> J = get6(rec, RC_J), M = get6(rec, RC_M);
     M3<D> F = get9(rec, RC_F);
@@ -725,7 +750,8 @@ TILE_FN bool pass2(const SlotRow& r, const Par& par, const Rec& rec, const Rec& 
         const Vec f = get3(rec, RC_X);
         S3<D> Ji;
         ok = invSym(J, Ji);
-        const Vec e = mul(Ji, mulT(E, f) - zw);
+        const bool freely = !MINV && (r.info & F_FREELY) != 0;
+        const Vec e = freely ? mul(Ji, -zw) : mul(Ji, mulT(E, f) - zw);
         M3<D> Y;  // J^-1 F
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -745,7 +771,7 @@ TILE_FN bool pass2(const SlotRow& r, const Par& par, const Rec& rec, const Rec& 
             M.zz -= F.a[2] * Y.a[2] + F.a[5] * Y.a[5] + F.a[8] * Y.a[8];
             zv = zv + mulT(F, e);
             if (!MINV) zv = zv + mul(M, gv);
-            pushMass(r, par, recP, l, reexpress(E, M), f, mul(E, zv));
+            pushMass(r, par, recP, l, reexpress(E, M), f, !freely, mul(E, zv));
         }
     } else if (CL == CL_FREE) {
         // P+ = 0: the body's acceleration follows from its own balance
@@ -774,7 +800,7 @@ TILE_FN bool pass2(const SlotRow& r, const Par& par, const Rec& rec, const Rec& 
         put3(rec, RC_X + 3, a);
         if (hasP) {
             const S3<D> none{0, 0, 0, 0, 0, 0};
-            pushMass(r, par, recP, l, none, fw, fv);
+            pushMass(r, par, recP, l, none, fw, true, fv);
         }
     } else {
         // one column after another, the outermost last: a joint of n mobilities
@@ -820,8 +846,8 @@ TILE_FN bool pass2(const SlotRow& r, const Par& par, const Rec& rec, const Rec& 
 
 // ------------------------------------------------------------------ pass 3
 // Base to tip: udot and the body's acceleration.
-template <int CL, bool MINV, class Out>
-TILE_FN void pass3(const Model& md, const SlotRow& r, const Par& par, const Rec& rec, const Rec& recP, Out& out) {
+template <int CL, bool MINV, class PA, class RC, class Out>
+TILE_FN void pass3(const Model& md, const SlotRow& r, const PA& par, const RC& rec, const RC& recP, Out& out) {
     const bool ci = (r.info & F_CI) != 0;
     Vec aw = zero(), av = MINV ? zero() : -md.g;
     if (r.parent >= 0) {

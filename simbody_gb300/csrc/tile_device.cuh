@@ -16,9 +16,19 @@
 
 namespace sbg {
 
+// LS: lane stride of the records (the widest a tile can be); SH: the tables
+// have no lanes (one topology per tile); YS: stride of the state columns, 0 =
+// the instance's own.
+template <int LS_, bool SH_, int YS_> struct TileCfg {
+    static constexpr int LS = LS_, YS = YS_;
+    static constexpr bool SH = SH_;
+};
+
 struct TileCtx {
     TileDesc d;
     double* rec;     // the lane's column of the tile's records
+    const int4* slots;  // the lane's column of the slot integers, parameters
+    const double* par;
     int lane, w;     // lane of the tile, warp of the block
     bool on;         // the lane holds an instance
     int inst;
@@ -28,136 +38,138 @@ __device__ __forceinline__ void tileSync(int W) {
     if (W == 1) __syncwarp(); else __syncthreads();
 }
 
+template <class CF> __device__ __forceinline__ void tileTables(const TileTables& TT, TileCtx& c) {
+    c.lane = threadIdx.x & 31;
+    c.w = threadIdx.x >> 5;
+    const int l = CF::SH || c.lane >= CF::LS ? 0 : c.lane;
+    c.slots = reinterpret_cast<const int4*>(TT.slots + c.d.slot0) + 2 * l;
+    c.par = TT.par + c.d.par0 + l;
+}
 // Tile `id` of a batch.
+template <class CF>
 __device__ __forceinline__ TileCtx tileCtx(const DevTables& T, const TileTables& TT, int id, double* recs) {
     TileCtx c;
     c.d = TT.desc[id];
-    c.lane = threadIdx.x & 31;
-    c.w = threadIdx.x >> 5;
+    tileTables<CF>(TT, c);
     c.on = c.lane < c.d.lanes;
-    c.rec = recs + c.d.rec0 + c.lane;
-    c.inst = c.on ? T.order[c.d.pos0 + c.lane] : 0;
+    c.rec = recs + c.d.rec0 + (c.on ? c.lane : 0);
+    c.inst = c.on ? T.order[c.d.pos0 + c.lane] : T.order[c.d.pos0];
     return c;
 }
 // The tile of one instance, in a tile set with one tile per instance, on the
 // block's own records.
-__device__ __forceinline__ TileCtx tileCtxOne(const TileTables& TT, int inst, double* recs) {
+template <class CF> __device__ __forceinline__ TileCtx tileCtxOne(const TileTables& TT, int inst, double* recs) {
     TileCtx c;
     c.d = TT.desc[inst];
-    c.lane = threadIdx.x & 31;
-    c.w = threadIdx.x >> 5;
+    tileTables<CF>(TT, c);
     c.on = c.lane == 0;
     c.rec = recs;
     c.inst = inst;
     return c;
 }
 
-// Class of the warp's body at a step (-1: none), and the lane's row of it
-// (false: none on this lane).
-__device__ __forceinline__ int tileClass(const TileTables& TT, const TileCtx& c, int step) {
-    return TT.cls[c.d.cls0 + step * TT.W + c.w];
+// The warp's slot at a step: its class (-1: none) and the lane's integers.
+struct TileSlot {
+    int cl;
+    int4 a, b;
+    __device__ __forceinline__ bool some() const { return a.x >= 0; }  // a body on this lane
+    __device__ __forceinline__ tile::SlotRow row() const { return tile::SlotRow{a.x, a.y, a.z, a.w, b.x, b.y, b.z}; }
+};
+template <class CF> __device__ __forceinline__ TileSlot tileSlot(const TileTables& TT, const TileCtx& c, int step) {
+    const int slot = step * TT.W + c.w;
+    const int4* s = c.slots + (int64_t)slot * (2 * (CF::SH ? 1 : CF::LS));
+    TileSlot t;
+    t.cl = TT.cls[c.d.cls0 + slot];
+    t.a = s[0];
+    t.b = s[1];
+    return t;
 }
-__device__ __forceinline__ bool tileRow(const TileTables& TT, const TileCtx& c, int slot, tile::SlotRow& r, tile::Par& par) {
-    const int64_t st = c.d.shared ? 1 : c.d.ls, l = c.d.shared ? 0 : c.lane;
-    const int32_t* s = TT.slots + c.d.slot0 + (int64_t)slot * tile::SI_COUNT * st + l;
-    r.qo = s[tile::SI_Q * st];
-    r.uo = s[tile::SI_U * st];
-    r.parent = s[tile::SI_PARENT * st];
-    r.info = s[tile::SI_INFO * st];
-    r.row = s[tile::SI_ROW * st];
-    r.kbeg = s[tile::SI_KBEG * st];
-    r.kcnt = s[tile::SI_KCNT * st];
-    par.p = TT.par + c.d.par0 + (int64_t)slot * tile::PR_COUNT * st + l;
-    par.ls = st;
-    return r.qo >= 0;
+
+// f(slot, row, parameters) for the warp's bodies in the order of the steps (or
+// back), the next step's integers loaded ahead; f runs on the lanes of `run`
+// that have a body at the step.
+template <class CF, bool FORWARD, class F>
+__device__ __forceinline__ void tileSweep(const TileTables& TT, const TileCtx& c, bool run, F f) {
+    constexpr int LN = CF::SH ? 1 : CF::LS;
+    const int n = c.d.nsteps, W = TT.W;
+    const int first = FORWARD ? 0 : n - 1, inc = FORWARD ? 1 : -1;
+    TileSlot t = tileSlot<CF>(TT, c, first);
+    for (int k = 0; k < n; ++k) {
+        const int step = first + inc * k;
+        const TileSlot next = tileSlot<CF>(TT, c, k + 1 < n ? step + inc : step);
+        if (t.cl >= 0 && run && t.some()) {
+            const int slot = step * W + c.w;
+            f(t.cl, slot, t.row(), tile::Par<LN>{c.par + (int64_t)slot * (tile::PR_COUNT * LN)});
+        }
+        tileSync(W);
+        t = next;
+    }
 }
 
 // One RHS of the tile's instances for which `active` holds; SINGULAR_D is
 // reported to the thread whose body met it. All warps of the block call it.
-template <bool MINV, class Src, class Out>
+template <class CF, bool MINV, class Src, class Out>
 __device__ __forceinline__ int tileRhs(const DevTables& T, const TileTables& TT, const TileCtx& c, const Src& src,
                                        Out& out, bool active) {
     using namespace tile;
-    const int W = TT.W, nsteps = c.d.nsteps;
-    const int64_t ls = c.d.ls, rs = TT.rsTotal;
+    constexpr int LN = CF::SH ? 1 : CF::LS;
+    typedef Rec<CF::LS> RC;
+    typedef Par<LN> PA;
     Model md;
     md.kpar = T.kpar64;
     md.rs = TT.rs;
     md.pose = !MINV && TT.pose;
-    md.bodyPar = nullptr;
-    md.g = zero();
-    int body0 = 0;
-    if (c.on) {
-        md.g = Vec{T.grav[3 * c.inst], T.grav[3 * c.inst + 1], T.grav[3 * c.inst + 2]};
-        body0 = T.ibody[c.inst];
-        md.bodyPar = T.par64 + (int64_t)body0 * kParamStride;
-    }
+    md.g = Vec{T.grav[3 * c.inst], T.grav[3 * c.inst + 1], T.grav[3 * c.inst + 2]};
+    const int body0 = T.ibody[c.inst];
+    md.bodyPar = T.par64 + (int64_t)body0 * kParamStride;
     const bool run = c.on && active;
     bool ok = true;
-    auto recOf = [&](int slot) { return Rec{c.rec + (int64_t)slot * rs * ls, ls}; };
-    for (int step = 0; step < nsteps; ++step) {
-        const int cl = tileClass(TT, c, step), slot = step * W + c.w;
-        SlotRow r;
-        Par par;
-        if (cl >= 0 && run && tileRow(TT, c, slot, r, par)) {
-            const Rec rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
-            // contact spheres are grouped by body row of the batch's body table
-            if (r.kcnt > 0 && md.pose) r.kbeg = T.kbeg[body0 + r.row];
-            switch (cl) {
-            case CL_PIN: pass1<CL_PIN, MINV>(md, r, par, rec, recP, src, out); break;
-            case CL_SLIDER: pass1<CL_SLIDER, MINV>(md, r, par, rec, recP, src, out); break;
-            case CL_UNIV: pass1<CL_UNIV, MINV>(md, r, par, rec, recP, src, out); break;
-            case CL_BALL: pass1<CL_BALL, MINV>(md, r, par, rec, recP, src, out); break;
-            case CL_FREE: pass1<CL_FREE, MINV>(md, r, par, rec, recP, src, out); break;
-            default: pass1<CL_GEN, MINV>(md, r, par, rec, recP, src, out); break;
-            }
+    const int64_t recSize = (int64_t)TT.rsTotal * CF::LS;
+    auto recOf = [&](int slot) { return RC{c.rec + slot * recSize}; };
+    tileSweep<CF, true>(TT, c, run, [&](int cl, int slot, SlotRow r, PA par) {
+        const RC rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
+        // contact spheres are grouped by body row of the batch's body table
+        if (md.pose && r.kcnt > 0) r.kbeg = T.kbeg[body0 + r.row];
+        switch (cl) {
+        case CL_PIN: pass1<CL_PIN, MINV>(md, r, par, rec, recP, src, out); break;
+        case CL_SLIDER: pass1<CL_SLIDER, MINV>(md, r, par, rec, recP, src, out); break;
+        case CL_UNIV: pass1<CL_UNIV, MINV>(md, r, par, rec, recP, src, out); break;
+        case CL_BALL: pass1<CL_BALL, MINV>(md, r, par, rec, recP, src, out); break;
+        case CL_FREE: pass1<CL_FREE, MINV>(md, r, par, rec, recP, src, out); break;
+        default: pass1<CL_GEN, MINV>(md, r, par, rec, recP, src, out); break;
         }
-        tileSync(W);
-    }
-    for (int step = nsteps - 1; step >= 0; --step) {
-        const int cl = tileClass(TT, c, step), slot = step * W + c.w;
-        SlotRow r;
-        Par par;
-        if (cl >= 0 && run && tileRow(TT, c, slot, r, par)) {
-            const Rec rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
-            switch (cl) {
-            case CL_PIN: ok &= pass2<CL_PIN, MINV>(r, par, rec, recP); break;
-            case CL_SLIDER: ok &= pass2<CL_SLIDER, MINV>(r, par, rec, recP); break;
-            case CL_UNIV: ok &= pass2<CL_UNIV, MINV>(r, par, rec, recP); break;
-            case CL_BALL: ok &= pass2<CL_BALL, MINV>(r, par, rec, recP); break;
-            case CL_FREE: ok &= pass2<CL_FREE, MINV>(r, par, rec, recP); break;
-            default: ok &= pass2<CL_GEN, MINV>(r, par, rec, recP); break;
-            }
+    });
+    tileSweep<CF, false>(TT, c, run, [&](int cl, int slot, SlotRow r, PA par) {
+        const RC rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
+        switch (cl) {
+        case CL_PIN: ok &= pass2<CL_PIN, MINV>(r, par, rec, recP); break;
+        case CL_SLIDER: ok &= pass2<CL_SLIDER, MINV>(r, par, rec, recP); break;
+        case CL_UNIV: ok &= pass2<CL_UNIV, MINV>(r, par, rec, recP); break;
+        case CL_BALL: ok &= pass2<CL_BALL, MINV>(r, par, rec, recP); break;
+        case CL_FREE: ok &= pass2<CL_FREE, MINV>(r, par, rec, recP); break;
+        default: ok &= pass2<CL_GEN, MINV>(r, par, rec, recP); break;
         }
-        tileSync(W);
-    }
-    for (int step = 0; step < nsteps; ++step) {
-        const int cl = tileClass(TT, c, step), slot = step * W + c.w;
-        SlotRow r;
-        Par par;
-        if (cl >= 0 && run && tileRow(TT, c, slot, r, par)) {
-            const Rec rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
-            switch (cl) {
-            case CL_PIN: pass3<CL_PIN, MINV>(md, r, par, rec, recP, out); break;
-            case CL_SLIDER: pass3<CL_SLIDER, MINV>(md, r, par, rec, recP, out); break;
-            case CL_UNIV: pass3<CL_UNIV, MINV>(md, r, par, rec, recP, out); break;
-            case CL_BALL: pass3<CL_BALL, MINV>(md, r, par, rec, recP, out); break;
-            case CL_FREE: pass3<CL_FREE, MINV>(md, r, par, rec, recP, out); break;
-            default: pass3<CL_GEN, MINV>(md, r, par, rec, recP, out); break;
-            }
+    });
+    tileSweep<CF, true>(TT, c, run, [&](int cl, int slot, SlotRow r, PA par) {
+        const RC rec = recOf(slot), recP = recOf(r.parent < 0 ? slot : r.parent);
+        switch (cl) {
+        case CL_PIN: pass3<CL_PIN, MINV>(md, r, par, rec, recP, out); break;
+        case CL_SLIDER: pass3<CL_SLIDER, MINV>(md, r, par, rec, recP, out); break;
+        case CL_UNIV: pass3<CL_UNIV, MINV>(md, r, par, rec, recP, out); break;
+        case CL_BALL: pass3<CL_BALL, MINV>(md, r, par, rec, recP, out); break;
+        case CL_FREE: pass3<CL_FREE, MINV>(md, r, par, rec, recP, out); break;
+        default: pass3<CL_GEN, MINV>(md, r, par, rec, recP, out); break;
         }
-        tileSync(W);
-    }
+    });
     return ok ? 0 : SBG_INST_SINGULAR_D;
 }
 
 // Calls f(row) for the lane's bodies that this warp owns.
-template <class F>
-__device__ __forceinline__ void tileBodies(const TileTables& TT, const TileCtx& c, F f) {
+template <class CF, class F>
+__device__ __forceinline__ void tileBodies(const TileTables& TT, const TileCtx& c, bool run, F f) {
     for (int step = 0; step < c.d.nsteps; ++step) {
-        tile::SlotRow r;
-        tile::Par par;
-        if (tileClass(TT, c, step) >= 0 && c.on && tileRow(TT, c, step * TT.W + c.w, r, par)) f(r);
+        const TileSlot t = tileSlot<CF>(TT, c, step);
+        if (t.cl >= 0 && run && t.some()) f(t.row());
     }
 }
 
@@ -189,61 +201,69 @@ __device__ __forceinline__ int tileReduce(const TileTables& TT, const TileCtx& c
 }
 
 // ----------------------------------------------------------- sources, sinks
-struct TileYSrc {
+// An instance's column: element k at k * YS from its base.
+template <int YS> struct TileCol {
+    int64_t base;
+    int stride, nq;
+    __device__ __forceinline__ TileCol(const DevTables& T, int inst)
+        : base(T.ybase[inst]), stride(YS ? YS : (int)T.ystride[inst]), nq(T.inq[inst]) {}
+    __device__ __forceinline__ int64_t at(int k) const { return base + (int64_t)k * (YS ? YS : stride); }
+    __device__ __forceinline__ int64_t atU(int k) const { return at(nq + k); }
+};
+template <int YS> struct TileYSrc {
+    TileCol<YS> c;
     const double* y;
-    int64_t base, stride;
-    int nq;
-    __device__ __forceinline__ double q(int k) const { return y[base + (int64_t)k * stride]; }
-    __device__ __forceinline__ double u(int k) const { return y[base + (int64_t)(nq + k) * stride]; }
+    __device__ __forceinline__ double q(int k) const { return y[c.at(k)]; }
+    __device__ __forceinline__ double u(int k) const { return y[c.atU(k)]; }
     __device__ __forceinline__ double fext(int) const { return 0.0; }
 };
-struct TileFSrc {  // M^-1 f: q and the given forces
-    const double* y;
-    const double* f;
-    int64_t base, stride;
-    int nq;
-    __device__ __forceinline__ double q(int k) const { return y[base + (int64_t)k * stride]; }
+template <int YS> struct TileFSrc {  // M^-1 f: q and the given forces
+    TileCol<YS> c;
+    const double *y, *f;
+    __device__ __forceinline__ double q(int k) const { return y[c.at(k)]; }
     __device__ __forceinline__ double u(int) const { return 0.0; }
-    __device__ __forceinline__ double fext(int k) const { return f[base + (int64_t)(nq + k) * stride]; }
+    __device__ __forceinline__ double fext(int k) const { return f[c.atU(k)]; }
 };
-// Stage input y0 + c * combo(f) of RK-Merson, formed while pass 1 loads it
-// (RungeKuttaMersonIntegrator.cpp:108-126).
-struct TileStageSrc {
-    const double* y;
-    const double *f0, *fa, *fb;
-    int64_t base, stride;
-    int nq, stage;
-    double c;
-    __device__ __forceinline__ double at(int k) const {
-        const int64_t e = base + (int64_t)k * stride;
-        const double y0 = y[e];
-        switch (stage) {
-        case 0: return y0;
-        case 1: return y0 + c * f0[e];                                    // h/3 f0
-        case 2: return y0 + c * (f0[e] + fa[e]);                          // h/6 (f0+f1)
-        case 3: return y0 + c * (f0[e] + 3.0 * fa[e]);                    // h/8 (f0+3f2)
-        default: return y0 + c * ((f0[e] - 3.0 * fa[e]) + 4.0 * fb[e]);   // h/2 (f0-3f2+4f3)
+// Stage input y0 + c * combo(f) of RK-Merson (RungeKuttaMersonIntegrator.cpp:
+// 108-126) into the plane yt, element by element over the block's warps. Formed
+// in the bodies' loads instead, its five cases made up most of the kernel's
+// code, which then ran from beyond the instruction cache.
+template <class CF>
+__device__ __forceinline__ void tileStageInput(const TileTables& TT, const TileCtx& c, const TileCol<CF::YS>& col, int ny,
+                                               bool run, int stage, double h, const double* y, const double* f0,
+                                               const double* fa, const double* fb, double* yt) {
+    const int W = TT.W;
+    auto all = [&](auto f) {
+        if (run) {
+#pragma unroll 4
+            for (int k = c.w; k < ny; k += W) {
+                const int64_t e = col.at(k);
+                yt[e] = f(e);
+            }
         }
-    }
-    __device__ __forceinline__ double q(int k) const { return at(k); }
-    __device__ __forceinline__ double u(int k) const { return at(nq + k); }
-    __device__ __forceinline__ double fext(int) const { return 0.0; }
-};
-struct TileOut {
+    };
+    if (stage == 0) all([&](int64_t e) { return y[e]; });
+    else if (stage == 1) all([&](int64_t e) { return y[e] + h * f0[e]; });                          // h/3 f0
+    else if (stage == 2) all([&](int64_t e) { return y[e] + h * (f0[e] + fa[e]); });                // h/6 (f0+f1)
+    else if (stage == 3) all([&](int64_t e) { return y[e] + h * (f0[e] + 3.0 * fa[e]); });          // h/8 (f0+3f2)
+    else all([&](int64_t e) { return y[e] + h * ((f0[e] - 3.0 * fa[e]) + 4.0 * fb[e]); });          // h/2 (f0-3f2+4f3)
+    tileSync(W);
+}
+template <int YS> struct TileOut {
+    TileCol<YS> c;
     double* f;
-    int64_t base, stride;
-    int nq;
     bool finite = true;
-    __device__ __forceinline__ void qdot(int k, double v) { f[base + (int64_t)k * stride] = v; finite &= tile::finiteBits(v); }
-    __device__ __forceinline__ void udot(int k, double v) { f[base + (int64_t)(nq + k) * stride] = v; finite &= tile::finiteBits(v); }
+    __device__ __forceinline__ TileOut(TileCol<YS> col, double* p) : c(col), f(p) {}
+    __device__ __forceinline__ void qdot(int k, double v) { f[c.at(k)] = v; finite &= tile::finiteBits(v); }
+    __device__ __forceinline__ void udot(int k, double v) { f[c.atU(k)] = v; finite &= tile::finiteBits(v); }
 };
-struct TileUOut {  // M^-1 f: u slots only
+template <int YS> struct TileUOut {  // M^-1 f: u slots only
+    TileCol<YS> c;
     double* f;
-    int64_t base, stride;
-    int nq;
     bool finite = true;
+    __device__ __forceinline__ TileUOut(TileCol<YS> col, double* p) : c(col), f(p) {}
     __device__ __forceinline__ void qdot(int, double) {}
-    __device__ __forceinline__ void udot(int k, double v) { f[base + (int64_t)(nq + k) * stride] = v; finite &= tile::finiteBits(v); }
+    __device__ __forceinline__ void udot(int k, double v) { f[c.atU(k)] = v; finite &= tile::finiteBits(v); }
 };
 
 // |q|^2 dq - q (q . dq): N N^-1 dq of the unnormalised quaternion q with unit
@@ -259,5 +279,15 @@ __device__ __forceinline__ double tileQuatErrSq(const double* q, const double* d
     }
     return s;
 }
+
+// Calls f(TileCfg) for the kind of the tiles of a batch whose state columns
+// have stride YS (0: each its own).
+template <int YS, class F> inline void tileDispatch(const TileSet& S, F f) {
+    if (S.tt.ls == 1) f(TileCfg<1, true, YS>());
+    else if (S.tt.ls == 8 && !S.tt.shared) f(TileCfg<8, false, YS>());
+    else if (S.tt.shared) f(TileCfg<32, true, YS>());
+    else f(TileCfg<32, false, YS>());
+}
+typedef TileCfg<1, true, 0> TileOne;  // one tile per instance
 
 }  // namespace sbg

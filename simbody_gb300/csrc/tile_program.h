@@ -13,10 +13,13 @@
 // and with them its results, do not depend on which tile it is in.
 #pragma once
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <map>
+#include <queue>
 #include <vector>
 
 #include "tile_core.cuh"
@@ -29,7 +32,73 @@ inline int tileCost(int cls, int n) {
     static const int c[tile::CL_COUNT] = {300, 205, 500, 390, 600, 400};
     return c[cls] + (cls == tile::CL_GEN ? 150 * n : 0);
 }
-constexpr int kTileStepCost = 60;  // a step's own latency (loads, barrier) in FP64 instructions
+// In FP64 instructions: what a step waits for its barrier, and what a body waits
+// for its loads; another warp of the sub-partition fills the latter.
+constexpr int kTileStepCost = 60, kTileBodyWait = 150;
+
+inline int tileClassOf(int info) {
+    using namespace tile;
+    const int type = info & 15;
+    const bool quat = (info & F_QUAT) != 0;
+    return type == SBG_PIN ? CL_PIN : type == SBG_SLIDER ? CL_SLIDER : type == SBG_UNIVERSAL ? CL_UNIV
+           : type == SBG_BALL && quat ? CL_BALL : type == SBG_FREE && quat ? CL_FREE : CL_GEN;
+}
+
+// Orders the instances of a batch so that a tile's trees have their mobilizers
+// in like numbers: at a step all lanes take one class, so a tile takes as many
+// steps of a class as its richest tree. Halves the set at the median of the
+// class whose work spreads most, down to tiles of 32 (and of 8 within them);
+// the tiles with the most work come first. work: per instance and class. 8,192
+// random trees: lanes busy 57 % in the order of size alone, 65 % in this one.
+inline void tileOrder(std::vector<int>& pos, const std::vector<std::array<float, tile::CL_COUNT>>& work) {
+    using namespace tile;
+    struct Rec {
+        static void split(int* a, int n, const std::vector<std::array<float, CL_COUNT>>& work) {
+            const int unit = n > 32 ? 32 : 8;
+            if (n <= 8) return;
+            int best = 0;
+            float spread = -1;
+            for (int c = 0; c < CL_COUNT; ++c) {
+                float lo = work[a[0]][c], hi = lo, sum = 0, sq = 0;
+                for (int k = 0; k < n; ++k) {
+                    const float v = work[a[k]][c];
+                    lo = std::min(lo, v);
+                    hi = std::max(hi, v);
+                    sum += v;
+                    sq += v * v;
+                }
+                const float s = hi > lo ? sq - sum * sum / n : -1;
+                if (s > spread) { spread = s; best = c; }
+            }
+            if (spread < 0) return;  // all alike
+            const int m = ((n + 2 * unit - 1) / (2 * unit)) * unit;
+            if (m >= n) return;
+            std::nth_element(a, a + m, a + n, [&](int x, int y) {
+                return work[x][best] != work[y][best] ? work[x][best] > work[y][best] : x < y;
+            });
+            split(a, m, work);
+            split(a + m, n - m, work);
+        }
+    };
+    const int n = (int)pos.size();
+    if (n == 0) return;
+    Rec::split(pos.data(), n, work);
+    std::vector<std::pair<float, int>> tiles;  // work of the richest instance, first position
+    for (int p = 0; p + 32 <= n; p += 32) {
+        float most = 0;
+        for (int k = p; k < p + 32; ++k) {
+            float t = 0;
+            for (float v : work[pos[k]]) t += v;
+            most = std::max(most, t);
+        }
+        tiles.push_back({-most, p});
+    }
+    std::sort(tiles.begin(), tiles.end());
+    std::vector<int> out;
+    for (const auto& t : tiles) out.insert(out.end(), pos.begin() + t.second, pos.begin() + t.second + 32);
+    out.insert(out.end(), pos.begin() + n / 32 * 32, pos.end());
+    pos.swap(out);
+}
 
 // The rows of one topology for the tile driver.
 struct TileRows {
@@ -46,10 +115,8 @@ struct TileRows {
         ints.assign((size_t)nb * SI_COUNT, 0);
         for (int r = 0; r < nb; ++r) {
             const double* b = &t.par[(size_t)r * kParamStride];
-            const int type = t.info[r] & 15, n = (t.info[r] >> 4) & 15;
-            const bool quat = (t.info[r] & F_QUAT) != 0;
-            cls[r] = type == SBG_PIN ? CL_PIN : type == SBG_SLIDER ? CL_SLIDER : type == SBG_UNIVERSAL ? CL_UNIV
-                     : type == SBG_BALL && quat ? CL_BALL : type == SBG_FREE && quat ? CL_FREE : CL_GEN;
+            const int n = (t.info[r] >> 4) & 15;
+            cls[r] = tileClassOf(t.info[r]);
             gen |= cls[r] == CL_GEN;
             cost[r] = tileCost(cls[r], n);
             parent[r] = t.parent[r];
@@ -95,7 +162,7 @@ struct TileRows {
             }
             int32_t* s = &ints[(size_t)r * SI_COUNT];
             s[SI_Q] = t.qoff[r]; s[SI_U] = t.uoff[r]; s[SI_PARENT] = parent[r];
-            s[SI_INFO] = t.info[r] | (ci ? F_CI : 0);
+            s[SI_INFO] = t.info[r] | (ci ? F_CI : 0) | (t.fcnt[r] == 0 ? F_FREELY : 0);
             s[SI_ROW] = r; s[SI_KBEG] = t.kbeg[r]; s[SI_KCNT] = t.kcnt[r];
             pose |= t.kcnt[r] > 0;
         }
@@ -118,7 +185,9 @@ struct TileSchedule {
     int nsteps = 0;
     std::vector<int32_t> cls;              // nsteps * W
     std::vector<std::vector<int>> row;     // per slot, per lane
-    int64_t length = 0, load = 0;          // FP64 instructions: of the longest warp step by step, of all warps
+    // FP64 instructions: length, step by step of the busiest sub-partition (a
+    // block's warps take the SM's four in turn); load, of the busiest one in all
+    int64_t length = 0, load = 0;
 
     TileSchedule(const std::vector<const TileRows*>& lanes, int W) {
         using namespace tile;
@@ -145,10 +214,17 @@ struct TileSchedule {
         int remaining = 0;
         for (int l = 0; l < nl; ++l) remaining += L[l].left;
         std::vector<std::vector<int>> done(nl);
+        std::vector<int> turn(W);                 // warps, the one with the least work so far first
+        std::vector<int64_t> sum(W, 0), sub(std::min(W, 4), 0);
+        for (int w = 0; w < W; ++w) turn[w] = w;
         while (remaining > 0) {
-            int64_t longest = 0;
+            std::vector<int64_t> stepSub(sub.size(), 0), stepBody(sub.size(), 0);
             for (auto& d : done) d.clear();
-            for (int w = 0; w < W; ++w) {
+            std::stable_sort(turn.begin(), turn.end(), [&](int a, int b) { return sum[a] < sum[b]; });
+            cls.resize(cls.size() + W, -1);
+            row.resize(row.size() + W, std::vector<int>(nl, -1));
+            for (int w : turn) {
+                const size_t slot = (size_t)nsteps * W + w;
                 // the class with the most work ready, weighted by how critical it is
                 double score[CL_COUNT] = {};
                 for (int l = 0; l < nl; ++l) {
@@ -166,9 +242,8 @@ struct TileSchedule {
                 int best = -1;
                 for (int c = 0; c < CL_COUNT; ++c)
                     if (score[c] > 0 && (best < 0 || score[c] > score[best])) best = c;
-                cls.push_back(best);
-                row.emplace_back(nl, -1);
-                if (best < 0) continue;
+                if (best < 0) break;
+                cls[slot] = best;
                 int stepCost = 0;
                 for (int l = 0; l < nl; ++l) {
                     auto& rd = L[l].ready;
@@ -179,29 +254,35 @@ struct TileSchedule {
                     if (at < 0) continue;
                     const int r = rd[at];
                     rd.erase(rd.begin() + at);
-                    row.back()[l] = r;
+                    row[slot][l] = r;
                     done[l].push_back(r);
                     --remaining;
                     stepCost = std::max(stepCost, lanes[l]->cost[r]);
                 }
-                load += stepCost + kTileStepCost;
-                longest = std::max<int64_t>(longest, stepCost + kTileStepCost);
+                sum[w] += stepCost;
+                sub[w % 4] += stepCost;
+                stepSub[w % 4] += stepCost;
+                stepBody[w % 4] = std::max<int64_t>(stepBody[w % 4], stepCost + kTileBodyWait);
             }
             for (int l = 0; l < nl; ++l)
                 for (int r : done[l])
                     for (int k : L[l].next[r])
                         if (--L[l].waits[k] == 0) L[l].ready.push_back(k);
-            length += longest;
+            length += std::max(*std::max_element(stepSub.begin(), stepSub.end()),
+                               *std::max_element(stepBody.begin(), stepBody.end())) + kTileStepCost;
             ++nsteps;
         }
+        load = *std::max_element(sub.begin(), sub.end()) + (int64_t)nsteps * kTileStepCost / 4;
     }
-    static constexpr double kCritical = 3.0;
+    static constexpr double kCritical = 1.0;
 };
 
 // The tables of a batch's tiles on the host. Parameters are gathered on the
 // device from the topologies' rows (parRow: row per slot and lane, -1: none).
 struct TileProgram {
     int W = 1, rs = 0, rsTotal = 0;
+    int ls = 32;           // lanes per tile
+    bool shared = false;   // every tile has one topology: tables without lanes
     bool pose = false;
     std::vector<TileDesc> desc;
     std::vector<int32_t> cls, slots, parRow;
@@ -209,25 +290,22 @@ struct TileProgram {
 
     // One tile over `topo` (topology per lane). rows: per topology, rowBase:
     // its first row in the parameter rows.
-    void add(int pos0, const std::vector<int>& topo, int ls, const std::vector<const TileRows*>& rows,
+    void add(int pos0, const std::vector<int>& topo, const std::vector<const TileRows*>& rows,
              const std::vector<int64_t>& rowBase) {
         using namespace tile;
-        const bool same = std::all_of(topo.begin(), topo.end(), [&](int k) { return k == topo[0]; });
         TileDesc d{};
         d.pos0 = pos0;
         d.lanes = (int)topo.size();
-        d.ls = ls;
-        d.shared = same;
         d.rec0 = recElems;
-        const auto it = same ? known.find(topo[0]) : known.end();
+        const auto it = shared ? known.find(topo[0]) : known.end();
         if (it != known.end()) {
             d.cls0 = it->second.cls0; d.nsteps = it->second.nsteps;
             d.slot0 = it->second.slot0; d.par0 = it->second.par0;
         } else {
             std::vector<const TileRows*> lanes;
-            for (int l = 0; l < (same ? 1 : d.lanes); ++l) lanes.push_back(rows[topo[l]]);
+            for (int l = 0; l < (shared ? 1 : d.lanes); ++l) lanes.push_back(rows[topo[l]]);
             const TileSchedule s(lanes, W);
-            const int st = same ? 1 : ls, nl = (int)lanes.size();
+            const int st = shared ? 1 : ls, nl = (int)lanes.size();
             const int64_t nslots = (int64_t)s.nsteps * W;
             d.nsteps = s.nsteps;
             d.cls0 = (int32_t)cls.size();
@@ -243,22 +321,22 @@ struct TileProgram {
                 for (int64_t k = 0; k < nslots; ++k)
                     if (s.row[k][l] >= 0) slotOf[s.row[k][l]] = (int)k;
                 for (int r = 0; r < t.nb; ++r) {
-                    int32_t* o = &slots[d.slot0 + (int64_t)slotOf[r] * SI_COUNT * st + l];
-                    for (int k = 0; k < SI_COUNT; ++k) o[(int64_t)k * st] = t.ints[(size_t)r * SI_COUNT + k];
-                    o[(int64_t)SI_PARENT * st] = t.parent[r] < 0 ? -1 : slotOf[t.parent[r]];
+                    int32_t* o = &slots[d.slot0 + ((int64_t)slotOf[r] * st + l) * SI_COUNT];
+                    std::copy_n(&t.ints[(size_t)r * SI_COUNT], SI_COUNT, o);
+                    o[SI_PARENT] = t.parent[r] < 0 ? -1 : slotOf[t.parent[r]];
                     parRow[d.par0 / PR_COUNT + (int64_t)slotOf[r] * st + l] = (int32_t)(rowBase[topo[l]] + r);
                 }
             }
-            // the lanes of a step agree on whether C is the identity
+            // the lanes of a step agree on these flags
             for (int64_t k = 0; k < nslots; ++k) {
-                int32_t* o = &slots[d.slot0 + (k * SI_COUNT + SI_INFO) * st];
-                bool ci = true;
-                for (int l = 0; l < nl; ++l) ci &= s.row[k][l] < 0 || (o[l] & F_CI);
-                if (!ci)
-                    for (int l = 0; l < nl; ++l)
-                        if (s.row[k][l] >= 0) o[l] &= ~F_CI;
+                int32_t* o = &slots[d.slot0 + k * st * SI_COUNT + SI_INFO];
+                int all = F_CI | F_FREELY;
+                for (int l = 0; l < nl; ++l)
+                    if (s.row[k][l] >= 0) all &= o[l * SI_COUNT];
+                for (int l = 0; l < nl; ++l)
+                    if (s.row[k][l] >= 0) o[l * SI_COUNT] &= ~(F_CI | F_FREELY) | all;
             }
-            if (same) known[topo[0]] = d;
+            if (shared) known[topo[0]] = d;
         }
         const int64_t n = (int64_t)d.nsteps * W * rsTotal * ls;
         recElems += n;
@@ -266,35 +344,55 @@ struct TileProgram {
         desc.push_back(d);
     }
 
-    // Instances per tile and warps per tile for `n` instances on `nsub` SM
-    // sub-partitions, topoAt[p] the topology at order position p: the shape
-    // with the least time by the schedule's FP64 instructions, on a sample of
-    // its tiles. A tile's warps wait for one another at each step (length);
-    // past one warp per sub-partition the warps' instructions add up (load).
-    // Fewer lanes per tile follow a lane's own tree better and more warps
-    // shorten the steps; both cost warps. Measured on 8,192 random trees.
-    static void shape(const std::vector<int>& topoAt, const std::vector<const TileRows*>& rows, int nsub, int& TW, int& W) {
+    // Instances per tile and warps per tile for a batch on `sms` SMs, topoAt[p]
+    // the topology at order position p: the shape with the least time by the
+    // schedule's FP64 instructions. Fewer lanes per tile follow a lane's own
+    // tree better and more warps shorten the steps; both take sub-partitions
+    // from other tiles. The lengths and loads of a sample of the tiles stand
+    // for all, dealt out in order to the SMs (or, of fewer than four warps, to
+    // the SM's shares): a share is done no sooner than its longest tile, the
+    // sum of its loads, or its tiles one after another on the warps that
+    // registers leave room for (eight an SM). Measured, ms, 8/32 lanes x 4/8
+    // warps: 8,192 random trees 35.3 36.0 12.6 13.7; 3,000 with contacts 26.9
+    // 26.6 13.3 12.6; 1,500 trees of 4 to 256 bodies 24.1 17.9 24.6 19.2.
+    static void shape(const std::vector<int>& topoAt, const std::vector<const TileRows*>& rows, int sms, int& TW, int& W) {
         const int n = (int)topoAt.size();
         double best = 0;
         TW = 32; W = 1;
         const bool same = std::all_of(topoAt.begin(), topoAt.end(), [&](int k) { return k == topoAt[0]; });
-        for (int tw : {32, 16, 8, 4, 2, 1}) {
+        for (int tw : {32, 8, 1}) {
             if (same && tw < 32) break;  // alignment is perfect at any width
             const int tiles = (n + tw - 1) / tw;
-            if (tw < 32 && tiles > 4 * nsub) break;
+            if (tw < 32 && tiles > 16 * sms) break;
             for (int w : {1, 2, 4, 8}) {
-                double length = 0, load = 0;
-                const int samples = std::min(tiles, same ? 1 : 4);
+                const int samples = std::min(tiles, same ? 1 : 6);
+                std::vector<double> len(samples), load(samples);
                 for (int s = 0; s < samples; ++s) {
-                    const int p0 = (int)((int64_t)tiles * s / samples) * tw;
+                    const int at = samples == 1 ? 0 : (int)((int64_t)(tiles - 1) * s / (samples - 1)), p0 = at * tw;
                     std::vector<const TileRows*> lanes;
                     for (int p = p0; p < std::min(n, p0 + (same ? 1 : tw)); ++p) lanes.push_back(rows[topoAt[p]]);
                     const TileSchedule sc(lanes, w);
-                    length += double(sc.length) / samples;
-                    load += double(sc.load) / samples;
+                    len[s] = (double)sc.length;
+                    load[s] = (double)sc.load;
                 }
-                const double waves = std::ceil(double(tiles) * w / nsub);
-                const double t = std::max(length, waves * load / w);
+                const int shares = sms * std::max(1, 4 / w);
+                const double resident = w == 8 ? 1 : 2;
+                std::vector<double> sum(shares, 0), row(shares, 0);
+                std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> q;
+                for (int k = 0; k < shares; ++k) q.push({0, k});
+                double t = 0;
+                for (int k = 0; k < tiles; ++k) {
+                    const double x = samples == 1 ? 0 : double(k) * (samples - 1) / std::max(1, tiles - 1);
+                    const int i = std::min((int)x, std::max(0, samples - 2)), j = std::min(i + 1, samples - 1);
+                    const double ln = len[i] + (x - i) * (len[j] - len[i]), ld = load[i] + (x - i) * (load[j] - load[i]);
+                    const int sh = q.top().second;
+                    q.pop();
+                    sum[sh] += ld;
+                    row[sh] += ln / resident;
+                    const double d = std::max(sum[sh], row[sh]);
+                    t = std::max({t, d, ln});
+                    q.push({d, sh});
+                }
                 if (best == 0 || t < 0.97 * best) { best = t; TW = tw; W = w; }
             }
         }
