@@ -53,14 +53,6 @@ template <class R> struct ScrTiled {
     R* p;
     __device__ __forceinline__ R& operator()(int rec, int f) const { return p[(rec + f) * kTile]; }
 };
-// Loop-closure records: element f of record rec at (rec + f) * s, with the
-// stride of the instance (32 inside a batch's interleaved tiles, 1 for an
-// instance whose record is its own).
-template <class R> struct ScrStrided {
-    R* p;
-    int s;
-    __device__ __forceinline__ R& operator()(int rec, int f) const { return p[(rec + f) * s]; }
-};
 template <class R> struct ScrRows {
     R* p;
     int P;  // rows of the instance
@@ -941,7 +933,7 @@ __device__ __forceinline__ void body5Free(const DevTables& T, int row, int rec, 
 // ---------------------------------------------------------------- drivers
 // Chain driver: one thread, rows in order; carries along chains, pushes into
 // the parent's record otherwise. Returns SBG_INST_* bits.
-template <class R, int NM, bool REF, bool LOOPS = false, class SC, class Src, class Out>
+template <class R, int NM, bool REF, class SC, class Src, class Out>
 __device__ __forceinline__ int rhsChain(const DevTables& T, int inst, const SC& S, const Src& src, Out& out) {
     static_assert(!REF || std::is_same<R, float>::value, "refinement is for the FP32 recursion");
     const int body0 = T.ibody[inst], nb = T.inb[inst];
@@ -961,8 +953,6 @@ __device__ __forceinline__ int rhsChain(const DevTables& T, int inst, const SC& 
                 storeKin(S, rec, carry);
                 storeC2(S, rec, zeroC2<R>());
             }
-            if constexpr (LOOPS)
-                if (info & F_LOOPBODY) storeKin(S, T.lrec[row], carry);
         }
     }
     bool ok = true;
@@ -997,11 +987,6 @@ __device__ __forceinline__ int rhsChain(const DevTables& T, int inst, const SC& 
             const A3<R> Ap = parent < 0 ? A3<R>{} : (info & F_CARRY) ? carry : loadA3<R>(S, T.srec[body0 + parent], REF);
             if (n == 6) body3Free<R, REF>(T, row, rec, S, out, Ap, parent >= 0, carry);
             else carry = body3<R, NM, REF>(T, row, rec, n, S, out, Ap, parent >= 0);
-            if constexpr (LOOPS)
-                if (info & F_LOOPBODY) {
-                    st3<R>(S, T.lrec[row], kSlotA, carry.w);
-                    st3<R>(S, T.lrec[row], kSlotA + 3, carry.v);
-                }
             if (info & F_MEMCHILD) {
                 storeA3(S, rec, carry, REF);
                 if constexpr (REF)
@@ -1283,39 +1268,30 @@ __device__ __forceinline__ int illConditioned(const DevTables& T, const Out& out
 }
 
 // One RHS of the instance owned by slot s, through either driver; LOOPS adds
-// the Ball loop-closure multipliers (FP64; one-thread or level-parallel driver).
+// the Ball loop-closure multipliers (FP64; level-parallel driver).
 template <class R, int NM, bool REF, bool GROUP, bool LOOPS = false, class Src, class Out>
 __device__ __forceinline__ int rhs(const DevTables& T, const Slot& s, R* scratch, const Src& src, Out& out) {
     if constexpr (LOOPS) {
-        static_assert(std::is_same<R, double>::value && !REF, "loop closures run in FP64");
+        static_assert(std::is_same<R, double>::value && !REF && GROUP, "loop closures: FP64, level-parallel driver");
         double* rec0 = scratch + T.sbase[s.inst];
-        if constexpr (GROUP) {
-            // tree passes on the group's lanes; the multiplier solve and the
-            // constraint sweeps (loop paths only) on its first lane, the
-            // Gram columns on its first three
-            // record-major rows (the first lane's serial loop work touches a
-            // few records many times: they stay in L1)
-            const ScrGen S{rec0, (int)T.sstride[s.inst], 1};
-            int st = rhsGroup<double, NM, false, true>(T, s.inst, S, src, out, s.gl, s.G, s.mask);
-            if (T.incons[s.inst] > 0) {
-                const LoopState L = loopStateRows(T, s.inst, rec0, nullptr, nullptr, nullptr, 0, 0);
-                int lst = 0;
-                if (s.G >= 3) lst = loopForwardDynamicsLanes<NM>(L, out, s.gl, s.mask);
-                else if (s.gl == 0) lst = loopForwardDynamics<NM, true>(L, out);
-                __syncwarp(s.mask);
-                lst = (int)__reduce_or_sync(s.mask, (unsigned)lst);
-                if (!(lst & SBG_INST_CHOLESKY_FAIL)) loopCorrectionOutRows<NM>(L, out, s.gl, s.G, s.mask);
-                st |= lst;
-            }
-            return st;
-        } else {
-            const int sst = (int)T.sstride[s.inst];
-            const ScrStrided<double> S{rec0, sst};
-            int st = rhsChain<double, NM, false, true>(T, s.inst, S, src, out);
-            if (T.incons[s.inst] > 0)
-                st |= loopForwardDynamics<NM>(loopStateChain(T, s.inst, rec0, sst, nullptr, nullptr, nullptr, 0, 0), out);
-            return st;
+        // tree passes on the group's lanes; the multiplier solve and the
+        // constraint sweeps (loop paths only) on its first lane, the
+        // Gram columns on its first three
+        // record-major rows (the first lane's serial loop work touches a
+        // few records many times: they stay in L1)
+        const ScrGen S{rec0, (int)T.sstride[s.inst], 1};
+        int st = rhsGroup<double, NM, false, true>(T, s.inst, S, src, out, s.gl, s.G, s.mask);
+        if (T.incons[s.inst] > 0) {
+            const LoopState L = loopStateRows(T, s.inst, rec0, nullptr, nullptr, nullptr, 0, 0);
+            int lst = 0;
+            if (s.G >= 3) lst = loopForwardDynamicsLanes<NM>(L, out, s.gl, s.mask);
+            else if (s.gl == 0) lst = loopForwardDynamics<NM, true>(L, out);
+            __syncwarp(s.mask);
+            lst = (int)__reduce_or_sync(s.mask, (unsigned)lst);
+            if (!(lst & SBG_INST_CHOLESKY_FAIL)) loopCorrectionOutRows<NM>(L, out, s.gl, s.G, s.mask);
+            st |= lst;
         }
+        return st;
     } else if constexpr (GROUP) {
         const ScrRows<R> S{scratch + T.sbase[s.inst], T.inb[s.inst]};
         int st = rhsGroup<R, NM, REF>(T, s.inst, S, src, out, s.gl, s.G, s.mask);
@@ -1478,15 +1454,13 @@ __global__ void __launch_bounds__(BS, MINB) rkMersonKernel(DevTables T, int firs
         if (!groupAll<GROUP>(o.finite, s)) st |= SBG_INST_NONFINITE;
         if constexpr (GROUP) __syncwarp(s.mask);  // the next stage reads what other lanes wrote
     };
-    // The loop-closure state of this instance (either driver's layout; only
-    // instantiated with R = double); its projections run on the first lane
-    // of a group. The stage planes fB/fC are free outside a step.
+    // The loop-closure state of this instance (only instantiated with R =
+    // double); its projections run on the first lane of a group. The stage planes fB/fC are free outside a step.
     auto loopState = [&]() {
         double* rec0 = reinterpret_cast<double*>(scratch) + T.sbase[inst];
         double* sv = reinterpret_cast<double*>(fB);
         double* dl = reinterpret_cast<double*>(fC);
-        if constexpr (GROUP) return loopStateRows(T, inst, rec0, y, sv, dl, base, stride);
-        else return loopStateChain(T, inst, rec0, (int)T.sstride[inst], y, sv, dl, base, stride);
+        return loopStateRows(T, inst, rec0, y, sv, dl, base, stride);
     };
     // Integrator::initialize with loop closures: forced position and
     // velocity projection (IntegratorRep.h:856-895).

@@ -119,6 +119,7 @@ struct sbg_batch_s {
     std::vector<int32_t> groupWidthKey;   // widest level of each group-segment instance
     int groupShift = -1;                  // G = pow2ceil(width) >> shift, clamped to [2, 32]
     int nGroupBlocks = 0;
+    int nLoopBlocks = 0, groupFirst = 0;  // block table: the loop-closure segment's blocks, then the group segment's
     int32_t* dBlkFirst = nullptr;
     int32_t* dBlkG = nullptr;
     cudaStream_t stream2 = nullptr;
@@ -165,7 +166,9 @@ struct sbg_batch_s {
     cudaEvent_t fbFork = nullptr, fbJoin = nullptr;
 
     Streams streams() const { return Streams{stream, stream2, evFork, evJoin}; }
-    LaunchPlan plan() const { return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop}; }
+    LaunchPlan plan() const {
+        return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop, 0, groupFirst, nLoopBlocks, 0};
+    }
     BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones}; }
     // kernels of one pass over the batch
     int segments() const {
@@ -200,11 +203,46 @@ struct sbg_batch_s {
         first.push_back(nChain + nLoop + ng);
         gs.push_back(0);
         nGroupBlocks = (int)gs.size() - 1;
-        cudaError_t e = cudaMemcpy(dBlkFirst, first.data(), first.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(dBlkG, gs.data(), gs.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        cudaError_t e = cudaMemcpy(dBlkFirst + groupFirst, first.data(), first.size() * sizeof(int32_t),
+                                   cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(dBlkG + groupFirst, gs.data(), gs.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cudaFail(e, "group block table");
         groupShift = shift;
         return SBG_OK;
+    }
+
+    // Lanes per instance of the loop-closure segment, in blocks of one warp: as
+    // many as the widest level (4 to 32: the Gram takes three), fewer while the
+    // segment has more warps than the GPU has sub-partitions, on which they
+    // share the FP64 pipe; and as few instances per warp as fit beside one
+    // another, whose multiplier solves run on one lane each and diverge.
+    int setLoopBlocks(const std::vector<int32_t>& ord) {
+        std::vector<int32_t> first, gs;
+        const int64_t subs = 4 * sms;
+        auto lanesOf = [&](int p) {
+            const int w = topos[topoOf[ord[p]]]->maxLevelWidth;
+            int G = 4;
+            while (G < 32 && G < w) G <<= 1;
+            while (G > 4 && (int64_t)nLoop * G > 32 * subs) G >>= 1;
+            return G;
+        };
+        const int per = (int)std::max<int64_t>(1, (nLoop + subs - 1) / subs);
+        for (int p = nChain; p < nChain + nLoop;) {
+            const int G = lanesOf(p);
+            first.push_back(p);
+            gs.push_back(G);
+            int q = p;
+            while (q < nChain + nLoop && q - p < std::min(per, 32 / G) && lanesOf(q) == G) ++q;
+            p = q;
+        }
+        nLoopBlocks = (int)gs.size();
+        first.push_back(nChain + nLoop);
+        gs.push_back(0);
+        groupFirst = nLoopBlocks + 1;
+        cudaError_t e = cudaMemcpy(dBlkFirst, first.data(), first.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(dBlkG, gs.data(), gs.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+        return e == cudaSuccess ? SBG_OK : cudaFail(e, "loop block table");
     }
 
     ~sbg_batch_s() {
@@ -725,7 +763,10 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         std::stable_sort(chainPos.begin(), chainPos.end(), [&](int a, int c) {
             return inb[a] != inb[c] ? inb[a] > inb[c] : instTopo[a] < instTopo[c];
         });
-        std::stable_sort(loopPos.begin(), loopPos.end(), [&](int a, int c) { return inb[a] > inb[c]; });
+        std::stable_sort(loopPos.begin(), loopPos.end(), [&](int a, int c) {
+            const int wa = topos[instTopo[a]]->maxLevelWidth, wc = topos[instTopo[c]]->maxLevelWidth;
+            return wa != wc ? wa > wc : inb[a] > inb[c];
+        });
         if (precision == SBG_PRECISION_FP64) {
             std::vector<std::array<float, tile::CL_COUNT>> per(b->topos.size()), work(ninst);
             for (size_t k = 0; k < per.size(); ++k) {
@@ -750,41 +791,40 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     std::copy(loopPos.begin(), loopPos.end(), order.begin() + b->nChain);
     std::copy(groupPos.begin(), groupPos.end(), order.begin() + b->nChain + b->nLoop);
     b->order = order;
-    // slot records of the loop-closure topologies follow their body records
-    std::vector<int32_t> lrec(parent.size(), -1), lslot(parent.size(), -1);
+    std::vector<int32_t> lslot(parent.size(), -1);
     for (int k = 0; k < ntopo; ++k) {
         if (used[k] < 0) continue;
-        const sbg_topology_s* t = topos[k];
-        for (int r = 0; r < t->nb; ++r)
-            if (t->lslot[r] >= 0) {
-                lrec[rowBase[k] + r] = (int32_t)(recTotal[k] + (int64_t)t->lslot[r] * kSlotSize);
-                lslot[rowBase[k] + r] = t->lslot[r];
-            }
+        for (int r = 0; r < topos[k]->nb; ++r) lslot[rowBase[k] + r] = topos[k]->lslot[r];
     }
     int64_t yOff = 0, sOff = 0, sOffLoop = 0;
-    // tiles of 32 chain-driver instances (the chain segment, then the
-    // loop-closure segment with its own FP64 scratch)
-    auto tile = [&](int p0, int p1, int64_t& sOffSeg, bool loops) {
-        for (int t0 = p0; t0 < p1; t0 += kTile) {
-            const int t1 = std::min(p1, t0 + kTile);
-            int64_t yw = 0, sw = 0;
-            for (int p = t0; p < t1; ++p) {
-                const int i = order[p];
-                const sbg_topology_s* t = topos[instTopo[i]];
-                yw = std::max<int64_t>(yw, inq[i] + inu[i]);
-                sw = std::max<int64_t>(sw, recTotal[instTopo[i]] + (loops ? (int64_t)t->nslots * kSlotSize : 0));
-            }
-            for (int p = t0; p < t1; ++p) {
-                const int i = order[p];
-                ybase[i] = yOff + (p - t0); ystride[i] = kTile;
-                sbase[i] = sOffSeg + (p - t0); sstride[i] = kTile;
-            }
-            yOff += yw * kTile;
-            sOffSeg += sw * kTile;
+    // tiles of 32 chain-driver instances
+    for (int t0 = 0; t0 < b->nChain; t0 += kTile) {
+        const int t1 = std::min(b->nChain, t0 + kTile);
+        int64_t yw = 0, sw = 0;
+        for (int p = t0; p < t1; ++p) {
+            const int i = order[p];
+            yw = std::max<int64_t>(yw, inq[i] + inu[i]);
+            sw = std::max<int64_t>(sw, recTotal[instTopo[i]]);
         }
-    };
-    tile(0, b->nChain, sOff, false);
-    tile(b->nChain, b->nChain + b->nLoop, sOffLoop, true);
+        for (int p = t0; p < t1; ++p) {
+            const int i = order[p];
+            ybase[i] = yOff + (p - t0); ystride[i] = kTile;
+            sbase[i] = sOff + (p - t0); sstride[i] = kTile;
+        }
+        yOff += yw * kTile;
+        sOff += sw * kTile;
+    }
+    // the loop-closure segment: contiguous columns, FP64 record-major rows of
+    // the instance's width (the bodies, then two slot records per constraint)
+    for (int p = b->nChain; p < b->nChain + b->nLoop; ++p) {
+        const int i = order[p];
+        const sbg_topology_s* t = topos[instTopo[i]];
+        ybase[i] = yOff; ystride[i] = 1;
+        yOff += t->nq + t->nu;
+        sstride[i] = rowsRecordWidth(*t, 3);
+        sbase[i] = sOffLoop;
+        sOffLoop += (t->nb + 2 * t->ncons) * sstride[i];
+    }
     // constraint tables
     std::vector<int32_t> lcons, icons(ninst, 0), incons(ninst, 0), consBase(ntopo, 0);
     std::vector<double> lst;
@@ -884,21 +924,22 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     if ((rc = b->upload(&T.cbeg, cbeg, "children table"))) return bail(rc);
     if ((rc = b->upload(&T.ccnt, ccnt, "children table"))) return bail(rc);
     if ((rc = b->upload(&T.clist, clist, "children table"))) return bail(rc);
-    if ((rc = b->upload(&T.lrec, lrec, "loop table"))) return bail(rc);
     if ((rc = b->upload(&T.lslot, lslot, "loop table"))) return bail(rc);
     if ((rc = b->upload(&T.lcons, lcons, "loop table"))) return bail(rc);
     if ((rc = b->upload(&T.lst, lst, "loop table"))) return bail(rc);
     if ((rc = b->upload(&T.icons, icons, "instance table"))) return bail(rc);
     if ((rc = b->upload(&T.incons, incons, "instance table"))) return bail(rc);
-    {   // group block table (capacity: one block per group instance + end)
+    {   // block table: the loop-closure segment's blocks and their end, then the
+        // group segment's (at most one block per instance)
         void* q = nullptr;
-        const size_t cap = (size_t)(ninst - b->nChain - b->nLoop) + 2;
+        const size_t cap = (size_t)(ninst - b->nChain) + 4;
         if ((rc = b->alloc(&q, cap * sizeof(int32_t), "group block table"))) return bail(rc);
         b->dBlkFirst = static_cast<int32_t*>(q);
         if ((rc = b->alloc(&q, cap * sizeof(int32_t), "group block table"))) return bail(rc);
         b->dBlkG = static_cast<int32_t*>(q);
         T.blkFirst = b->dBlkFirst;
         T.blkG = b->dBlkG;
+        if (b->nLoop > 0 && (rc = b->setLoopBlocks(order))) return bail(rc);
         if ((rc = b->setGroupShift(1))) return bail(rc);
     }
     const int64_t* dOff = nullptr;

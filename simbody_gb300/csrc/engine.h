@@ -117,7 +117,6 @@ struct DevTables {
     const int32_t* blkFirst; // per group block: first order position (+ end)
     const int32_t* blkG;     // per group block: lanes per instance
     // loop closures
-    const int32_t* lrec;     // per body row: slot record offset, -1 if none
     const int32_t* lcons;    // per constraint: local row of body 1, of body 2 (-1 = Ground)
     const double* lst;       // per constraint: station 1 (in body 1), station 2 (in body 2)
     const int32_t* lslot;    // per body row: slot index of a loop body (-1 = none): level-parallel layout

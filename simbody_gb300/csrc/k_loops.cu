@@ -1,47 +1,32 @@
-// k_loops.cu -- kernels of the loop-closure segments (FP64): realize with
-// Constraint::Ball multipliers and the tree M^-1 of those instances on the
-// one-thread driver, and the level-parallel driver's realize and RK-Merson
-// (the one-thread RK-Merson is in k_rkloops.cu).
+// k_loops.cu -- kernels of the loop-closure segments (FP64) on the
+// level-parallel driver: the tree passes on the lanes of each instance's
+// group, the Gram columns on three of them, the multiplier solve and the
+// projections on its first. Blocks [loopGroupFirst, +nLoopGroupBlocks) of the
+// block table; records record-major (width in T.sstride). The server's blocks
+// have 128 threads, a batch's one warp. 300 trees of 20 to 40 bodies, a fifth
+// with closures, two steps: 18.0 ms; 62.0 ms with one thread per instance,
+// whose lanes ran the tree passes and up to four closures' sweeps in turn.
 #include "abi_device.cuh"
 
 namespace sbg {
 
-
-void realizeLoop(const KArgs& a, cudaStream_t s) {
-    double* sc = static_cast<double*>(a.scratchLoop);
-    const int first = a.P->nChain;
-    const Launch1D L = spread(a.P->nLoop, 128);
-    if (a.P->nm == 1)
-        realizeKernel<double, 1, false, false, 1, true><<<L.grid, L.block, 0, s>>>(*a.T, first, a.P->nLoop, a.y, a.ydot, sc, a.status);
-    else
-        realizeKernel<double, 3, false, false, 1, true><<<L.grid, L.block, 0, s>>>(*a.T, first, a.P->nLoop, a.y, a.ydot, sc, a.status);
-}
-
-void minvLoop(const KArgs& a, cudaStream_t s) {
-    double* sc = static_cast<double*>(a.scratchLoop);
-    const int first = a.P->nChain;
-    const Launch1D L = spread(a.P->nLoop, 128);
-    if (a.P->nm == 1)
-        minvKernel<double, 1, false><<<L.grid, L.block, 0, s>>>(*a.T, first, a.P->nLoop, a.y, a.f, a.ydot, sc, a.status);
-    else
-        minvKernel<double, 3, false><<<L.grid, L.block, 0, s>>>(*a.T, first, a.P->nLoop, a.y, a.f, a.ydot, sc, a.status);
-}
-
-// Loop-closure instances on the level-parallel driver (FP64): tree passes on
-// the lanes of each instance's group, the multiplier solve and projections on
-// its first lane. Blocks [loopGroupFirst, +nLoopGroupBlocks) of the block
-// table; FP64 scratch and stage planes, records record-major (width in
-// T.sstride).
-void rkLoopGroup(const KArgs& a, cudaStream_t s) {
+void rkLoopGroup(const KArgs& a, int threads, cudaStream_t s) {
     if (a.P->nLoopGroupBlocks <= 0) return;
-    rkMersonKernel<double, 3, false, true, 1, true><<<a.P->nLoopGroupBlocks, 128, 0, s>>>(
+    rkMersonKernel<double, 3, false, true, 1, true><<<a.P->nLoopGroupBlocks, threads, 0, s>>>(
         *a.T, a.P->loopGroupFirst, 0, a.ystate, a.time, static_cast<double*>(a.fbufLoop), a.fplane,
         static_cast<double*>(a.scratchLoop), a.status, a.h, a.step, a.accuracy, a.consTol, a.projectEveryStep);
 }
-void realizeLoopGroup(const KArgs& a, cudaStream_t s) {
+void realizeLoopGroup(const KArgs& a, int threads, cudaStream_t s) {
     if (a.P->nLoopGroupBlocks <= 0) return;
-    realizeKernel<double, 3, false, true, 1, true><<<a.P->nLoopGroupBlocks, 128, 0, s>>>(
+    realizeKernel<double, 3, false, true, 1, true><<<a.P->nLoopGroupBlocks, threads, 0, s>>>(
         *a.T, a.P->loopGroupFirst, 0, a.y, a.ydot, static_cast<double*>(a.scratchLoop), a.status);
+}
+// The tree's M^-1 f (without constraints) of these instances; its records are
+// field-major in the same memory.
+void minvLoopGroup(const KArgs& a, int threads, cudaStream_t s) {
+    if (a.P->nLoopGroupBlocks <= 0) return;
+    minvKernel<double, 3, true><<<a.P->nLoopGroupBlocks, threads, 0, s>>>(
+        *a.T, a.P->loopGroupFirst, 0, a.y, a.f, a.ydot, static_cast<double*>(a.scratchLoop), a.status);
 }
 
 }  // namespace sbg

@@ -13,13 +13,10 @@ cudaError_t launchTreeOp(const DevTables& T, const LaunchPlan& P, const OpIO& io
         if (P.nm == 1) treeOpKernel<1, 0><<<L.grid, L.block, 0, s>>>(T, 0, P.nChain, y, scratch, io, status);
         else treeOpKernel<3, 0><<<L.grid, L.block, 0, s>>>(T, 0, P.nChain, y, scratch, io, status);
     }
-    if (P.nLoop > 0) {
-        const Launch1D L = spread(P.nLoop, 128);
-        if (P.nm == 1) treeOpKernel<1, 1><<<L.grid, L.block, 0, s>>>(T, P.nChain, P.nLoop, y, scratchLoop, io, status);
-        else treeOpKernel<3, 1><<<L.grid, L.block, 0, s>>>(T, P.nChain, P.nLoop, y, scratchLoop, io, status);
-    }
+    if (P.nLoopGroupBlocks > 0)
+        treeOpKernel<3, 1><<<P.nLoopGroupBlocks, 32, 0, s>>>(T, P.loopGroupFirst, 0, y, scratchLoop, io, status);
     if (P.nGroupBlocks > 0)
-        treeOpKernel<3, 2><<<P.nGroupBlocks, 128, 0, s>>>(T, P.groupFirst, 0, y, scratch, io, status);
+        treeOpKernel<3, 1><<<P.nGroupBlocks, 128, 0, s>>>(T, P.groupFirst, 0, y, scratch, io, status);
     return cudaGetLastError();
 }
 

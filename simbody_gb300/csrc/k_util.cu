@@ -159,7 +159,7 @@ cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision
                           const BatchBufs& B, int32_t* status, const Streams& s) {
     KArgs a = baseArgs(T, P, B, status);
     a.y = y; a.ydot = ydot;
-    auto loops = [&](cudaStream_t st) { realizeLoop(a, st); };
+    auto loops = [&](cudaStream_t st) { realizeLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
         return tilesThenLoops(P, s, [&](cudaStream_t st) { realizeTiles(a, *B.tiles, 0, B.tiles->ntiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
@@ -176,7 +176,7 @@ cudaError_t launchMInv(const DevTables& T, const LaunchPlan& P, int precision, c
                        double* out, const BatchBufs& B, int32_t* status, const Streams& s) {
     KArgs a = baseArgs(T, P, B, status);
     a.y = y; a.f = f; a.ydot = out;
-    auto loops = [&](cudaStream_t st) { minvLoop(a, st); };
+    auto loops = [&](cudaStream_t st) { minvLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
         return tilesThenLoops(P, s, [&](cudaStream_t st) { minvTiles(a, *B.tiles, st); }, loops);
     return forkJoin(P, s, [&](cudaStream_t st) { minv32Chain(a, st); }, loops,
@@ -189,7 +189,7 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
     KArgs a = baseArgs(T, P, B, status);
     a.ystate = y; a.time = time; a.h = h; a.step = step; a.accuracy = accuracy; a.consTol = consTol;
     a.projectEveryStep = projectEveryStep;
-    auto loops = [&](cudaStream_t st) { rkLoop(a, st); };
+    auto loops = [&](cudaStream_t st) { rkLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
         return tilesThenLoops(P, s, [&](cudaStream_t st) { rkTiles(a, *B.tiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;

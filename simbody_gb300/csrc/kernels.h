@@ -162,11 +162,10 @@ void minv32Group(const KArgs& a, cudaStream_t s);
 void rk64Group(const KArgs& a, cudaStream_t s);
 void rk32Chain(const KArgs& a, bool refine, cudaStream_t s);
 void rk32Group(const KArgs& a, bool refine, cudaStream_t s);
-void realizeLoop(const KArgs& a, cudaStream_t s);  // k_loops.cu
-void minvLoop(const KArgs& a, cudaStream_t s);
-void rkLoop(const KArgs& a, cudaStream_t s);
-void rkLoopWidth1(const KArgs& a, cudaStream_t s);  // k_rkloops1.cu: rkLoop for batch width 1
-void rkLoopGroup(const KArgs& a, cudaStream_t s);      // loop closures, level-parallel driver
+// Loop closures, level-parallel driver (k_loops.cu), blocks of `threads`.
+void rkLoopGroup(const KArgs& a, int threads, cudaStream_t s);
+void realizeLoopGroup(const KArgs& a, int threads, cudaStream_t s);
+void minvLoopGroup(const KArgs& a, int threads, cudaStream_t s);
 cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
                              StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
                              cudaStream_t s);
@@ -176,6 +175,5 @@ cudaError_t launchFillInt(int32_t* p, int n, int v, cudaStream_t s);
 // *out = instances with steps left in a one-step integration call
 cudaError_t launchCountUnfinished(int n, const int32_t* stepsLeft, const double* time, const int32_t* status,
                                   double tStop, int32_t* out, cudaStream_t s);
-void realizeLoopGroup(const KArgs& a, cudaStream_t s);
 
 }  // namespace sbg

@@ -1,4 +1,4 @@
-// loops_device.cuh -- Constraint::Ball loop closures on the FP64 chain
+// loops_device.cuh -- Constraint::Ball loop closures on the FP64 level-parallel
 // driver: the multipliers of the loop forward dynamics and the integrator's
 // position and velocity projections. Textually included by abi_device.cuh
 // inside namespace sbg (it uses that file's records, kinematics and sweeps).
@@ -41,11 +41,9 @@
 // eps off the path. Skipped rows would have contributed exact zeros, so the
 // results are the same as full sweeps.
 
-// Loop-closure records through either driver's layout: element f of record
-// rec at rec * a + f * b, with (a, b) = (s, s) for the interleaved tiles of
-// the one-thread driver (stride s) and (W, 1) for the record-major rows of
-// the level-parallel driver (record width W; the bodies, then the slot
-// records).
+// Loop-closure records: element f of record rec at rec * a + f * b, (a, b) =
+// (W, 1) for the record-major rows of the level-parallel driver (record width
+// W; the bodies, then the slot records).
 template <class R> struct ScrGenT {
     R* p;
     int a, b;
@@ -66,25 +64,18 @@ struct LoopState {
     double* save;
     double* delta;
     int64_t base, stride;
-    bool rows;  // level-parallel layout: record = local row, slots after the bodies
     int body0, nb;
-    // record of body row `row`, slot record of a loop body row
-    __device__ __forceinline__ int rec(int row) const { return rows ? row - body0 : T.srec[row]; }
-    __device__ __forceinline__ int slot(int row) const { return rows ? nb + T.lslot[row] : T.lrec[row]; }
+    // record of body row `row` (its local row), slot record of a loop body row
+    __device__ __forceinline__ int rec(int row) const { return row - body0; }
+    __device__ __forceinline__ int slot(int row) const { return nb + T.lslot[row]; }
 };
-// The state of instance `inst` over records at `scratch` (its record base):
-// one-thread layout with stride s, or the level-parallel layout.
-__device__ __forceinline__ LoopState loopStateChain(const DevTables& T, int inst, double* scratch, int s, double* y,
-                                                    double* save, double* delta, int64_t base, int64_t stride) {
-    return LoopState{T, inst, SC64{scratch, s, s}, y, save, delta, base, stride, false, T.ibody[inst], T.inb[inst]};
-}
 // The level-parallel layout of an instance with loop closures: one record
 // per row (the bodies, then 2 slot records per constraint), record-major
 // with the record width in T.sstride (element f of row r at r * W + f).
 __device__ __forceinline__ int loopRows(const DevTables& T, int inst) { return T.inb[inst] + 2 * T.incons[inst]; }
 __device__ __forceinline__ LoopState loopStateRows(const DevTables& T, int inst, double* scratch, double* y,
                                                    double* save, double* delta, int64_t base, int64_t stride) {
-    return LoopState{T, inst, SC64{scratch, (int)T.sstride[inst], 1}, y, save, delta, base, stride, true,
+    return LoopState{T, inst, SC64{scratch, (int)T.sstride[inst], 1}, y, save, delta, base, stride,
                      T.ibody[inst], T.inb[inst]};
 }
 

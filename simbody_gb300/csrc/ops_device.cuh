@@ -186,22 +186,18 @@ __device__ __forceinline__ int treeOp(const DevTables& T, int inst, const SC& S,
     return finite ? 0 : SBG_INST_NONFINITE;
 }
 
-// SEG 0: one-thread instances in 32-wide interleaved tiles; 1: the loop-closure
-// segment (one thread, records at stride sstride); 2: the level-parallel
-// segment (field-major rows).
+// SEG 0: one-thread instances in 32-wide interleaved tiles; 1: the
+// level-parallel and the loop-closure segments (field-major rows).
 template <int NM, int SEG>
 __global__ void __launch_bounds__(128) treeOpKernel(DevTables T, int first, int count, const double* __restrict__ y,
                                                    double* __restrict__ scratch, OpIO io,
                                                    int32_t* __restrict__ status) {
-    const Slot s = SEG == 2 ? groupSlot(T, first) : chainSlot(T, first, count);
+    const Slot s = SEG == 1 ? groupSlot(T, first) : chainSlot(T, first, count);
     if (s.inst < 0) return;
     const int body0 = T.ibody[s.inst];
     int st;
     if constexpr (SEG == 0) {
         const ScrTiled<double> S{scratch + T.sbase[s.inst]};
-        st = treeOp<NM>(T, s.inst, S, [&](int lb) { return (int)T.srec[body0 + lb]; }, y, io, 0, 1, 0u);
-    } else if constexpr (SEG == 1) {
-        const ScrStrided<double> S{scratch + T.sbase[s.inst], (int)T.sstride[s.inst]};
         st = treeOp<NM>(T, s.inst, S, [&](int lb) { return (int)T.srec[body0 + lb]; }, y, io, 0, 1, 0u);
     } else {
         const ScrRows<double> S{scratch + T.sbase[s.inst], T.inb[s.inst]};

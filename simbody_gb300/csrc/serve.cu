@@ -162,7 +162,7 @@ struct ServeReq {
     int32_t fp64Steps = 0; // 1: its RHS switched to FP64 (an ill-conditioned M)
 };
 
-enum RowTable { R_PARENT = 0, R_INFO, R_QOFF, R_UOFF, R_SREC, R_FBEG, R_FCNT, R_LREC, R_CBEG, R_CCNT, R_CLIST, R_LEV,
+enum RowTable { R_PARENT = 0, R_INFO, R_QOFF, R_UOFF, R_SREC, R_FBEG, R_FCNT, R_CBEG, R_CCNT, R_CLIST, R_LEV,
                 R_LSLOT, R_KBEG, R_KCNT, kRowTables };
 
 struct TickRec {
@@ -292,8 +292,7 @@ void buildImage(const sbg_topology_s& t, ServeReq& r, Footprint& fp) {
     r.loops = t.ncons > 0;
     r.G = groupLanes(t);
     for (int k = 0; k < 3; ++k) r.grav[k] = t.gravity[k];
-    int64_t recTotal = 0;
-    const std::vector<int32_t> srec = paddedRecords(t, 3, &recTotal);
+    const std::vector<int32_t> srec = paddedRecords(t, 3, nullptr);
     r.rowsI.assign((size_t)kRowTables * rows, 0);
     auto at = [&](int table, int row) -> int32_t& { return r.rowsI[(size_t)table * rows + row]; };
     for (int i = 0; i < nb; ++i) {
@@ -304,7 +303,6 @@ void buildImage(const sbg_topology_s& t, ServeReq& r, Footprint& fp) {
         at(R_SREC, i) = srec[i];
         at(R_FBEG, i) = t.fbeg[i];  // request-relative: + force base at admission
         at(R_FCNT, i) = t.fcnt[i];
-        at(R_LREC, i) = t.lslot[i] >= 0 ? (int32_t)(recTotal + (int64_t)t.lslot[i] * kSlotSize) : -1;
         at(R_LSLOT, i) = t.lslot[i];
         at(R_CBEG, i) = t.cbeg[i];  // request-relative: + row base at admission
         at(R_CCNT, i) = t.ccnt[i];
@@ -604,7 +602,6 @@ int laneCreate(const sbg_server_config* cfg, int64_t budget, std::chrono::steady
     T.srec = s->rowsI[R_SREC];
     T.fbeg = s->rowsI[R_FBEG];
     T.fcnt = s->rowsI[R_FCNT];
-    T.lrec = s->rowsI[R_LREC];
     T.lslot = s->rowsI[R_LSLOT];
     T.cbeg = s->rowsI[R_CBEG];
     T.ccnt = s->rowsI[R_CCNT];
@@ -836,7 +833,7 @@ int laneIssue(ServeLane* s) {
             ++s->launches;
         }
         if (nLoopBlocks > 0) {
-            rkLoopGroup(a, m);
+            rkLoopGroup(a, 128, m);
             ++s->launches;
         }
         if (both) {
