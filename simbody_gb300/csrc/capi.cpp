@@ -43,8 +43,11 @@ const int kNQ[SBG_NUM_MOBILIZERS] = {1, 1, 2, 4, 7, 3, 3, 2, 3, 6, 0, 1};
 const int kNU[SBG_NUM_MOBILIZERS] = {1, 1, 2, 3, 6, 3, 3, 2, 3, 6, 0, 1};
 
 // Host buffers the caller allocated page-locked (cudaMallocHost,
-// cudaHostRegister, a pinned torch tensor) are copied to and from directly;
-// pageable ones go through the batch's pinned staging buffer.
+// cudaHostRegister, a pinned torch tensor) are copied to and from directly, and
+// so are pageable ones where the GPU uses the host's page tables (Grace): 16 MB
+// up takes 102 us then, 756 us by way of a pinned staging buffer (88 us from
+// pinned memory); down 96 and 1,259 us. Elsewhere pageable buffers go through
+// the batch's staging buffer.
 bool isPinned(const void* p) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -90,6 +93,7 @@ struct sbg_batch_s {
     std::vector<int64_t> hostYOff, hostUOff;  // packed host offsets (n+1)
     std::vector<int64_t> hostBOff;            // bodies before each instance (n+1)
     int64_t nyTotal = 0, nuTotal = 0, colElems = 0;
+    int maxCol = 0;                           // elements of the longest state column
     std::vector<DevBuf> bufs;
     int64_t devBytes = 0;
     DevTables T{};
@@ -109,7 +113,9 @@ struct sbg_batch_s {
     void* fbufLoop = nullptr;     // FP64 stage derivatives of that segment (fbuf itself in FP64 batches)
     int nLoop = 0;                // order positions [nChain, nChain + nLoop)
     int64_t scratchElems = 0;
-    double* hostPinned = nullptr;  // pinned host staging (nyTotal)
+    bool pageable = false;         // the GPU copies to and from pageable host memory itself
+    double* hostPinned = nullptr;  // pinned host staging, allocated when first needed
+    size_t hostPinnedBytes = 0;
     bool stateSet = false;
     bool integrating = false;  // an integration has run since the state was last set: it can be continued
     bool realized = false;     // ydot holds the realize of the current state (qdotdot can be formed)
@@ -126,9 +132,10 @@ struct sbg_batch_s {
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
     bool orderIdentity = false;         // launch order = instance order (a one-topology chain batch)
     // pipelined host realize: pipe[0] (= stream) uploads the chunks in order,
-    // pipe[1..3] compute them, pipe[4] downloads them in order; per chunk an
+    // pipe[2..] compute them, pipe[1] downloads them in order; per chunk an
     // event when its upload and when its gather is done
-    cudaStream_t pipe[5] = {};
+    static constexpr int kPipe = 10;
+    cudaStream_t pipe[kPipe] = {};
     cudaEvent_t pipeEv[2][16] = {};
     cudaEvent_t pipeStart = nullptr, pipeEnd = nullptr;
     cudaEvent_t evT0 = nullptr, evT1 = nullptr;
@@ -141,12 +148,11 @@ struct sbg_batch_s {
     std::vector<int32_t> topoOf;             // per instance, its index in topos
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
+    TileSet tiles32{};                       // FP32 forms: the chain segment's tiles (kernel variant 9)
     int tileWidth = kTile;                   // instances per tile of `tiles`
-    // tree operators (allocated on first use): FP64 scratch, device operands and results in the host packing,
+    // tree operators (allocated on first use): device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
-    void* opsScratch = nullptr;
     double* opsDev = nullptr;
-    double* opsHost = nullptr;
     int64_t opsElems = 0;
     int64_t* dHostBOff = nullptr;
     cudaEvent_t evOp0 = nullptr, evOp1 = nullptr;  // bracket the last tree operator's kernels
@@ -165,11 +171,19 @@ struct sbg_batch_s {
     cudaStream_t fbStream = nullptr;
     cudaEvent_t fbFork = nullptr, fbJoin = nullptr;
 
+    // Packing of the state columns: which order positions are interleaved.
+    Packing packing() const {
+        return Packing{&T, nChain, precision == SBG_PRECISION_FP64 ? nChain + nLoop : ninst, ninst, maxCol};
+    }
+    int packLaunches() const {
+        return (nChain > 0) + (nLoop > 0 || (precision != SBG_PRECISION_FP64 && ninst > nChain)) +
+               (precision == SBG_PRECISION_FP64 && ninst > nChain + nLoop);
+    }
     Streams streams() const { return Streams{stream, stream2, evFork, evJoin}; }
     LaunchPlan plan() const {
         return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop, 0, groupFirst, nLoopBlocks, 0};
     }
-    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones}; }
+    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones, &tiles32}; }
     // kernels of one pass over the batch
     int segments() const {
         if (precision == SBG_PRECISION_FP64) return (tiles.ntiles > 0) + (nLoop > 0);
@@ -250,7 +264,6 @@ struct sbg_batch_s {
         for (auto& b : bufs) cudaFree(b.p);
         for (sbg_topology_s* t : topos) releaseTopology(t);
         if (hostPinned) cudaFreeHost(hostPinned);
-        if (opsHost) cudaFreeHost(opsHost);
         if (realizeGraph) cudaGraphExecDestroy(realizeGraph);
         if (evFork) cudaEventDestroy(evFork);
         if (evT0) cudaEventDestroy(evT0);
@@ -262,7 +275,7 @@ struct sbg_batch_s {
         if (fbJoin) cudaEventDestroy(fbJoin);
         if (fbStream) cudaStreamDestroy(fbStream);
         if (stream2) cudaStreamDestroy(stream2);
-        for (int k = 1; k < 5; ++k)
+        for (int k = 1; k < kPipe; ++k)
             if (pipe[k]) cudaStreamDestroy(pipe[k]);
         for (auto& row : pipeEv)
             for (cudaEvent_t e : row)
@@ -270,6 +283,25 @@ struct sbg_batch_s {
         if (pipeStart) cudaEventDestroy(pipeStart);
         if (pipeEnd) cudaEventDestroy(pipeEnd);
         if (stream) cudaStreamDestroy(stream);
+    }
+    // Where copies of `bytes` from or to the caller's buffer go: the buffer, or
+    // the staging buffer from its byte `at` on (null: no memory).
+    void* hostSide(const void* p, size_t bytes, size_t at = 0) {
+        if (pageable || isPinned(p)) return const_cast<void*>(p);
+        if (hostPinnedBytes < at + bytes) {
+            void* q = nullptr;
+            if (cudaMallocHost(&q, at + bytes) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            if (hostPinned) {
+                std::memcpy(q, hostPinned, std::min(at, hostPinnedBytes));
+                cudaFreeHost(hostPinned);
+            }
+            hostPinned = static_cast<double*>(q);
+            hostPinnedBytes = at + bytes;
+        }
+        return reinterpret_cast<char*>(hostPinned) + at;
     }
     int alloc(void** out, size_t bytes, const char* what) {
         if (budget > 0 && devBytes + (int64_t)bytes > budget)
@@ -578,6 +610,7 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
             }
     }
     out->ntiles = (int)P.desc.size();
+    out->sms = sms;
     out->tt.W = P.W;
     out->tt.ls = P.ls;
     out->tt.shared = P.shared;
@@ -627,6 +660,51 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     return SBG_OK;
 }
 
+// The chain segment's tiles of the FP32 forms, where some tree branches.
+static int buildTiles32(sbg_batch b) {
+    using namespace tile;
+    std::vector<TileRows> store;
+    std::vector<const TileRows*> rows(b->topos.size(), nullptr);
+    const std::vector<int64_t> rowBase(b->topos.size(), 0);
+    store.reserve(b->topos.size());
+    std::vector<int> at;
+    bool wide = false, six = false;
+    for (int p = 0; p < b->nChain; ++p) {
+        const int k = b->topoOf[b->order[p]];
+        at.push_back(k);
+        wide |= !b->topos[k]->chain;
+        if (rows[k]) continue;
+        store.emplace_back(*b->topos[k], true);
+        rows[k] = &store.back();
+        six |= rows[k]->gen;
+    }
+    if (!wide) return SBG_OK;
+    TileProgram P;
+    P.rs = P.rsTotal = scratchRecordSize(six ? 6 : b->nm);
+    P.W = TileProgram::warps32(at, rows, b->sms);
+    if (const char* v = std::getenv("SBG_TILE32")) P.W = std::max(1, std::min(8, std::atoi(v)));  // tuning override
+    P.shared = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
+    for (int p = 0; p < b->nChain; p += kTile)
+        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, rowBase);
+    TileSet& S = b->tiles32;
+    S.sms = b->sms;
+    S.tt.W = P.W;
+    S.tt.ls = kTile;
+    S.tt.shared = P.shared;
+    S.tt.rs = S.tt.rsTotal = P.rsTotal;
+    int rc;
+    if ((rc = b->upload(&S.tt.desc, P.desc, "tile table"))) return rc;
+    if ((rc = b->upload(&S.tt.cls, P.cls, "tile table"))) return rc;
+    if ((rc = b->upload(&S.tt.slots, P.slots, "tile table"))) return rc;
+    void* p = nullptr;
+    if ((rc = b->alloc(&p, P.recElems * sizeof(float), "tile records"))) return rc;
+    S.recs = static_cast<double*>(p);
+    if ((rc = b->alloc(&p, b->colElems * sizeof(double), "stage input"))) return rc;
+    S.yt = static_cast<double*>(p);
+    S.ntiles = (int)P.desc.size();
+    return SBG_OK;
+}
+
 extern "C" {
 
 int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
@@ -666,6 +744,10 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
+        int access = 0, tables = 0;
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
+        b->pageable = access && tables;
         if (e != cudaSuccess) return bail(cudaFail(e, "stream/event creation"));
     }
 
@@ -748,6 +830,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         inq[i] = t->nq;
         inu[i] = t->nu;
         b->topoOf[i] = used[instTopo[i]];
+        b->maxCol = std::max(b->maxCol, t->nq + t->nu);
         ilev[i] = levBase[instTopo[i]];
         inlev[i] = t->nlevels;
         for (int k = 0; k < 3; ++k) grav[3 * i + k] = t->gravity[k];
@@ -879,7 +962,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     if (precision == SBG_PRECISION_FP64) b->variant = 1;  // FP64 needs every register
     if (const char* v = std::getenv("SBG_VARIANT")) {  // tuning override
         const int want = std::atoi(v);
-        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 ? want : 1;
+        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 || want == 9 ? want : 1;
     }
 
     int rc = 0;
@@ -972,6 +1055,8 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if ((rc = buildTiles(b, false, &b->tiles))) return bail(rc);
     } else {
         if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
+        if ((rc = buildTiles32(b))) return bail(rc);
+        if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
         if (precision == SBG_PRECISION_MIXED) {
             // FP64 tiles for the instances whose refinement reports an
             // ill-conditioned M, and the count of those recomputed
@@ -990,10 +1075,6 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if (precision == SBG_PRECISION_FP64) b->fbufLoop = b->fbuf;
         else if ((rc = b->alloc(&b->fbufLoop, 4 * b->colElems * sizeof(double), "loop stage derivatives")))
             return bail(rc);
-    }
-    {
-        cudaError_t e = cudaMallocHost(&b->hostPinned, std::max<int64_t>(b->nyTotal, 1) * sizeof(double));
-        if (e != cudaSuccess) return bail(cudaFail(e, "cudaMallocHost"));
     }
     cudaError_t e = cudaMemsetAsync(b->time, 0, std::max<int64_t>(ninst, 1) * sizeof(double), b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->status, 0, std::max<int64_t>(ninst, 1) * sizeof(int32_t), b->stream);
@@ -1024,26 +1105,31 @@ int sbg_batch_device_bytes(sbg_batch b, int64_t* bytes) {
 void* sbg_batch_stream(sbg_batch b) { return b ? (void*)b->stream : nullptr; }
 int64_t sbg_batch_launch_count(sbg_batch b) { return b ? b->launches : 0; }
 
-int sbg_batch_set_state(sbg_batch b, const double* t, const double* y) {
-    if (!b || !y) return fail(SBG_ERR_INVALID, "null argument");
-    SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
-    const size_t bytes = b->nyTotal * sizeof(double);
-    const double* src = y;
-    if (!isPinned(y)) {
-        std::memcpy(b->hostPinned, y, bytes);
-        src = b->hostPinned;
-    }
+// The state upload of a call: y into the columns, the times (null: zero).
+static int uploadState(sbg_batch b, const double* t, const double* y) {
+    const size_t bytes = b->nyTotal * sizeof(double), tbytes = b->ninst * sizeof(double);
+    void* src = b->hostSide(y, bytes);
+    if (!src) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    if (src != y) std::memcpy(src, y, bytes);
     SBG_CUDA(cudaMemcpyAsync(b->staging, src, bytes, cudaMemcpyHostToDevice, b->stream), "state upload");
-    SBG_CUDA(launchScatter(b->T, b->dHostYOff, b->staging, b->y, 0, b->stream), "state scatter");
-    ++b->launches;
+    SBG_CUDA(launchScatter(b->packing(), b->dHostYOff, b->staging, b->y, 0, b->stream), "state scatter");
+    b->launches += b->packLaunches();
     if (t) {
-        SBG_CUDA(cudaStreamSynchronize(b->stream), "state upload");
-        std::memcpy(b->hostPinned, t, b->ninst * sizeof(double));
-        SBG_CUDA(cudaMemcpyAsync(b->time, b->hostPinned, b->ninst * sizeof(double), cudaMemcpyHostToDevice, b->stream),
-                 "time upload");
+        if (src != y) SBG_CUDA(cudaStreamSynchronize(b->stream), "state upload");
+        void* ts = b->hostSide(t, tbytes);
+        if (!ts) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+        if (ts != t) std::memcpy(ts, t, tbytes);
+        SBG_CUDA(cudaMemcpyAsync(b->time, ts, tbytes, cudaMemcpyHostToDevice, b->stream), "time upload");
     } else {
         SBG_CUDA(cudaMemsetAsync(b->time, 0, std::max(b->ninst, 1) * sizeof(double), b->stream), "time reset");
     }
+    return SBG_OK;
+}
+
+int sbg_batch_set_state(sbg_batch b, const double* t, const double* y) {
+    if (!b || !y) return fail(SBG_ERR_INVALID, "null argument");
+    SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
+    if (int rc = uploadState(b, t, y)) return rc;
     SBG_CUDA(cudaStreamSynchronize(b->stream), "state upload");
     b->stateSet = true;
     b->integrating = false;
@@ -1055,14 +1141,18 @@ int sbg_batch_get_state(sbg_batch b, double* t, double* y) {
     if (!b || !y) return fail(SBG_ERR_INVALID, "null argument");
     if (!b->stateSet) return fail(SBG_ERR_STATE, "no state has been set");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
-    SBG_CUDA(launchGather(b->T, b->dHostYOff, b->y, b->staging, 0, b->stream), "state gather");
-    ++b->launches;
-    double* dst = isPinned(y) ? y : b->hostPinned;
-    SBG_CUDA(cudaMemcpyAsync(dst, b->staging, b->nyTotal * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
-             "state download");
+    SBG_CUDA(launchGather(b->packing(), b->dHostYOff, b->y, b->staging, 0, b->stream), "state gather");
+    b->launches += b->packLaunches();
+    const size_t bytes = b->nyTotal * sizeof(double);
+    void* dst = b->hostSide(y, bytes);
+    if (!dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    SBG_CUDA(cudaMemcpyAsync(dst, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream), "state download");
+    if (t && b->pageable)
+        SBG_CUDA(cudaMemcpyAsync(t, b->time, b->ninst * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "time download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "state download");
-    if (dst != y) std::memcpy(y, b->hostPinned, b->nyTotal * sizeof(double));
-    if (t) SBG_CUDA(cudaMemcpy(t, b->time, b->ninst * sizeof(double), cudaMemcpyDeviceToHost), "time download");
+    if (dst != y) std::memcpy(y, dst, bytes);
+    if (t && !b->pageable)
+        SBG_CUDA(cudaMemcpy(t, b->time, b->ninst * sizeof(double), cudaMemcpyDeviceToHost), "time download");
     return SBG_OK;
 }
 
@@ -1113,7 +1203,8 @@ static int tuneVariant(sbg_batch b) {
     }
     if (!fixedVariant && b->precision != SBG_PRECISION_FP64) {
         int bestVariant = 1;
-        for (int v : {4, 7, 8}) {
+        for (int v : {4, 7, 8, 9}) {
+            if (v == 9 && !b->tiles32.ntiles) continue;
             if (v >= 7 && b->nChain == 0) continue;  // 64-thread blocks exist for the chain driver only
             if (v == 8 && !b->stagedOk) continue;
             b->variant = v;
@@ -1157,18 +1248,20 @@ int sbg_realize_acceleration_async(sbg_batch b) {
 int sbg_batch_get_ydot(sbg_batch b, double* ydot, int32_t* status) {
     if (!b) return fail(SBG_ERR_INVALID, "null batch");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
-    double* dst = ydot && isPinned(ydot) ? ydot : b->hostPinned;
+    const size_t bytes = b->nyTotal * sizeof(double);
+    void* dst = nullptr;
     if (ydot) {
-        SBG_CUDA(launchGather(b->T, b->dHostYOff, b->ydot, b->staging, 0, b->stream), "derivative gather");
-        ++b->launches;
-        SBG_CUDA(cudaMemcpyAsync(dst, b->staging, b->nyTotal * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
-                 "derivative download");
+        dst = b->hostSide(ydot, bytes);
+        if (!dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+        SBG_CUDA(launchGather(b->packing(), b->dHostYOff, b->ydot, b->staging, 0, b->stream), "derivative gather");
+        b->launches += b->packLaunches();
+        SBG_CUDA(cudaMemcpyAsync(dst, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream), "derivative download");
     }
     if (status)
         SBG_CUDA(cudaMemcpyAsync(status, b->status, b->ninst * sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream),
                  "status download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "derivative download");
-    if (ydot && dst != ydot) std::memcpy(ydot, b->hostPinned, b->nyTotal * sizeof(double));
+    if (dst && dst != ydot) std::memcpy(ydot, dst, bytes);
     return SBG_OK;
 }
 
@@ -1181,7 +1274,7 @@ int sbg_realize_acceleration(sbg_batch b, double* ydot, int32_t* status) {
 // State::updY + realize(Stage::Acceleration) + getYDot from and to host
 // buffers in one call. For a batch whose instances all run the one-thread
 // driver in instance order, the instances are cut into tile-aligned chunks:
-// one stream uploads the chunks in order, three streams scatter, realize and
+// one stream uploads the chunks in order, others scatter, realize and
 // gather them as their uploads land, and one stream downloads them in order
 // as they finish. The copies of one direction thus go one chunk at a time at
 // the link's full rate (concurrent copies would share it, so that the first
@@ -1199,22 +1292,23 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     const bool pipelined = b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 &&
                            (b->tuned || b->precision == SBG_PRECISION_FP64) && nchunks > 1 &&
                            b->ninst >= nchunks * kTile;
-    if (!pipelined) {
-        if (int rc = sbg_batch_set_state(b, nullptr, y)) return rc;
-        return sbg_realize_acceleration(b, ydot, status);
-    }
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
-    const size_t bytes = b->nyTotal * sizeof(double);
-    const double* src = y;
-    if (!isPinned(y)) {
-        std::memcpy(b->hostPinned, y, bytes);
-        src = b->hostPinned;
+    if (!pipelined) {
+        if (int rc = uploadState(b, nullptr, y)) return rc;
+        b->stateSet = true;
+        b->integrating = false;
+        if (int rc = sbg_realize_acceleration_async(b)) return rc;
+        return sbg_batch_get_ydot(b, ydot, status);  // waits for the upload too
     }
-    const bool dstPinned = isPinned(ydot);
-    double* dst = dstPinned ? ydot : b->hostPinned;
-    const bool stPinned = status && isPinned(status);
+    const size_t bytes = b->nyTotal * sizeof(double);
+    double* src = static_cast<double*>(b->hostSide(y, bytes));
+    double* dst = static_cast<double*>(b->hostSide(ydot, bytes));
+    if (!src || !dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    if (src != y) std::memcpy(src, y, bytes);
+    const bool stDirect = status && (b->pageable || isPinned(status));
     b->pipe[0] = b->stream;
-    for (int k = 1; k < 5; ++k)
+    const int lanes = std::min(nchunks, b->kPipe - 2);  // compute streams
+    for (int k = 1; k < 2 + lanes; ++k)
         if (!b->pipe[k]) SBG_CUDA(cudaStreamCreateWithFlags(&b->pipe[k], cudaStreamNonBlocking), "streams");
     for (auto& row : b->pipeEv)
         for (cudaEvent_t& e : row)
@@ -1223,11 +1317,11 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
         SBG_CUDA(cudaEventCreateWithFlags(&b->pipeStart, cudaEventDisableTiming), "events");
         SBG_CUDA(cudaEventCreateWithFlags(&b->pipeEnd, cudaEventDisableTiming), "events");
     }
-    cudaStream_t up = b->pipe[0], down = b->pipe[4];
+    cudaStream_t up = b->pipe[0], down = b->pipe[1];
     SBG_CUDA(cudaMemsetAsync(b->time, 0, std::max(b->ninst, 1) * sizeof(double), up), "time reset");
     // every stream starts after the work already queued on the batch stream
     SBG_CUDA(cudaEventRecord(b->pipeStart, up), "pipeline");
-    for (int k = 1; k < 5; ++k) SBG_CUDA(cudaStreamWaitEvent(b->pipe[k], b->pipeStart, 0), "pipeline");
+    for (int k = 1; k < 2 + lanes; ++k) SBG_CUDA(cudaStreamWaitEvent(b->pipe[k], b->pipeStart, 0), "pipeline");
     const int tiles = (b->ninst + kTile - 1) / kTile;
     KArgs a{};
     a.T = &b->T;
@@ -1235,17 +1329,18 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     a.ydot = b->ydot;
     a.scratch = b->scratch;
     a.status = b->status;
+    a.tiles32 = &b->tiles32;
     for (int c = 0; c < nchunks; ++c) {
         const int i0 = std::min(b->ninst, (int)((int64_t)tiles * c / nchunks) * kTile);
         const int i1 = std::min(b->ninst, (int)((int64_t)tiles * (c + 1) / nchunks) * kTile);
         if (i1 <= i0) continue;
         const int64_t o0 = b->hostYOff[i0], o1 = b->hostYOff[i1];
-        cudaStream_t st = b->pipe[1 + c % 3];
+        cudaStream_t st = b->pipe[2 + c % lanes];
         SBG_CUDA(cudaMemcpyAsync(b->staging + o0, src + o0, (o1 - o0) * sizeof(double), cudaMemcpyHostToDevice, up),
                  "state upload");
         SBG_CUDA(cudaEventRecord(b->pipeEv[0][c], up), "pipeline");
         SBG_CUDA(cudaStreamWaitEvent(st, b->pipeEv[0][c], 0), "pipeline");
-        SBG_CUDA(launchScatter(b->T, b->dHostYOff, b->staging, b->y, 0, st, i0, i1 - i0), "state scatter");
+        SBG_CUDA(launchScatter(b->packing(), b->dHostYOff, b->staging, b->y, 0, st, i0, i1 - i0), "state scatter");
         LaunchPlan P = b->plan();
         P.chainFirst = i0;
         P.nChain = i1 - i0;
@@ -1256,29 +1351,36 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
         } else {
             realize32Chain(a, b->precision == SBG_PRECISION_MIXED, st);
             if (b->precision == SBG_PRECISION_MIXED) {
-                const int share = b->ones.blocks / 3;  // three streams' chunks at a time
-                realizeFallbackTiles(a, b->ones, i0, i1 - i0, (c % 3) * share, share, st);
+                const int share = b->ones.blocks / lanes;  // of the chunks under way together
+                realizeFallbackTiles(a, b->ones, i0, i1 - i0, (c % lanes) * share, share, st);
             }
         }
         SBG_CUDA(cudaGetLastError(), "realize launch");
-        SBG_CUDA(launchGather(b->T, b->dHostYOff, b->ydot, b->staging, 0, st, i0, i1 - i0), "derivative gather");
+        SBG_CUDA(launchGather(b->packing(), b->dHostYOff, b->ydot, b->staging, 0, st, i0, i1 - i0), "derivative gather");
         SBG_CUDA(cudaEventRecord(b->pipeEv[1][c], st), "pipeline");
+        b->launches += 1 + 2 * b->packLaunches() + (b->precision == SBG_PRECISION_MIXED ? 1 : 0);
+    }
+    // after every chunk is under way: a copy to pageable memory may hold the host
+    for (int c = 0; c < nchunks; ++c) {
+        const int i0 = std::min(b->ninst, (int)((int64_t)tiles * c / nchunks) * kTile);
+        const int i1 = std::min(b->ninst, (int)((int64_t)tiles * (c + 1) / nchunks) * kTile);
+        if (i1 <= i0) continue;
+        const int64_t o0 = b->hostYOff[i0], o1 = b->hostYOff[i1];
         SBG_CUDA(cudaStreamWaitEvent(down, b->pipeEv[1][c], 0), "pipeline");
         SBG_CUDA(cudaMemcpyAsync(dst + o0, b->staging + o0, (o1 - o0) * sizeof(double), cudaMemcpyDeviceToHost, down),
                  "derivative download");
-        if (stPinned)
+        if (stDirect)
             SBG_CUDA(cudaMemcpyAsync(status + i0, b->status + i0, (i1 - i0) * sizeof(int32_t), cudaMemcpyDeviceToHost,
                                      down), "status download");
-        b->launches += 3 + (b->precision == SBG_PRECISION_MIXED ? 1 : 0);
     }
-    if (status && !stPinned)
+    if (status && !stDirect)
         SBG_CUDA(cudaMemcpyAsync(status, b->status, b->ninst * sizeof(int32_t), cudaMemcpyDeviceToHost, down),
                  "status download");
     // the batch stream continues after the downloads
     SBG_CUDA(cudaEventRecord(b->pipeEnd, down), "pipeline");
     SBG_CUDA(cudaStreamWaitEvent(b->stream, b->pipeEnd, 0), "pipeline");
     SBG_CUDA(cudaStreamSynchronize(down), "pipelined realize");
-    if (!dstPinned) std::memcpy(ydot, b->hostPinned, bytes);
+    if (dst != ydot) std::memcpy(ydot, dst, bytes);
     b->stateSet = true;
     b->integrating = false;
     b->realized = true;
@@ -1290,41 +1392,39 @@ int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
     if (!b->stateSet) return fail(SBG_ERR_STATE, "no state has been set");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     const size_t bytes = b->nuTotal * sizeof(double);
-    std::memcpy(b->hostPinned, f, bytes);
-    SBG_CUDA(cudaMemcpyAsync(b->staging, b->hostPinned, bytes, cudaMemcpyHostToDevice, b->stream), "force upload");
-    SBG_CUDA(launchScatter(b->T, b->dHostUOff, b->staging, b->fcol, 1, b->stream), "force scatter");
+    void* src = b->hostSide(f, bytes);
+    if (!src) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    if (src != f) std::memcpy(src, f, bytes);
+    SBG_CUDA(cudaMemcpyAsync(b->staging, src, bytes, cudaMemcpyHostToDevice, b->stream), "force upload");
+    SBG_CUDA(launchScatter(b->packing(), b->dHostUOff, b->staging, b->fcol, 1, b->stream), "force scatter");
     SBG_CUDA(launchMInv(b->T, b->plan(), b->precision, b->y, b->fcol, b->ydot, b->bufsArg(), b->status, b->streams()),
              "M^-1 kernel launch");
     b->realized = false;  // the result went to the derivative columns
-    SBG_CUDA(launchGather(b->T, b->dHostUOff, b->ydot, b->staging, 1, b->stream), "result gather");
-    b->launches += 2 + b->segments();
-    SBG_CUDA(cudaMemcpyAsync(b->hostPinned, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream), "result download");
+    SBG_CUDA(launchGather(b->packing(), b->dHostUOff, b->ydot, b->staging, 1, b->stream), "result gather");
+    b->launches += 2 * b->packLaunches() + b->segments();
+    void* dst = b->hostSide(outp, bytes);
+    if (!dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    SBG_CUDA(cudaMemcpyAsync(dst, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream), "result download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "M^-1");
-    std::memcpy(outp, b->hostPinned, bytes);
+    if (dst != outp) std::memcpy(outp, dst, bytes);
     return SBG_OK;
 }
 
 // ------------------------------------------------------------ tree operators
 // Device operands of a tree operator in the host packing: x [nu] | fmob [nu] |
-// fbody [6 nb] | out [max(nu, 10 nb)], mirrored in pinned host memory.
+// fbody [6 nb] | out [max(nu, 10 nb)].
 static int ensureTreeOps(sbg_batch b) {
     const int64_t nu = b->nuTotal, nbT = b->hostBOff[b->ninst];
     const int64_t need = 2 * nu + 6 * nbT + std::max<int64_t>(nu, 10 * nbT);
     if (b->opsDev && b->opsElems >= need) return SBG_OK;
     int rc;
     void* p = nullptr;
-    if (!b->opsScratch && b->scratchElems > 0)
-        if ((rc = b->alloc(&b->opsScratch, b->scratchElems * sizeof(double), "tree-operator scratch"))) return rc;
+    if (!b->tiles.ntiles && (rc = buildTiles(b, false, &b->tiles))) return rc;  // a mixed batch's
     if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
     b->opsDev = static_cast<double*>(p);
     const int64_t* dOff = nullptr;
     if ((rc = b->upload(&dOff, b->hostBOff, "offsets"))) return rc;
     b->dHostBOff = const_cast<int64_t*>(dOff);
-    cudaError_t e = cudaMallocHost(&b->opsHost, std::max<int64_t>(need, 1) * sizeof(double));
-    if (e != cudaSuccess) {
-        b->opsHost = nullptr;
-        return cudaFail(e, "cudaMallocHost");
-    }
     b->opsElems = need;
     if (!b->evOp0) {
         SBG_CUDA(cudaEventCreate(&b->evOp0), "event");
@@ -1345,11 +1445,12 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     double* dB = dF + nu;
     double* dOut = dB + 6 * nbT;
     const int64_t nOut = kind == OP_JV ? 6 * nbT : (kind == OP_COMPOSITE ? 10 * nbT : nu);
-    double* hX = b->opsHost;
     auto up = [&](const double* src, double* dDst, int64_t n, const char* what) -> int {
         if (!src || n == 0) return SBG_OK;
-        double* h = hX + (dDst - b->opsDev);
-        std::memcpy(h, src, n * sizeof(double));
+        if (!b->pageable) SBG_CUDA(cudaStreamSynchronize(b->stream), what);  // hostSide may move the buffer
+        void* h = b->hostSide(src, n * sizeof(double), (dDst - b->opsDev) * sizeof(double));
+        if (!h) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+        if (h != src) std::memcpy(h, src, n * sizeof(double));
         SBG_CUDA(cudaMemcpyAsync(dDst, h, n * sizeof(double), cudaMemcpyHostToDevice, b->stream), what);
         return SBG_OK;
     };
@@ -1357,20 +1458,21 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     if (int rc = up(fmob, dF, nu, "mobility force upload")) return rc;
     if (int rc = up(fbody, dB, 6 * nbT, "body force upload")) return rc;
     OpIO io{kind, x ? dX : nullptr, fmob ? dF : nullptr, fbody ? dB : nullptr, dOut, b->dHostUOff, b->dHostBOff};
-    double* sc = static_cast<double*>(b->opsScratch);
     SBG_CUDA(cudaEventRecord(b->evOp0, b->stream), "event");
-    SBG_CUDA(launchTreeOp(b->T, b->plan(), io, b->y, sc, static_cast<double*>(b->scratchLoop), b->status, b->stream),
+    SBG_CUDA(launchTreeOp(b->T, b->plan(), b->tiles, io, b->y, static_cast<double*>(b->scratchLoop), b->status, b->stream),
              "tree-operator kernel launch");
     SBG_CUDA(cudaEventRecord(b->evOp1, b->stream), "event");
-    b->launches += b->segments();
-    double* hOut = hX + (dOut - b->opsDev);
+    b->launches += (b->tiles.ntiles > 0) + (b->nLoop > 0);
+    if (!b->pageable) SBG_CUDA(cudaStreamSynchronize(b->stream), "tree operator");  // hostSide may move the buffer
+    void* hOut = nOut > 0 ? b->hostSide(out, nOut * sizeof(double), (dOut - b->opsDev) * sizeof(double)) : out;
+    if (!hOut) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
     if (nOut > 0)
         SBG_CUDA(cudaMemcpyAsync(hOut, dOut, nOut * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "result download");
     if (status && b->ninst > 0)
         SBG_CUDA(cudaMemcpyAsync(status, b->status, b->ninst * sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream),
                  "status download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "tree operator");
-    std::memcpy(out, hOut, nOut * sizeof(double));
+    if (hOut != out) std::memcpy(out, hOut, nOut * sizeof(double));
     return SBG_OK;
 }
 
@@ -1530,7 +1632,7 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
         if (!b->tiles.ntiles)
             if (int rc = buildTiles(b, false, &b->tiles)) return rc;
         const BatchBufs B64{nullptr, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64, b->colElems,
-                            &b->tiles, &b->ones};
+                            &b->tiles, &b->ones, nullptr};
         const StepCtl step{nsteps >= 0 ? nsteps : -1, 0, tStop, 0, 0};
         SBG_CUDA(launchRKMerson(Tk, P, SBG_PRECISION_FP64, b->y, b->time, B64, b->status, h, step, acc, ctol, pes,
                                 b->streams()),
@@ -1661,10 +1763,12 @@ int sbg_batch_get_qdotdot(sbg_batch b, double* qdotdot) {
     const int64_t nqT = b->nyTotal - b->nuTotal;
     SBG_CUDA(launchQDotDot(b->T, b->dHostQOff, b->y, b->ydot, b->staging, b->stream), "qdotdot kernel launch");
     ++b->launches;
-    SBG_CUDA(cudaMemcpyAsync(b->hostPinned, b->staging, nqT * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
+    void* dst = b->hostSide(qdotdot, nqT * sizeof(double));
+    if (!dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
+    SBG_CUDA(cudaMemcpyAsync(dst, b->staging, nqT * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
              "qdotdot download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "qdotdot");
-    std::memcpy(qdotdot, b->hostPinned, nqT * sizeof(double));
+    if (dst != qdotdot) std::memcpy(qdotdot, dst, nqT * sizeof(double));
     return SBG_OK;
 }
 

@@ -8,11 +8,13 @@ namespace {
 
 template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
-    realizeTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int tile0,
+    realizeTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int tile0, int ntiles,
                       const double* __restrict__ y, double* __restrict__ ydot, double* __restrict__ recs,
                       int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
-    const TileCtx c = tileCtx<CF>(T, TT, tile0 + blockIdx.x, recs);
+    const int id = tileId(TT, tile0, ntiles);
+    if (id < 0) return;
+    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
     const TileYSrc<CF::YS> src{{T, c.inst}, y};
     TileOut<CF::YS> out(src.c, ydot);
     int st = tileRhs<CF, false>(T, TT, c, src, out, true);
@@ -23,11 +25,14 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
-    minvTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, const double* __restrict__ y,
+    minvTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int ntiles,
+                   const double* __restrict__ y,
                    const double* __restrict__ f, double* __restrict__ o, double* __restrict__ recs,
                    int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
-    const TileCtx c = tileCtx<CF>(T, TT, blockIdx.x, recs);
+    const int id = tileId(TT, 0, ntiles);
+    if (id < 0) return;
+    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
     const TileFSrc<CF::YS> src{{T, c.inst}, y, f};
     TileUOut<CF::YS> out(src.c, o);
     int st = tileRhs<CF, true>(T, TT, c, src, out, true);
@@ -75,14 +80,16 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s) {
     if (ntiles <= 0) return;
+    const TileLaunch L(S, ntiles);
     tileDispatch<kTile>(S, [&](auto cf) {
-        realizeTileKernel<decltype(cf)><<<ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, tile0, a.y, a.ydot, S.recs, a.status);
+        realizeTileKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, tile0, ntiles, a.y, a.ydot, S.recs, a.status);
     });
 }
 void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s) {
     if (S.ntiles <= 0) return;
+    const TileLaunch L(S, S.ntiles);
     tileDispatch<kTile>(S, [&](auto cf) {
-        minvTileKernel<decltype(cf)><<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, a.y, a.f, a.ydot, S.recs, a.status);
+        minvTileKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, S.ntiles, a.y, a.f, a.ydot, S.recs, a.status);
     });
 }
 void realizeFallbackTiles(const KArgs& a, const TileSet& S, int first, int count, int block0, int blocks, cudaStream_t s) {

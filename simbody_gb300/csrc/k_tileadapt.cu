@@ -57,10 +57,12 @@ namespace {
 template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     rkAdaptiveTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT,
-                         double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
+                         int ntiles, double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
                          int32_t* __restrict__ status, const __grid_constant__ AdaptCtl ac) {
     __shared__ TileShare<5> sh;
-    const TileCtx c = tileCtx<CF>(T, TT, blockIdx.x, recs);
+    const int id = tileId(TT, 0, ntiles);
+    if (id < 0) return;
+    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
     const TileCol<CF::YS> col(T, c.inst);
     const int nq = col.nq, nu = T.inu[c.inst];
     double *f0 = fbuf, *fA = fbuf + fplane, *fB = fbuf + 2 * fplane, *fC = fbuf + 3 * fplane, *yt = fbuf + 4 * fplane;
@@ -238,8 +240,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 void rkAdaptiveTiles(const KArgs& a, const TileSet& S, const AdaptCtl& ac, cudaStream_t s) {
     if (S.ntiles <= 0) return;
+    const TileLaunch L(S, S.ntiles);
     tileDispatch<kTile>(S, [&](auto cf) {
-        rkAdaptiveTileKernel<decltype(cf)><<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, S.recs, a.ystate, a.time,
+        rkAdaptiveTileKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, S.ntiles, S.recs, a.ystate, a.time,
                                                                             static_cast<double*>(a.fbuf), a.fplane,
                                                                             a.status, ac);
     });

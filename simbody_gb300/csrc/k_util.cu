@@ -2,6 +2,8 @@
 // precision dispatch of the launchers.
 #include "abi_device.cuh"
 
+#include <algorithm>
+
 namespace sbg {
 
 // Integrator::initialize forces a projection: quaternions are normalized
@@ -95,23 +97,97 @@ cudaError_t launchQDotDot(const DevTables& T, const int64_t* qHost, const double
 
 // Pack/unpack between the host's per-instance packing and the columns.
 // part 0: all of [q,u]; part 1: the u slots only (nu values per instance).
-__global__ void scatterKernel(DevTables T, const int64_t* __restrict__ hostOff, const double* __restrict__ packed,
-                              double* __restrict__ cols, int part, int inst0) {
-    const int inst = inst0 + blockIdx.x;
+// Contiguous columns: one block per instance.
+template <bool SCATTER>
+__global__ void __launch_bounds__(128) packKernel(const __grid_constant__ DevTables T, const int64_t* __restrict__ hostOff,
+                                                  const double* __restrict__ src, double* __restrict__ dst, int part,
+                                                  int pos0) {
+    const int inst = T.order[pos0 + blockIdx.x];
     const int nq = T.inq[inst];
     const int cnt = part == 0 ? nq + T.inu[inst] : T.inu[inst];
-    const int c0 = part == 0 ? 0 : nq;
-    const int64_t base = T.ybase[inst], stride = T.ystride[inst], off = hostOff[inst];
-    for (int k = threadIdx.x; k < cnt; k += blockDim.x) cols[base + (int64_t)(c0 + k) * stride] = packed[off + k];
+    const int64_t base = T.ybase[inst] + (part == 0 ? 0 : nq), off = hostOff[inst];
+    for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
+        if (SCATTER) dst[base + k] = src[off + k];
+        else dst[off + k] = src[base + k];
+    }
 }
-__global__ void gatherKernel(DevTables T, const int64_t* __restrict__ hostOff, const double* __restrict__ cols,
-                             double* __restrict__ packed, int part, int inst0) {
-    const int inst = inst0 + blockIdx.x;
-    const int nq = T.inq[inst];
-    const int cnt = part == 0 ? nq + T.inu[inst] : T.inu[inst];
-    const int c0 = part == 0 ? 0 : nq;
-    const int64_t base = T.ybase[inst], stride = T.ystride[inst], off = hostOff[inst];
-    for (int k = threadIdx.x; k < cnt; k += blockDim.x) packed[off + k] = cols[base + (int64_t)(c0 + k) * stride];
+// Interleaved columns: the 32 instances of a tile by 32 elements at a time
+// through shared memory, so that both sides move whole 256-byte rows. Bound by
+// DRAM: 65,536 columns of 224 elements up in ?? us and down in ?? us, against
+// 92 and 83 us with each instance's elements written 256 bytes apart.
+template <bool SCATTER>
+__global__ void __launch_bounds__(256) packTileKernel(const __grid_constant__ DevTables T,
+                                                      const int64_t* __restrict__ hostOff,
+                                                      const double* __restrict__ src, double* __restrict__ dst, int part,
+                                                      int pos0, int count) {
+    __shared__ double sm[32][33];
+    __shared__ int64_t off[32], col[32];
+    __shared__ int cnt[32], most;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w == 0) {
+        const int p = blockIdx.x * kTile + lane;
+        int n = 0;
+        if (p < count) {
+            const int inst = T.order[pos0 + p], nq = T.inq[inst], nu = T.inu[inst];
+            n = part == 0 ? nq + nu : nu;
+            off[lane] = hostOff[inst];
+            col[lane] = T.ybase[inst] + (part == 0 ? 0 : (int64_t)nq * kTile);
+        }
+        cnt[lane] = n;
+        n = __reduce_max_sync(0xffffffffu, n);
+        if (lane == 0) most = n;
+    }
+    __syncthreads();
+    for (int k0 = 32 * blockIdx.y; k0 < most; k0 += 32 * gridDim.y) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = w + 8 * r;
+            if (SCATTER) {  // row of instance i
+                if (k0 + lane < cnt[i]) sm[i][lane] = src[off[i] + k0 + lane];
+            } else {        // element k0 + i of all
+                if (k0 + i < cnt[lane]) sm[i][lane] = src[col[lane] + (int64_t)(k0 + i) * kTile];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = w + 8 * r;
+            if (SCATTER) {
+                if (k0 + i < cnt[lane]) dst[col[lane] + (int64_t)(k0 + i) * kTile] = sm[lane][i];
+            } else {
+                if (k0 + lane < cnt[i]) dst[off[i] + k0 + lane] = sm[lane][i];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <bool SCATTER>
+static cudaError_t launchPack(const Packing& P, const int64_t* hostOff, const double* src, double* dst, int part,
+                              cudaStream_t s, int pos0, int count) {
+    auto tiles = [&](int p0, int n) {
+        if (n <= 0) return;
+        const int nt = (n + kTile - 1) / kTile, rows = (P.maxCol + 31) / 32;
+        const int split = std::max(1, std::min(rows, 1024 / nt));  // few tiles: their elements over several blocks
+        packTileKernel<SCATTER><<<dim3(nt, split), 256, 0, s>>>(*P.T, hostOff, src, dst, part, p0, n);
+    };
+    if (count >= 0) {
+        tiles(pos0, count);
+    } else {
+        tiles(0, P.tiles0);
+        if (P.tiles1 > P.tiles0)
+            packKernel<SCATTER><<<P.tiles1 - P.tiles0, 128, 0, s>>>(*P.T, hostOff, src, dst, part, P.tiles0);
+        tiles(P.tiles1, P.ninst - P.tiles1);
+    }
+    return cudaGetLastError();
+}
+cudaError_t launchScatter(const Packing& P, const int64_t* hostOff, const double* packed, double* cols, int part,
+                          cudaStream_t s, int pos0, int count) {
+    return launchPack<true>(P, hostOff, packed, cols, part, s, pos0, count);
+}
+cudaError_t launchGather(const Packing& P, const int64_t* hostOff, const double* cols, double* packed, int part,
+                         cudaStream_t s, int pos0, int count) {
+    return launchPack<false>(P, hostOff, cols, packed, part, s, pos0, count);
 }
 
 // Run the chain segment, then the loop-closure segment, on the main stream
@@ -144,7 +220,7 @@ static cudaError_t forkJoin(const LaunchPlan& P, const Streams& s, FC chain, FL 
 static KArgs baseArgs(const DevTables& T, const LaunchPlan& P, const BatchBufs& B, int32_t* status) {
     KArgs a{};
     a.T = &T; a.P = &P; a.scratch = B.scratch; a.scratchLoop = B.scratchLoop; a.fbuf = B.fbuf;
-    a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status;
+    a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status; a.tiles32 = B.tiles32;
     return a;
 }
 // FP64: the tiles, then the loop-closure segment, on the main stream.
@@ -262,22 +338,6 @@ cudaError_t launchNormalizeQuat(const DevTables& T, double* y, cudaStream_t s) {
     const int blocks = (T.ninst + 3) / 4;
     if (blocks == 0) return cudaSuccess;
     normalizeQuatKernel<<<blocks, 128, 0, s>>>(T, y);
-    return cudaGetLastError();
-}
-
-cudaError_t launchScatter(const DevTables& T, const int64_t* hostOff, const double* packed, double* cols, int part,
-                          cudaStream_t s, int inst0, int count) {
-    if (count < 0) count = T.ninst - inst0;
-    if (count <= 0) return cudaSuccess;
-    scatterKernel<<<count, 128, 0, s>>>(T, hostOff, packed, cols, part, inst0);
-    return cudaGetLastError();
-}
-
-cudaError_t launchGather(const DevTables& T, const int64_t* hostOff, const double* cols, double* packed, int part,
-                         cudaStream_t s, int inst0, int count) {
-    if (count < 0) count = T.ninst - inst0;
-    if (count <= 0) return cudaSuccess;
-    gatherKernel<<<count, 128, 0, s>>>(T, hostOff, cols, packed, part, inst0);
     return cudaGetLastError();
 }
 

@@ -11,6 +11,8 @@
 // sub-partitions. Records live in global memory, field by field across the
 // lanes; their loads are short beside a step's FP64 instructions.
 #pragma once
+#include <algorithm>
+
 #include "kernels.h"
 #include "tile_program.h"
 
@@ -29,21 +31,39 @@ struct TileCtx {
     double* rec;     // the lane's column of the tile's records
     const int4* slots;  // the lane's column of the slot integers, parameters
     const double* par;
-    int lane, w;     // lane of the tile, warp of the block
+    int lane, w;     // lane and warp of the tile
+    int sub;         // tile of the block
     bool on;         // the lane holds an instance
     int inst;
 };
 
-__device__ __forceinline__ void tileSync(int W) {
-    if (W == 1) __syncwarp(); else __syncthreads();
+// Tiles of fewer than four warps share a block where there are more of them
+// than SMs, so that the block's warps take the SM's sub-partitions in turn:
+// single-warp blocks landed two on one sub-partition beside an empty one when
+// other kernels' blocks came and went (20,000 FP64 chains in two chunks 1.64
+// ms, 1.27 ms so); while there are SMs for all, each its own (1,024 pendulums
+// 9.3 ms, four to a block 10.1 ms).
+inline int tilesPerBlock(const TileSet& S, int sms) {
+    return S.tt.W >= 4 ? 1 : std::max(1, std::min(4 / S.tt.W, (S.ntiles + sms - 1) / sms));
+}
+__device__ __forceinline__ void tileSync(int W, const TileCtx& c) {
+    if (W == 1) __syncwarp();
+    else if (W == 2) asm volatile("bar.sync %0, 64;" ::"r"(1 + c.sub) : "memory");
+    else __syncthreads();
 }
 
 template <class CF> __device__ __forceinline__ void tileTables(const TileTables& TT, TileCtx& c) {
     c.lane = threadIdx.x & 31;
-    c.w = threadIdx.x >> 5;
+    c.sub = (threadIdx.x >> 5) / TT.W;
+    c.w = (threadIdx.x >> 5) - c.sub * TT.W;
     const int l = CF::SH || c.lane >= CF::LS ? 0 : c.lane;
     c.slots = reinterpret_cast<const int4*>(TT.slots + c.d.slot0) + 2 * l;
     c.par = TT.par + c.d.par0 + l;
+}
+// The warp's tile among [tile0, tile0 + count), -1 past the end.
+__device__ __forceinline__ int tileId(const TileTables& TT, int tile0, int count) {
+    const int k = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / TT.W;
+    return k < count ? tile0 + k : -1;
 }
 // Tile `id` of a batch.
 template <class CF>
@@ -101,7 +121,7 @@ __device__ __forceinline__ void tileSweep(const TileTables& TT, const TileCtx& c
             const int slot = step * W + c.w;
             f(t.cl, slot, t.row(), tile::Par<LN>{c.par + (int64_t)slot * (tile::PR_COUNT * LN)});
         }
-        tileSync(W);
+        tileSync(W, c);
         t = next;
     }
 }
@@ -184,19 +204,20 @@ template <int N>
 __device__ __forceinline__ int tileReduce(const TileTables& TT, const TileCtx& c, TileShare<N>& sh, double* v, int bits) {
     if (TT.W == 1) return bits;
 #pragma unroll
-    for (int k = 0; k < N; ++k) sh.v[k][c.w][c.lane] = v[k];
-    sh.bits[c.w][c.lane] = bits;
-    __syncthreads();
+    for (int k = 0; k < N; ++k) sh.v[k][c.sub * TT.W + c.w][c.lane] = v[k];
+    sh.bits[c.sub * TT.W + c.w][c.lane] = bits;
+    tileSync(TT.W, c);
     int b = 0;
     double s[N > 0 ? N : 1] = {};
     for (int w = 0; w < TT.W; ++w) {
+        const int i = c.sub * TT.W + w;
 #pragma unroll
-        for (int k = 0; k < N; ++k) s[k] = w == 0 ? sh.v[k][0][c.lane] : s[k] + sh.v[k][w][c.lane];
-        b |= sh.bits[w][c.lane];
+        for (int k = 0; k < N; ++k) s[k] = w == 0 ? sh.v[k][i][c.lane] : s[k] + sh.v[k][i][c.lane];
+        b |= sh.bits[i][c.lane];
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k] = s[k];
-    __syncthreads();  // the arrays may be written again
+    tileSync(TT.W, c);  // the arrays may be written again
     return b;
 }
 
@@ -228,10 +249,10 @@ template <int YS> struct TileFSrc {  // M^-1 f: q and the given forces
 // 108-126) into the plane yt, element by element over the block's warps. Formed
 // in the bodies' loads instead, its five cases made up most of the kernel's
 // code, which then ran from beyond the instruction cache.
-template <class CF>
+template <class CF, class F>
 __device__ __forceinline__ void tileStageInput(const TileTables& TT, const TileCtx& c, const TileCol<CF::YS>& col, int ny,
-                                               bool run, int stage, double h, const double* y, const double* f0,
-                                               const double* fa, const double* fb, double* yt) {
+                                               bool run, int stage, double h, const double* y, const F* f0, const F* fa,
+                                               const F* fb, double* yt) {
     const int W = TT.W;
     auto all = [&](auto f) {
         if (run) {
@@ -243,11 +264,13 @@ __device__ __forceinline__ void tileStageInput(const TileTables& TT, const TileC
         }
     };
     if (stage == 0) all([&](int64_t e) { return y[e]; });
-    else if (stage == 1) all([&](int64_t e) { return y[e] + h * f0[e]; });                          // h/3 f0
-    else if (stage == 2) all([&](int64_t e) { return y[e] + h * (f0[e] + fa[e]); });                // h/6 (f0+f1)
-    else if (stage == 3) all([&](int64_t e) { return y[e] + h * (f0[e] + 3.0 * fa[e]); });          // h/8 (f0+3f2)
-    else all([&](int64_t e) { return y[e] + h * ((f0[e] - 3.0 * fa[e]) + 4.0 * fb[e]); });          // h/2 (f0-3f2+4f3)
-    tileSync(W);
+    else if (stage == 1) all([&](int64_t e) { return y[e] + h * double(f0[e]); });                          // h/3 f0
+    else if (stage == 2) all([&](int64_t e) { return y[e] + h * (double(f0[e]) + double(fa[e])); });                // h/6 (f0+f1)
+    else if (stage == 3) all([&](int64_t e) { return y[e] + h * (double(f0[e]) + 3.0 * double(fa[e])); });          // h/8 (f0+3f2)
+    else all([&](int64_t e) {                                                                       // h/2 (f0-3f2+4f3)
+        return y[e] + h * ((double(f0[e]) - 3.0 * double(fa[e])) + 4.0 * double(fb[e]));
+    });
+    tileSync(W, c);
 }
 template <int YS> struct TileOut {
     TileCol<YS> c;
@@ -288,6 +311,15 @@ template <int YS, class F> inline void tileDispatch(const TileSet& S, F f) {
     else if (S.tt.shared) f(TileCfg<32, true, YS>());
     else f(TileCfg<32, false, YS>());
 }
+// Grid and block of a launch over `ntiles` of the set's tiles.
+struct TileLaunch {
+    int grid, block;
+    TileLaunch(const TileSet& S, int ntiles) {
+        const int per = tilesPerBlock(S, S.sms);
+        grid = (ntiles + per - 1) / per;
+        block = 32 * S.tt.W * per;
+    }
+};
 typedef TileCfg<1, true, 0> TileOne;  // one tile per instance
 
 }  // namespace sbg

@@ -122,7 +122,7 @@ __device__ __forceinline__ void rkTile(const DevTables& T, const TileTables& TT,
             tileBodies<CF>(TT, c, renorm, [&](const tile::SlotRow& r) {
                 if (r.info & F_QUAT) tileNormalize(y, col, r.qo);
             });
-        tileSync(TT.W);
+        tileSync(TT.W, c);
     }
     if (c.on && c.w == 0) {
         if (T.stepsLeft) T.stepsLeft[c.inst] = left;
@@ -138,18 +138,21 @@ __device__ __forceinline__ void rkTile(const DevTables& T, const TileTables& TT,
 
 template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
-    rkTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, double* __restrict__ recs,
-                 double* y, double* __restrict__ time, double* fbuf, int64_t fplane, int32_t* __restrict__ status,
+    rkTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int ntiles,
+                 double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane, int32_t* __restrict__ status,
                  double h, StepCtl sc, double accuracy, double consTol, int pes) {
     __shared__ TileShare<4> sh;
-    const TileCtx c = tileCtx<CF>(T, TT, blockIdx.x, recs);
+    const int id = tileId(TT, 0, ntiles);
+    if (id < 0) return;
+    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
     rkTile<CF, false>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
 }
 
 template <int YS> void rkTilesWith(const KArgs& a, const TileSet& S, cudaStream_t s) {
     if (S.ntiles <= 0) return;
+    const TileLaunch L(S, S.ntiles);
     tileDispatch<YS>(S, [&](auto cf) {
-        rkTileKernel<decltype(cf)><<<S.ntiles, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, S.recs, a.ystate, a.time,
+        rkTileKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, S.ntiles, S.recs, a.ystate, a.time,
                                                                     static_cast<double*>(a.fbuf), a.fplane, a.status, a.h,
                                                                     a.step, a.accuracy, a.consTol, a.projectEveryStep);
     });
