@@ -148,10 +148,10 @@ struct sbg_batch_s {
     std::vector<int32_t> topoOf;             // per instance, its index in topos
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
-    TileSet tiles32{};                       // FP32 forms: the chain segment's tiles (kernel variant 9)
     int tileWidth = kTile;                   // instances per tile of `tiles`
-    // tree operators (allocated on first use): device operands and results in the host packing,
+    // tree operators (allocated on first use): FP64 scratch, device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
+    void* opsScratch = nullptr;
     double* opsDev = nullptr;
     int64_t opsElems = 0;
     int64_t* dHostBOff = nullptr;
@@ -183,7 +183,7 @@ struct sbg_batch_s {
     LaunchPlan plan() const {
         return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop, 0, groupFirst, nLoopBlocks, 0};
     }
-    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones, &tiles32}; }
+    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones}; }
     // kernels of one pass over the batch
     int segments() const {
         if (precision == SBG_PRECISION_FP64) return (tiles.ntiles > 0) + (nLoop > 0);
@@ -660,51 +660,6 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     return SBG_OK;
 }
 
-// The chain segment's tiles of the FP32 forms, where some tree branches.
-static int buildTiles32(sbg_batch b) {
-    using namespace tile;
-    std::vector<TileRows> store;
-    std::vector<const TileRows*> rows(b->topos.size(), nullptr);
-    const std::vector<int64_t> rowBase(b->topos.size(), 0);
-    store.reserve(b->topos.size());
-    std::vector<int> at;
-    bool wide = false, six = false;
-    for (int p = 0; p < b->nChain; ++p) {
-        const int k = b->topoOf[b->order[p]];
-        at.push_back(k);
-        wide |= !b->topos[k]->chain;
-        if (rows[k]) continue;
-        store.emplace_back(*b->topos[k], true);
-        rows[k] = &store.back();
-        six |= rows[k]->gen;
-    }
-    if (!wide) return SBG_OK;
-    TileProgram P;
-    P.rs = P.rsTotal = scratchRecordSize(six ? 6 : b->nm);
-    P.W = TileProgram::warps32(at, rows, b->sms);
-    if (const char* v = std::getenv("SBG_TILE32")) P.W = std::max(1, std::min(8, std::atoi(v)));  // tuning override
-    P.shared = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
-    for (int p = 0; p < b->nChain; p += kTile)
-        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, rowBase);
-    TileSet& S = b->tiles32;
-    S.sms = b->sms;
-    S.tt.W = P.W;
-    S.tt.ls = kTile;
-    S.tt.shared = P.shared;
-    S.tt.rs = S.tt.rsTotal = P.rsTotal;
-    int rc;
-    if ((rc = b->upload(&S.tt.desc, P.desc, "tile table"))) return rc;
-    if ((rc = b->upload(&S.tt.cls, P.cls, "tile table"))) return rc;
-    if ((rc = b->upload(&S.tt.slots, P.slots, "tile table"))) return rc;
-    void* p = nullptr;
-    if ((rc = b->alloc(&p, P.recElems * sizeof(float), "tile records"))) return rc;
-    S.recs = static_cast<double*>(p);
-    if ((rc = b->alloc(&p, b->colElems * sizeof(double), "stage input"))) return rc;
-    S.yt = static_cast<double*>(p);
-    S.ntiles = (int)P.desc.size();
-    return SBG_OK;
-}
-
 extern "C" {
 
 int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
@@ -962,7 +917,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     if (precision == SBG_PRECISION_FP64) b->variant = 1;  // FP64 needs every register
     if (const char* v = std::getenv("SBG_VARIANT")) {  // tuning override
         const int want = std::atoi(v);
-        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 || want == 9 ? want : 1;
+        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 ? want : 1;
     }
 
     int rc = 0;
@@ -1055,8 +1010,6 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if ((rc = buildTiles(b, false, &b->tiles))) return bail(rc);
     } else {
         if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
-        if ((rc = buildTiles32(b))) return bail(rc);
-        if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
         if (precision == SBG_PRECISION_MIXED) {
             // FP64 tiles for the instances whose refinement reports an
             // ill-conditioned M, and the count of those recomputed
@@ -1203,8 +1156,7 @@ static int tuneVariant(sbg_batch b) {
     }
     if (!fixedVariant && b->precision != SBG_PRECISION_FP64) {
         int bestVariant = 1;
-        for (int v : {4, 7, 8, 9}) {
-            if (v == 9 && !b->tiles32.ntiles) continue;
+        for (int v : {4, 7, 8}) {
             if (v >= 7 && b->nChain == 0) continue;  // 64-thread blocks exist for the chain driver only
             if (v == 8 && !b->stagedOk) continue;
             b->variant = v;
@@ -1329,7 +1281,6 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     a.ydot = b->ydot;
     a.scratch = b->scratch;
     a.status = b->status;
-    a.tiles32 = &b->tiles32;
     for (int c = 0; c < nchunks; ++c) {
         const int i0 = std::min(b->ninst, (int)((int64_t)tiles * c / nchunks) * kTile);
         const int i1 = std::min(b->ninst, (int)((int64_t)tiles * (c + 1) / nchunks) * kTile);
@@ -1419,7 +1370,8 @@ static int ensureTreeOps(sbg_batch b) {
     if (b->opsDev && b->opsElems >= need) return SBG_OK;
     int rc;
     void* p = nullptr;
-    if (!b->tiles.ntiles && (rc = buildTiles(b, false, &b->tiles))) return rc;  // a mixed batch's
+    if (!b->opsScratch && b->scratchElems > 0)
+        if ((rc = b->alloc(&b->opsScratch, b->scratchElems * sizeof(double), "tree-operator scratch"))) return rc;
     if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
     b->opsDev = static_cast<double*>(p);
     const int64_t* dOff = nullptr;
@@ -1458,11 +1410,12 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     if (int rc = up(fmob, dF, nu, "mobility force upload")) return rc;
     if (int rc = up(fbody, dB, 6 * nbT, "body force upload")) return rc;
     OpIO io{kind, x ? dX : nullptr, fmob ? dF : nullptr, fbody ? dB : nullptr, dOut, b->dHostUOff, b->dHostBOff};
+    double* sc = static_cast<double*>(b->opsScratch);
     SBG_CUDA(cudaEventRecord(b->evOp0, b->stream), "event");
-    SBG_CUDA(launchTreeOp(b->T, b->plan(), b->tiles, io, b->y, static_cast<double*>(b->scratchLoop), b->status, b->stream),
+    SBG_CUDA(launchTreeOp(b->T, b->plan(), io, b->y, sc, static_cast<double*>(b->scratchLoop), b->status, b->stream),
              "tree-operator kernel launch");
     SBG_CUDA(cudaEventRecord(b->evOp1, b->stream), "event");
-    b->launches += (b->tiles.ntiles > 0) + (b->nLoop > 0);
+    b->launches += b->segments();
     if (!b->pageable) SBG_CUDA(cudaStreamSynchronize(b->stream), "tree operator");  // hostSide may move the buffer
     void* hOut = nOut > 0 ? b->hostSide(out, nOut * sizeof(double), (dOut - b->opsDev) * sizeof(double)) : out;
     if (!hOut) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
@@ -1632,7 +1585,7 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
         if (!b->tiles.ntiles)
             if (int rc = buildTiles(b, false, &b->tiles)) return rc;
         const BatchBufs B64{nullptr, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64, b->colElems,
-                            &b->tiles, &b->ones, nullptr};
+                            &b->tiles, &b->ones};
         const StepCtl step{nsteps >= 0 ? nsteps : -1, 0, tStop, 0, 0};
         SBG_CUDA(launchRKMerson(Tk, P, SBG_PRECISION_FP64, b->y, b->time, B64, b->status, h, step, acc, ctol, pes,
                                 b->streams()),

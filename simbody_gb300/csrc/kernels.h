@@ -50,7 +50,6 @@ struct BatchBufs {
     int64_t fplane;
     const TileSet* tiles;  // FP64: the chain and group segments' tiles
     const TileSet* ones;   // mixed form: one FP64 tile per instance
-    const TileSet* tiles32;  // FP32 forms: the chain segment's tiles (variant 9)
 };
 cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision, const double* y, double* ydot,
                           const BatchBufs& B, int32_t* status, const Streams& s);
@@ -62,8 +61,8 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
 // Tree operators (k_ops.cu, ops_device.cuh). Operands in the host packing:
 // u-like arrays nu values per instance at uoff[inst]; body arrays one entry
 // per mobilized body, in descriptor body order, from boff[inst] (6 values per
-// SpatialVec, 10 per spatial inertia). S: the batch's FP64 tiles; scratchLoop
-// the loop segment's records.
+// SpatialVec, 10 per spatial inertia). scratch is FP64 scratch laid out like
+// the batch's own (its element offsets), scratchLoop the loop segment's.
 enum : int { OP_RESIDUAL = 0, OP_MV = 1, OP_JV = 2, OP_JTF = 3, OP_COMPOSITE = 4 };
 struct OpIO {
     int kind;
@@ -74,9 +73,8 @@ struct OpIO {
     const int64_t* uoff;
     const int64_t* boff;
 };
-cudaError_t launchTreeOp(const DevTables& T, const LaunchPlan& P, const TileSet& S, const OpIO& io, const double* y,
+cudaError_t launchTreeOp(const DevTables& T, const LaunchPlan& P, const OpIO& io, const double* y, double* scratch,
                          double* scratchLoop, int32_t* status, cudaStream_t s);
-void treeOpTiles(const DevTables& T, const TileSet& S, const OpIO& io, const double* y, int32_t* status, cudaStream_t s);
 cudaError_t launchNormalizeQuat(const DevTables& T, double* y, cudaStream_t s);
 // qdotdot of every instance from the resident y and ydot, nq values per
 // instance at qHost[inst] of out.
@@ -149,11 +147,7 @@ struct KArgs {
     double h, accuracy, consTol;
     StepCtl step;
     int projectEveryStep;
-    const TileSet* tiles32;
 };
-// Tile driver, FP32 forms (k_tile32.cu, k_tilerk32.cu): variant 9 of the chain segment.
-void realizeTiles32(const KArgs& a, const TileSet& S, bool refine, int tile0, int ntiles, cudaStream_t s);
-void rkTiles32(const KArgs& a, const TileSet& S, bool refine, cudaStream_t s);
 // Tile driver, FP64 (k_tile.cu, k_tilerk.cu, k_tileadapt.cu).
 void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s);
 void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s);
