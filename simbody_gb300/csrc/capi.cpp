@@ -149,9 +149,8 @@ struct sbg_batch_s {
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
     int tileWidth = kTile;                   // instances per tile of `tiles`
-    // tree operators (allocated on first use): FP64 scratch, device operands and results in the host packing,
+    // tree operators (allocated on first use): device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
-    void* opsScratch = nullptr;
     double* opsDev = nullptr;
     int64_t opsElems = 0;
     int64_t* dHostBOff = nullptr;
@@ -1370,8 +1369,7 @@ static int ensureTreeOps(sbg_batch b) {
     if (b->opsDev && b->opsElems >= need) return SBG_OK;
     int rc;
     void* p = nullptr;
-    if (!b->opsScratch && b->scratchElems > 0)
-        if ((rc = b->alloc(&b->opsScratch, b->scratchElems * sizeof(double), "tree-operator scratch"))) return rc;
+    if (!b->tiles.ntiles && (rc = buildTiles(b, false, &b->tiles))) return rc;  // a mixed batch's
     if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
     b->opsDev = static_cast<double*>(p);
     const int64_t* dOff = nullptr;
@@ -1410,12 +1408,11 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     if (int rc = up(fmob, dF, nu, "mobility force upload")) return rc;
     if (int rc = up(fbody, dB, 6 * nbT, "body force upload")) return rc;
     OpIO io{kind, x ? dX : nullptr, fmob ? dF : nullptr, fbody ? dB : nullptr, dOut, b->dHostUOff, b->dHostBOff};
-    double* sc = static_cast<double*>(b->opsScratch);
     SBG_CUDA(cudaEventRecord(b->evOp0, b->stream), "event");
-    SBG_CUDA(launchTreeOp(b->T, b->plan(), io, b->y, sc, static_cast<double*>(b->scratchLoop), b->status, b->stream),
+    SBG_CUDA(launchTreeOp(b->T, b->plan(), b->tiles, io, b->y, static_cast<double*>(b->scratchLoop), b->status, b->stream),
              "tree-operator kernel launch");
     SBG_CUDA(cudaEventRecord(b->evOp1, b->stream), "event");
-    b->launches += b->segments();
+    b->launches += (b->tiles.ntiles > 0) + (b->nLoop > 0);
     if (!b->pageable) SBG_CUDA(cudaStreamSynchronize(b->stream), "tree operator");  // hostSide may move the buffer
     void* hOut = nOut > 0 ? b->hostSide(out, nOut * sizeof(double), (dOut - b->opsDev) * sizeof(double)) : out;
     if (!hOut) return fail(SBG_ERR_NOMEM, "out of pinned host memory");

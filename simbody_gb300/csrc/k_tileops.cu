@@ -9,7 +9,6 @@
 // body takes about 150 (M x) to 300 (composite inertias), the sweeps in Ground
 // axes about 400 to 700, and mobilizers don't diverge. 6,000 trees of 20 to 40
 // bodies, inverse dynamics: 2.07 ms for the kernel before, ?? ms now.
-#include "ops_device.cuh"
 #include "tile_device.cuh"
 
 namespace sbg {
@@ -294,8 +293,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 void treeOpTiles(const DevTables& T, const TileSet& S, const OpIO& io, const double* y, int32_t* status, cudaStream_t s) {
     if (S.ntiles <= 0) return;
+    const TileLaunch L(S, S.ntiles);
     tileDispatch<0>(S, [&](auto cf) {
-        tileOpKernel<decltype(cf)><<<tileGrid(S, S.ntiles), tileBlock(S), 0, s>>>(T, S.tt, S.ntiles, y, S.recs, io, status);
+        tileOpKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(T, S.tt, S.ntiles, y, S.recs, io, status);
     });
 }
 

@@ -61,8 +61,8 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
 // Tree operators (k_ops.cu, ops_device.cuh). Operands in the host packing:
 // u-like arrays nu values per instance at uoff[inst]; body arrays one entry
 // per mobilized body, in descriptor body order, from boff[inst] (6 values per
-// SpatialVec, 10 per spatial inertia). scratch is FP64 scratch laid out like
-// the batch's own (its element offsets), scratchLoop the loop segment's.
+// SpatialVec, 10 per spatial inertia). S: the batch's FP64 tiles; scratchLoop
+// the loop segment's records.
 enum : int { OP_RESIDUAL = 0, OP_MV = 1, OP_JV = 2, OP_JTF = 3, OP_COMPOSITE = 4 };
 struct OpIO {
     int kind;
@@ -73,8 +73,9 @@ struct OpIO {
     const int64_t* uoff;
     const int64_t* boff;
 };
-cudaError_t launchTreeOp(const DevTables& T, const LaunchPlan& P, const OpIO& io, const double* y, double* scratch,
+cudaError_t launchTreeOp(const DevTables& T, const LaunchPlan& P, const TileSet& S, const OpIO& io, const double* y,
                          double* scratchLoop, int32_t* status, cudaStream_t s);
+void treeOpTiles(const DevTables& T, const TileSet& S, const OpIO& io, const double* y, int32_t* status, cudaStream_t s);
 cudaError_t launchNormalizeQuat(const DevTables& T, double* y, cudaStream_t s);
 // qdotdot of every instance from the resident y and ydot, nq values per
 // instance at qHost[inst] of out.

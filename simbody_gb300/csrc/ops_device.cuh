@@ -11,8 +11,8 @@
 // kinematics for the residual, and the body accelerations
 // A = ~Phi A_parent + H x [+ a]), then one tip to base (body forces
 // F = own + sum Phi_c F_c, tau = ~H F - f; or the composite inertias). The
-// bodies of a level are spread over the G lanes of the instance's group
-// (G = 1 for the one-thread layouts); a parent pulls its children's results
+// bodies of a level are spread over the G lanes of the instance's group; a
+// parent pulls its children's results
 // after a level barrier. Each body's record holds its kinematics [0,18), the
 // body1 fields [18,42), H at kRecH, and the operator's A [42,48) and F
 // [48,54) (composite inertias: [42,52)).
@@ -39,21 +39,6 @@ struct OpSink {
     template <class R> __device__ __forceinline__ void qdot(int, R) {}
     template <class R> __device__ __forceinline__ void udot(int, R) {}
 };
-
-// Unit inertia of a unit point mass at p (MassProperties.h:458-466, 866-867).
-__device__ __forceinline__ S3<double> pointMassUnit(V3<double> p) {
-    const double xx = p.x * p.x, yy = p.y * p.y, zz = p.z * p.z;
-    return S3<double>{yy + zz, xx + zz, xx + yy, -p.x * p.y, -p.x * p.z, -p.y * p.z};
-}
-__device__ __forceinline__ S3<double> operator+(const S3<double>& a, const S3<double>& b) {
-    return S3<double>{a.xx + b.xx, a.yy + b.yy, a.zz + b.zz, a.xy + b.xy, a.xz + b.xz, a.yz + b.yz};
-}
-__device__ __forceinline__ S3<double> operator-(const S3<double>& a, const S3<double>& b) {
-    return S3<double>{a.xx - b.xx, a.yy - b.yy, a.zz - b.zz, a.xy - b.xy, a.xz - b.xz, a.yz - b.yz};
-}
-__device__ __forceinline__ S3<double> operator*(double s, const S3<double>& a) {
-    return S3<double>{s * a.xx, s * a.yy, s * a.zz, s * a.xy, s * a.xz, s * a.yz};
-}
 
 // rec(lb): record of local row lb in the instance's scratch.
 template <int NM, class SC, class RecOf>
@@ -186,24 +171,15 @@ __device__ __forceinline__ int treeOp(const DevTables& T, int inst, const SC& S,
     return finite ? 0 : SBG_INST_NONFINITE;
 }
 
-// SEG 0: one-thread instances in 32-wide interleaved tiles; 1: the
-// level-parallel and the loop-closure segments (field-major rows).
-template <int NM, int SEG>
-__global__ void __launch_bounds__(128) treeOpKernel(DevTables T, int first, int count, const double* __restrict__ y,
+// The instances of the level-parallel layout (field-major rows).
+__global__ void __launch_bounds__(128) treeOpKernel(DevTables T, int first, const double* __restrict__ y,
                                                    double* __restrict__ scratch, OpIO io,
                                                    int32_t* __restrict__ status) {
-    const Slot s = SEG == 1 ? groupSlot(T, first) : chainSlot(T, first, count);
+    const Slot s = groupSlot(T, first);
     if (s.inst < 0) return;
-    const int body0 = T.ibody[s.inst];
-    int st;
-    if constexpr (SEG == 0) {
-        const ScrTiled<double> S{scratch + T.sbase[s.inst]};
-        st = treeOp<NM>(T, s.inst, S, [&](int lb) { return (int)T.srec[body0 + lb]; }, y, io, 0, 1, 0u);
-    } else {
-        const ScrRows<double> S{scratch + T.sbase[s.inst], T.inb[s.inst]};
-        st = treeOp<NM>(T, s.inst, S, [](int lb) { return lb; }, y, io, s.gl, s.G, s.mask);
-        st = (int)__reduce_or_sync(s.mask, (unsigned)st);
-    }
+    const ScrRows<double> S{scratch + T.sbase[s.inst], T.inb[s.inst]};
+    int st = treeOp<3>(T, s.inst, S, [](int lb) { return lb; }, y, io, s.gl, s.G, s.mask);
+    st = (int)__reduce_or_sync(s.mask, (unsigned)st);
     if (s.gl == 0) status[s.inst] = st;
 }
 

@@ -116,4 +116,19 @@ template <class R> __host__ __device__ __forceinline__ AB<R> abshift(const AB<R>
     return o;
 }
 
+// Unit inertia of a unit point mass at p (MassProperties.h:458-466, 866-867).
+__host__ __device__ __forceinline__ S3<double> pointMassUnit(V3<double> p) {
+    const double xx = p.x * p.x, yy = p.y * p.y, zz = p.z * p.z;
+    return S3<double>{yy + zz, xx + zz, xx + yy, -p.x * p.y, -p.x * p.z, -p.y * p.z};
+}
+__host__ __device__ __forceinline__ S3<double> operator+(const S3<double>& a, const S3<double>& b) {
+    return S3<double>{a.xx + b.xx, a.yy + b.yy, a.zz + b.zz, a.xy + b.xy, a.xz + b.xz, a.yz + b.yz};
+}
+__host__ __device__ __forceinline__ S3<double> operator-(const S3<double>& a, const S3<double>& b) {
+    return S3<double>{a.xx - b.xx, a.yy - b.yy, a.zz - b.zz, a.xy - b.xy, a.xz - b.xz, a.yz - b.yz};
+}
+__host__ __device__ __forceinline__ S3<double> operator*(double s, const S3<double>& a) {
+    return S3<double>{s * a.xx, s * a.yy, s * a.zz, s * a.xy, s * a.xz, s * a.yz};
+}
+
 }  // namespace sbg

@@ -36,8 +36,9 @@ enum : int { CL_PIN = 0, CL_SLIDER, CL_UNIV, CL_BALL, CL_FREE, CL_GEN, CL_COUNT 
 // Parameters of a body (doubles), in M axes about the origin of M.
 //   C = R of the inboard frame F in the parent's M axes, d = its origin there
 //   mobility forces folded per mobility: f_j = S_j - K_j q_j - B_j u_j
+//   p_MB, the body's origin
 enum : int { PR_M = 0, PR_MC = 1, PR_J = 4, PR_C = 10, PR_D = 19, PR_PITCH = 22, PR_K = 23, PR_S = 29, PR_B = 35,
-             PR_COUNT = 41 };
+             PR_PMB = 41, PR_COUNT = 44 };
 // Integers of a body: q and u slots, slot of the parent (-1 = Ground), info
 // word (body table), body row, contacts.
 enum : int { SI_Q = 0, SI_U, SI_PARENT, SI_INFO, SI_ROW, SI_KBEG, SI_KCNT, SI_COUNT = 8 };

@@ -155,6 +155,7 @@ struct TileRows {
                 o[PR_D + i] = PR[3 * i] * pPF[0] + PR[3 * i + 1] * pPF[1] + PR[3 * i + 2] * pPF[2] + Pp[i];
             }
             o[PR_PITCH] = b[34];
+            for (int i = 0; i < 3; ++i) o[PR_PMB + i] = pMB[i];
             for (int k = t.fbeg[r]; k < t.fbeg[r] + t.fcnt[r]; ++k) {
                 const int j = t.fkw[k] & 255;
                 if ((t.fkw[k] >> 8) == 0) { o[PR_K + j] += t.fcoef[k]; o[PR_S + j] += t.fcoef[k] * t.fq0[k]; }
