@@ -26,11 +26,11 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 CU_UNITS = ["k_r32c.cu", "k_r32cr.cu", "k_r32s.cu", "k_r32g.cu", "k_rk64.cu", "k_rk32c.cu", "k_rk32cr.cu", "k_rk32g.cu",
             "k_util.cu", "k_noalloc.cu", "k_loops.cu", "k_ops.cu", "k_tile.cu", "k_tilerk.cu", "k_tilerkmixed.cu",
-            "k_tileadapt.cu", "k_tileops.cu", "serve.cu"]
+            "k_tileadapt.cu", "k_tileops.cu", "k_tile32.cu", "k_tilerk32.cu", "serve.cu"]
 HOST_UNITS = ["capi.cpp"]
 HEADERS = ["abi_device.cuh", "loops_device.cuh", "spatial.cuh", "engine.h", "kernels.h", "topology_internal.h",
            "serve_sched.h", "ops_device.cuh", "rk32c_launch.cuh",
-           "r32c_launch.cuh", "tile_core.cuh", "tile_device.cuh", "tilerk_device.cuh", "tile_program.h", "steps_device.cuh"]
+           "r32c_launch.cuh", "tile_core.cuh", "tile_device.cuh", "tilerk_device.cuh", "tile32_device.cuh", "tile_program.h", "steps_device.cuh"]
 
 
 def _nvcc() -> str:

@@ -1243,6 +1243,20 @@ __device__ __forceinline__ Slot groupSlot(const DevTables& T, int blk0) {
 
 #include "loops_device.cuh"
 
+// SBG_INST_ILL_CONDITIONED by the instance's largest |udot0| and correction.
+__device__ __forceinline__ int illConditionedBy(const DevTables& T, int inst, float um, float dm) {
+    const float tol = (T.fbList || T.ictl) ? kIllConditionedStep : kIllConditioned;
+    if (T.kcnt) {
+        // Contact spheres: the indentation is a small difference of body
+        // positions, which FP32 kinematics resolve to about 1e-5 of it, so
+        // these instances take the FP64 path of the mixed form.
+        const int b0 = T.ibody[inst], nb = T.inb[inst];
+        for (int r = 0; r < nb; ++r)
+            if (T.info[b0 + r] & F_CONTACT) return SBG_INST_ILL_CONDITIONED;
+    }
+    return dm > tol * um ? SBG_INST_ILL_CONDITIONED : 0;
+}
+
 // Mixed form: SBG_INST_ILL_CONDITIONED when the refinement correction exceeds
 // kIllConditioned of udot0 (max-norms over the instance, i.e. over the lanes
 // of its group). The correction is about cond(M) times the FP32 rounding, so
@@ -1255,16 +1269,7 @@ __device__ __forceinline__ int illConditioned(const DevTables& T, const Out& out
         um = __uint_as_float(__reduce_max_sync(s.mask, __float_as_uint(um)));
         dm = __uint_as_float(__reduce_max_sync(s.mask, __float_as_uint(dm)));
     }
-    const float tol = (T.fbList || T.ictl) ? kIllConditionedStep : kIllConditioned;
-    if (T.kcnt) {
-        // Contact spheres: the indentation is a small difference of body
-        // positions, which FP32 kinematics resolve to about 1e-5 of it, so
-        // these instances take the FP64 path of the mixed form.
-        const int b0 = T.ibody[s.inst], nb = T.inb[s.inst];
-        for (int r = 0; r < nb; ++r)
-            if (T.info[b0 + r] & F_CONTACT) return SBG_INST_ILL_CONDITIONED;
-    }
-    return dm > tol * um ? SBG_INST_ILL_CONDITIONED : 0;
+    return illConditionedBy(T, s.inst, um, dm);
 }
 
 // One RHS of the instance owned by slot s, through either driver; LOOPS adds

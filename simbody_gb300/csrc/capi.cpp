@@ -86,7 +86,7 @@ struct sbg_batch_s {
     int sms = 1;
     int nm = 3;
     bool tiled = false;
-    int variant = 0;  // kernel variant: 0 = not tuned yet, else 1, 4, 7 or 8 (see LaunchPlan)
+    int variant = 0;  // kernel variant: 0 = not tuned yet, else 1, 4, 7, 8 or 9 (see LaunchPlan)
     bool stagedOk = false;  // variant 8 applies: one shared chain topology without Free bodies
     cudaStream_t stream = nullptr;
     std::vector<int32_t> instTopo;
@@ -148,6 +148,7 @@ struct sbg_batch_s {
     std::vector<int32_t> topoOf;             // per instance, its index in topos
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
+    TileSet tiles32{};                       // FP32 forms: the chain segment's tiles (kernel variant 9)
     int tileWidth = kTile;                   // instances per tile of `tiles`
     // tree operators (allocated on first use): device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
@@ -182,7 +183,7 @@ struct sbg_batch_s {
     LaunchPlan plan() const {
         return LaunchPlan{nChain, nGroupBlocks, nm, variant == 0 ? 1 : variant, nLoop, 0, groupFirst, nLoopBlocks, 0};
     }
-    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones}; }
+    BatchBufs bufsArg() const { return BatchBufs{scratch, scratchLoop, fbuf, fbufLoop, colElems, &tiles, &ones, &tiles32}; }
     // kernels of one pass over the batch
     int segments() const {
         if (precision == SBG_PRECISION_FP64) return (tiles.ntiles > 0) + (nLoop > 0);
@@ -659,6 +660,51 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     return SBG_OK;
 }
 
+// The chain segment's tiles of the FP32 forms, where some tree branches.
+static int buildTiles32(sbg_batch b) {
+    using namespace tile;
+    std::vector<TileRows> store;
+    std::vector<const TileRows*> rows(b->topos.size(), nullptr);
+    const std::vector<int64_t> rowBase(b->topos.size(), 0);
+    store.reserve(b->topos.size());
+    std::vector<int> at;
+    bool wide = false, six = false;
+    for (int p = 0; p < b->nChain; ++p) {
+        const int k = b->topoOf[b->order[p]];
+        at.push_back(k);
+        wide |= !b->topos[k]->chain;
+        if (rows[k]) continue;
+        store.emplace_back(*b->topos[k], true);
+        rows[k] = &store.back();
+        six |= rows[k]->gen;
+    }
+    if (!wide) return SBG_OK;
+    TileProgram P;
+    P.rs = P.rsTotal = scratchRecordSize(six ? 6 : b->nm);
+    P.W = TileProgram::warps32(at, rows, b->sms);
+    if (const char* v = std::getenv("SBG_TILE32")) P.W = std::max(1, std::min(8, std::atoi(v)));  // tuning override
+    P.shared = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
+    for (int p = 0; p < b->nChain; p += kTile)
+        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, rowBase);
+    TileSet& S = b->tiles32;
+    S.sms = b->sms;
+    S.tt.W = P.W;
+    S.tt.ls = kTile;
+    S.tt.shared = P.shared;
+    S.tt.rs = S.tt.rsTotal = P.rsTotal;
+    int rc;
+    if ((rc = b->upload(&S.tt.desc, P.desc, "tile table"))) return rc;
+    if ((rc = b->upload(&S.tt.cls, P.cls, "tile table"))) return rc;
+    if ((rc = b->upload(&S.tt.slots, P.slots, "tile table"))) return rc;
+    void* p = nullptr;
+    if ((rc = b->alloc(&p, P.recElems * sizeof(float), "tile records"))) return rc;
+    S.recs = static_cast<double*>(p);
+    if ((rc = b->alloc(&p, b->colElems * sizeof(double), "stage input"))) return rc;
+    S.yt = static_cast<double*>(p);
+    S.ntiles = (int)P.desc.size();
+    return SBG_OK;
+}
+
 extern "C" {
 
 int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
@@ -916,7 +962,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     if (precision == SBG_PRECISION_FP64) b->variant = 1;  // FP64 needs every register
     if (const char* v = std::getenv("SBG_VARIANT")) {  // tuning override
         const int want = std::atoi(v);
-        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 ? want : 1;
+        b->variant = want == 8 ? (b->stagedOk ? 8 : 7) : want == 4 || want == 7 || want == 9 ? want : 1;
     }
 
     int rc = 0;
@@ -1009,6 +1055,8 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if ((rc = buildTiles(b, false, &b->tiles))) return bail(rc);
     } else {
         if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
+        if ((rc = buildTiles32(b))) return bail(rc);
+        if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
         if (precision == SBG_PRECISION_MIXED) {
             // FP64 tiles for the instances whose refinement reports an
             // ill-conditioned M, and the count of those recomputed
@@ -1139,6 +1187,10 @@ static int tuneVariant(sbg_batch b) {
         SBG_CUDA(cudaEventCreate(&b->evT0), "tuner");
         SBG_CUDA(cudaEventCreate(&b->evT1), "tuner");
     }
+    // the tile driver beat the one-thread variants at every size of branching
+    // trees (realize, us, variant 7 / tiles: 64 trees 528 / 224, 4,096 884 / 553,
+    // 16,384 1428 / 935)
+    if (b->variant == 0 && b->tiles32.ntiles) b->variant = 9;
     const bool fixedVariant = b->variant != 0;
     if (!fixedVariant) b->variant = 1;
     float best = 1e30f, ms = 0;
@@ -1280,6 +1332,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     a.ydot = b->ydot;
     a.scratch = b->scratch;
     a.status = b->status;
+    a.tiles32 = &b->tiles32;
     for (int c = 0; c < nchunks; ++c) {
         const int i0 = std::min(b->ninst, (int)((int64_t)tiles * c / nchunks) * kTile);
         const int i1 = std::min(b->ninst, (int)((int64_t)tiles * (c + 1) / nchunks) * kTile);
@@ -1582,7 +1635,7 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
         if (!b->tiles.ntiles)
             if (int rc = buildTiles(b, false, &b->tiles)) return rc;
         const BatchBufs B64{nullptr, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64, b->colElems,
-                            &b->tiles, &b->ones};
+                            &b->tiles, &b->ones, nullptr};
         const StepCtl step{nsteps >= 0 ? nsteps : -1, 0, tStop, 0, 0};
         SBG_CUDA(launchRKMerson(Tk, P, SBG_PRECISION_FP64, b->y, b->time, B64, b->status, h, step, acc, ctol, pes,
                                 b->streams()),

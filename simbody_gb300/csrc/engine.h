@@ -194,7 +194,7 @@ struct LaunchPlan {
     int nChain;
     int nGroupBlocks;
     int nm;
-    int variant;  // 1: registers as needed; 4: at most 128 registers (FP32 only); 7: 64-thread blocks; 8: 7 staged (realize)
+    int variant;  // 1: registers as needed; 4: at most 128 registers (FP32 only); 7: 64-thread blocks; 8: 7 staged (realize); 9: tiles
     int nLoop;    // order positions [nChain, nChain + nLoop): instances with loop closures (FP64 chain driver)
     int chainFirst;  // first order position of the chain segment launch (a sub-range of it: pipelined realize)
     int groupFirst;  // first block of the level-parallel launch in the block table
@@ -229,6 +229,7 @@ struct TileSet {
     double* recs;
     int32_t blocks;
     int64_t recStride;
+    double* yt;            // FP32 forms: the stage input of RK-Merson (a column plane)
 };
 
 }  // namespace sbg

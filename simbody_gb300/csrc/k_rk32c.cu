@@ -6,7 +6,8 @@
 namespace sbg {
 
 void rk32Chain(const KArgs& a, bool refine, cudaStream_t s) {
-    if (refine) rk32ChainRefined(a, s);
+    if (a.P->variant == 9) rkTiles32(a, *a.tiles32, refine, s);
+    else if (refine) rk32ChainRefined(a, s);
     else rk32ChainPick<false>(a, s);
 }
 

@@ -7,7 +7,7 @@ namespace sbg {
 namespace {
 
 template <class CF, int NM, bool REF>
-__global__ void __launch_bounds__(32 * kTileMaxWarps, 2)
+__global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
     realizeTile32Kernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int tile0, int ntiles,
                         const double* __restrict__ y, double* __restrict__ ydot, float* __restrict__ recs,
                         int32_t* __restrict__ status) {

@@ -7,7 +7,7 @@ namespace sbg {
 namespace {
 
 template <class CF, int NM, bool REF>
-__global__ void __launch_bounds__(32 * kTileMaxWarps, 2)
+__global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
     rkTile32Kernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int ntiles,
                    float* __restrict__ recs, double* y, double* yt, double* __restrict__ time, float* fbuf, int64_t fplane,
                    int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol, int pes) {

@@ -220,7 +220,7 @@ static cudaError_t forkJoin(const LaunchPlan& P, const Streams& s, FC chain, FL 
 static KArgs baseArgs(const DevTables& T, const LaunchPlan& P, const BatchBufs& B, int32_t* status) {
     KArgs a{};
     a.T = &T; a.P = &P; a.scratch = B.scratch; a.scratchLoop = B.scratchLoop; a.fbuf = B.fbuf;
-    a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status;
+    a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status; a.tiles32 = B.tiles32;
     return a;
 }
 // FP64: the tiles, then the loop-closure segment, on the main stream.

@@ -50,6 +50,7 @@ struct BatchBufs {
     int64_t fplane;
     const TileSet* tiles;  // FP64: the chain and group segments' tiles
     const TileSet* ones;   // mixed form: one FP64 tile per instance
+    const TileSet* tiles32;  // FP32 forms: the chain segment's tiles (variant 9)
 };
 cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision, const double* y, double* ydot,
                           const BatchBufs& B, int32_t* status, const Streams& s);
@@ -148,7 +149,11 @@ struct KArgs {
     double h, accuracy, consTol;
     StepCtl step;
     int projectEveryStep;
+    const TileSet* tiles32;
 };
+// Tile driver, FP32 forms (k_tile32.cu, k_tilerk32.cu): variant 9 of the chain segment.
+void realizeTiles32(const KArgs& a, const TileSet& S, bool refine, int tile0, int ntiles, cudaStream_t s);
+void rkTiles32(const KArgs& a, const TileSet& S, bool refine, cudaStream_t s);
 // Tile driver, FP64 (k_tile.cu, k_tilerk.cu, k_tileadapt.cu).
 void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s);
 void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s);

@@ -249,10 +249,10 @@ template <int YS> struct TileFSrc {  // M^-1 f: q and the given forces
 // 108-126) into the plane yt, element by element over the block's warps. Formed
 // in the bodies' loads instead, its five cases made up most of the kernel's
 // code, which then ran from beyond the instruction cache.
-template <class CF>
+template <class CF, class F>
 __device__ __forceinline__ void tileStageInput(const TileTables& TT, const TileCtx& c, const TileCol<CF::YS>& col, int ny,
-                                               bool run, int stage, double h, const double* y, const double* f0,
-                                               const double* fa, const double* fb, double* yt) {
+                                               bool run, int stage, double h, const double* y, const F* f0, const F* fa,
+                                               const F* fb, double* yt) {
     const int W = TT.W;
     auto all = [&](auto f) {
         if (run) {
@@ -264,10 +264,12 @@ __device__ __forceinline__ void tileStageInput(const TileTables& TT, const TileC
         }
     };
     if (stage == 0) all([&](int64_t e) { return y[e]; });
-    else if (stage == 1) all([&](int64_t e) { return y[e] + h * f0[e]; });                          // h/3 f0
-    else if (stage == 2) all([&](int64_t e) { return y[e] + h * (f0[e] + fa[e]); });                // h/6 (f0+f1)
-    else if (stage == 3) all([&](int64_t e) { return y[e] + h * (f0[e] + 3.0 * fa[e]); });          // h/8 (f0+3f2)
-    else all([&](int64_t e) { return y[e] + h * ((f0[e] - 3.0 * fa[e]) + 4.0 * fb[e]); });          // h/2 (f0-3f2+4f3)
+    else if (stage == 1) all([&](int64_t e) { return y[e] + h * double(f0[e]); });                          // h/3 f0
+    else if (stage == 2) all([&](int64_t e) { return y[e] + h * (double(f0[e]) + double(fa[e])); });                // h/6 (f0+f1)
+    else if (stage == 3) all([&](int64_t e) { return y[e] + h * (double(f0[e]) + 3.0 * double(fa[e])); });          // h/8 (f0+3f2)
+    else all([&](int64_t e) {                                                                       // h/2 (f0-3f2+4f3)
+        return y[e] + h * ((double(f0[e]) - 3.0 * double(fa[e])) + 4.0 * double(fb[e]));
+    });
     tileSync(W, c);
 }
 template <int YS> struct TileOut {

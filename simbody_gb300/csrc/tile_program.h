@@ -108,8 +108,29 @@ struct TileRows {
     std::vector<double> par;       // PR_COUNT per row
     std::vector<int32_t> ints;     // SI_COUNT per row, the parent's row in SI_PARENT
 
-    explicit TileRows(const sbg_topology_s& t) : nb(t.nb) {
+    explicit TileRows(const sbg_topology_s& t, bool fp32 = false) : nb(t.nb) {
         using namespace tile;
+        if (fp32) {
+            // the FP32 routines have two widths, and the chain driver's order in
+            // which children add to their parent: falling rows, tip to base
+            cls.resize(nb); parent.assign(t.parent.begin(), t.parent.end()); prevSib.assign(nb, -1);
+            height.assign(nb, 0); cost.resize(nb);
+            ints.assign((size_t)nb * SI_COUNT, 0);
+            for (int r = 0; r < nb; ++r) {
+                const bool six = ((t.info[r] >> 4) & 15) == 6;
+                cls[r] = six ? CL_FREE : CL_BALL;
+                gen |= six;
+                cost[r] = six ? 900 : 300;
+                int32_t* s = &ints[(size_t)r * SI_COUNT];
+                s[SI_Q] = t.qoff[r]; s[SI_U] = t.uoff[r]; s[SI_PARENT] = parent[r]; s[SI_INFO] = t.info[r]; s[SI_ROW] = r;
+                for (int k = 1; k < t.ccnt[r]; ++k) prevSib[t.clist[t.cbeg[r] + k]] = t.clist[t.cbeg[r] + k - 1];
+            }
+            for (int r = nb - 1; r >= 0; --r) {
+                height[r] += cost[r];
+                if (parent[r] >= 0) height[parent[r]] = std::max(height[parent[r]], height[r]);
+            }
+            return;
+        }
         cls.resize(nb); parent.resize(nb); prevSib.assign(nb, -1); height.assign(nb, 0); cost.resize(nb);
         par.assign((size_t)nb * PR_COUNT, 0.0);
         ints.assign((size_t)nb * SI_COUNT, 0);
@@ -397,6 +418,30 @@ struct TileProgram {
                 if (best == 0 || t < 0.97 * best) { best = t; TW = tw; W = w; }
             }
         }
+    }
+
+    // Warps per tile of the FP32 forms, whose tiles are bound by latency: the
+    // fewest steps, while the GPU holds the warps at once (8 an SM; at 128
+    // registers, 16 an SM, the spills cost more than the warps gave). Realize of
+    // random trees, us, 2 / 4 / 8 warps: 512 trees 355 / 259 / 258, 4,096 633 /
+    // 553 / 569, 16,384 935 / 1007 / 1582.
+    static int warps32(const std::vector<int>& topoAt, const std::vector<const TileRows*>& rows, int sms) {
+        const int n = (int)topoAt.size(), tiles = (n + 31) / 32;
+        int W = 1;
+        double best = 0;
+        for (int w : {1, 2, 4}) {
+            double steps = 0;
+            const int samples = std::min(tiles, 4);
+            for (int s = 0; s < samples; ++s) {
+                std::vector<const TileRows*> lanes;
+                const int p0 = (int)((int64_t)tiles * s / samples) * 32;
+                for (int p = p0; p < std::min(n, p0 + 32); ++p) lanes.push_back(rows[topoAt[p]]);
+                steps += double(TileSchedule(lanes, w).nsteps) / samples;
+            }
+            const double t = steps * std::max(1.0, double(tiles) * w / (8 * sms));
+            if (best == 0 || t < 0.95 * best) { best = t; W = w; }
+        }
+        return W;
     }
 
 private:

@@ -50,3 +50,28 @@ def test_shared_topology_in_any_tile(engine, n):
     b = Batch(topo, which)
     got, st = b.realize_acceleration_from(np.concatenate([own[k] for k in which]))
     assert (st == 0).all() and np.array_equal(got, np.concatenate([alone[k] for k in which]))
+
+
+def _with_variant(monkeypatch, w, precision, variant, run):
+    monkeypatch.setenv("SBG_VARIANT", str(variant))
+    b, y0 = engine_batch(w, precision)
+    b.set_state(y0)
+    out = run(b)
+    assert b.kernel_variant == variant
+    return out
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 70])
+@pytest.mark.parametrize("precision", ["mixed", "mixed_fast"])
+def test_fp32_tiles_match_the_one_thread_driver_bitwise(engine, monkeypatch, precision, n):
+    for config in (3, 4, 6, 8):
+        w = Workload(config, n)
+
+        def run(b):
+            d, st = b.realize_acceleration()
+            sr = b.rk_merson_fixed(w.h, 3)
+            y, t = b.get_state()
+            return d, st, sr, y, t
+
+        for a, c in zip(_with_variant(monkeypatch, w, precision, 7, run), _with_variant(monkeypatch, w, precision, 9, run)):
+            np.testing.assert_array_equal(a, c)
