@@ -145,6 +145,7 @@ struct sbg_batch_s {
     // batches; mixed ones once an integration has switched to FP64), and one
     // tile per instance (mixed batches)
     std::vector<sbg_topology_s*> topos;      // the topologies used, held
+    std::vector<int32_t> rowBase;            // per topology used, its first row in the body table
     std::vector<int32_t> topoOf;             // per instance, its index in topos
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
@@ -562,17 +563,13 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     const int sms = b->sms;
     std::vector<TileRows> store;
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
-    std::vector<int64_t> rowBase(b->topos.size(), 0);
-    std::vector<double> par;
     store.reserve(b->topos.size());
     TileProgram P;
     bool gen = false;
     for (size_t k = 0; k < b->topos.size(); ++k) {
         if (b->topos[k]->ncons > 0) continue;  // the loop-closure segment's
-        store.emplace_back(*b->topos[k]);
+        store.emplace_back(*b->topos[k], false);
         rows[k] = &store.back();
-        rowBase[k] = (int64_t)par.size() / PR_COUNT;
-        par.insert(par.end(), rows[k]->par.begin(), rows[k]->par.end());
         gen |= rows[k]->gen;
         P.pose |= rows[k]->pose;
     }
@@ -590,7 +587,7 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
         std::vector<TileDesc> per(b->ninst, TileDesc{});
         for (int i = 0; i < b->ninst; ++i) {
             if (b->topos[b->topoOf[i]]->ncons > 0) continue;
-            P.add(0, {b->topoOf[i]}, rows, rowBase);
+            P.add(0, {b->topoOf[i]}, rows, b->rowBase);
             per[i] = P.desc.back();
             per[i].rec0 = 0;
         }
@@ -606,7 +603,7 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
             for (int p = seg.first; p < seg.second; p += TW) {
                 std::vector<int> lanes;
                 for (int k = p; k < std::min(seg.second, p + TW); ++k) lanes.push_back(b->topoOf[b->order[k]]);
-                P.add(p, lanes, rows, rowBase);
+                P.add(p, lanes, rows, b->rowBase);
             }
     }
     out->ntiles = (int)P.desc.size();
@@ -626,24 +623,16 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     const int64_t nPar = (int64_t)P.parRow.size() * PR_COUNT;
     if ((rc = b->alloc(&p, std::max<int64_t>(nPar, 1) * sizeof(double), "tile parameters"))) return rc;
     out->tt.par = static_cast<double*>(p);
-    if (P.shared) {  // tables without lanes: the rows in slot order
-        std::vector<double> v(std::max<int64_t>(nPar, 1));
-        for (size_t k = 0; k < P.parRow.size(); ++k)
-            if (P.parRow[k] >= 0) std::copy_n(&par[(size_t)P.parRow[k] * PR_COUNT], PR_COUNT, &v[k * PR_COUNT]);
-        SBG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice), "tile parameters");
-    } else {
-        void *dRow = nullptr, *dPar = nullptr;
+    {
+        void* dRow = nullptr;
         cudaError_t e = cudaMalloc(&dRow, std::max<size_t>(P.parRow.size(), 1) * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMalloc(&dPar, par.size() * sizeof(double));
         if (e == cudaSuccess)
-            e = cudaMemcpy(dRow, P.parRow.data(), P.parRow.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(dPar, par.data(), par.size() * sizeof(double), cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(dRow, P.parRow.data(), P.parRow.size() * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream);
         if (e == cudaSuccess)
-            e = launchTilePar(out->tt, out->ntiles, static_cast<int32_t*>(dRow), static_cast<double*>(dPar),
-                              PR_COUNT, static_cast<double*>(p), b->stream);
+            e = launchTilePar(b->T, static_cast<int32_t*>(dRow), (int64_t)P.parRow.size(), P.shared ? 1 : P.ls,
+                              static_cast<double*>(p), b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         cudaFree(dRow);
-        cudaFree(dPar);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return cudaFail(e, "tile parameters");
@@ -665,7 +654,6 @@ static int buildTiles32(sbg_batch b) {
     using namespace tile;
     std::vector<TileRows> store;
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
-    const std::vector<int64_t> rowBase(b->topos.size(), 0);
     store.reserve(b->topos.size());
     std::vector<int> at;
     bool wide = false, six = false;
@@ -685,7 +673,7 @@ static int buildTiles32(sbg_batch b) {
     if (const char* v = std::getenv("SBG_TILE32")) P.W = std::max(1, std::min(8, std::atoi(v)));  // tuning override
     P.shared = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
     for (int p = 0; p < b->nChain; p += kTile)
-        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, rowBase);
+        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, b->rowBase);
     TileSet& S = b->tiles32;
     S.sms = b->sms;
     S.tt.W = P.W;
@@ -758,7 +746,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     // distinct topologies used, concatenated body tables
     std::vector<int> used(ntopo, -1);
     std::vector<int64_t> recTotal(ntopo, 0);
-    std::vector<int32_t> parent, info, qoff, uoff, srec, fbeg, fcnt, fkw, bidx, kbeg, kcnt;
+    std::vector<int32_t> parent, info, qoff, uoff, srec, fbeg, fcnt, fkw, bidx, row0, kbeg, kcnt;
     std::vector<double> par, fcoef, fq0, kpar;
     std::vector<int32_t> rowBase(ntopo, 0);
     for (int i = 0; i < ninst; ++i) {
@@ -775,6 +763,8 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         qoff.insert(qoff.end(), t->qoff.begin(), t->qoff.end());
         uoff.insert(uoff.end(), t->uoff.begin(), t->uoff.end());
         bidx.insert(bidx.end(), t->bodyOfRow.begin(), t->bodyOfRow.end());
+        row0.resize(parent.size(), rowBase[k]);
+        b->rowBase.push_back(rowBase[k]);
         const std::vector<int32_t> pr = paddedRecords(*t, nm, &recTotal[k]);
         srec.insert(srec.end(), pr.begin(), pr.end());
         for (int32_t fb : t->fbeg) fbeg.push_back(fb + fOff);
@@ -975,6 +965,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     if ((rc = b->upload(&T.uoff, uoff, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.srec, srec, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.bidx, bidx, "body table"))) return bail(rc);
+    if ((rc = b->upload(&T.row0, row0, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.fbeg, fbeg, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.fcnt, fcnt, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.par64, par, "parameters"))) return bail(rc);

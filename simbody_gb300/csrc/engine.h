@@ -120,6 +120,7 @@ struct DevTables {
     const int32_t* lcons;    // per constraint: local row of body 1, of body 2 (-1 = Ground)
     const double* lst;       // per constraint: station 1 (in body 1), station 2 (in body 2)
     const int32_t* lslot;    // per body row: slot index of a loop body (-1 = none): level-parallel layout
+    const int32_t* row0;     // per body row: first row of its topology
     const int32_t* bidx;     // per body row: index of the body in its system description (tree operators)
     // FP64 mirror of the scratch with the same element offsets (mixed batches
     // and the server's mixed lane; null otherwise): where the mixed form's

@@ -1,6 +1,7 @@
 // k_util.cu -- state packing kernels, quaternion normalization and the
 // precision dispatch of the launchers.
 #include "abi_device.cuh"
+#include "tile_core.cuh"
 
 #include <algorithm>
 
@@ -283,26 +284,68 @@ cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, do
     return cudaGetLastError();
 }
 
-// Parameters of the tiles' slots from the topologies' rows, across the lanes.
-__global__ void tileParKernel(const TileDesc* __restrict__ desc, int ntiles, int W, int ls,
-                              const int32_t* __restrict__ parRow, const double* __restrict__ rows, int count,
-                              double* __restrict__ par) {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const TileDesc d = desc[t];
-        const int64_t n = (int64_t)d.nsteps * W * ls, p0 = d.par0 / count;
-        for (int64_t k = threadIdx.x; k < n; k += blockDim.x) {
-            const int row = parRow[p0 + k];
-            if (row < 0) continue;
-            double* o = par + d.par0 + (k / ls) * count * ls + k % ls;
-            for (int f = 0; f < count; ++f) o[(int64_t)f * ls] = rows[(int64_t)row * count + f];
+// Parameters of the tiles' slots (tile_core.cuh) from the body table: entry k
+// is lane k % ls of slot k / ls, parRow[k] its row (-1: none).
+__global__ void __launch_bounds__(128) tileParKernel(const __grid_constant__ DevTables T,
+                                                     const int32_t* __restrict__ parRow, int64_t n, int ls,
+                                                     double* __restrict__ par) {
+    using namespace tile;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        const int row = parRow[k];
+        if (row < 0) continue;
+        double* o = par + (k / ls) * PR_COUNT * ls + k % ls;
+        auto put = [&](int f, double v) { o[(int64_t)f * ls] = v; };
+        const double* b = T.par64 + (int64_t)row * kParamStride;
+        const int parent = T.parent[row];
+        M3<double> RMB, PR = ident3<double>(), RPF;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            RMB.a[i] = b[22 + i];
+            RPF.a[i] = b[10 + i];
         }
+        const V3<double> com = mk3(b[1], b[2], b[3]), pMB = mk3(b[31], b[32], b[33]), pPF = mk3(b[19], b[20], b[21]);
+        V3<double> pP = z3<double>();
+        if (parent >= 0) {
+            const double* p = T.par64 + (int64_t)(T.row0[row] + parent) * kParamStride;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) PR.a[i] = p[22 + i];
+            pP = mk3(p[31], p[32], p[33]);
+        }
+        const double m = b[0];
+        const V3<double> c = mul(RMB, com) + pMB;
+        // unit inertia about the mass centre in body axes, turned to M axes, then about M's origin
+        const S3<double> G{b[4], b[5], b[6], b[7], b[8], b[9]};
+        const S3<double> J = m * (reexpress(RMB, G - pointMassUnit(com)) + pointMassUnit(c));
+        const M3<double> C = mul(PR, RPF);
+        const V3<double> d = mul(PR, pPF) + pP;
+        put(PR_M, m);
+        put(PR_MC, m * c.x); put(PR_MC + 1, m * c.y); put(PR_MC + 2, m * c.z);
+        put(PR_J, J.xx); put(PR_J + 1, J.yy); put(PR_J + 2, J.zz);
+        put(PR_J + 3, J.xy); put(PR_J + 4, J.xz); put(PR_J + 5, J.yz);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) put(PR_C + i, C.a[i]);
+        put(PR_D, d.x); put(PR_D + 1, d.y); put(PR_D + 2, d.z);
+        put(PR_PITCH, b[34]);
+        put(PR_PMB, pMB.x); put(PR_PMB + 1, pMB.y); put(PR_PMB + 2, pMB.z);
+        double K[6] = {}, S[6] = {}, B[6] = {};
+        for (int f = T.fbeg[row]; f < T.fbeg[row] + T.fcnt[row]; ++f) {
+            const int which = T.fkind_which[f] & 255;
+            const bool damper = (T.fkind_which[f] >> 8) != 0;
+            const double v = T.fcoef64[f], q0 = T.fq064[f];
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                if (j == which) {
+                    if (damper) B[j] += v;
+                    else { K[j] += v; S[j] += v * q0; }
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 6; ++j) { put(PR_K + j, K[j]); put(PR_S + j, S[j]); put(PR_B + j, B[j]); }
     }
 }
-cudaError_t launchTilePar(const TileTables& tt, int ntiles, const int32_t* parRow, const double* rows, int count,
-                          double* par, cudaStream_t s) {
-    if (ntiles <= 0) return cudaSuccess;
-    tileParKernel<<<ntiles < 4096 ? ntiles : 4096, 256, 0, s>>>(tt.desc, ntiles, tt.W, tt.shared ? 1 : tt.ls, parRow, rows,
-                                                                count, par);
+cudaError_t launchTilePar(const DevTables& T, const int32_t* parRow, int64_t n, int ls, double* par, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    tileParKernel<<<(int)std::min<int64_t>((n + 127) / 128, 16384), 128, 0, s>>>(T, parRow, n, ls, par);
     return cudaGetLastError();
 }
 

@@ -184,8 +184,7 @@ void minvLoopGroup(const KArgs& a, int threads, cudaStream_t s);
 cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
                              StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
                              cudaStream_t s);
-cudaError_t launchTilePar(const TileTables& tt, int ntiles, const int32_t* parRow, const double* rows, int count,
-                          double* par, cudaStream_t s);
+cudaError_t launchTilePar(const DevTables& T, const int32_t* parRow, int64_t n, int ls, double* par, cudaStream_t s);
 cudaError_t launchFillInt(int32_t* p, int n, int v, cudaStream_t s);
 // *out = instances with steps left in a one-step integration call
 cudaError_t launchCountUnfinished(int n, const int32_t* stepsLeft, const double* time, const int32_t* status,

@@ -100,166 +100,116 @@ inline void tileOrder(std::vector<int>& pos, const std::vector<std::array<float,
     pos.swap(out);
 }
 
-// The rows of one topology for the tile driver.
+// The rows of one topology for the tile driver. The FP32 routines have two
+// widths, and the chain driver's order in which children add to their parent
+// (falling rows, tip to base); the FP64 ones a class per mobilizer, and
+// siblings in the order of falling height.
 struct TileRows {
     int nb = 0;
     bool pose = false, gen = false;
-    std::vector<int> cls, parent, prevSib, height, cost;
-    std::vector<double> par;       // PR_COUNT per row
-    std::vector<int32_t> ints;     // SI_COUNT per row, the parent's row in SI_PARENT
+    const sbg_topology_s* t = nullptr;
+    std::vector<int16_t> cls;
+    std::vector<int> height, cost;
+    std::vector<int32_t> info;          // info words with the tile driver's flags
+    std::vector<int> waits;             // parent and sibling that come before, per row
+    std::vector<int> next0, next;       // rows that wait for row r: next[next0[r]] ...
 
-    explicit TileRows(const sbg_topology_s& t, bool fp32 = false) : nb(t.nb) {
+    TileRows(const sbg_topology_s& topo, bool fp32) : nb(topo.nb), t(&topo) {
         using namespace tile;
-        if (fp32) {
-            // the FP32 routines have two widths, and the chain driver's order in
-            // which children add to their parent: falling rows, tip to base
-            cls.resize(nb); parent.assign(t.parent.begin(), t.parent.end()); prevSib.assign(nb, -1);
-            height.assign(nb, 0); cost.resize(nb);
-            ints.assign((size_t)nb * SI_COUNT, 0);
-            for (int r = 0; r < nb; ++r) {
-                const bool six = ((t.info[r] >> 4) & 15) == 6;
-                cls[r] = six ? CL_FREE : CL_BALL;
-                gen |= six;
-                cost[r] = six ? 900 : 300;
-                int32_t* s = &ints[(size_t)r * SI_COUNT];
-                s[SI_Q] = t.qoff[r]; s[SI_U] = t.uoff[r]; s[SI_PARENT] = parent[r]; s[SI_INFO] = t.info[r]; s[SI_ROW] = r;
-                for (int k = 1; k < t.ccnt[r]; ++k) prevSib[t.clist[t.cbeg[r] + k]] = t.clist[t.cbeg[r] + k - 1];
-            }
-            for (int r = nb - 1; r >= 0; --r) {
-                height[r] += cost[r];
-                if (parent[r] >= 0) height[parent[r]] = std::max(height[parent[r]], height[r]);
-            }
-            return;
-        }
-        cls.resize(nb); parent.resize(nb); prevSib.assign(nb, -1); height.assign(nb, 0); cost.resize(nb);
-        par.assign((size_t)nb * PR_COUNT, 0.0);
-        ints.assign((size_t)nb * SI_COUNT, 0);
+        cls.resize(nb); height.assign(nb, 0); cost.resize(nb); info.resize(nb); waits.assign(nb, 0);
         for (int r = 0; r < nb; ++r) {
-            const double* b = &t.par[(size_t)r * kParamStride];
-            const int n = (t.info[r] >> 4) & 15;
-            cls[r] = tileClassOf(t.info[r]);
+            const int n = (t->info[r] >> 4) & 15, p = t->parent[r];
+            info[r] = t->info[r];
+            if (fp32) {
+                cls[r] = n == 6 ? CL_FREE : CL_BALL;
+                gen |= n == 6;
+                cost[r] = n == 6 ? 900 : 300;
+                continue;
+            }
+            cls[r] = (int16_t)tileClassOf(t->info[r]);
             gen |= cls[r] == CL_GEN;
             cost[r] = tileCost(cls[r], n);
-            parent[r] = t.parent[r];
-            double* o = &par[(size_t)r * PR_COUNT];
-            const double m = b[0], *RMB = b + 22, *pMB = b + 31;
-            double c[3], Gm[9], T[9];
-            for (int i = 0; i < 3; ++i) c[i] = RMB[3 * i] * b[1] + RMB[3 * i + 1] * b[2] + RMB[3 * i + 2] * b[3] + pMB[i];
-            // about the mass centre in body axes, turned to M axes, then about M's origin
-            const double com2 = b[1] * b[1] + b[2] * b[2] + b[3] * b[3];
-            const double G[9] = {b[4], b[7], b[8], b[7], b[5], b[9], b[8], b[9], b[6]};
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) Gm[3 * i + j] = G[3 * i + j] - ((i == j ? com2 : 0.0) - b[1 + i] * b[1 + j]);
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j)
-                    T[3 * i + j] = RMB[3 * i] * Gm[j] + RMB[3 * i + 1] * Gm[3 + j] + RMB[3 * i + 2] * Gm[6 + j];
-            const double c2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2];
-            auto J = [&](int i, int j) {
-                const double g = T[3 * i] * RMB[3 * j] + T[3 * i + 1] * RMB[3 * j + 1] + T[3 * i + 2] * RMB[3 * j + 2];
-                return m * (g + ((i == j ? c2 : 0.0) - c[i] * c[j]));
-            };
-            o[PR_M] = m;
-            for (int i = 0; i < 3; ++i) o[PR_MC + i] = m * c[i];
-            o[PR_J] = J(0, 0); o[PR_J + 1] = J(1, 1); o[PR_J + 2] = J(2, 2);
-            o[PR_J + 3] = J(0, 1); o[PR_J + 4] = J(0, 2); o[PR_J + 5] = J(1, 2);
-            static const double eye[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, nil[3] = {0, 0, 0};
-            const double* PR = parent[r] < 0 ? eye : &t.par[(size_t)parent[r] * kParamStride + 22];
-            const double* Pp = parent[r] < 0 ? nil : &t.par[(size_t)parent[r] * kParamStride + 31];
-            const double *RPF = b + 10, *pPF = b + 19;
-            bool ci = true;
-            for (int i = 0; i < 3; ++i) {
-                for (int j = 0; j < 3; ++j) {
-                    const double v = PR[3 * i] * RPF[j] + PR[3 * i + 1] * RPF[3 + j] + PR[3 * i + 2] * RPF[6 + j];
-                    o[PR_C + 3 * i + j] = v;
-                    ci &= v == (i == j ? 1.0 : 0.0);
-                }
-                o[PR_D + i] = PR[3 * i] * pPF[0] + PR[3 * i + 1] * pPF[1] + PR[3 * i + 2] * pPF[2] + Pp[i];
+            pose |= t->kcnt[r] > 0;
+            // C = R_MB of the parent times R_PF
+            bool ci = (t->info[r] & F_RPF_I) && (p < 0 || (t->info[p] & F_RMB_I));
+            if (!ci && p >= 0) {
+                const double *PR = &t->par[(size_t)p * kParamStride + 22], *RPF = &t->par[(size_t)r * kParamStride + 10];
+                ci = true;
+                for (int i = 0; i < 3; ++i)
+                    for (int j = 0; j < 3; ++j)
+                        ci &= PR[3 * i] * RPF[j] + PR[3 * i + 1] * RPF[3 + j] + PR[3 * i + 2] * RPF[6 + j] == (i == j);
             }
-            o[PR_PITCH] = b[34];
-            for (int i = 0; i < 3; ++i) o[PR_PMB + i] = pMB[i];
-            for (int k = t.fbeg[r]; k < t.fbeg[r] + t.fcnt[r]; ++k) {
-                const int j = t.fkw[k] & 255;
-                if ((t.fkw[k] >> 8) == 0) { o[PR_K + j] += t.fcoef[k]; o[PR_S + j] += t.fcoef[k] * t.fq0[k]; }
-                else o[PR_B + j] += t.fcoef[k];
-            }
-            int32_t* s = &ints[(size_t)r * SI_COUNT];
-            s[SI_Q] = t.qoff[r]; s[SI_U] = t.uoff[r]; s[SI_PARENT] = parent[r];
-            s[SI_INFO] = t.info[r] | (ci ? F_CI : 0) | (t.fcnt[r] == 0 ? F_FREELY : 0);
-            s[SI_ROW] = r; s[SI_KBEG] = t.kbeg[r]; s[SI_KCNT] = t.kcnt[r];
-            pose |= t.kcnt[r] > 0;
+            info[r] |= (ci ? F_CI : 0) | (t->fcnt[r] == 0 ? F_FREELY : 0);
         }
         for (int r = nb - 1; r >= 0; --r) {
-            height[r] += cost[r] + kTileStepCost;
-            if (parent[r] >= 0) height[parent[r]] = std::max(height[parent[r]], height[r]);
+            height[r] += cost[r] + (fp32 ? 0 : kTileStepCost);
+            if (t->parent[r] >= 0) height[t->parent[r]] = std::max(height[t->parent[r]], height[r]);
         }
-        // siblings in the order of falling height
+        // a body waits for its parent and for the sibling before it
+        std::vector<int> sib(nb, -1), kids;
         for (int r = 0; r < nb; ++r) {
-            std::vector<int> kids(t.clist.begin() + t.cbeg[r], t.clist.begin() + t.cbeg[r] + t.ccnt[r]);
-            std::stable_sort(kids.begin(), kids.end(), [&](int a, int b) { return height[a] > height[b]; });
-            for (size_t k = 1; k < kids.size(); ++k) prevSib[kids[k]] = kids[k - 1];
+            kids.assign(t->clist.begin() + t->cbeg[r], t->clist.begin() + t->cbeg[r] + t->ccnt[r]);
+            if (!fp32) std::stable_sort(kids.begin(), kids.end(), [&](int x, int y) { return height[x] > height[y]; });
+            for (size_t k = 1; k < kids.size(); ++k) sib[kids[k - 1]] = kids[k];
         }
+        next0.reserve(nb + 1);
+        next.reserve(2 * nb);
+        for (int r = 0; r < nb; ++r) {
+            next0.push_back((int)next.size());
+            next.insert(next.end(), t->clist.begin() + t->cbeg[r], t->clist.begin() + t->cbeg[r] + t->ccnt[r]);
+            if (sib[r] >= 0) next.push_back(sib[r]);
+        }
+        next0.push_back((int)next.size());
+        for (int k : next) ++waits[k];
     }
 };
 
 // Schedule of one tile: classes of (step, warp), and the row each lane takes
 // there (-1: none).
 struct TileSchedule {
-    int nsteps = 0;
+    int nsteps = 0, lanes = 0;
     std::vector<int32_t> cls;              // nsteps * W
-    std::vector<std::vector<int>> row;     // per slot, per lane
+    std::vector<int> row;                  // per slot and lane
     // FP64 instructions: length, step by step of the busiest sub-partition (a
     // block's warps take the SM's four in turn); load, of the busiest one in all
     int64_t length = 0, load = 0;
+    static constexpr double kCritical = 1.0;
 
-    TileSchedule(const std::vector<const TileRows*>& lanes, int W) {
+    TileSchedule(const std::vector<const TileRows*>& rows, int W) : lanes((int)rows.size()) {
         using namespace tile;
-        const int nl = (int)lanes.size();
-        struct Lane {
-            std::vector<int> ready;            // ready rows, in falling height
-            std::vector<int> waits;            // parent and sibling still to come, per row
-            std::vector<std::vector<int>> next;
-            int left;
-        };
-        std::vector<Lane> L(nl);
-        for (int l = 0; l < nl; ++l) {
-            const TileRows& t = *lanes[l];
-            L[l].waits.assign(t.nb, 0);
-            L[l].next.resize(t.nb);
-            L[l].left = t.nb;
-            for (int r = 0; r < t.nb; ++r) {
-                if (t.parent[r] >= 0) { ++L[l].waits[r]; L[l].next[t.parent[r]].push_back(r); }
-                if (t.prevSib[r] >= 0) { ++L[l].waits[r]; L[l].next[t.prevSib[r]].push_back(r); }
-            }
-            for (int r = 0; r < t.nb; ++r)
-                if (!L[l].waits[r]) L[l].ready.push_back(r);
-        }
+        const int nl = lanes;
+        std::vector<std::vector<int>> ready(nl), waits(nl), done(nl);
         int remaining = 0;
-        for (int l = 0; l < nl; ++l) remaining += L[l].left;
-        std::vector<std::vector<int>> done(nl);
-        std::vector<int> turn(W);                 // warps, the one with the least work so far first
-        std::vector<int64_t> sum(W, 0), sub(std::min(W, 4), 0);
+        for (int l = 0; l < nl; ++l) {
+            waits[l] = rows[l]->waits;
+            remaining += rows[l]->nb;
+            for (int r = 0; r < rows[l]->nb; ++r)
+                if (!waits[l][r]) ready[l].push_back(r);
+        }
+        std::vector<int> turn(W);  // warps, the one with the least work so far first
+        std::vector<int64_t> sum(W, 0), sub(std::min(W, 4), 0), stepSub, stepBody;
         for (int w = 0; w < W; ++w) turn[w] = w;
         while (remaining > 0) {
-            std::vector<int64_t> stepSub(sub.size(), 0), stepBody(sub.size(), 0);
+            stepSub.assign(sub.size(), 0);
+            stepBody.assign(sub.size(), 0);
             for (auto& d : done) d.clear();
             std::stable_sort(turn.begin(), turn.end(), [&](int a, int b) { return sum[a] < sum[b]; });
             cls.resize(cls.size() + W, -1);
-            row.resize(row.size() + W, std::vector<int>(nl, -1));
+            row.resize(row.size() + (size_t)W * nl, -1);
             for (int w : turn) {
                 const size_t slot = (size_t)nsteps * W + w;
                 // the class with the most work ready, weighted by how critical it is
                 double score[CL_COUNT] = {};
                 for (int l = 0; l < nl; ++l) {
-                    if (L[l].ready.empty()) continue;
-                    bool seen[CL_COUNT] = {};
-                    int top = 0;
-                    for (int r : L[l].ready) top = std::max(top, lanes[l]->height[r]);
-                    for (int r : L[l].ready) {
-                        const int c = lanes[l]->cls[r];
-                        if (seen[c]) continue;
-                        seen[c] = true;
-                        score[c] += 1.0 + kCritical * lanes[l]->height[r] / top;
+                    if (ready[l].empty()) continue;
+                    const TileRows& t = *rows[l];
+                    int most[CL_COUNT] = {}, top = 0;
+                    for (int r : ready[l]) {
+                        most[t.cls[r]] = std::max(most[t.cls[r]], t.height[r]);
+                        top = std::max(top, t.height[r]);
                     }
+                    for (int c = 0; c < CL_COUNT; ++c)
+                        if (most[c]) score[c] += 1.0 + kCritical * most[c] / top;
                 }
                 int best = -1;
                 for (int c = 0; c < CL_COUNT; ++c)
@@ -268,39 +218,40 @@ struct TileSchedule {
                 cls[slot] = best;
                 int stepCost = 0;
                 for (int l = 0; l < nl; ++l) {
-                    auto& rd = L[l].ready;
+                    const TileRows& t = *rows[l];
+                    auto& rd = ready[l];
                     int at = -1;
                     for (int k = 0; k < (int)rd.size(); ++k)
-                        if (lanes[l]->cls[rd[k]] == best &&
-                            (at < 0 || lanes[l]->height[rd[k]] > lanes[l]->height[rd[at]])) at = k;
+                        if (t.cls[rd[k]] == best && (at < 0 || t.height[rd[k]] > t.height[rd[at]])) at = k;
                     if (at < 0) continue;
                     const int r = rd[at];
                     rd.erase(rd.begin() + at);
-                    row[slot][l] = r;
+                    row[slot * nl + l] = r;
                     done[l].push_back(r);
                     --remaining;
-                    stepCost = std::max(stepCost, lanes[l]->cost[r]);
+                    stepCost = std::max(stepCost, t.cost[r]);
                 }
                 sum[w] += stepCost;
                 sub[w % 4] += stepCost;
                 stepSub[w % 4] += stepCost;
                 stepBody[w % 4] = std::max<int64_t>(stepBody[w % 4], stepCost + kTileBodyWait);
             }
-            for (int l = 0; l < nl; ++l)
+            for (int l = 0; l < nl; ++l) {
+                const TileRows& t = *rows[l];
                 for (int r : done[l])
-                    for (int k : L[l].next[r])
-                        if (--L[l].waits[k] == 0) L[l].ready.push_back(k);
+                    for (int k = t.next0[r]; k < t.next0[r + 1]; ++k)
+                        if (--waits[l][t.next[k]] == 0) ready[l].push_back(t.next[k]);
+            }
             length += std::max(*std::max_element(stepSub.begin(), stepSub.end()),
                                *std::max_element(stepBody.begin(), stepBody.end())) + kTileStepCost;
             ++nsteps;
         }
         load = *std::max_element(sub.begin(), sub.end()) + (int64_t)nsteps * kTileStepCost / 4;
     }
-    static constexpr double kCritical = 1.0;
 };
 
-// The tables of a batch's tiles on the host. Parameters are gathered on the
-// device from the topologies' rows (parRow: row per slot and lane, -1: none).
+// The tables of a batch's tiles on the host. Parameters are formed on the
+// device from the body table (parRow: its row per slot and lane, -1: none).
 struct TileProgram {
     int W = 1, rs = 0, rsTotal = 0;
     int ls = 32;           // lanes per tile
@@ -311,9 +262,9 @@ struct TileProgram {
     int64_t recElems = 0, maxTile = 0;  // record doubles of all tiles, of the largest
 
     // One tile over `topo` (topology per lane). rows: per topology, rowBase:
-    // its first row in the parameter rows.
+    // its first row in the body table.
     void add(int pos0, const std::vector<int>& topo, const std::vector<const TileRows*>& rows,
-             const std::vector<int64_t>& rowBase) {
+             const std::vector<int32_t>& rowBase) {
         using namespace tile;
         TileDesc d{};
         d.pos0 = pos0;
@@ -340,13 +291,16 @@ struct TileProgram {
             for (int l = 0; l < nl; ++l) {
                 const TileRows& t = *lanes[l];
                 slotOf.assign(t.nb, -1);
-                for (int64_t k = 0; k < nslots; ++k)
-                    if (s.row[k][l] >= 0) slotOf[s.row[k][l]] = (int)k;
-                for (int r = 0; r < t.nb; ++r) {
-                    int32_t* o = &slots[d.slot0 + ((int64_t)slotOf[r] * st + l) * SI_COUNT];
-                    std::copy_n(&t.ints[(size_t)r * SI_COUNT], SI_COUNT, o);
-                    o[SI_PARENT] = t.parent[r] < 0 ? -1 : slotOf[t.parent[r]];
-                    parRow[d.par0 / PR_COUNT + (int64_t)slotOf[r] * st + l] = (int32_t)(rowBase[topo[l]] + r);
+                for (int64_t k = 0; k < nslots; ++k) {
+                    const int r = s.row[k * nl + l];
+                    if (r < 0) continue;
+                    slotOf[r] = (int)k;  // a parent's slot comes before
+                    int32_t* o = &slots[d.slot0 + (k * st + l) * SI_COUNT];
+                    o[SI_Q] = t.t->qoff[r]; o[SI_U] = t.t->uoff[r];
+                    o[SI_PARENT] = t.t->parent[r] < 0 ? -1 : slotOf[t.t->parent[r]];
+                    o[SI_INFO] = t.info[r]; o[SI_ROW] = r;
+                    o[SI_KBEG] = t.t->kbeg[r]; o[SI_KCNT] = t.t->kcnt[r];
+                    parRow[d.par0 / PR_COUNT + k * st + l] = rowBase[topo[l]] + r;
                 }
             }
             // the lanes of a step agree on these flags
@@ -354,9 +308,9 @@ struct TileProgram {
                 int32_t* o = &slots[d.slot0 + k * st * SI_COUNT + SI_INFO];
                 int all = F_CI | F_FREELY;
                 for (int l = 0; l < nl; ++l)
-                    if (s.row[k][l] >= 0) all &= o[l * SI_COUNT];
+                    if (s.row[k * nl + l] >= 0) all &= o[l * SI_COUNT];
                 for (int l = 0; l < nl; ++l)
-                    if (s.row[k][l] >= 0) o[l * SI_COUNT] &= ~(F_CI | F_FREELY) | all;
+                    if (s.row[k * nl + l] >= 0) o[l * SI_COUNT] &= ~(F_CI | F_FREELY) | all;
             }
             if (shared) known[topo[0]] = d;
         }
