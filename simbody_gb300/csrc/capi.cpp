@@ -228,7 +228,7 @@ struct sbg_batch_s {
     }
 
     // Lanes per instance of the loop-closure segment, in blocks of one warp: as
-    // many as the widest level (4 to 32: the Gram takes three), fewer while the
+    // many as the widest level and the Gram's columns (4 to 32), fewer while the
     // segment has more warps than the GPU has sub-partitions, on which they
     // share the FP64 pipe; and as few instances per warp as fit beside one
     // another, whose multiplier solves run on one lane each and diverge.
@@ -236,7 +236,8 @@ struct sbg_batch_s {
         std::vector<int32_t> first, gs;
         const int64_t subs = 4 * sms;
         auto lanesOf = [&](int p) {
-            const int w = topos[topoOf[ord[p]]]->maxLevelWidth;
+            const sbg_topology_s* t = topos[topoOf[ord[p]]];
+            const int w = std::max(t->maxLevelWidth, 3 * t->ncons);
             int G = 4;
             while (G < 32 && G < w) G <<= 1;
             while (G > 4 && (int64_t)nLoop * G > 32 * subs) G >>= 1;
@@ -894,7 +895,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         const sbg_topology_s* t = topos[instTopo[i]];
         ybase[i] = yOff; ystride[i] = 1;
         yOff += t->nq + t->nu;
-        sstride[i] = rowsRecordWidth(*t, 3);
+        sstride[i] = rowsRecordWidth(*t, 3) + kLoopExt;
         sbase[i] = sOffLoop;
         sOffLoop += (t->nb + 2 * t->ncons) * sstride[i];
     }
@@ -958,6 +959,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     int rc = 0;
     DevTables& T = b->T;
     T.ninst = ninst;
+    T.loopExt = 1;
     std::vector<float> par32(par.begin(), par.end()), fcoef32(fcoef.begin(), fcoef.end()), fq032(fq0.begin(), fq0.end());
     if ((rc = b->upload(&T.parent, parent, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.info, info, "body table"))) return bail(rc);

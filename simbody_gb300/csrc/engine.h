@@ -75,6 +75,8 @@ enum : int {
 constexpr int kSlotA = 18, kSlotB = 24, kSlotF = 30, kSlotB3 = 36, kSlotF3 = 48, kSlotSize = 60;
 constexpr int kMaxLoopCons = 4;             // Ball constraints per instance
 constexpr int kMaxLoopEq = 3 * kMaxLoopCons;
+// A record's extension for Gram columns 3 to 11 (18 values each, loops_device.cuh).
+constexpr int kLoopExt = 18 * (kMaxLoopEq - 3);
 constexpr int F_MEMACC = F_MEMCHILD;
 
 // Warp tile of the shared-topology scratch layout.
@@ -121,6 +123,7 @@ struct DevTables {
     const double* lst;       // per constraint: station 1 (in body 1), station 2 (in body 2)
     const int32_t* lslot;    // per body row: slot index of a loop body (-1 = none): level-parallel layout
     const int32_t* row0;     // per body row: first row of its topology
+    int32_t loopExt;         // the loop-closure records (sstride wide) end in kLoopExt more values
     const int32_t* bidx;     // per body row: index of the body in its system description (tree operators)
     // FP64 mirror of the scratch with the same element offsets (mixed batches
     // and the server's mixed lane; null otherwise): where the mixed form's

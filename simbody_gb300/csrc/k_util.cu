@@ -224,12 +224,22 @@ static KArgs baseArgs(const DevTables& T, const LaunchPlan& P, const BatchBufs& 
     a.fbufLoop = B.fbufLoop; a.fplane = B.fplane; a.status = status; a.tiles32 = B.tiles32;
     return a;
 }
-// FP64: the tiles, then the loop-closure segment, on the main stream.
+// FP64: the tiles on the main stream and the loop-closure segment beside them
+// on the side stream.
 template <class FT, class FL>
-static cudaError_t tilesThenLoops(const LaunchPlan& P, const Streams& s, FT tiles, FL loops) {
+static cudaError_t tilesAndLoops(const LaunchPlan& P, const TileSet& S, const Streams& s, FT tiles, FL loops) {
+    if (P.nLoop == 0 || S.ntiles == 0) {
+        if (P.nLoop > 0) loops(s.main); else tiles(s.main);
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaEventRecord(s.fork, s.main);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s.side, s.fork, 0);
+    if (e != cudaSuccess) return e;
+    loops(s.side);
     tiles(s.main);
-    if (P.nLoop > 0) loops(s.main);
-    return cudaGetLastError();
+    e = cudaEventRecord(s.join, s.side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s.main, s.join, 0);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision, const double* y, double* ydot,
@@ -238,7 +248,7 @@ cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision
     a.y = y; a.ydot = ydot;
     auto loops = [&](cudaStream_t st) { realizeLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
-        return tilesThenLoops(P, s, [&](cudaStream_t st) { realizeTiles(a, *B.tiles, 0, B.tiles->ntiles, st); }, loops);
+        return tilesAndLoops(P, *B.tiles, s, [&](cudaStream_t st) { realizeTiles(a, *B.tiles, 0, B.tiles->ntiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
     const cudaError_t e = forkJoin(P, s, [&](cudaStream_t st) { realize32Chain(a, ref, st); }, loops,
                                    [&](cudaStream_t st) { realize32Group(a, ref, st); });
@@ -255,7 +265,7 @@ cudaError_t launchMInv(const DevTables& T, const LaunchPlan& P, int precision, c
     a.y = y; a.f = f; a.ydot = out;
     auto loops = [&](cudaStream_t st) { minvLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
-        return tilesThenLoops(P, s, [&](cudaStream_t st) { minvTiles(a, *B.tiles, st); }, loops);
+        return tilesAndLoops(P, *B.tiles, s, [&](cudaStream_t st) { minvTiles(a, *B.tiles, st); }, loops);
     return forkJoin(P, s, [&](cudaStream_t st) { minv32Chain(a, st); }, loops,
                     [&](cudaStream_t st) { minv32Group(a, st); });
 }
@@ -268,7 +278,7 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
     a.projectEveryStep = projectEveryStep;
     auto loops = [&](cudaStream_t st) { rkLoopGroup(a, 32, st); };
     if (precision == SBG_PRECISION_FP64)
-        return tilesThenLoops(P, s, [&](cudaStream_t st) { rkTiles(a, *B.tiles, st); }, loops);
+        return tilesAndLoops(P, *B.tiles, s, [&](cudaStream_t st) { rkTiles(a, *B.tiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
     return forkJoin(P, s, [&](cudaStream_t st) { rk32Chain(a, ref, st); }, loops,
                     [&](cudaStream_t st) { rk32Group(a, ref, st); });

@@ -65,6 +65,7 @@ struct LoopState {
     double* delta;
     int64_t base, stride;
     int body0, nb;
+    int ext;  // offset in a record of the fields of Gram columns 3 to 11 (0: none)
     // record of body row `row` (its local row), slot record of a loop body row
     __device__ __forceinline__ int rec(int row) const { return row - body0; }
     __device__ __forceinline__ int slot(int row) const { return nb + T.lslot[row]; }
@@ -76,7 +77,7 @@ __device__ __forceinline__ int loopRows(const DevTables& T, int inst) { return T
 __device__ __forceinline__ LoopState loopStateRows(const DevTables& T, int inst, double* scratch, double* y,
                                                    double* save, double* delta, int64_t base, int64_t stride) {
     return LoopState{T, inst, SC64{scratch, (int)T.sstride[inst], 1}, y, save, delta, base, stride,
-                     T.ibody[inst], T.inb[inst]};
+                     T.ibody[inst], T.inb[inst], T.loopExt ? (int)T.sstride[inst] - kLoopExt : 0};
 }
 
 // The weights of a sweep that applies none (kMInvSweep; see PosWeights).
@@ -398,6 +399,19 @@ __device__ __forceinline__ int slotB(int k) { return k == 0 ? kSlotB : kSlotB3 +
 __device__ __forceinline__ int recEpsK(int eEps, int k) { return k == 0 ? eEps : kRecA + 6 * (k - 1); }
 __device__ __forceinline__ int recZaccK(int k) { return k == 0 ? kRecZacc : (k == 1 ? kRecPc : kRecPacc); }
 
+// Fields of column k of up to twelve that run side by side: the three above,
+// then those of the extension (body record: eps, z accumulator, outward
+// acceleration; slot record: F, B).
+__device__ __forceinline__ int colF(const LoopState& L, int k) { return k < 3 ? slotF(k) : L.ext + 18 * (k - 3); }
+__device__ __forceinline__ int colB(const LoopState& L, int k) { return k < 3 ? slotB(k) : L.ext + 18 * (k - 3) + 6; }
+__device__ __forceinline__ int colEps(const LoopState& L, int eEps, int k) {
+    return k < 3 ? recEpsK(eEps, k) : L.ext + 18 * (k - 3);
+}
+__device__ __forceinline__ int colZacc(const LoopState& L, int k) {
+    return k < 3 ? recZaccK(k) : L.ext + 18 * (k - 3) + 6;
+}
+__device__ __forceinline__ int colOut(const LoopState& L, int k) { return k < 3 ? 6 * k : L.ext + 18 * (k - 3) + 12; }
+
 __device__ __forceinline__ void loopZeroAcc3(const LoopState& L) {
     const DevTables& T = L.T;
     const int body0 = T.ibody[L.inst], nb = T.inb[L.inst];
@@ -421,10 +435,11 @@ __device__ __forceinline__ void loopClearForces3(const LoopState& L) {
         }
     }
 }
-__device__ __forceinline__ void loopAddForceK(const SC64& S, int slot, V3d r, V3d F, int k) {
+__device__ __forceinline__ void loopAddForceK(const LoopState& L, int slot, V3d r, V3d F, int k) {
     if (slot < 0) return;
-    st3<double>(S, slot, slotF(k), ld3<double>(S, slot, slotF(k)) + cross(r, F));
-    st3<double>(S, slot, slotF(k) + 3, ld3<double>(S, slot, slotF(k) + 3) + F);
+    const int f = colF(L, k);
+    st3<double>(L.S, slot, f, ld3<double>(L.S, slot, f) + cross(r, F));
+    st3<double>(L.S, slot, f + 3, ld3<double>(L.S, slot, f + 3) + F);
 }
 
 template <int N, int KIND>
@@ -624,10 +639,10 @@ template <int N, int KIND>
 __device__ __forceinline__ void loopIn1(const LoopState& L, int row, int rec, int n, int info, int k, V3d& zw, V3d& zv) {
     const SC64& S = L.S;
     const int eDI = kRecH + 7 * N, eG = eDI + N * N, eEps = eG + 6 * N;
-    const int fE = recEpsK(eEps, k);
+    const int fE = colEps(L, eEps, k);
     if (info & F_LOOPBODY) {
         const int sl = L.slot(row);
-        const V3d tw = ld3<double>(S, sl, slotF(k)), tv = ld3<double>(S, sl, slotF(k) + 3);
+        const V3d tw = ld3<double>(S, sl, colF(L, k)), tv = ld3<double>(S, sl, colF(L, k) + 3);
         if (KIND == kMInvSweep) { zw = zw - tw; zv = zv - tv; }
         else { zw = zw + tw; zv = zv + tv; }
     }
@@ -657,7 +672,7 @@ template <int N, int KIND>
 __device__ __forceinline__ void loopOut1(const LoopState& L, int rec, int n, bool hasParent, int k, V3d& Aw, V3d& Av) {
     const SC64& S = L.S;
     const int eDI = kRecH + 7 * N, eG = eDI + N * N, eEps = eG + 6 * N;
-    const int fE = recEpsK(eEps, k);
+    const int fE = colEps(L, eEps, k);
     const V3d l = ld3<double>(S, rec, kRecL);
     const V3d Apw = hasParent ? Aw : z3<double>();
     const V3d Apv = hasParent ? Av + cross(Aw, l) : z3<double>();
@@ -696,13 +711,13 @@ __device__ __noinline__ void loopOut16(const LoopState& L, int rec, bool hasPare
     loopOut1<6, KIND>(L, rec, 6, hasParent, k, Aw, Av);
 }
 
-// Column k of the three-column sweep (loopSweep3), on one lane.
+// Column k of up to twelve (as column k % 3 of loopSweep3), on one lane.
 template <int NM, int KIND, class Wt>
 __device__ __forceinline__ void loopSweepColumn(const LoopState& L, const Wt& wt, int k) {
     const DevTables& T = L.T;
     const SC64& S = L.S;
     const int body0 = T.ibody[L.inst], nb = T.inb[L.inst];
-    const int fZ = recZaccK(k);
+    const int fZ = colZacc(L, k), fO = colOut(L, k), fB = colB(L, k);
     {
         V3d cw = z3<double>(), cv = z3<double>();
         bool have = false;
@@ -726,7 +741,7 @@ __device__ __forceinline__ void loopSweepColumn(const LoopState& L, const Wt& wt
             if (n == 6) loopIn16<KIND>(L, row, rec, info, k, zw, zv);
             else loopIn1<NM, KIND>(L, row, rec, n, info, k, zw, zv);
             if constexpr (KIND == kJacSweep) {
-                const int fE = recEpsK(recEps(recN(n, NM)), k);
+                const int fE = colEps(L, recEps(recN(n, NM)), k);
                 double g[6];
                 for (int j = 0; j < n; ++j) g[j] = S(rec, fE + j);
                 wt.apply(row, n, g);
@@ -757,16 +772,16 @@ __device__ __forceinline__ void loopSweepColumn(const LoopState& L, const Wt& wt
             V3d pw = aw, pv = av;
             if (hp && !(info & F_CARRY)) {
                 const int pr = L.rec(body0 + parent);
-                pw = ld3<double>(S, pr, 6 * k);
-                pv = ld3<double>(S, pr, 6 * k + 3);
+                pw = ld3<double>(S, pr, fO);
+                pv = ld3<double>(S, pr, fO + 3);
             }
             if (n == 6) loopOut16<KIND>(L, rec, hp, k, pw, pv);
             else loopOut1<NM, KIND>(L, rec, n, hp, k, pw, pv);
             if (info & F_LOOPBODY) {
-                st3<double>(S, L.slot(row), slotB(k), pw);
-                st3<double>(S, L.slot(row), slotB(k) + 3, pv);
+                st3<double>(S, L.slot(row), fB, pw);
+                st3<double>(S, L.slot(row), fB + 3, pv);
             }
-            if (info & F_MEMCHILD) { st3<double>(S, rec, 6 * k, pw); st3<double>(S, rec, 6 * k + 3, pv); }
+            if (info & F_MEMCHILD) { st3<double>(S, rec, fO, pw); st3<double>(S, rec, fO + 3, pv); }
             aw = pw;
             av = pv;
         }
@@ -914,8 +929,8 @@ __device__ __forceinline__ void loopGram(const LoopState& L, const Wt& wt, doubl
         for (int k = 0; k < 3; ++k) {
             V3d e = z3<double>();
             if (k == 0) e.x = 1.0; else if (k == 1) e.y = 1.0; else e.z = 1.0;
-            loopAddForceK(L.S, Gc.s2, Gc.r2, e, k);
-            loopAddForceK(L.S, Gc.s1, Gc.r1, -e, k);
+            loopAddForceK(L, Gc.s2, Gc.r2, e, k);
+            loopAddForceK(L, Gc.s1, Gc.r1, -e, k);
         }
         loopSweep3<NM, KIND>(L, wt);
         for (int i = 0; i < nc; ++i) {
@@ -930,58 +945,61 @@ __device__ __forceinline__ void loopGram(const LoopState& L, const Wt& wt, doubl
     }
 }
 
-// loopGram with lane k < 3 of the group (gl, mask: the lane's index in the
-// group and the group's lanes; absolute lane = the warp lane) sweeping
-// column k of every constraint. A is filled on the group's first lane only;
-// every lane of the group must call.
+// loopGram with the columns on lanes of the group (gl, mask: the lane's index
+// in the group and the group's lanes; absolute lane = the warp lane): all 3 m
+// of m constraints side by side where the records have their fields and the
+// group the lanes, else the three of one constraint after another. A column
+// sweeps the paths of every constraint in either case, so side by side they
+// take one sweep's FP64 instructions instead of m. A is filled on the group's
+// first lane only; every lane of the group must call.
 template <int NM, int KIND, class Wt>
 __device__ __forceinline__ void loopGramLanes(const LoopState& L, const Wt& wt, double* A, int gl, unsigned mask) {
     const DevTables& T = L.T;
     const int nc = T.incons[L.inst];
     const int base = (int)(threadIdx.x & 31) - gl;
-    const bool act = gl < 3;
-    const int k = act ? gl : 0;
+    const bool wide = L.ext > 0 && __popc(mask) >= 3 * nc;
+    const int lanes = wide ? 3 * nc : 3, rounds = wide ? 1 : nc;
+    const bool act = gl < lanes;
+    const int k = act ? gl : 0, axis = k % 3;
+    const int fF = colF(L, k), fB = colB(L, k), fZ = colZacc(L, k);
     if (act) {  // this column's accumulators held tree-pass values
         const int body0 = T.ibody[L.inst], nb = T.inb[L.inst];
         for (int lb = 0; lb < nb; ++lb) {
             const int row = body0 + lb;
             if ((T.info[row] & (F_MEMCHILD | F_LOOPPATH)) == (F_MEMCHILD | F_LOOPPATH)) {
-                st3<double>(L.S, L.rec(row), recZaccK(k), z3<double>());
-                st3<double>(L.S, L.rec(row), recZaccK(k) + 3, z3<double>());
+                st3<double>(L.S, L.rec(row), fZ, z3<double>());
+                st3<double>(L.S, L.rec(row), fZ + 3, z3<double>());
             }
         }
     }
-    for (int c = 0; c < nc; ++c) {
+    for (int round = 0; round < rounds; ++round) {
         if (act) {
             for (int c2 = 0; c2 < nc; ++c2) {
                 int s1, s2;
                 loopSlots(L, c2, s1, s2);
-                if (s1 >= 0) { st3<double>(L.S, s1, slotF(k), z3<double>()); st3<double>(L.S, s1, slotF(k) + 3, z3<double>()); }
-                if (s2 >= 0) { st3<double>(L.S, s2, slotF(k), z3<double>()); st3<double>(L.S, s2, slotF(k) + 3, z3<double>()); }
+                if (s1 >= 0) { st3<double>(L.S, s1, fF, z3<double>()); st3<double>(L.S, s1, fF + 3, z3<double>()); }
+                if (s2 >= 0) { st3<double>(L.S, s2, fF, z3<double>()); st3<double>(L.S, s2, fF + 3, z3<double>()); }
             }
-            const LoopGeom Gc = loopGeom(L, c);
+            const LoopGeom Gc = loopGeom(L, wide ? k / 3 : round);
             V3d e = z3<double>();
-            if (k == 0) e.x = 1.0; else if (k == 1) e.y = 1.0; else e.z = 1.0;
-            loopAddForceK(L.S, Gc.s2, Gc.r2, e, k);
-            loopAddForceK(L.S, Gc.s1, Gc.r1, -e, k);
+            if (axis == 0) e.x = 1.0; else if (axis == 1) e.y = 1.0; else e.z = 1.0;
+            loopAddForceK(L, Gc.s2, Gc.r2, e, k);
+            loopAddForceK(L, Gc.s1, Gc.r1, -e, k);
             loopSweepColumn<NM, KIND>(L, wt, k);
         }
         for (int i = 0; i < nc; ++i) {
             V3d d = z3<double>();
             if (act) {
                 const LoopGeom G = loopGeom(L, i);
-                d = slotPoint(L.S, G.s2, slotB(k), G.r2) - slotPoint(L.S, G.s1, slotB(k), G.r1);
+                d = slotPoint(L.S, G.s2, fB, G.r2) - slotPoint(L.S, G.s1, fB, G.r1);
             }
             const double v[3] = {d.x, d.y, d.z};
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const double v1 = __shfl_sync(mask, v[r], base + 1), v2 = __shfl_sync(mask, v[r], base + 2);
-                if (gl == 0) {
-                    A[(3 * i + r) * kMaxLoopEq + 3 * c] = v[r];
-                    A[(3 * i + r) * kMaxLoopEq + 3 * c + 1] = v1;
-                    A[(3 * i + r) * kMaxLoopEq + 3 * c + 2] = v2;
+            for (int r = 0; r < 3; ++r)
+                for (int col = 0; col < lanes; ++col) {
+                    const double x = __shfl_sync(mask, v[r], base + col);
+                    if (gl == 0) A[(3 * i + r) * kMaxLoopEq + 3 * round + col] = x;
                 }
-            }
         }
     }
 }
