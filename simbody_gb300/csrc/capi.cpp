@@ -559,18 +559,21 @@ int sbg_topology_default_state(sbg_topology t, double* y) {
 // The tile set of a batch's FP64 work: the chain and group segments' tiles, or
 // (single) one tile per instance that isn't in the loop-closure segment, with
 // records for every block of a launch that fills the GPU.
-static int buildTiles(sbg_batch b, bool single, TileSet* out) {
+static int buildTilesOf(sbg_batch b, bool single, TileSet* out) {
     using namespace tile;
     const int sms = b->sms;
-    std::vector<TileRows> store;
+    std::vector<TileRows> store(b->topos.size());
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
-    store.reserve(b->topos.size());
     TileProgram P;
     bool gen = false;
+    int64_t nRows = 0;
+    for (const sbg_topology_s* t : b->topos) nRows += t->nb;
+    tileParallel((int)b->topos.size(), nRows, [&](int k) {
+        if (b->topos[k]->ncons == 0) store[k] = TileRows(*b->topos[k], false);  // else the loop-closure segment's
+    });
     for (size_t k = 0; k < b->topos.size(); ++k) {
-        if (b->topos[k]->ncons > 0) continue;  // the loop-closure segment's
-        store.emplace_back(*b->topos[k], false);
-        rows[k] = &store.back();
+        if (b->topos[k]->ncons > 0) continue;
+        rows[k] = &store[k];
         gen |= rows[k]->gen;
         P.pose |= rows[k]->pose;
     }
@@ -585,27 +588,43 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
         P.W = 4;  // one warp per sub-partition
         P.ls = 1;
         P.shared = true;
+        std::vector<TileProgram::Lanes> kinds;  // one tile per topology stands for its instances
+        std::vector<int> kindOf(b->topos.size(), -1);
+        for (int i = 0; i < b->ninst; ++i) {
+            const int k = b->topoOf[i];
+            if (!rows[k] || kindOf[k] >= 0) continue;
+            kindOf[k] = (int)kinds.size();
+            kinds.push_back({0, {k}});
+        }
+        P.build(kinds, rows, b->rowBase);
         std::vector<TileDesc> per(b->ninst, TileDesc{});
         for (int i = 0; i < b->ninst; ++i) {
-            if (b->topos[b->topoOf[i]]->ncons > 0) continue;
-            P.add(0, {b->topoOf[i]}, rows, b->rowBase);
-            per[i] = P.desc.back();
+            if (kindOf[b->topoOf[i]] < 0) continue;
+            per[i] = P.desc[kindOf[b->topoOf[i]]];
             per[i].rec0 = 0;
         }
         P.desc.swap(per);
     } else {
         int TW = 32;
         TileProgram::shape(at, rows, sms, TW, P.W);
-        if (const char* v = std::getenv("SBG_TILE")) std::sscanf(v, "%d,%d", &TW, &P.W);  // tuning override
+        const bool same = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
+        if (const char* v = std::getenv("SBG_TILE")) {  // tuning override: lanes,warps
+            int tw = 0, w = 0;
+            if (std::sscanf(v, "%d,%d", &tw, &w) == 2 && (tw == 1 || tw == 32 || (tw == 8 && !same)) && w >= 1 && w <= 8) {
+                TW = tw;
+                P.W = w;
+            }
+        }
         b->tileWidth = TW;
         P.ls = TW;
-        P.shared = TW == 1 || std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
+        P.shared = TW == 1 || same;
+        std::vector<TileProgram::Lanes> tiles;
         for (const auto& seg : {std::make_pair(0, b->nChain), std::make_pair(b->nChain + b->nLoop, b->ninst)})
             for (int p = seg.first; p < seg.second; p += TW) {
-                std::vector<int> lanes;
-                for (int k = p; k < std::min(seg.second, p + TW); ++k) lanes.push_back(b->topoOf[b->order[k]]);
-                P.add(p, lanes, rows, b->rowBase);
+                tiles.push_back({p, {}});
+                for (int k = p; k < std::min(seg.second, p + TW); ++k) tiles.back().topo.push_back(b->topoOf[b->order[k]]);
             }
+        P.build(tiles, rows, b->rowBase);
     }
     out->ntiles = (int)P.desc.size();
     out->sms = sms;
@@ -651,7 +670,7 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
 }
 
 // The chain segment's tiles of the FP32 forms, where some tree branches.
-static int buildTiles32(sbg_batch b) {
+static int buildTiles32Of(sbg_batch b) {
     using namespace tile;
     std::vector<TileRows> store;
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
@@ -673,8 +692,10 @@ static int buildTiles32(sbg_batch b) {
     P.W = TileProgram::warps32(at, rows, b->sms);
     if (const char* v = std::getenv("SBG_TILE32")) P.W = std::max(1, std::min(8, std::atoi(v)));  // tuning override
     P.shared = std::all_of(at.begin(), at.end(), [&](int k) { return k == at[0]; });
+    std::vector<TileProgram::Lanes> tiles;
     for (int p = 0; p < b->nChain; p += kTile)
-        P.add(p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile)), rows, b->rowBase);
+        tiles.push_back({p, std::vector<int>(at.begin() + p, at.begin() + std::min(b->nChain, p + kTile))});
+    P.build(tiles, rows, b->rowBase);
     TileSet& S = b->tiles32;
     S.sms = b->sms;
     S.tt.W = P.W;
@@ -692,6 +713,27 @@ static int buildTiles32(sbg_batch b) {
     S.yt = static_cast<double*>(p);
     S.ntiles = (int)P.desc.size();
     return SBG_OK;
+}
+
+// Also called when a batch is in use (tree operators and FP64 steps of a mixed
+// one): no memory for the tables is a status there, not an exception, and
+// leaves the batch without the tiles, which the next call tries to build again.
+static int buildTiles(sbg_batch b, bool single, TileSet* out) {
+    try {
+        TileSet S{};
+        const int rc = buildTilesOf(b, single, &S);
+        if (rc == SBG_OK) *out = S;
+        return rc;
+    } catch (const std::exception& e) {
+        return fail(SBG_ERR_NOMEM, std::string("tile tables: ") + e.what());
+    }
+}
+static int buildTiles32(sbg_batch b) {
+    try {
+        return buildTiles32Of(b);
+    } catch (const std::exception& e) {
+        return fail(SBG_ERR_NOMEM, std::string("tile tables: ") + e.what());
+    }
 }
 
 extern "C" {
@@ -1290,11 +1332,18 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
                            b->ninst >= nchunks * kTile;
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     if (!pipelined) {
-        if (int rc = uploadState(b, nullptr, y)) return rc;
-        b->stateSet = true;
-        b->integrating = false;
-        if (int rc = sbg_realize_acceleration_async(b)) return rc;
-        return sbg_batch_get_ydot(b, ydot, status);  // waits for the upload too
+        int rc = uploadState(b, nullptr, y);
+        if (!rc) {
+            b->stateSet = true;
+            b->integrating = false;
+            rc = sbg_realize_acceleration_async(b);
+        }
+        if (!rc) rc = sbg_batch_get_ydot(b, ydot, status);  // waits for the upload too
+        if (rc) {  // the caller's buffers are not in use after the return
+            cudaStreamSynchronize(b->stream);
+            cudaGetLastError();
+        }
+        return rc;
     }
     const size_t bytes = b->nyTotal * sizeof(double);
     double* src = static_cast<double*>(b->hostSide(y, bytes));

@@ -75,3 +75,18 @@ def test_fp32_tiles_match_the_one_thread_driver_bitwise(engine, monkeypatch, pre
 
         for a, c in zip(_with_variant(monkeypatch, w, precision, 7, run), _with_variant(monkeypatch, w, precision, 9, run)):
             np.testing.assert_array_equal(a, c)
+
+
+def test_no_budget_for_the_operators_tiles_is_an_error_each_time(engine):
+    # a mixed batch builds the FP64 tiles at its first tree operator; the budget is what the batch itself takes
+    w = Workload(3, 33)
+    topo = [Topology(w.systems[k], keepalive=w) for k in range(w.nsys)]
+    need = Batch(topo, w.instance_system, precision="mixed").device_bytes
+    b = Batch(topo, w.instance_system, precision="mixed", device_budget_bytes=need)
+    b.set_state(w.y0)
+    ydot, st = b.realize_acceleration()
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="budget"):
+            b.multiply_by_m(np.ones(b.u_offsets[-1]))
+    again, st2 = b.realize_acceleration()
+    assert (st == 0).all() and np.array_equal(ydot, again) and np.array_equal(st, st2)
