@@ -30,7 +30,7 @@ CU_UNITS = ["k_r32c.cu", "k_r32cr.cu", "k_r32s.cu", "k_r32g.cu", "k_rk64.cu", "k
 HOST_UNITS = ["capi.cpp"]
 HEADERS = ["abi_device.cuh", "loops_device.cuh", "spatial.cuh", "engine.h", "kernels.h", "topology_internal.h",
            "serve_sched.h", "ops_device.cuh", "rk32c_launch.cuh",
-           "r32c_launch.cuh", "tile_core.cuh", "tile_device.cuh", "tilerk_device.cuh", "tile32_device.cuh", "tile_program.h", "steps_device.cuh"]
+           "r32c_launch.cuh", "tile_core.cuh", "tile_device.cuh", "tilerk_device.cuh", "tile32_device.cuh", "stage_device.cuh", "tile_program.h", "steps_device.cuh"]
 
 
 def _nvcc() -> str:

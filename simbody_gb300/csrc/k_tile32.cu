@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
     const TileCtx c = tileCtx<CF>(T, TT, id, nullptr);
     const YSrc src{y, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
     YdOut out{ydot, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
-    int st = tileRhs32<CF, NM, REF>(T, TT, c, recs, src, out, true);
+    int st = tileRhs32<CF, NM, REF>(T, TT, c, recs, tileStage<NM>(), src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
     st = tileReduce<0>(TT, c, sh, nullptr, st);
     if constexpr (REF) st |= tileIll(T, TT, c, mx, out);
@@ -28,12 +28,13 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
 template <int NM, bool REF> void go(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s) {
     const TileLaunch L(S, ntiles);
     float* recs = reinterpret_cast<float*>(S.recs);
-    if (S.tt.shared)
-        realizeTile32Kernel<TileCfg<32, true, 0>, NM, REF><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, tile0, ntiles, a.y, a.ydot,
-                                                                                     recs, a.status);
-    else
-        realizeTile32Kernel<TileCfg<32, false, 0>, NM, REF><<<L.grid, L.block, 0, s>>>(*a.T, S.tt, tile0, ntiles, a.y,
-                                                                                      a.ydot, recs, a.status);
+    auto launch = [&](auto cf) {
+        auto* const kernel = realizeTile32Kernel<decltype(cf), NM, REF>;
+        kernel<<<L.grid, L.block, tileStageBytes<NM>(kernel, L.block), s>>>(*a.T, S.tt, tile0, ntiles, a.y, a.ydot, recs,
+                                                                            a.status);
+    };
+    if (S.tt.shared) launch(TileCfg<32, true, 0>());
+    else launch(TileCfg<32, false, 0>());
 }
 
 }  // namespace

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
             tileStageInput<CF>(TT, c, col, nq + nu, going, stg, cc, y, f0, stg >= 3 ? fB : fA, fC, yt);
             const YSrc src{yt, col.base, col.stride, nq};
             FOut<float> out{stg == 0 ? f0 : stg == 2 ? fB : stg == 3 ? fC : fA, col.base, col.stride, nq};
-            bits |= tileRhs32<CF, NM, REF>(T, TT, c, recs, src, out, going);
+            bits |= tileRhs32<CF, NM, REF>(T, TT, c, recs, tileStage<NM>(), src, out, going);
             if (!out.finite) bits |= SBG_INST_NONFINITE;
             if constexpr (REF) ill |= tileIll(T, TT, c, mx, out);
         }
@@ -141,14 +141,14 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
 template <int NM, bool REF> void go(const KArgs& a, const TileSet& S, cudaStream_t s) {
     const TileLaunch L(S, S.ntiles);
     float *fb = static_cast<float*>(a.fbuf), *recs = reinterpret_cast<float*>(S.recs);
-    if (S.tt.shared)
-        rkTile32Kernel<TileCfg<32, true, 0>, NM, REF><<<L.grid, L.block, 0, s>>>(
+    auto launch = [&](auto cf) {
+        auto* const kernel = rkTile32Kernel<decltype(cf), NM, REF>;
+        kernel<<<L.grid, L.block, tileStageBytes<NM>(kernel, L.block), s>>>(
             *a.T, S.tt, S.ntiles, recs, a.ystate, S.yt, a.time, fb, a.fplane, a.status, a.h, a.step, a.accuracy, a.consTol,
             a.projectEveryStep);
-    else
-        rkTile32Kernel<TileCfg<32, false, 0>, NM, REF><<<L.grid, L.block, 0, s>>>(
-            *a.T, S.tt, S.ntiles, recs, a.ystate, S.yt, a.time, fb, a.fplane, a.status, a.h, a.step, a.accuracy, a.consTol,
-            a.projectEveryStep);
+    };
+    if (S.tt.shared) launch(TileCfg<32, true, 0>());
+    else launch(TileCfg<32, false, 0>());
 }
 
 }  // namespace
