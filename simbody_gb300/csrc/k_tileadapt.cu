@@ -59,7 +59,10 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
     rkAdaptiveTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT,
                          int ntiles, double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
                          int32_t* __restrict__ status, const __grid_constant__ AdaptCtl ac) {
+    // One array per type: the block's tiles each keep to their own part of an
+    // array and do not wait for one another.
     __shared__ TileShare<5> sh;
+    __shared__ TileShare<0> shFin;
     const int id = tileId(TT, 0, ntiles);
     if (id < 0) return;
     const TileCtx c = tileCtx<CF>(T, TT, id, recs);
@@ -217,8 +220,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                     if (!tile::finiteBits(y1v)) fin |= SBG_INST_NONFINITE;
                 }
             });
-        double none[1];
-        fin = tileReduce<0>(TT, c, reinterpret_cast<TileShare<0>&>(sh), none, fin);
+        fin = tileReduce<0>(TT, c, shFin, nullptr, fin);
         if (take) {
             st |= fin;
             tc = t1;
