@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
     TileOut<CF::YS> out(src.c, ydot);
     int st = tileRhs<CF, false>(T, TT, c, src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
-    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    st = tileReduce(TT, c, sh, st);
     if (c.on && c.w == 0) status[c.inst] = st;
 }
 
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
     TileUOut<CF::YS> out(src.c, o);
     int st = tileRhs<CF, true>(T, TT, c, src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
-    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    st = tileReduce(TT, c, sh, st);
     if (c.on && c.w == 0) status[c.inst] = st;
 }
 
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
             TileOut<0> out(src.c, ydot);
             int st = tileRhs<TileOne, false>(T, TT, c, src, out, true);
             if (!out.finite) st |= SBG_INST_NONFINITE;
-            st = tileReduce<0>(TT, c, sh, nullptr, st);
+            st = tileReduce(TT, c, sh, st);
             if (c.on && c.w == 0) {
                 status[c.inst] = st;
                 atomicAdd(T.fallbacks, 1ULL);

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
     YdOut out{ydot, T.ybase[c.inst], T.ystride[c.inst], T.inq[c.inst]};
     int st = tileRhs32<CF, NM, REF>(T, TT, c, recs, tileStage<NM>(), src, out, true);
     if (!out.finite) st |= SBG_INST_NONFINITE;
-    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    st = tileReduce(TT, c, sh, st);
     if constexpr (REF) st |= tileIll(T, TT, c, mx, out);
     if (c.on && c.w == 0) status[c.inst] = st;
 }

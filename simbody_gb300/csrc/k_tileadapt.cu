@@ -59,10 +59,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
     rkAdaptiveTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT,
                          int ntiles, double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
                          int32_t* __restrict__ status, const __grid_constant__ AdaptCtl ac) {
-    // One array per type: the block's tiles each keep to their own part of an
-    // array and do not wait for one another.
     __shared__ TileShare<5> sh;
-    __shared__ TileShare<0> shFin;
     const int id = tileId(TT, 0, ntiles);
     if (id < 0) return;
     const TileCtx c = tileCtx<CF>(T, TT, id, recs);
@@ -119,10 +116,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
             return y0 + h6 * ((a0 + 4.0 * aC) + aA);
         };
         // error norm and quaternion errors of y1, y untouched
-        double v[5] = {0, 0, 0, 0, 0};  // sq, su, squat, nquat, sq after the projection
         tileBodies<CF>(TT, c, going, [&](const tile::SlotRow& r) {
                 const int nqb = slotQ(r.info), n = (r.info >> 4) & 15;
-                double q1[4], dq[4], extra = 0;
+                double q1[4], dq[4], sq = 0, sqP = 0, extra = 0, su = 0;
 #pragma unroll
                 for (int j = 0; j < 7; ++j)
                     if (j < nqb) {
@@ -133,10 +129,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                         if (j >= 4 || !(r.info & F_QUAT)) extra += dj * dj;
                     }
                 if (r.info & F_QUAT) {
-                    v[0] += tileQuatErrSq(q1, dq);
+                    sq = tileQuatErrSq(q1, dq);
                     const double len = sqrt(q1[0] * q1[0] + q1[1] * q1[1] + q1[2] * q1[2] + q1[3] * q1[3]);
-                    v[2] += (len - 1) * (len - 1);
-                    v[3] += 1;
+                    yt[col.at(r.qo + 1)] = (len - 1) * (len - 1);
                     // the same after normalization, the radial part of dq removed
                     double qn[4], dqn[4];
 #pragma unroll
@@ -144,10 +139,8 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                     const double d = dq[0] * qn[0] + dq[1] * qn[1] + dq[2] * qn[2] + dq[3] * qn[3];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) dqn[k] = dq[k] - d * qn[k];
-                    v[4] += tileQuatErrSq(qn, dqn);
+                    sqP = tileQuatErrSq(qn, dqn);
                 }
-                v[0] += extra;
-                v[4] += extra;
                 for (int j = 0; j < n; ++j) {
                     const int64_t e = col.atU(r.uo + j);
                     double ysv;
@@ -155,10 +148,17 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                     const double vi = fabs(y[e]);
                     double d = 0.2 * fabs(y1v - ysv);
                     if (vi > 1) d = d / vi;  // calcRelativeScaling, frozen at step start
-                    v[1] += d * d;
+                    su += d * d;
+                }
+                if (n > 0) {  // tileSums
+                    yt[col.at(r.qo)] = sq + extra;
+                    if (r.info & F_QUAT) yt[col.at(r.qo + 2)] = sqP + extra;
+                    yt[col.atU(r.uo)] = su;
                 }
             });
-        bits = tileReduce<5>(TT, c, sh, v, bits);
+        bits = tileReduce(TT, c, sh, bits);
+        double v[5];  // sq, su, squat, nquat, sq after the projection
+        tileSums(T, TT, c, sh, col, yt, going, v);
         bool take = false, proj = false;
         if (going) {
             st |= bits;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                     if (!tile::finiteBits(y1v)) fin |= SBG_INST_NONFINITE;
                 }
             });
-        fin = tileReduce<0>(TT, c, shFin, nullptr, fin);
+        fin = tileReduce(TT, c, sh, fin);
         if (take) {
             st |= fin;
             tc = t1;

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
             }
         });
     int st = finite ? 0 : SBG_INST_NONFINITE;
-    st = tileReduce<0>(TT, c, sh, nullptr, st);
+    st = tileReduce(TT, c, sh, st);
     if (c.on && c.w == 0) status[c.inst] = st;
 }
 

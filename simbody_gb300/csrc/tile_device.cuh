@@ -193,32 +193,70 @@ __device__ __forceinline__ void tileBodies(const TileTables& TT, const TileCtx& 
     }
 }
 
-// Per-lane sums and status bits over the block's warps, the same on every
-// warp (warps in order).
+// Per-lane status bits over the tile's warps, the same on every warp.
 constexpr int kTileMaxWarps = 8;
 template <int N> struct TileShare {
-    double v[N > 0 ? N : 1][kTileMaxWarps][32];
+    double v[N > 0 ? N : 1][kTileMaxWarps][32];  // tileSums: per sum, tile of the block and lane
     int bits[kTileMaxWarps][32];
 };
 template <int N>
-__device__ __forceinline__ int tileReduce(const TileTables& TT, const TileCtx& c, TileShare<N>& sh, double* v, int bits) {
+__device__ __forceinline__ int tileReduce(const TileTables& TT, const TileCtx& c, TileShare<N>& sh, int bits) {
     if (TT.W == 1) return bits;
-#pragma unroll
-    for (int k = 0; k < N; ++k) sh.v[k][c.sub * TT.W + c.w][c.lane] = v[k];
     sh.bits[c.sub * TT.W + c.w][c.lane] = bits;
     tileSync(TT.W, c);
     int b = 0;
-    double s[N > 0 ? N : 1] = {};
-    for (int w = 0; w < TT.W; ++w) {
-        const int i = c.sub * TT.W + w;
-#pragma unroll
-        for (int k = 0; k < N; ++k) s[k] = w == 0 ? sh.v[k][i][c.lane] : s[k] + sh.v[k][i][c.lane];
-        b |= sh.bits[i][c.lane];
-    }
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = s[k];
-    tileSync(TT.W, c);  // the arrays may be written again
+    for (int w = 0; w < TT.W; ++w) b |= sh.bits[c.sub * TT.W + w][c.lane];
+    tileSync(TT.W, c);  // the array may be written again
     return b;
+}
+
+// Sums over an instance's bodies of the error norms and projection gates, in
+// the order of its rows whatever the tile's schedule: added up by the warps
+// that the schedule deals the bodies to, an instance's step sizes would depend
+// on the other instances of its tile. Each body has left its parts in the
+// column plane `part` (tileReduce after it makes them visible to every warp): at
+// its first u slot the u error; at its first q slot the q error, and for a
+// quaternion at the next two the error of its length and the q error after
+// normalization. v: q error, u error, length errors, number of quaternions, q
+// error after normalization (N = 5). A warp takes every W-th sum: all of them
+// on one warp are 4 FP64 additions and as many loads a body, about 5 us a step of
+// 30 bodies.
+template <int N, class Col>
+__device__ __forceinline__ void tileSums(const DevTables& T, const TileTables& TT, const TileCtx& c, TileShare<N>& sh,
+                                         const Col& col, const double* part, bool run, double* v) {
+    const int body0 = T.ibody[c.inst], nb = run ? T.inb[c.inst] : 0;
+    // f(info, q slot, u slot) of the rows with mobilities
+    auto sum = [&](auto f) {
+        double s = 0;
+#pragma unroll 4
+        for (int r = body0; r < body0 + nb; ++r) {
+            const int info = T.info[r];
+            if ((info >> 4) & 15) s += f(info, T.qoff[r], T.uoff[r]);
+        }
+        return s;
+    };
+    auto one = [&](int k) -> double {
+        if (k == 0) return sum([&](int, int q, int) { return part[col.at(q)]; });
+        if (k == 1) return sum([&](int, int, int u) { return part[col.atU(u)]; });
+        if (k == 2) return sum([&](int info, int q, int) { return info & F_QUAT ? part[col.at(q + 1)] : 0.0; });
+        if (k == 3) {
+            int n = 0;
+            for (int r = body0; r < body0 + nb; ++r) n += (T.info[r] & F_QUAT) != 0;
+            return n;
+        }
+        return sum([&](int info, int q, int) { return part[col.at(info & F_QUAT ? q + 2 : q)]; });
+    };
+    const int W = TT.W;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        if (W == 1) v[k] = one(k);
+        else if (k % W == c.w) sh.v[k][c.sub][c.lane] = one(k);
+    }
+    if (W == 1) return;
+    tileSync(W, c);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = sh.v[k][c.sub][c.lane];
+    tileSync(W, c);  // the arrays and the plane may be written again
 }
 
 // ----------------------------------------------------------- sources, sinks

@@ -63,10 +63,9 @@ __device__ __forceinline__ void rkTile(const DevTables& T, const TileTables& TT,
         // y1 = y0 + h/6 (f0 + 4 f3 + f4); yerr = 0.2 |y1 - ysave|; error norm
         // (RungeKuttaMersonIntegrator.cpp:124-139, IntegratorRep.h:454-523)
         const double h6 = hs / 6, h2 = hs / 2;
-        double v[4] = {0, 0, 0, 0};  // sq, su, squat, nquat
         tileBodies<CF>(TT, c, going, [&](const tile::SlotRow& r) {
                 const int nqb = slotQ(r.info), n = (r.info >> 4) & 15;
-                double q1[4], dq[4], extra = 0;
+                double q1[4], dq[4], sq = 0, extra = 0, su = 0;
 #pragma unroll
                 for (int j = 0; j < 7; ++j)
                     if (j < nqb) {
@@ -81,12 +80,10 @@ __device__ __forceinline__ void rkTile(const DevTables& T, const TileTables& TT,
                         if (j >= 4 || !(r.info & F_QUAT)) extra += dj * dj;
                     }
                 if (r.info & F_QUAT) {
-                    v[0] += tileQuatErrSq(q1, dq);
+                    sq = tileQuatErrSq(q1, dq);
                     const double len = sqrt(q1[0] * q1[0] + q1[1] * q1[1] + q1[2] * q1[2] + q1[3] * q1[3]);
-                    v[2] += (len - 1) * (len - 1);
-                    v[3] += 1;
+                    yt[col.at(r.qo + 1)] = (len - 1) * (len - 1);
                 }
-                v[0] += extra;
                 for (int j = 0; j < n; ++j) {
                     const int64_t e = col.atU(r.uo + j);
                     const double y0 = y[e], a0 = f0[e], aB = fB[e], aC = fC[e], aA = fA[e];
@@ -95,12 +92,18 @@ __device__ __forceinline__ void rkTile(const DevTables& T, const TileTables& TT,
                     const double vi = fabs(y0);
                     double d = 0.2 * fabs(y1v - ys);
                     if (vi > 1) d = d / vi;  // calcRelativeScaling, frozen at step start
-                    v[1] += d * d;
+                    su += d * d;
                     y[e] = y1v;
                     if (!tile::finiteBits(y1v)) bits |= SBG_INST_NONFINITE;
                 }
+                if (n > 0) {  // tileSums
+                    yt[col.at(r.qo)] = sq + extra;
+                    yt[col.atU(r.uo)] = su;
+                }
             });
-        bits = tileReduce<4>(TT, c, sh, v, bits);
+        bits = tileReduce(TT, c, sh, bits);
+        double v[4];  // sq, su, squat, nquat
+        tileSums(T, TT, c, sh, col, yt, going, v);
         bool renorm = false;
         if (going) {
             st |= bits;

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from simbody_gb300 import Batch, Topology, Workload
+from simbody_gb300 import Batch, Topology, Workload, engine_batch
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +83,28 @@ def test_error_controlled_tiles_that_share_a_block(engine, monkeypatch, tree, wa
     ry = ry.reshape(len(sample), -1)
     # 1e-10: the tolerance of fixed and error-controlled steps against the oracle
     assert (np.linalg.norm(yo[sample] - ry, axis=1) <= 1e-10 * np.linalg.norm(ry, axis=1)).all()
+
+
+@pytest.mark.parametrize("config", [3, 6, 7, 8])
+def test_steps_do_not_depend_on_the_other_instances(engine, config):
+    """The error norms and projection gates are sums over an instance's bodies
+    in its own order: alone, among others and with other neighbours it takes
+    the same steps to the last bit."""
+    w = Workload(config, 96)
+
+    def run(idx):
+        b, y0 = engine_batch(w, "fp64", instances=idx)
+        b.set_state(y0)
+        _, stats = b.rk_merson_adaptive(0.03, accuracy=1e-4)
+        ya, ta = b.get_state()
+        b.set_state(y0)
+        b.rk_merson_fixed(w.h, 3)
+        yf, _ = b.get_state()
+        cut = [slice(b.y_offsets[k], b.y_offsets[k + 1]) for k in range(len(idx))]
+        return {i: (stats[k], ta[k], ya[cut[k]], yf[cut[k]]) for k, i in enumerate(idx)}
+
+    among = run(list(range(96)))
+    for idx in [[k] for k in (0, 7, 40, 95)] + [list(range(95, -1, -5))]:
+        for i, got in run(idx).items():
+            for a, b in zip(got, among[i]):
+                np.testing.assert_array_equal(a, b)
