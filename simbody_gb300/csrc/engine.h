@@ -213,6 +213,10 @@ struct TileDesc {
     int32_t nsteps, cls0;  // classes at cls0 + step * W + warp
     int64_t slot0, par0, rec0;
 };
+// Entry of the table that the tiles' parameters are formed from: a row of the
+// body table, with this bit where the host found the rotation from the body's
+// inboard frame to its parent's mobilizer frame to be the identity.
+constexpr int32_t kParIdentity = 1 << 30;
 struct TileTables {
     const TileDesc* desc;
     const int32_t* cls;

@@ -295,14 +295,14 @@ cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, do
 }
 
 // Parameters of the tiles' slots (tile_core.cuh) from the body table: entry k
-// is lane k % ls of slot k / ls, parRow[k] its row (-1: none).
+// is lane k % ls of slot k / ls, parRow[k] its row and kParIdentity (-1: none).
 __global__ void __launch_bounds__(128) tileParKernel(const __grid_constant__ DevTables T,
                                                      const int32_t* __restrict__ parRow, int64_t n, int ls,
                                                      double* __restrict__ par) {
     using namespace tile;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-        const int row = parRow[k];
-        if (row < 0) continue;
+        if (parRow[k] < 0) continue;
+        const int row = parRow[k] & ~kParIdentity;
         double* o = par + (k / ls) * PR_COUNT * ls + k % ls;
         auto put = [&](int f, double v) { o[(int64_t)f * ls] = v; };
         const double* b = T.par64 + (int64_t)row * kParamStride;
@@ -326,7 +326,9 @@ __global__ void __launch_bounds__(128) tileParKernel(const __grid_constant__ Dev
         // unit inertia about the mass centre in body axes, turned to M axes, then about M's origin
         const S3<double> G{b[4], b[5], b[6], b[7], b[8], b[9]};
         const S3<double> J = m * (reexpress(RMB, G - pointMassUnit(com)) + pointMassUnit(c));
-        const M3<double> C = mul(PR, RPF);
+        // The identity where the host's product is, whatever this one rounds to: a
+        // lane applies C or leaves it out by what the other lanes of its step do.
+        const M3<double> C = (parRow[k] & kParIdentity) ? ident3<double>() : mul(PR, RPF);
         const V3<double> d = mul(PR, pPF) + pP;
         put(PR_M, m);
         put(PR_MC, m * c.x); put(PR_MC + 1, m * c.y); put(PR_MC + 2, m * c.z);

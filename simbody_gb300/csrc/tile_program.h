@@ -287,7 +287,8 @@ struct TileSchedule {
 };
 
 // The tables of a batch's tiles on the host. Parameters are formed on the
-// device from the body table (parRow: its row per slot and lane, -1: none).
+// device from the body table (parRow: its row and kParIdentity per slot and
+// lane, -1: none).
 struct TileProgram {
     int W = 1, rs = 0, rsTotal = 0;
     int ls = 32;           // lanes per tile
@@ -373,7 +374,7 @@ struct TileProgram {
                     o[SI_PARENT] = t.t->parent[r] < 0 ? -1 : slotOf[t.t->parent[r]];
                     o[SI_INFO] = t.info[r]; o[SI_ROW] = r;
                     o[SI_KBEG] = t.t->kbeg[r]; o[SI_KCNT] = t.t->kcnt[r];
-                    bodies[k * st + l] = rowBase[topo[l]] + r;
+                    bodies[k * st + l] = (rowBase[topo[l]] + r) | ((t.info[r] & F_CI) ? kParIdentity : 0);
                 }
             }
             // the lanes of a step agree on these flags

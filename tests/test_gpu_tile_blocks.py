@@ -3,11 +3,14 @@ soon as there are more tiles than SMs, and nothing orders one against the
 other. Every tile kernel, on two and on four tiles a block, gives each instance
 the bits it has with one tile a block, and a sample agrees with the CPU
 oracle."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from oracle import oracle as O
 from simbody_gb300 import Batch, Topology, Workload, engine_batch
+from simbody_gb300 import _native as Nat
 
 pytestmark = pytest.mark.gpu
 
@@ -108,3 +111,36 @@ def test_steps_do_not_depend_on_the_other_instances(engine, config):
         for i, got in run(idx).items():
             for a, b in zip(got, among[i]):
                 np.testing.assert_array_equal(a, b)
+
+
+def _pins(angle):
+    """Four pins in a row whose frames are turned by +angle on the parent's side
+    and back on the child's: the rotation between them is the identity up to
+    rounding."""
+    c, s = np.cos(angle), np.sin(angle)
+    bodies = (Nat.BodyDesc * 4)()
+    for k, b in enumerate(bodies):
+        b.parent, b.mobilizer, b.mass = k, Nat.SBG_PIN, 1.0
+        b.com[0], b.com[1] = 0.3, 0.1
+        b.unit_inertia[0], b.unit_inertia[1], b.unit_inertia[2] = 0.2, 0.3, 0.4
+        for X, sg in ((b.X_PF, -1), (b.X_BM, 1)):
+            X[0] = X[4] = c
+            X[1], X[3] = -sg * s, sg * s
+            X[8] = 1.0
+        b.X_PF[9] = 0.5
+    d = Nat.SystemDesc(4, 0, 0, 0, (C.c_double * 3)(0, -9.8, 0), bodies, None, None)
+    return Topology(d, keepalive=bodies)
+
+
+def test_frames_that_cancel_up_to_rounding(engine):
+    """A body whose inboard frame is aligned with its parent's mobilizer frame
+    skips that rotation, unless a neighbour in the tile needs one: the bits are
+    the same."""
+    angles = np.linspace(0.01, 3.1, 60)
+    topo = [_pins(a) for a in angles]
+    y = np.linspace(-1, 1, 8 * len(topo)).reshape(len(topo), 8)
+    among, st = Batch(topo, np.arange(len(topo), dtype=np.int32)).realize_acceleration_from(y.ravel())
+    assert (st == 0).all()
+    for k, t in enumerate(topo):
+        alone, _ = Batch([t], np.zeros(1, np.int32)).realize_acceleration_from(y[k])
+        np.testing.assert_array_equal(alone, among.reshape(-1, 8)[k])
