@@ -339,20 +339,26 @@ __global__ void __launch_bounds__(128) tileParKernel(const __grid_constant__ Dev
         put(PR_D, d.x); put(PR_D + 1, d.y); put(PR_D + 2, d.z);
         put(PR_PITCH, b[34]);
         put(PR_PMB, pMB.x); put(PR_PMB + 1, pMB.y); put(PR_PMB + 2, pMB.z);
-        double K[6] = {}, S[6] = {}, B[6] = {};
-        for (int f = T.fbeg[row]; f < T.fbeg[row] + T.fcnt[row]; ++f) {
-            const int which = T.fkind_which[f] & 255;
-            const bool damper = (T.fkind_which[f] >> 8) != 0;
-            const double v = T.fcoef64[f], q0 = T.fq064[f];
+        // Q0: the rest position of the mobility's stiffest spring
+        double K[6] = {}, S[6] = {}, B[6] = {}, Q0[6] = {}, stiff[6] = {};
+        auto forces = [&](auto use) {
+            for (int f = T.fbeg[row]; f < T.fbeg[row] + T.fcnt[row]; ++f) {
+                const int which = T.fkind_which[f] & 255;
+                const bool damper = (T.fkind_which[f] >> 8) != 0;
 #pragma unroll
-            for (int j = 0; j < 6; ++j)
-                if (j == which) {
-                    if (damper) B[j] += v;
-                    else { K[j] += v; S[j] += v * q0; }
-                }
-        }
+                for (int j = 0; j < 6; ++j)
+                    if (j == which) use(j, damper, T.fcoef64[f], T.fq064[f]);
+            }
+        };
+        forces([&](int j, bool damper, double v, double q0) {
+            if (!damper && fabs(v) > stiff[j]) { stiff[j] = fabs(v); Q0[j] = q0; }
+        });
+        forces([&](int j, bool damper, double v, double q0) {
+            if (damper) B[j] += v;
+            else { K[j] += v; S[j] += v * (q0 - Q0[j]); }
+        });
 #pragma unroll
-        for (int j = 0; j < 6; ++j) { put(PR_K + j, K[j]); put(PR_S + j, S[j]); put(PR_B + j, B[j]); }
+        for (int j = 0; j < 6; ++j) { put(PR_K + j, K[j]); put(PR_S + j, S[j]); put(PR_B + j, B[j]); put(PR_Q0 + j, Q0[j]); }
     }
 }
 cudaError_t launchTilePar(const DevTables& T, const int32_t* parRow, int64_t n, int ls, double* par, cudaStream_t s) {

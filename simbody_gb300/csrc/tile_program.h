@@ -174,7 +174,11 @@ struct TileRows {
                     for (int j = 0; j < 3; ++j)
                         ci &= PR[3 * i] * RPF[j] + PR[3 * i + 1] * RPF[3 + j] + PR[3 * i + 2] * RPF[6 + j] == (i == j);
             }
-            info[r] |= (ci ? F_CI : 0) | (t->fcnt[r] == 0 ? F_FREELY : 0);
+            unsigned springs = 0, dampers = 0;
+            for (int f = t->fbeg[r]; f < t->fbeg[r] + t->fcnt[r]; ++f)
+                if (t->fcoef[f] != 0) ((t->fkw[f] >> 8) ? dampers : springs) |= 1u << (t->fkw[f] & 255);
+            const bool all = (springs & dampers) == (1u << n) - 1;  // each mobility has both
+            info[r] |= (ci ? F_CI : 0) | (t->fcnt[r] == 0 ? F_FREELY : 0) | (all ? F_FORCES : 0);
         }
         for (int r = nb - 1; r >= 0; --r) {
             height[r] += cost[r] + (fp32 ? 0 : kTileStepCost);
@@ -380,11 +384,11 @@ struct TileProgram {
             // the lanes of a step agree on these flags
             for (int64_t k = 0; k < nslots; ++k) {
                 int32_t* o = table + k * st * SI_COUNT + SI_INFO;
-                int all = F_CI | F_FREELY;
+                int all = F_CI | F_FREELY | F_FORCES;
                 for (int l = 0; l < nl; ++l)
                     if (s.row[k * nl + l] >= 0) all &= o[l * SI_COUNT];
                 for (int l = 0; l < nl; ++l)
-                    if (s.row[k * nl + l] >= 0) o[l * SI_COUNT] &= ~(F_CI | F_FREELY) | all;
+                    if (s.row[k * nl + l] >= 0) o[l * SI_COUNT] &= ~(F_CI | F_FREELY | F_FORCES) | all;
             }
         });
     }
