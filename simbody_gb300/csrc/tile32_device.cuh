@@ -144,10 +144,12 @@ template <int NM> __device__ __forceinline__ float* tileStage() {
     return reinterpret_cast<float*>(stageRaw) + (threadIdx.x >> 5) * TileSets<NM>::warpFloats;
 }
 template <int NM, class K> inline size_t tileStageBytes(K kernel, int block) {
-    const size_t bytes = (size_t)(block / 32) * TileSets<NM>::warpFloats * sizeof(float);
-    if (bytes > 32 * 1024)  // beside the static arrays of the kernel
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return bytes;
+    constexpr size_t warpBytes = TileSets<NM>::warpFloats * sizeof(float);
+    // The limit is the kernel's in the whole process, whichever batch launches it
+    // on whichever thread: always the widest block's. An error is left for the
+    // launch's cudaGetLastError.
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kTileMaxWarps * warpBytes));
+    return (block / 32) * warpBytes;
 }
 
 // The largest |udot0| and correction over the tile's warps, per lane.
