@@ -154,7 +154,6 @@ struct sbg_batch_s {
     // tree operators (allocated on first use): device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
     double* opsDev = nullptr;
-    int64_t opsElems = 0;
     int64_t* dHostBOff = nullptr;
     cudaEvent_t evOp0 = nullptr, evOp1 = nullptr;  // bracket the last tree operator's kernels
     // one-step launches of a mixed batch integration (allocated on first use)
@@ -305,6 +304,15 @@ struct sbg_batch_s {
         }
         return reinterpret_cast<char*>(hostPinned) + at;
     }
+    // Frees what has been allocated since bufs had n entries and devBytes was
+    // `bytes`: a step of several allocations is made whole or not at all.
+    void release(size_t n, int64_t bytes) {
+        while (bufs.size() > n) {
+            cudaFree(bufs.back().p);
+            bufs.pop_back();
+        }
+        devBytes = bytes;
+    }
     int alloc(void** out, size_t bytes, const char* what) {
         if (budget > 0 && devBytes + (int64_t)bytes > budget)
             return fail(SBG_ERR_BUDGET, std::string("device budget exceeded allocating ") + what);
@@ -333,6 +341,18 @@ struct sbg_batch_s {
         return SBG_OK;
     }
 };
+
+namespace {
+// Gives back what is allocated in its scope unless keep() is reached.
+struct AllocScope {
+    sbg_batch b;
+    size_t n;
+    int64_t bytes;
+    explicit AllocScope(sbg_batch b_) : b(b_), n(b_->bufs.size()), bytes(b_->devBytes) {}
+    ~AllocScope() { if (b) b->release(n, bytes); }
+    void keep() { b = nullptr; }
+};
+}  // namespace
 
 extern "C" {
 
@@ -717,13 +737,16 @@ static int buildTiles32Of(sbg_batch b) {
 
 // Also called when a batch is in use (tree operators and FP64 steps of a mixed
 // one): no memory for the tables is a status there, not an exception, and
-// leaves the batch without the tiles, which the next call tries to build again.
+// leaves the batch as it was; the next call tries to build them again.
 static int buildTiles(sbg_batch b, bool single, TileSet* out) {
     try {
+        AllocScope scope(b);
         TileSet S{};
         const int rc = buildTilesOf(b, single, &S);
-        if (rc == SBG_OK) *out = S;
-        return rc;
+        if (rc != SBG_OK) return rc;
+        scope.keep();
+        *out = S;
+        return SBG_OK;
     } catch (const std::exception& e) {
         return fail(SBG_ERR_NOMEM, std::string("tile tables: ") + e.what());
     }
@@ -1459,22 +1482,23 @@ int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
 // Device operands of a tree operator in the host packing: x [nu] | fmob [nu] |
 // fbody [6 nb] | out [max(nu, 10 nb)].
 static int ensureTreeOps(sbg_batch b) {
+    if (b->opsDev) return SBG_OK;
     const int64_t nu = b->nuTotal, nbT = b->hostBOff[b->ninst];
     const int64_t need = 2 * nu + 6 * nbT + std::max<int64_t>(nu, 10 * nbT);
-    if (b->opsDev && b->opsElems >= need) return SBG_OK;
+    if (!b->evOp0) SBG_CUDA(cudaEventCreate(&b->evOp0), "event");
+    if (!b->evOp1) SBG_CUDA(cudaEventCreate(&b->evOp1), "event");
+    AllocScope scope(b);
     int rc;
+    TileSet tiles = b->tiles;
+    if (!tiles.ntiles && (rc = buildTiles(b, false, &tiles))) return rc;  // a mixed batch's
     void* p = nullptr;
-    if (!b->tiles.ntiles && (rc = buildTiles(b, false, &b->tiles))) return rc;  // a mixed batch's
     if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
-    b->opsDev = static_cast<double*>(p);
     const int64_t* dOff = nullptr;
     if ((rc = b->upload(&dOff, b->hostBOff, "offsets"))) return rc;
+    scope.keep();
+    b->tiles = tiles;
+    b->opsDev = static_cast<double*>(p);
     b->dHostBOff = const_cast<int64_t*>(dOff);
-    b->opsElems = need;
-    if (!b->evOp0) {
-        SBG_CUDA(cudaEventCreate(&b->evOp0), "event");
-        SBG_CUDA(cudaEventCreate(&b->evOp1), "event");
-    }
     return SBG_OK;
 }
 
@@ -1594,31 +1618,37 @@ static int64_t stepsToReach(double t0, double tStop, double h) {
 // Buffers of the one-step launches of a mixed batch integration (allocated
 // on first use): the two FP64-mode lists and their lengths, the per-instance
 // FP64 modes and step counters, the FP64 stage planes, the list kernel's
-// stream and events.
+// stream and events, and the FP64 tiles that take over when the integration
+// switches, so that it cannot run out of memory after its first steps.
 static int ensureFallbackSteps(sbg_batch b) {
     if (b->fbList) return SBG_OK;
-    void* p = nullptr;
+    if (!b->fbStream) SBG_CUDA(cudaStreamCreateWithFlags(&b->fbStream, cudaStreamNonBlocking), "stream");
+    if (!b->fbFork) SBG_CUDA(cudaEventCreateWithFlags(&b->fbFork, cudaEventDisableTiming), "event");
+    if (!b->fbJoin) SBG_CUDA(cudaEventCreateWithFlags(&b->fbJoin, cudaEventDisableTiming), "event");
+    AllocScope scope(b);
     int rc;
+    TileSet tiles = b->tiles;
+    if (!tiles.ntiles && (rc = buildTiles(b, false, &tiles))) return rc;
+    void *lists, *count, *modes, *left, *steps, *planes, *taken;
     const int64_t n = b->ninst;
-    if ((rc = b->alloc(&p, 2 * n * sizeof(int32_t), "FP64 lists"))) return rc;
-    b->fbList = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, 4 * sizeof(int32_t), "FP64 list lengths"))) return rc;
-    b->fbCount = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, 2 * n * sizeof(int32_t), "FP64 modes"))) return rc;
-    b->fbMode = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, n * sizeof(int32_t), "FP64 step counters"))) return rc;
-    b->fbLeft = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, n * sizeof(int32_t), "step counters"))) return rc;
-    b->stepsLeft = static_cast<int32_t*>(p);
-    if ((rc = b->alloc(&p, 5 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
+    if ((rc = b->alloc(&lists, 2 * n * sizeof(int32_t), "FP64 lists"))) return rc;
+    if ((rc = b->alloc(&count, 4 * sizeof(int32_t), "FP64 list lengths"))) return rc;
+    if ((rc = b->alloc(&modes, 2 * n * sizeof(int32_t), "FP64 modes"))) return rc;
+    if ((rc = b->alloc(&left, n * sizeof(int32_t), "FP64 step counters"))) return rc;
+    if ((rc = b->alloc(&steps, n * sizeof(int32_t), "step counters"))) return rc;
+    if ((rc = b->alloc(&planes, 5 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
         return rc;
-    b->fbuf64 = static_cast<double*>(p);
-    if ((rc = b->alloc(&p, sizeof(unsigned long long), "FP64 step counter"))) return rc;
-    b->fbSteps = static_cast<unsigned long long*>(p);
-    SBG_CUDA(cudaMemsetAsync(b->fbSteps, 0, sizeof(unsigned long long), b->stream), "FP64 step counter");
-    SBG_CUDA(cudaStreamCreateWithFlags(&b->fbStream, cudaStreamNonBlocking), "stream");
-    SBG_CUDA(cudaEventCreateWithFlags(&b->fbFork, cudaEventDisableTiming), "event");
-    SBG_CUDA(cudaEventCreateWithFlags(&b->fbJoin, cudaEventDisableTiming), "event");
+    if ((rc = b->alloc(&taken, sizeof(unsigned long long), "FP64 step counter"))) return rc;
+    SBG_CUDA(cudaMemsetAsync(taken, 0, sizeof(unsigned long long), b->stream), "FP64 step counter");
+    scope.keep();
+    b->tiles = tiles;
+    b->fbCount = static_cast<int32_t*>(count);
+    b->fbMode = static_cast<int32_t*>(modes);
+    b->fbLeft = static_cast<int32_t*>(left);
+    b->stepsLeft = static_cast<int32_t*>(steps);
+    b->fbuf64 = static_cast<double*>(planes);
+    b->fbSteps = static_cast<unsigned long long*>(taken);
+    b->fbList = static_cast<int32_t*>(lists);
     return SBG_OK;
 }
 
@@ -1674,8 +1704,6 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
     // The FP64 persistent kernels take every instance's remaining steps once
     // the integration has switched.
     auto allFp64 = [&]() -> int {
-        if (!b->tiles.ntiles)
-            if (int rc = buildTiles(b, false, &b->tiles)) return rc;
         const BatchBufs B64{nullptr, b->scratchLoop, b->fbuf64, b->fbufLoop ? b->fbufLoop : b->fbuf64, b->colElems,
                             &b->tiles, &b->ones, nullptr};
         const StepCtl step{nsteps >= 0 ? nsteps : -1, 0, tStop, 0, 0};
