@@ -1257,6 +1257,11 @@ __device__ __forceinline__ int illConditionedBy(const DevTables& T, int inst, fl
     return dm > tol * um ? SBG_INST_ILL_CONDITIONED : 0;
 }
 
+// A mixed realize's ill-conditioned instances, counted for its FP64 recomputation.
+__device__ __forceinline__ void countFlagged(const DevTables& T, int st) {
+    if (T.flagged && (st & SBG_INST_ILL_CONDITIONED)) atomicAdd(T.flagged, 1);
+}
+
 // Mixed form: SBG_INST_ILL_CONDITIONED when the refinement correction exceeds
 // kIllConditioned of udot0 (max-norms over the instance, i.e. over the lanes
 // of its group). The correction is about cond(M) times the FP32 rounding, so
@@ -1325,7 +1330,10 @@ __global__ void __launch_bounds__(BS, MINB) realizeKernel(DevTables T, int first
     YdOut out{ydot, T.ybase[s.inst], T.ystride[s.inst], T.inq[s.inst]};
     int st = rhs<R, NM, REF, GROUP, LOOPS>(T, s, scratch, src, out);
     if (!groupAll<GROUP>(out.finite, s)) st |= SBG_INST_NONFINITE;
-    if (s.gl == 0) status[s.inst] = st;
+    if (s.gl == 0) {
+        status[s.inst] = st;
+        if constexpr (REF) countFlagged(T, st);
+    }
 }
 
 template <class R, int NM, bool GROUP>

@@ -150,7 +150,6 @@ struct sbg_batch_s {
     std::vector<int32_t> order;              // order position -> instance
     TileSet tiles{}, ones{};
     TileSet tiles32{};                       // FP32 forms: the chain segment's tiles (kernel variant 9)
-    int tileWidth = kTile;                   // instances per tile of `tiles`
     // tree operators (allocated on first use): device operands and results in the host packing,
     // their pinned host staging, and the per-instance packing offsets
     double* opsDev = nullptr;
@@ -190,9 +189,10 @@ struct sbg_batch_s {
         return (nChain > 0) + (nLoop > 0) + (nGroupBlocks > 0);
     }
     // kernels of one realize: the segments, and in the mixed form the FP64
-    // recomputation pass after the chain and the level-parallel segment
+    // recomputation passes after the chain and the level-parallel segment
     int realizeLaunches() const {
-        return segments() + (precision == SBG_PRECISION_MIXED ? (nChain > 0) + (nGroupBlocks > 0) : 0);
+        auto fallback = [&](int count) { return count > 0 ? 1 + fullTiles(tiles, count) : 0; };
+        return segments() + (precision == SBG_PRECISION_MIXED ? fallback(nChain) + fallback(ninst - nChain - nLoop) : 0);
     }
 
     // Lanes per instance of the group segment: blocks of 128 threads hold
@@ -635,7 +635,6 @@ static int buildTilesOf(sbg_batch b, bool single, TileSet* out) {
                 P.W = w;
             }
         }
-        b->tileWidth = TW;
         P.ls = TW;
         P.shared = TW == 1 || same;
         std::vector<TileProgram::Lanes> tiles;
@@ -1118,10 +1117,14 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         if (precision == SBG_PRECISION_MIXED) {
             // FP64 tiles for the instances whose refinement reports an
             // ill-conditioned M, and the count of those recomputed
+            // (a batch of few takes them one to a block: its tiles are built when
+            // steps or operators need them)
             if ((rc = buildTiles(b, true, &b->ones))) return bail(rc);
-            if ((rc = b->alloc(&p, sizeof(unsigned long long), "fallback counter"))) return bail(rc);
+            if (ninst > 2 * b->sms && (rc = buildTiles(b, false, &b->tiles))) return bail(rc);
+            if ((rc = b->alloc(&p, 2 * sizeof(unsigned long long), "fallback counters"))) return bail(rc);
             T.fallbacks = static_cast<unsigned long long*>(p);
-            const cudaError_t ez = cudaMemset(p, 0, sizeof(unsigned long long));
+            T.flagged = reinterpret_cast<int32_t*>(T.fallbacks + 1);
+            const cudaError_t ez = cudaMemset(p, 0, 2 * sizeof(unsigned long long));
             if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counter"));
         }
     }
@@ -1387,6 +1390,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     }
     cudaStream_t up = b->pipe[0], down = b->pipe[1];
     SBG_CUDA(cudaMemsetAsync(b->time, 0, std::max(b->ninst, 1) * sizeof(double), up), "time reset");
+    if (b->T.flagged) SBG_CUDA(cudaMemsetAsync(b->T.flagged, 0, sizeof(int32_t), up), "flag count reset");
     // every stream starts after the work already queued on the batch stream
     SBG_CUDA(cudaEventRecord(b->pipeStart, up), "pipeline");
     for (int k = 1; k < 2 + lanes; ++k) SBG_CUDA(cudaStreamWaitEvent(b->pipe[k], b->pipeStart, 0), "pipeline");
@@ -1414,19 +1418,20 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
         P.nChain = i1 - i0;
         a.P = &P;
         if (b->precision == SBG_PRECISION_FP64) {  // chunks start at multiples of 32, so of the tile width
-            const int t0 = i0 / b->tileWidth, t1 = (i1 + b->tileWidth - 1) / b->tileWidth;
+            const int TW = b->tiles.tt.ls, t0 = i0 / TW, t1 = (i1 + TW - 1) / TW;
             realizeTiles(a, b->tiles, t0, t1 - t0, st);
         } else {
             realize32Chain(a, b->precision == SBG_PRECISION_MIXED, st);
             if (b->precision == SBG_PRECISION_MIXED) {
                 const int share = b->ones.blocks / lanes;  // of the chunks under way together
-                realizeFallbackTiles(a, b->ones, i0, i1 - i0, (c % lanes) * share, share, st);
+                const int TW = std::max(1, b->tiles.tt.ls), t0 = i0 / TW, t1 = (i1 + TW - 1) / TW;
+                realizeFallbackTiles(a, b->tiles, t0, t1 - t0, b->ones, i0, i1 - i0, (c % lanes) * share, share, st);
             }
         }
         SBG_CUDA(cudaGetLastError(), "realize launch");
         SBG_CUDA(launchGather(b->packing(), b->dHostYOff, b->ydot, b->staging, 0, st, i0, i1 - i0), "derivative gather");
         SBG_CUDA(cudaEventRecord(b->pipeEv[1][c], st), "pipeline");
-        b->launches += 1 + 2 * b->packLaunches() + (b->precision == SBG_PRECISION_MIXED ? 1 : 0);
+        b->launches += 1 + 2 * b->packLaunches() + (b->precision == SBG_PRECISION_MIXED ? 1 + fullTiles(b->tiles, i1 - i0) : 0);
     }
     // after every chunk is under way: a copy to pageable memory may hold the host
     for (int c = 0; c < nchunks; ++c) {
@@ -1740,12 +1745,12 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
             SBG_CUDA(launchRKMerson(Tk, P, b->precision, b->y, b->time, b->bufsArg(), b->status, h, step, acc, ctol, pes,
                                     b->streams()),
                      "RK-Merson kernel launch");
-            SBG_CUDA(launchRKFp64List(Tk, b->ones, b->y, b->time, b->status, h, step, acc, ctol, pes, b->colElems,
+            SBG_CUDA(launchRKFp64List(Tk, b->tiles, b->ones, b->y, b->time, b->status, h, step, acc, ctol, pes, b->colElems,
                                       b->fbStream),
                      "FP64 list kernel launch");
             SBG_CUDA(cudaEventRecord(b->fbJoin, b->fbStream), "join");
             SBG_CUDA(cudaStreamWaitEvent(b->stream, b->fbJoin, 0), "join");
-            b->launches += b->segments() + 1;
+            b->launches += b->segments() + 1 + fullTiles(b->tiles, n);
         }
         SBG_CUDA(launchCountUnfinished(n, Tk.stepsLeft, b->time, b->status, tStop, b->fbCount + 2, b->stream),
                  "unfinished count");

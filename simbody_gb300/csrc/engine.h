@@ -125,12 +125,12 @@ struct DevTables {
     const int32_t* row0;     // per body row: first row of its topology
     int32_t loopExt;         // the loop-closure records (sstride wide) end in kLoopExt more values
     const int32_t* bidx;     // per body row: index of the body in its system description (tree operators)
-    // FP64 mirror of the scratch with the same element offsets (mixed batches
-    // and the server's mixed lane; null otherwise): where the mixed form's
-    // refinement reports an ill-conditioned M the RHS is recomputed in FP64
-    // on these records.
+    // FP64 mirror of the scratch with the same element offsets (the server's
+    // mixed lane; null otherwise): where the mixed form's refinement reports an
+    // ill-conditioned M the RHS is recomputed in FP64 on these records.
     double* scratch64;
     unsigned long long* fallbacks;  // instances recomputed in FP64 by realize (cumulative; null = none)
+    int32_t* flagged;               // those that this call's mixed realize has flagged (null = not counted)
     const int32_t* icons;    // per instance: first constraint
     const int32_t* incons;   // per instance: number of constraints
     // per-instance integration control (the serving loop; null in a batch,

@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(BS, MINB)
     if constexpr (REF) st |= illConditioned<false>(T, out, Slot{inst, 0, 1, 0u});
     if (!out.finite) st |= SBG_INST_NONFINITE;
     status[inst] = st;
+    if constexpr (REF) countFlagged(T, st);
 }
 
 template <int NM, bool REF> void goStaged(const KArgs& a, cudaStream_t s) {

@@ -22,7 +22,10 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 1)
     if (!out.finite) st |= SBG_INST_NONFINITE;
     st = tileReduce(TT, c, sh, st);
     if constexpr (REF) st |= tileIll(T, TT, c, mx, out);
-    if (c.on && c.w == 0) status[c.inst] = st;
+    if (c.on && c.w == 0) {
+        status[c.inst] = st;
+        if constexpr (REF) countFlagged(T, st);
+    }
 }
 
 template <int NM, bool REF> void go(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaStream_t s) {

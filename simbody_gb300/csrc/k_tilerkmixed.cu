@@ -9,15 +9,33 @@ void rkTilesMixed(const KArgs& a, const TileSet& S, cudaStream_t s) { rkTilesWit
 
 namespace {
 
-// The instances in FP64 mode at this launch (T.fbList), one at a time per
-// block on the block's own records (TT: one tile per instance).
+// The instances in FP64 mode at this launch on the batch's tiles, where the list
+// is longer than `few` (fullTiles).
+template <class CF>
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
-    rkTileListKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, double* __restrict__ recs,
-                     int64_t recStride, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
-                     int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol, int pes) {
+    rkTileListedKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int ntiles, int few,
+                       double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane,
+                       int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol, int pes) {
+    __shared__ TileShare<4> sh;
+    if (T.fbCount[sc.launch & 1] <= few) return;
+    const int id = tileId(TT, 0, ntiles);
+    if (id < 0) return;
+    TileCtx c = tileCtx<CF>(T, TT, id, recs);
+    c.on = c.on && T.fbMode[(int64_t)(sc.launch & 1) * T.ninst + c.inst];
+    rkTile<CF, true>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
+}
+
+// The instances of a list (T.fbList) of up to `few`, one at a time per block on
+// the block's own records (TT: one tile per instance).
+__global__ void __launch_bounds__(32 * kTileMaxWarps)
+    rkTileListKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int few,
+                     double* __restrict__ recs, int64_t recStride, double* y, double* __restrict__ time, double* fbuf,
+                     int64_t fplane, int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol,
+                     int pes) {
     __shared__ TileShare<4> sh;
     const int32_t* list = T.fbList + (int64_t)(sc.launch & 1) * T.ninst;
     const int n = T.fbCount[sc.launch & 1];
+    if (n > few) return;
     for (int g = blockIdx.x; g < n; g += gridDim.x) {
         const TileCtx c = tileCtxOne<TileOne>(TT, list[g], recs + recStride * blockIdx.x);
         rkTile<TileOne, true>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
@@ -27,11 +45,20 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 
 }  // namespace
 
-void rkTilesList(const KArgs& a, const TileSet& S, cudaStream_t s) {
-    const int blocks = a.T->ninst < S.blocks ? a.T->ninst : S.blocks;
+void rkTilesList(const KArgs& a, const TileSet& S, const TileSet& ones, cudaStream_t s) {
+    const int blocks = a.T->ninst < ones.blocks ? a.T->ninst : ones.blocks;
     if (blocks <= 0) return;
-    rkTileListKernel<<<blocks, 32 * S.tt.W, 0, s>>>(*a.T, S.tt, S.recs, S.recStride, a.ystate, a.time, a.T->fbuf64, a.fplane,
-                                                    a.status, a.h, a.step, a.accuracy, a.consTol, a.projectEveryStep);
+    const bool full = fullTiles(S, a.T->ninst);
+    if (full)
+        tileDispatch<0>(S, [&](auto cf) {
+            const TileLaunch L(S, S.ntiles);
+            rkTileListedKernel<decltype(cf)><<<L.grid, L.block, 0, s>>>(
+                *a.T, S.tt, S.ntiles, fewInstances(S), S.recs, a.ystate, a.time, a.T->fbuf64, a.fplane, a.status, a.h, a.step,
+                a.accuracy, a.consTol, a.projectEveryStep);
+        });
+    rkTileListKernel<<<blocks, 32 * ones.tt.W, 0, s>>>(*a.T, ones.tt, full ? fewInstances(S) : a.T->ninst, ones.recs,
+                                                       ones.recStride, a.ystate, a.time, a.T->fbuf64, a.fplane, a.status,
+                                                       a.h, a.step, a.accuracy, a.consTol, a.projectEveryStep);
 }
 
 }  // namespace sbg

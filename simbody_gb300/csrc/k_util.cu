@@ -250,12 +250,17 @@ cudaError_t launchRealize(const DevTables& T, const LaunchPlan& P, int precision
     if (precision == SBG_PRECISION_FP64)
         return tilesAndLoops(P, *B.tiles, s, [&](cudaStream_t st) { realizeTiles(a, *B.tiles, 0, B.tiles->ntiles, st); }, loops);
     const bool ref = precision == SBG_PRECISION_MIXED;
-    const cudaError_t e = forkJoin(P, s, [&](cudaStream_t st) { realize32Chain(a, ref, st); }, loops,
-                                   [&](cudaStream_t st) { realize32Group(a, ref, st); });
+    cudaError_t e = cudaSuccess;
+    if (ref && fullTiles(*B.tiles, T.ninst)) e = cudaMemsetAsync(T.flagged, 0, sizeof(int32_t), s.main);
+    if (e == cudaSuccess)
+        e = forkJoin(P, s, [&](cudaStream_t st) { realize32Chain(a, ref, st); }, loops,
+                     [&](cudaStream_t st) { realize32Group(a, ref, st); });
     if (e != cudaSuccess || !ref) return e;
-    if (P.nChain > 0) realizeFallbackTiles(a, *B.ones, 0, P.nChain, 0, B.ones->blocks, s.main);
-    const int group0 = P.nChain + P.nLoop;
-    if (P.nGroupBlocks > 0) realizeFallbackTiles(a, *B.ones, group0, T.ninst - group0, 0, B.ones->blocks, s.main);
+    const TileSet& S = *B.tiles;  // the chain segment's tiles, then the group segment's
+    const int group0 = P.nChain + P.nLoop, chainTiles = S.ntiles ? (P.nChain + S.tt.ls - 1) / S.tt.ls : 0;
+    realizeFallbackTiles(a, S, 0, chainTiles, *B.ones, 0, P.nChain, 0, B.ones->blocks, s.main);
+    realizeFallbackTiles(a, S, chainTiles, S.ntiles - chainTiles, *B.ones, group0, T.ninst - group0, 0, B.ones->blocks,
+                         s.main);
     return cudaGetLastError();
 }
 
@@ -284,13 +289,13 @@ cudaError_t launchRKMerson(const DevTables& T, const LaunchPlan& P, int precisio
                     [&](cudaStream_t st) { rk32Group(a, ref, st); });
 }
 
-cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
+cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, const TileSet& ones, double* y, double* time, int32_t* status, double h,
                              StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
                              cudaStream_t s) {
     KArgs a{};
     a.T = &T; a.ystate = y; a.time = time; a.status = status; a.h = h; a.step = step;
     a.accuracy = accuracy; a.consTol = consTol; a.projectEveryStep = projectEveryStep; a.fplane = fplane;
-    rkTilesList(a, S, s);
+    rkTilesList(a, S, ones, s);
     return cudaGetLastError();
 }
 

@@ -48,7 +48,7 @@ struct BatchBufs {
     void* fbuf;          // RK stage derivatives (R), 4 planes of fplane elements
     void* fbufLoop;      // FP64 stage derivatives of the loop-closure segment, 4 planes
     int64_t fplane;
-    const TileSet* tiles;  // FP64: the chain and group segments' tiles
+    const TileSet* tiles;  // FP64: the chain and group segments' tiles (mixed form: for its FP64 work)
     const TileSet* ones;   // mixed form: one FP64 tile per instance
     const TileSet* tiles32;  // FP32 forms: the chain segment's tiles (variant 9)
 };
@@ -159,13 +159,24 @@ void realizeTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, cudaS
 void minvTiles(const KArgs& a, const TileSet& S, cudaStream_t s);
 void rkTiles(const KArgs& a, const TileSet& S, cudaStream_t s);
 void rkAdaptiveTiles(const KArgs& a, const TileSet& S, const AdaptCtl& ac, cudaStream_t s);
+// FP64 work on some of a batch's instances (a mixed batch's ill-conditioned
+// ones). An FP64 instruction costs the same for one lane as for 32: up to two
+// instances an SM run one to a block, side by side and in the time of one; of
+// more, the batch's tiles take them, idle lanes and all. Mixed realize, us, one to
+// a block / tiles: 12,000 trees with 12 contact trees among them 976 / 1129, with
+// 120 and 14 in a hundred tiles 1802 / 1461, 4,000 contact trees 45231 / 1093 (by
+// one thread each 3957).
+inline int fewInstances(const TileSet& S) { return 2 * S.sms; }
+inline bool fullTiles(const TileSet& S, int count) { return S.ntiles > 0 && S.tt.ls > 1 && count > fewInstances(S); }
 // FP64 recomputation of the instances at order positions [first, first +
-// count) that a mixed realize flagged SBG_INST_ILL_CONDITIONED, on the records
-// of the set's blocks [block0, block0 + blocks).
-void realizeFallbackTiles(const KArgs& a, const TileSet& S, int first, int count, int block0, int blocks, cudaStream_t s);
+// count) that a mixed realize flagged SBG_INST_ILL_CONDITIONED: many of them on
+// the batch's tiles [tile0, tile0 + ntiles), which hold these positions, else one
+// to a block, on the records of the blocks [block0, block0 + blocks) of `ones`.
+void realizeFallbackTiles(const KArgs& a, const TileSet& S, int tile0, int ntiles, const TileSet& ones, int first, int count,
+                          int block0, int blocks, cudaStream_t s);
 // One FP64 RK-Merson step for each instance in FP64 mode at this launch
-// (T.fbList[launch & 1]).
-void rkTilesList(const KArgs& a, const TileSet& S, cudaStream_t s);
+// (T.fbList[launch & 1]): many on the batch's tiles S, few one to a block.
+void rkTilesList(const KArgs& a, const TileSet& S, const TileSet& ones, cudaStream_t s);
 void realize32Chain(const KArgs& a, bool refine, cudaStream_t s);
 // Variant 8: the chain driver with record fields staged through shared
 // memory (one shared chain topology, no Free bodies, segment start a
@@ -181,7 +192,7 @@ void rk32Group(const KArgs& a, bool refine, cudaStream_t s);
 void rkLoopGroup(const KArgs& a, int threads, cudaStream_t s);
 void realizeLoopGroup(const KArgs& a, int threads, cudaStream_t s);
 void minvLoopGroup(const KArgs& a, int threads, cudaStream_t s);
-cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, double* y, double* time, int32_t* status, double h,
+cudaError_t launchRKFp64List(const DevTables& T, const TileSet& S, const TileSet& ones, double* y, double* time, int32_t* status, double h,
                              StepCtl step, double accuracy, double consTol, int projectEveryStep, int64_t fplane,
                              cudaStream_t s);
 cudaError_t launchTilePar(const DevTables& T, const int32_t* parRow, int64_t n, int ls, double* par, cudaStream_t s);
