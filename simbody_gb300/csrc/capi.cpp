@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <numeric>
 #include <string>
@@ -576,11 +577,32 @@ int sbg_topology_default_state(sbg_topology t, double* y) {
 // --------------------------------------------------------------------- batch
 }  // extern "C"
 
-// The tile set of a batch's FP64 work: the chain and group segments' tiles, or
-// (single) one tile per instance that isn't in the loop-closure segment, with
-// records for every block of a launch that fills the GPU.
-static int buildTilesOf(sbg_batch b, bool single, TileSet* out) {
+// Operands of the tree operators, buffers of a mixed integration's launches.
+static int64_t treeOpElems(sbg_batch b) {
+    const int64_t nu = b->nuTotal, nbT = b->hostBOff[b->ninst];
+    return std::max<int64_t>(1, 2 * nu + 6 * nbT + std::max<int64_t>(nu, 10 * nbT));
+}
+static int64_t fallbackStepsBytes(sbg_batch b) {
+    return (6 * (int64_t)b->ninst + 4) * sizeof(int32_t) +
+           5 * std::max<int64_t>(b->colElems, 1) * sizeof(double) + sizeof(unsigned long long);
+}
+// What later calls on the batch allocate beside the tiles.
+static int64_t lazyBytes(sbg_batch b) {
+    int64_t n = treeOpElems(b) * sizeof(double) + (b->ninst + 1) * sizeof(int64_t);
+    if (b->precision == SBG_PRECISION_MIXED) n += fallbackStepsBytes(b);
+    if (b->precision == SBG_PRECISION_FP64) n += 2 * (int64_t)b->ninst * sizeof(int64_t);  // adaptStats
+    return n;
+}
+
+// The tile set of a batch's FP64 work. Wide: the chain and group segments'
+// tiles. Ones: one tile per instance that isn't in the loop-closure segment, on
+// tables per topology and on records for the blocks of a launch that fills the
+// GPU. Lean: the same on one warp, whose tables have no empty slots, and on the
+// records that the device budget leaves room for.
+enum TileKind { kTilesWide, kTilesOnes, kTilesLean };
+static int buildTilesOf(sbg_batch b, TileKind kind, TileSet* out) {
     using namespace tile;
+    const bool single = kind != kTilesWide;
     const int sms = b->sms;
     std::vector<TileRows> store(b->topos.size());
     std::vector<const TileRows*> rows(b->topos.size(), nullptr);
@@ -605,7 +627,7 @@ static int buildTilesOf(sbg_batch b, bool single, TileSet* out) {
     *out = TileSet{};
     if (at.empty()) return SBG_OK;
     if (single) {
-        P.W = 4;  // one warp per sub-partition
+        P.W = kind == kTilesLean ? 1 : 4;  // one warp per sub-partition
         P.ls = 1;
         P.shared = true;
         std::vector<TileProgram::Lanes> kinds;  // one tile per topology stands for its instances
@@ -679,11 +701,19 @@ static int buildTilesOf(sbg_batch b, bool single, TileSet* out) {
     }
     int64_t recElems = P.recElems;
     if (single) {
-        out->blocks = 4 * sms;
-        out->recStride = P.maxTile;
-        recElems = (int64_t)out->blocks * out->recStride;
+        out->tt.recStride = P.maxTile;
+        out->blocks = std::min(b->ninst, 4 * sms);
+        const int64_t each = P.maxTile * sizeof(double);
+        if (kind == kTilesLean && b->budget > 0)
+            out->blocks = (int)std::max<int64_t>(1, std::min<int64_t>(out->blocks,
+                                                                      (b->budget - b->devBytes - lazyBytes(b)) / each));
+        recElems = out->blocks * P.maxTile;
     }
-    if ((rc = b->alloc(&p, std::max<int64_t>(recElems, 1) * sizeof(double), "FP64 records"))) return rc;
+    while ((rc = b->alloc(&p, std::max<int64_t>(recElems, 1) * sizeof(double), "FP64 records"))) {
+        if (kind != kTilesLean || out->blocks == 1) return rc;
+        out->blocks = (out->blocks + 1) / 2;  // the GPU itself is full
+        recElems = out->blocks * P.maxTile;
+    }
     out->recs = static_cast<double*>(p);
     return SBG_OK;
 }
@@ -737,11 +767,11 @@ static int buildTiles32Of(sbg_batch b) {
 // Also called when a batch is in use (tree operators and FP64 steps of a mixed
 // one): no memory for the tables is a status there, not an exception, and
 // leaves the batch as it was; the next call tries to build them again.
-static int buildTiles(sbg_batch b, bool single, TileSet* out) {
+static int buildTiles(sbg_batch b, TileKind kind, TileSet* out) {
     try {
         AllocScope scope(b);
         TileSet S{};
-        const int rc = buildTilesOf(b, single, &S);
+        const int rc = buildTilesOf(b, kind, &S);
         if (rc != SBG_OK) return rc;
         scope.keep();
         *out = S;
@@ -750,6 +780,61 @@ static int buildTiles(sbg_batch b, bool single, TileSet* out) {
         return fail(SBG_ERR_NOMEM, std::string("tile tables: ") + e.what());
     }
 }
+static bool noRoom(int rc) { return rc == SBG_ERR_BUDGET || rc == SBG_ERR_NOMEM; }
+
+// The chain and group segments one instance at a time, on the tables and records
+// of `ones`: what a batch falls back to where its wide tiles do not fit. Their
+// records, one per body and lane, and their slots without a body take up to three
+// times the memory of one record per body.
+static int tilesFromOnes(sbg_batch b, const TileSet& ones, TileSet* out) {
+    std::vector<TileDesc> all(std::max(ones.ntiles, 1)), desc;
+    SBG_CUDA(cudaMemcpy(all.data(), ones.tt.desc, ones.ntiles * sizeof(TileDesc), cudaMemcpyDeviceToHost), "tile table");
+    for (int p = 0; p < b->ninst; ++p) {
+        if (p >= b->nChain && p < b->nChain + b->nLoop) continue;
+        desc.push_back(all[b->order[p]]);
+        desc.back().pos0 = p;
+    }
+    *out = ones;
+    out->ntiles = (int)desc.size();
+    return b->upload(&out->tt.desc, desc, "tile table");
+}
+static int buildTilesLean(sbg_batch b, TileSet* ones, TileSet* tiles) {
+    AllocScope scope(b);
+    TileSet o = *ones, t{};
+    int rc;
+    try {
+        if (!o.ntiles && (rc = buildTiles(b, kTilesLean, &o))) return rc;
+        if (o.ntiles && (rc = tilesFromOnes(b, o, &t))) return rc;
+    } catch (const std::exception& e) {
+        return fail(SBG_ERR_NOMEM, std::string("tile tables: ") + e.what());
+    }
+    scope.keep();
+    *ones = o;
+    *tiles = t;
+    return SBG_OK;
+}
+// make() allocates what a call needs, all of it or nothing, beside the batch's FP64
+// tiles, which are built now where the batch has none: wide, or where that does
+// not leave room, lean.
+template <class F> static int withTiles(sbg_batch b, F make) {
+    const TileSet tiles = b->tiles, ones = b->ones;
+    int rc = SBG_OK;
+    for (const bool lean : {false, true}) {
+        AllocScope scope(b);
+        if (!b->tiles.ntiles)
+            rc = lean ? buildTilesLean(b, &b->ones, &b->tiles) : buildTiles(b, kTilesWide, &b->tiles);
+        if (rc == SBG_OK) rc = make();
+        if (rc == SBG_OK) {
+            scope.keep();
+            return rc;
+        }
+        b->tiles = tiles;
+        b->ones = ones;
+        if (!noRoom(rc) || tiles.ntiles) break;
+    }
+    return rc;
+}
+
 static int buildTiles32(sbg_batch b) {
     try {
         return buildTiles32Of(b);
@@ -758,10 +843,10 @@ static int buildTiles32(sbg_batch b) {
     }
 }
 
-extern "C" {
-
-int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
-                     const sbg_batch_config* cfg, sbg_batch* out) {
+// lean: without what makes a batch faster and larger (the tiles of the FP32 forms,
+// wide FP64 tiles, the records' fields for Gram columns side by side).
+static int createBatch(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
+                       const sbg_batch_config* cfg, bool lean, sbg_batch* out) {
     if (!topos || ntopo < 1 || !instTopo || ninst < 0 || !out) return fail(SBG_ERR_INVALID, "bad batch arguments");
     const int precision = cfg ? cfg->precision : SBG_PRECISION_FP64;
     if (precision != SBG_PRECISION_FP64 && precision != SBG_PRECISION_MIXED && precision != SBG_PRECISION_MIXED_FAST)
@@ -790,7 +875,8 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     b->ninst = ninst;
     b->instTopo.assign(instTopo, instTopo + ninst);
     b->topoOf.resize(ninst);
-    auto bail = [&](int rc) { delete b; return rc; };
+    std::unique_ptr<sbg_batch_s> owner(b);
+    auto bail = [&](int rc) { return rc; };
     {
         cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking);
@@ -959,7 +1045,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         const sbg_topology_s* t = topos[instTopo[i]];
         ybase[i] = yOff; ystride[i] = 1;
         yOff += t->nq + t->nu;
-        sstride[i] = rowsRecordWidth(*t, 3) + kLoopExt;
+        sstride[i] = rowsRecordWidth(*t, 3) + (lean ? 0 : loopExtOf(t->ncons));
         sbase[i] = sOffLoop;
         sOffLoop += (t->nb + 2 * t->ncons) * sstride[i];
     }
@@ -1023,7 +1109,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     int rc = 0;
     DevTables& T = b->T;
     T.ninst = ninst;
-    T.loopExt = 1;
+    T.loopExt = lean ? 0 : 1;
     std::vector<float> par32(par.begin(), par.end()), fcoef32(fcoef.begin(), fcoef.end()), fq032(fq0.begin(), fq0.end());
     if ((rc = b->upload(&T.parent, parent, "body table"))) return bail(rc);
     if ((rc = b->upload(&T.info, info, "body table"))) return bail(rc);
@@ -1072,7 +1158,7 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     {   // block table: the loop-closure segment's blocks and their end, then the
         // group segment's (at most one block per instance)
         void* q = nullptr;
-        const size_t cap = (size_t)(ninst - b->nChain) + 4;
+        const size_t cap = (size_t)(ninst - b->nChain) + (b->nLoop > 0 ? 4 : 2);
         if ((rc = b->alloc(&q, cap * sizeof(int32_t), "group block table"))) return bail(rc);
         b->dBlkFirst = static_cast<int32_t*>(q);
         if ((rc = b->alloc(&q, cap * sizeof(int32_t), "group block table"))) return bail(rc);
@@ -1108,26 +1194,9 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
     b->status = static_cast<int32_t*>(p);
     if ((rc = b->alloc(&p, std::max<int64_t>(b->nyTotal, 1) * sizeof(double), "staging"))) return bail(rc);
     b->staging = static_cast<double*>(p);
-    if (precision == SBG_PRECISION_FP64) {
-        if ((rc = buildTiles(b, false, &b->tiles))) return bail(rc);
-    } else {
-        if ((rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch"))) return bail(rc);
-        if ((rc = buildTiles32(b))) return bail(rc);
-        if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
-        if (precision == SBG_PRECISION_MIXED) {
-            // FP64 tiles for the instances whose refinement reports an
-            // ill-conditioned M, and the count of those recomputed
-            // (a batch of few takes them one to a block: its tiles are built when
-            // steps or operators need them)
-            if ((rc = buildTiles(b, true, &b->ones))) return bail(rc);
-            if (ninst > 2 * b->sms && (rc = buildTiles(b, false, &b->tiles))) return bail(rc);
-            if ((rc = b->alloc(&p, 2 * sizeof(unsigned long long), "fallback counters"))) return bail(rc);
-            T.fallbacks = static_cast<unsigned long long*>(p);
-            T.flagged = reinterpret_cast<int32_t*>(T.fallbacks + 1);
-            const cudaError_t ez = cudaMemset(p, 0, 2 * sizeof(unsigned long long));
-            if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counter"));
-        }
-    }
+    if (precision != SBG_PRECISION_FP64 &&
+        (rc = b->alloc(&b->scratch, std::max<int64_t>(b->scratchElems, 1) * rsz, "scratch")))
+        return bail(rc);
     // FP64: and the stage input
     const int planes = precision == SBG_PRECISION_FP64 ? 5 : 4;
     if ((rc = b->alloc(&b->fbuf, planes * std::max<int64_t>(b->colElems, 1) * rsz, "stage derivatives"))) return bail(rc);
@@ -1137,12 +1206,42 @@ int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* in
         else if ((rc = b->alloc(&b->fbufLoop, 4 * b->colElems * sizeof(double), "loop stage derivatives")))
             return bail(rc);
     }
+    if (precision == SBG_PRECISION_MIXED) {  // instances recomputed in FP64, in all and flagged by this call
+        if ((rc = b->alloc(&p, 2 * sizeof(unsigned long long), "fallback counters"))) return bail(rc);
+        T.fallbacks = static_cast<unsigned long long*>(p);
+        T.flagged = reinterpret_cast<int32_t*>(T.fallbacks + 1);
+        const cudaError_t ez = cudaMemset(p, 0, 2 * sizeof(unsigned long long));
+        if (ez != cudaSuccess) return bail(cudaFail(ez, "fallback counters"));
+    }
+    // The tiles, last: lean ones take what the rest leaves. A mixed batch has FP64
+    // tiles for the instances whose refinement reports an ill-conditioned M; of
+    // few instances they go one to a block, and the wide tiles are built when
+    // steps or operators need them.
+    if (precision != SBG_PRECISION_FP64 && !lean && (rc = buildTiles32(b))) return bail(rc);
+    if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
+    if (precision == SBG_PRECISION_MIXED && (rc = buildTiles(b, lean ? kTilesLean : kTilesOnes, &b->ones))) return bail(rc);
+    if (precision == SBG_PRECISION_FP64 || (precision == SBG_PRECISION_MIXED && (lean || ninst > 2 * b->sms))) {
+        rc = lean ? buildTilesLean(b, &b->ones, &b->tiles) : buildTiles(b, kTilesWide, &b->tiles);
+        if (rc) return bail(rc);
+    }
     cudaError_t e = cudaMemsetAsync(b->time, 0, std::max<int64_t>(ninst, 1) * sizeof(double), b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->status, 0, std::max<int64_t>(ninst, 1) * sizeof(int32_t), b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return bail(cudaFail(e, "batch initialisation"));
-    *out = b;
+    *out = owner.release();
     return SBG_OK;
+}
+
+extern "C" {
+
+int sbg_batch_create(const sbg_topology* topos, int32_t ntopo, const int32_t* instTopo, int32_t ninst,
+                     const sbg_batch_config* cfg, sbg_batch* out) {
+    try {
+        const int rc = createBatch(topos, ntopo, instTopo, ninst, cfg, false, out);
+        return noRoom(rc) ? createBatch(topos, ntopo, instTopo, ninst, cfg, true, out) : rc;
+    } catch (const std::exception& e) {
+        return fail(SBG_ERR_NOMEM, std::string("batch tables: ") + e.what());
+    }
 }
 
 int sbg_batch_destroy(sbg_batch b) {
@@ -1353,7 +1452,10 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     // one per SM sub-partition: chunks of half as many still run side by side
     if (b->precision == SBG_PRECISION_FP64)
         nchunks = std::min<int64_t>(nchunks, b->tiles.ntiles / (2 * b->sms));
-    const bool pipelined = b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 &&
+    // (records that blocks share are one launch's at a time)
+    const bool apart = b->precision == SBG_PRECISION_FP64 ? !b->tiles.tt.recStride
+                                                          : b->precision != SBG_PRECISION_MIXED || b->ones.blocks >= nchunks;
+    const bool pipelined = apart && b->orderIdentity && b->nGroupBlocks == 0 && b->nLoop == 0 &&
                            (b->tuned || b->precision == SBG_PRECISION_FP64) && nchunks > 1 &&
                            b->ninst >= nchunks * kTile;
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
@@ -1488,23 +1590,18 @@ int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
 // fbody [6 nb] | out [max(nu, 10 nb)].
 static int ensureTreeOps(sbg_batch b) {
     if (b->opsDev) return SBG_OK;
-    const int64_t nu = b->nuTotal, nbT = b->hostBOff[b->ninst];
-    const int64_t need = 2 * nu + 6 * nbT + std::max<int64_t>(nu, 10 * nbT);
     if (!b->evOp0) SBG_CUDA(cudaEventCreate(&b->evOp0), "event");
     if (!b->evOp1) SBG_CUDA(cudaEventCreate(&b->evOp1), "event");
-    AllocScope scope(b);
-    int rc;
-    TileSet tiles = b->tiles;
-    if (!tiles.ntiles && (rc = buildTiles(b, false, &tiles))) return rc;  // a mixed batch's
-    void* p = nullptr;
-    if ((rc = b->alloc(&p, std::max<int64_t>(need, 1) * sizeof(double), "tree-operator operands"))) return rc;
-    const int64_t* dOff = nullptr;
-    if ((rc = b->upload(&dOff, b->hostBOff, "offsets"))) return rc;
-    scope.keep();
-    b->tiles = tiles;
-    b->opsDev = static_cast<double*>(p);
-    b->dHostBOff = const_cast<int64_t*>(dOff);
-    return SBG_OK;
+    return withTiles(b, [&]() -> int {
+        void* p = nullptr;
+        const int64_t* dOff = nullptr;
+        int rc;
+        if ((rc = b->alloc(&p, treeOpElems(b) * sizeof(double), "tree-operator operands"))) return rc;
+        if ((rc = b->upload(&dOff, b->hostBOff, "offsets"))) return rc;
+        b->opsDev = static_cast<double*>(p);
+        b->dHostBOff = const_cast<int64_t*>(dOff);
+        return SBG_OK;
+    });
 }
 
 static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob, const double* fbody, double* out,
@@ -1630,31 +1727,28 @@ static int ensureFallbackSteps(sbg_batch b) {
     if (!b->fbStream) SBG_CUDA(cudaStreamCreateWithFlags(&b->fbStream, cudaStreamNonBlocking), "stream");
     if (!b->fbFork) SBG_CUDA(cudaEventCreateWithFlags(&b->fbFork, cudaEventDisableTiming), "event");
     if (!b->fbJoin) SBG_CUDA(cudaEventCreateWithFlags(&b->fbJoin, cudaEventDisableTiming), "event");
-    AllocScope scope(b);
-    int rc;
-    TileSet tiles = b->tiles;
-    if (!tiles.ntiles && (rc = buildTiles(b, false, &tiles))) return rc;
-    void *lists, *count, *modes, *left, *steps, *planes, *taken;
-    const int64_t n = b->ninst;
-    if ((rc = b->alloc(&lists, 2 * n * sizeof(int32_t), "FP64 lists"))) return rc;
-    if ((rc = b->alloc(&count, 4 * sizeof(int32_t), "FP64 list lengths"))) return rc;
-    if ((rc = b->alloc(&modes, 2 * n * sizeof(int32_t), "FP64 modes"))) return rc;
-    if ((rc = b->alloc(&left, n * sizeof(int32_t), "FP64 step counters"))) return rc;
-    if ((rc = b->alloc(&steps, n * sizeof(int32_t), "step counters"))) return rc;
-    if ((rc = b->alloc(&planes, 5 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
-        return rc;
-    if ((rc = b->alloc(&taken, sizeof(unsigned long long), "FP64 step counter"))) return rc;
-    SBG_CUDA(cudaMemsetAsync(taken, 0, sizeof(unsigned long long), b->stream), "FP64 step counter");
-    scope.keep();
-    b->tiles = tiles;
-    b->fbCount = static_cast<int32_t*>(count);
-    b->fbMode = static_cast<int32_t*>(modes);
-    b->fbLeft = static_cast<int32_t*>(left);
-    b->stepsLeft = static_cast<int32_t*>(steps);
-    b->fbuf64 = static_cast<double*>(planes);
-    b->fbSteps = static_cast<unsigned long long*>(taken);
-    b->fbList = static_cast<int32_t*>(lists);
-    return SBG_OK;
+    return withTiles(b, [&]() -> int {
+        int rc;
+        void *lists, *count, *modes, *left, *steps, *planes, *taken;
+        const int64_t n = b->ninst;
+        if ((rc = b->alloc(&lists, 2 * n * sizeof(int32_t), "FP64 lists"))) return rc;
+        if ((rc = b->alloc(&count, 4 * sizeof(int32_t), "FP64 list lengths"))) return rc;
+        if ((rc = b->alloc(&modes, 2 * n * sizeof(int32_t), "FP64 modes"))) return rc;
+        if ((rc = b->alloc(&left, n * sizeof(int32_t), "FP64 step counters"))) return rc;
+        if ((rc = b->alloc(&steps, n * sizeof(int32_t), "step counters"))) return rc;
+        if ((rc = b->alloc(&planes, 5 * std::max<int64_t>(b->colElems, 1) * sizeof(double), "FP64 stage derivatives")))
+            return rc;
+        if ((rc = b->alloc(&taken, sizeof(unsigned long long), "FP64 step counter"))) return rc;
+        SBG_CUDA(cudaMemsetAsync(taken, 0, sizeof(unsigned long long), b->stream), "FP64 step counter");
+        b->fbCount = static_cast<int32_t*>(count);
+        b->fbMode = static_cast<int32_t*>(modes);
+        b->fbLeft = static_cast<int32_t*>(left);
+        b->stepsLeft = static_cast<int32_t*>(steps);
+        b->fbuf64 = static_cast<double*>(planes);
+        b->fbSteps = static_cast<unsigned long long*>(taken);
+        b->fbList = static_cast<int32_t*>(lists);
+        return SBG_OK;
+    });
 }
 
 // Launches per window of the FP64 share test of a mixed batch integration.

@@ -75,8 +75,12 @@ enum : int {
 constexpr int kSlotA = 18, kSlotB = 24, kSlotF = 30, kSlotB3 = 36, kSlotF3 = 48, kSlotSize = 60;
 constexpr int kMaxLoopCons = 4;             // Ball constraints per instance
 constexpr int kMaxLoopEq = 3 * kMaxLoopCons;
-// A record's extension for Gram columns 3 to 11 (18 values each, loops_device.cuh).
-constexpr int kLoopExt = 18 * (kMaxLoopEq - 3);
+// A record's extension for the Gram columns of `ncons` constraints from the
+// fourth on (18 values each, loops_device.cuh).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int loopExtOf(int ncons) { return ncons > 1 ? 18 * (3 * ncons - 3) : 0; }
 constexpr int F_MEMACC = F_MEMCHILD;
 
 // Warp tile of the shared-topology scratch layout.
@@ -123,7 +127,7 @@ struct DevTables {
     const double* lst;       // per constraint: station 1 (in body 1), station 2 (in body 2)
     const int32_t* lslot;    // per body row: slot index of a loop body (-1 = none): level-parallel layout
     const int32_t* row0;     // per body row: first row of its topology
-    int32_t loopExt;         // the loop-closure records (sstride wide) end in kLoopExt more values
+    int32_t loopExt;         // the loop-closure records (sstride wide) end in loopExtOf() more values
     const int32_t* bidx;     // per body row: index of the body in its system description (tree operators)
     // FP64 mirror of the scratch with the same element offsets (the server's
     // mixed lane; null otherwise): where the mixed form's refinement reports an
@@ -228,15 +232,16 @@ struct TileTables {
                            // level-parallel segment keeps contiguous columns)
     int32_t rs, rsTotal;   // doubles of a body's record without and with the Ground pose
     int32_t pose;          // some body carries contact spheres
+    int64_t recStride;     // 0: each tile has records of its own (TileDesc::rec0); else those that a block
+                           // sweeps one after another share its recStride doubles
 };
-// A batch's tiles with their records; or one tile per instance, swept one at a
-// time by each of `blocks` blocks on records of its own (recStride doubles).
+// A batch's tiles with their records; or one tile per instance, on the records
+// of `blocks` blocks.
 struct TileSet {
     TileTables tt;
     int32_t ntiles, sms;
     double* recs;
     int32_t blocks;
-    int64_t recStride;
     double* yt;            // FP32 forms: the stage input of RK-Merson (a column plane)
 };
 

@@ -16,21 +16,20 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                       int32_t* __restrict__ status, int few) {
     __shared__ TileShare<0> sh;
     if (FLAGGED && *T.flagged <= few) return;
-    const int id = tileId(TT, tile0, ntiles);
-    if (id < 0) return;
-    TileCtx c = tileCtx<CF>(T, TT, id, recs);
-    if constexpr (FLAGGED) {
-        c.on = c.on && (status[c.inst] & SBG_INST_ILL_CONDITIONED);
-        const int n = __popc(__ballot_sync(0xffffffffu, c.on));
-        if (n == 0) return;  // every warp of the tile counts the same
-        if (c.w == 0 && c.lane == 0) atomicAdd(T.fallbacks, (unsigned long long)n);
-    }
-    const TileYSrc<CF::YS> src{{T, c.inst}, y};
-    TileOut<CF::YS> out(src.c, ydot);
-    int st = tileRhs<CF, false>(T, TT, c, src, out, true);
-    if (!out.finite) st |= SBG_INST_NONFINITE;
-    st = tileReduce(TT, c, sh, st);
-    if (c.on && c.w == 0) status[c.inst] = st;
+    forTiles<CF>(T, TT, tile0, ntiles, recs, [&](TileCtx c) {
+        if constexpr (FLAGGED) {
+            c.on = c.on && (status[c.inst] & SBG_INST_ILL_CONDITIONED);
+            const int n = __popc(__ballot_sync(0xffffffffu, c.on));
+            if (n == 0) return;  // every warp of the tile counts the same
+            if (c.w == 0 && c.lane == 0) atomicAdd(T.fallbacks, (unsigned long long)n);
+        }
+        const TileYSrc<CF::YS> src{{T, c.inst}, y};
+        TileOut<CF::YS> out(src.c, ydot);
+        int st = tileRhs<CF, false>(T, TT, c, src, out, true);
+        if (!out.finite) st |= SBG_INST_NONFINITE;
+        st = tileReduce(TT, c, sh, st);
+        if (c.on && c.w == 0) status[c.inst] = st;
+    });
 }
 
 template <class CF>
@@ -40,15 +39,14 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                    const double* __restrict__ f, double* __restrict__ o, double* __restrict__ recs,
                    int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
-    const int id = tileId(TT, 0, ntiles);
-    if (id < 0) return;
-    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
-    const TileFSrc<CF::YS> src{{T, c.inst}, y, f};
-    TileUOut<CF::YS> out(src.c, o);
-    int st = tileRhs<CF, true>(T, TT, c, src, out, true);
-    if (!out.finite) st |= SBG_INST_NONFINITE;
-    st = tileReduce(TT, c, sh, st);
-    if (c.on && c.w == 0) status[c.inst] = st;
+    forTiles<CF>(T, TT, 0, ntiles, recs, [&](const TileCtx& c) {
+        const TileFSrc<CF::YS> src{{T, c.inst}, y, f};
+        TileUOut<CF::YS> out(src.c, o);
+        int st = tileRhs<CF, true>(T, TT, c, src, out, true);
+        if (!out.finite) st |= SBG_INST_NONFINITE;
+        st = tileReduce(TT, c, sh, st);
+        if (c.on && c.w == 0) status[c.inst] = st;
+    });
 }
 
 // The instances at order positions [first, first + count) whose mixed realize
@@ -59,7 +57,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     realizeFallbackTileKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int first,
                               int count, const double* __restrict__ y, double* __restrict__ ydot,
-                              double* __restrict__ recs, int64_t recStride, int32_t* __restrict__ status) {
+                              double* __restrict__ recs, int32_t* __restrict__ status) {
     __shared__ TileShare<0> sh;
     __shared__ int list[32 * kTileMaxWarps], n;
     for (int64_t k0 = 0; blockIdx.x + k0 * gridDim.x < count; k0 += blockDim.x) {
@@ -72,7 +70,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
         }
         __syncthreads();
         for (int k = 0; k < n; ++k) {
-            const TileCtx c = tileCtxOne<TileOne>(TT, list[k], recs + recStride * blockIdx.x);
+            const TileCtx c = tileCtxOne<TileOne>(TT, list[k], recs + TT.recStride * blockIdx.x);
             const TileYSrc<0> src{{T, c.inst}, y};
             TileOut<0> out(src.c, ydot);
             int st = tileRhs<TileOne, false>(T, TT, c, src, out, true);
@@ -114,7 +112,7 @@ void realizeFallbackTiles(const KArgs& a, const TileSet& S, int tile0, int ntile
                                                                              a.status, fewInstances(S));
         });
     realizeFallbackTileKernel<<<count < blocks ? count : blocks, 32 * ones.tt.W, 0, s>>>(
-        *a.T, ones.tt, first, count, a.y, a.ydot, ones.recs + ones.recStride * block0, ones.recStride, a.status);
+        *a.T, ones.tt, first, count, a.y, a.ydot, ones.recs + ones.tt.recStride * block0, a.status);
 }
 
 }  // namespace sbg

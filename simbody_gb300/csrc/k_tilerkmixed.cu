@@ -18,18 +18,17 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                        int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol, int pes) {
     __shared__ TileShare<4> sh;
     if (T.fbCount[sc.launch & 1] <= few) return;
-    const int id = tileId(TT, 0, ntiles);
-    if (id < 0) return;
-    TileCtx c = tileCtx<CF>(T, TT, id, recs);
-    c.on = c.on && T.fbMode[(int64_t)(sc.launch & 1) * T.ninst + c.inst];
-    rkTile<CF, true>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
+    forTiles<CF>(T, TT, 0, ntiles, recs, [&](TileCtx c) {
+        c.on = c.on && T.fbMode[(int64_t)(sc.launch & 1) * T.ninst + c.inst];
+        rkTile<CF, true>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
+    });
 }
 
 // The instances of a list (T.fbList) of up to `few`, one at a time per block on
 // the block's own records (TT: one tile per instance).
 __global__ void __launch_bounds__(32 * kTileMaxWarps)
     rkTileListKernel(const __grid_constant__ DevTables T, const __grid_constant__ TileTables TT, int few,
-                     double* __restrict__ recs, int64_t recStride, double* y, double* __restrict__ time, double* fbuf,
+                     double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf,
                      int64_t fplane, int32_t* __restrict__ status, double h, StepCtl sc, double accuracy, double consTol,
                      int pes) {
     __shared__ TileShare<4> sh;
@@ -37,7 +36,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
     const int n = T.fbCount[sc.launch & 1];
     if (n > few) return;
     for (int g = blockIdx.x; g < n; g += gridDim.x) {
-        const TileCtx c = tileCtxOne<TileOne>(TT, list[g], recs + recStride * blockIdx.x);
+        const TileCtx c = tileCtxOne<TileOne>(TT, list[g], recs + TT.recStride * blockIdx.x);
         rkTile<TileOne, true>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
         __syncthreads();
     }
@@ -56,8 +55,7 @@ void rkTilesList(const KArgs& a, const TileSet& S, const TileSet& ones, cudaStre
                 *a.T, S.tt, S.ntiles, fewInstances(S), S.recs, a.ystate, a.time, a.T->fbuf64, a.fplane, a.status, a.h, a.step,
                 a.accuracy, a.consTol, a.projectEveryStep);
         });
-    rkTileListKernel<<<blocks, 32 * ones.tt.W, 0, s>>>(*a.T, ones.tt, full ? fewInstances(S) : a.T->ninst, ones.recs,
-                                                       ones.recStride, a.ystate, a.time, a.T->fbuf64, a.fplane, a.status,
+    rkTileListKernel<<<blocks, 32 * ones.tt.W, 0, s>>>(*a.T, ones.tt, full ? fewInstances(S) : a.T->ninst, ones.recs, a.ystate, a.time, a.T->fbuf64, a.fplane, a.status,
                                                        a.h, a.step, a.accuracy, a.consTol, a.projectEveryStep);
 }
 

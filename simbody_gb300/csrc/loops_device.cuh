@@ -77,7 +77,8 @@ __device__ __forceinline__ int loopRows(const DevTables& T, int inst) { return T
 __device__ __forceinline__ LoopState loopStateRows(const DevTables& T, int inst, double* scratch, double* y,
                                                    double* save, double* delta, int64_t base, int64_t stride) {
     return LoopState{T, inst, SC64{scratch, (int)T.sstride[inst], 1}, y, save, delta, base, stride,
-                     T.ibody[inst], T.inb[inst], T.loopExt ? (int)T.sstride[inst] - kLoopExt : 0};
+                     T.ibody[inst], T.inb[inst],
+                     T.loopExt && T.incons[inst] > 1 ? (int)T.sstride[inst] - loopExtOf(T.incons[inst]) : 0};
 }
 
 // The weights of a sweep that applies none (kMInvSweep; see PosWeights).

@@ -44,7 +44,7 @@ struct TileCtx {
 // ms, 1.27 ms so); while there are SMs for all, each its own (1,024 pendulums
 // 9.3 ms, four to a block 10.1 ms).
 inline int tilesPerBlock(const TileSet& S, int sms) {
-    return S.tt.W >= 4 ? 1 : std::max(1, std::min(4 / S.tt.W, (S.ntiles + sms - 1) / sms));
+    return S.tt.W >= 4 || S.tt.recStride ? 1 : std::max(1, std::min(4 / S.tt.W, (S.ntiles + sms - 1) / sms));
 }
 __device__ __forceinline__ void tileSync(int W, const TileCtx& c) {
     if (W == 1) __syncwarp();
@@ -60,11 +60,6 @@ template <class CF> __device__ __forceinline__ void tileTables(const TileTables&
     c.slots = reinterpret_cast<const int4*>(TT.slots + c.d.slot0) + 2 * l;
     c.par = TT.par + c.d.par0 + l;
 }
-// The warp's tile among [tile0, tile0 + count), -1 past the end.
-__device__ __forceinline__ int tileId(const TileTables& TT, int tile0, int count) {
-    const int k = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / TT.W;
-    return k < count ? tile0 + k : -1;
-}
 // Tile `id` of a batch.
 template <class CF>
 __device__ __forceinline__ TileCtx tileCtx(const DevTables& T, const TileTables& TT, int id, double* recs) {
@@ -75,6 +70,28 @@ __device__ __forceinline__ TileCtx tileCtx(const DevTables& T, const TileTables&
     c.rec = recs + c.d.rec0 + (c.on ? c.lane : 0);
     c.inst = c.on ? T.order[c.d.pos0 + c.lane] : T.order[c.d.pos0];
     return c;
+}
+// The warp's tile among [tile0, tile0 + count), -1 past the end.
+__device__ __forceinline__ int tileId(const TileTables& TT, int tile0, int count) {
+    const int k = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / TT.W;
+    return k < count ? tile0 + k : -1;
+}
+// f(tile) for the warp's tile among [tile0, tile0 + count), if any; where blocks
+// share records (TT.recStride), for every gridDim-th tile from the block's on.
+template <class CF, class F>
+__device__ __forceinline__ void forTiles(const DevTables& T, const TileTables& TT, int tile0, int count, double* recs, F f) {
+    int id = tileId(TT, tile0, count);
+    if (id < 0) return;
+    if constexpr (CF::LS == 1) {
+        for (const int end = tile0 + count; id < end; id += TT.recStride ? gridDim.x : count) {
+            TileCtx c = tileCtx<CF>(T, TT, id, recs);
+            if (TT.recStride) c.rec = recs + TT.recStride * blockIdx.x;
+            f(c);
+            tileSync(TT.W, c);
+        }
+    } else {
+        f(tileCtx<CF>(T, TT, id, recs));
+    }
 }
 // The tile of one instance, in a tile set with one tile per instance, on the
 // block's own records.
@@ -354,7 +371,7 @@ struct TileLaunch {
     int grid, block;
     TileLaunch(const TileSet& S, int ntiles) {
         const int per = tilesPerBlock(S, S.sms);
-        grid = (ntiles + per - 1) / per;
+        grid = S.tt.recStride ? std::min(ntiles, S.blocks) : (ntiles + per - 1) / per;
         block = 32 * S.tt.W * per;
     }
 };

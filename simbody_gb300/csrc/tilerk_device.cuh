@@ -145,10 +145,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
                  double* __restrict__ recs, double* y, double* __restrict__ time, double* fbuf, int64_t fplane, int32_t* __restrict__ status,
                  double h, StepCtl sc, double accuracy, double consTol, int pes) {
     __shared__ TileShare<4> sh;
-    const int id = tileId(TT, 0, ntiles);
-    if (id < 0) return;
-    const TileCtx c = tileCtx<CF>(T, TT, id, recs);
-    rkTile<CF, false>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
+    forTiles<CF>(T, TT, 0, ntiles, recs, [&](const TileCtx& c) {
+        rkTile<CF, false>(T, TT, c, sh, y, time, fbuf, fplane, status, h, sc, accuracy, consTol, pes != 0);
+    });
 }
 
 template <int YS> void rkTilesWith(const KArgs& a, const TileSet& S, cudaStream_t s) {
