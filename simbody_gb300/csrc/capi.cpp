@@ -305,6 +305,14 @@ struct sbg_batch_s {
         }
         return reinterpret_cast<char*>(hostPinned) + at;
     }
+    // Waits for everything under way on the batch's streams.
+    void drain() {
+        for (cudaStream_t s : {stream, stream2, fbStream})
+            if (s) cudaStreamSynchronize(s);
+        for (int k = 1; k < kPipe; ++k)
+            if (pipe[k]) cudaStreamSynchronize(pipe[k]);
+        cudaGetLastError();
+    }
     // Frees what has been allocated since bufs had n entries and devBytes was
     // `bytes`: a step of several allocations is made whole or not at all.
     void release(size_t n, int64_t bytes) {
@@ -344,6 +352,14 @@ struct sbg_batch_s {
 };
 
 namespace {
+// A call that copies from or to the caller's memory: on a return without done()
+// (an error) no such copy is under way any more.
+struct CopyScope {
+    sbg_batch b;
+    explicit CopyScope(sbg_batch b_) : b(b_) {}
+    ~CopyScope() { if (b) b->drain(); }
+    int done() { b = nullptr; return SBG_OK; }
+};
 // Gives back what is allocated in its scope unless keep() is reached.
 struct AllocScope {
     sbg_batch b;
@@ -1289,18 +1305,20 @@ static int uploadState(sbg_batch b, const double* t, const double* y) {
 int sbg_batch_set_state(sbg_batch b, const double* t, const double* y) {
     if (!b || !y) return fail(SBG_ERR_INVALID, "null argument");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
+    CopyScope copies(b);
     if (int rc = uploadState(b, t, y)) return rc;
     SBG_CUDA(cudaStreamSynchronize(b->stream), "state upload");
     b->stateSet = true;
     b->integrating = false;
     b->realized = false;
-    return SBG_OK;
+    return copies.done();
 }
 
 int sbg_batch_get_state(sbg_batch b, double* t, double* y) {
     if (!b || !y) return fail(SBG_ERR_INVALID, "null argument");
     if (!b->stateSet) return fail(SBG_ERR_STATE, "no state has been set");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
+    CopyScope copies(b);
     SBG_CUDA(launchGather(b->packing(), b->dHostYOff, b->y, b->staging, 0, b->stream), "state gather");
     b->launches += b->packLaunches();
     const size_t bytes = b->nyTotal * sizeof(double);
@@ -1313,7 +1331,7 @@ int sbg_batch_get_state(sbg_batch b, double* t, double* y) {
     if (dst != y) std::memcpy(y, dst, bytes);
     if (t && !b->pageable)
         SBG_CUDA(cudaMemcpy(t, b->time, b->ninst * sizeof(double), cudaMemcpyDeviceToHost), "time download");
-    return SBG_OK;
+    return copies.done();
 }
 
 // Tuner: the FP32 kernels come in two register budgets (all the registers
@@ -1413,6 +1431,7 @@ int sbg_batch_get_ydot(sbg_batch b, double* ydot, int32_t* status) {
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     const size_t bytes = b->nyTotal * sizeof(double);
     void* dst = nullptr;
+    CopyScope copies(b);
     if (ydot) {
         dst = b->hostSide(ydot, bytes);
         if (!dst) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
@@ -1425,7 +1444,7 @@ int sbg_batch_get_ydot(sbg_batch b, double* ydot, int32_t* status) {
                  "status download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "derivative download");
     if (dst && dst != ydot) std::memcpy(ydot, dst, bytes);
-    return SBG_OK;
+    return copies.done();
 }
 
 int sbg_realize_acceleration(sbg_batch b, double* ydot, int32_t* status) {
@@ -1459,6 +1478,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
                            (b->tuned || b->precision == SBG_PRECISION_FP64) && nchunks > 1 &&
                            b->ninst >= nchunks * kTile;
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
+    CopyScope copies(b);
     if (!pipelined) {
         int rc = uploadState(b, nullptr, y);
         if (!rc) {
@@ -1467,11 +1487,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
             rc = sbg_realize_acceleration_async(b);
         }
         if (!rc) rc = sbg_batch_get_ydot(b, ydot, status);  // waits for the upload too
-        if (rc) {  // the caller's buffers are not in use after the return
-            cudaStreamSynchronize(b->stream);
-            cudaGetLastError();
-        }
-        return rc;
+        return rc ? rc : copies.done();
     }
     const size_t bytes = b->nyTotal * sizeof(double);
     double* src = static_cast<double*>(b->hostSide(y, bytes));
@@ -1559,7 +1575,7 @@ int sbg_realize_acceleration_host(sbg_batch b, const double* y, double* ydot, in
     b->stateSet = true;
     b->integrating = false;
     b->realized = true;
-    return SBG_OK;
+    return copies.done();
 }
 
 int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
@@ -1567,6 +1583,7 @@ int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
     if (!b->stateSet) return fail(SBG_ERR_STATE, "no state has been set");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     const size_t bytes = b->nuTotal * sizeof(double);
+    CopyScope copies(b);
     void* src = b->hostSide(f, bytes);
     if (!src) return fail(SBG_ERR_NOMEM, "out of pinned host memory");
     if (src != f) std::memcpy(src, f, bytes);
@@ -1582,7 +1599,7 @@ int sbg_multiply_by_minv(sbg_batch b, const double* f, double* outp) {
     SBG_CUDA(cudaMemcpyAsync(dst, b->staging, bytes, cudaMemcpyDeviceToHost, b->stream), "result download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "M^-1");
     if (dst != outp) std::memcpy(outp, dst, bytes);
-    return SBG_OK;
+    return copies.done();
 }
 
 // ------------------------------------------------------------ tree operators
@@ -1616,6 +1633,7 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
     double* dB = dF + nu;
     double* dOut = dB + 6 * nbT;
     const int64_t nOut = kind == OP_JV ? 6 * nbT : (kind == OP_COMPOSITE ? 10 * nbT : nu);
+    CopyScope copies(b);
     auto up = [&](const double* src, double* dDst, int64_t n, const char* what) -> int {
         if (!src || n == 0) return SBG_OK;
         if (!b->pageable) SBG_CUDA(cudaStreamSynchronize(b->stream), what);  // hostSide may move the buffer
@@ -1644,7 +1662,7 @@ static int runTreeOp(sbg_batch b, int kind, const double* x, const double* fmob,
                  "status download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "tree operator");
     if (hOut != out) std::memcpy(out, hOut, nOut * sizeof(double));
-    return SBG_OK;
+    return copies.done();
 }
 
 int sbg_batch_fallback_count(sbg_batch b, int64_t* n) {
@@ -1793,9 +1811,11 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
     } else {
         // steps to tStop from the earliest instance time, by the kernels' rule
         std::vector<double> t0(n);
+        CopyScope copies(b);
         SBG_CUDA(cudaMemcpyAsync(t0.data(), b->time, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
                  "time download");
         SBG_CUDA(cudaStreamSynchronize(b->stream), "time download");
+        copies.done();
         target = stepsToReach(*std::min_element(t0.begin(), t0.end()), tStop, h);
     }
     const LaunchPlan P = b->plan();
@@ -1849,9 +1869,11 @@ static int rkMersonMixedSteps(sbg_batch b, double h, int32_t nsteps, double tSto
         SBG_CUDA(launchCountUnfinished(n, Tk.stepsLeft, b->time, b->status, tStop, b->fbCount + 2, b->stream),
                  "unfinished count");
         int32_t left = 0;
+        CopyScope copies(b);
         SBG_CUDA(cudaMemcpyAsync(&left, b->fbCount + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream),
                  "unfinished count");
         SBG_CUDA(cudaStreamSynchronize(b->stream), "unfinished count");
+        copies.done();
         if (left == 0) break;
         if (L >= limit) return fail(SBG_ERR_CUDA, "mixed integration did not finish its steps");
         target = L + 4;
@@ -1933,6 +1955,7 @@ int sbg_batch_get_qdotdot(sbg_batch b, double* qdotdot) {
     if (!b->realized) return fail(SBG_ERR_STATE, "the current state has not been realized through Acceleration");
     SBG_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     const int64_t nqT = b->nyTotal - b->nuTotal;
+    CopyScope copies(b);
     SBG_CUDA(launchQDotDot(b->T, b->dHostQOff, b->y, b->ydot, b->staging, b->stream), "qdotdot kernel launch");
     ++b->launches;
     void* dst = b->hostSide(qdotdot, nqT * sizeof(double));
@@ -1941,7 +1964,7 @@ int sbg_batch_get_qdotdot(sbg_batch b, double* qdotdot) {
              "qdotdot download");
     SBG_CUDA(cudaStreamSynchronize(b->stream), "qdotdot");
     if (dst != qdotdot) std::memcpy(qdotdot, dst, nqT * sizeof(double));
-    return SBG_OK;
+    return copies.done();
 }
 
 int sbg_rk_merson_adaptive(sbg_batch b, double t_final, const sbg_adaptive_opts* opts, int32_t* status,
