@@ -289,7 +289,7 @@ struct sbg_batch_s {
     // Where copies of `bytes` from or to the caller's buffer go: the buffer, or
     // the staging buffer from its byte `at` on (null: no memory).
     void* hostSide(const void* p, size_t bytes, size_t at = 0) {
-        if (pageable || isPinned(p)) return const_cast<void*>(p);
+        if (bytes == 0 || pageable || isPinned(p)) return const_cast<void*>(p);
         if (hostPinnedBytes < at + bytes) {
             void* q = nullptr;
             if (cudaMallocHost(&q, at + bytes) != cudaSuccess) {

@@ -4,6 +4,8 @@ with pageable host memory copied in place and by way of the staging buffer.
 
   - A call that returns an error has no copy from or to the caller's memory
     under way, and the same call succeeds afterwards.
+  - Batches without instances, or whose bodies have no coordinates, take the
+    calls that copy states in both modes.
 """
 import ctypes as C
 import subprocess
@@ -121,6 +123,21 @@ def test_no_copy_is_under_way_after_an_error(host, precision, n, pageable):
         else:
             pytest.fail(f"{name}: more runtime calls than expected")
     assert failed > 20
+    host.sbg_batch_destroy(b)
+    host.sbg_topology_destroy(topo)
+    host.fake_pageable(1)
+
+
+@pytest.mark.parametrize("pageable", [1, 0])
+@pytest.mark.parametrize("precision", [N.PRECISION_FP64, N.PRECISION_MIXED, N.PRECISION_MIXED_FAST])
+@pytest.mark.parametrize("n,mobilizers", [(0, [N.SBG_PIN]), (3, [N.SBG_WELD, N.SBG_WELD])])
+def test_batches_without_coordinates(host, precision, pageable, n, mobilizers):
+    host.fake_pageable(pageable)
+    topo = _topology(host, mobilizers)
+    b = _batch(host, topo, n, precision)
+    nu = 0 if n else 1
+    for name, call in _calls(host, b, n, nu, nu, len(mobilizers)).items():
+        assert call() == 0, (name, host.sbg_last_error())
     host.sbg_batch_destroy(b)
     host.sbg_topology_destroy(topo)
     host.fake_pageable(1)
