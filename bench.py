@@ -59,6 +59,8 @@ def _args():
     p.add_argument("--serve-sustained-rate", type=float, default=20.0,
                    help="arrival rate of the sustained serving run (requests/s)")
     p.add_argument("--serve-budget-gb", type=float, default=40.0)
+    p.add_argument("--section-seconds", type=float, default=900.0,
+                   help="time for the sections after the headline; then the line is printed without the rest")
     p.add_argument("--serve-deadline", type=float, default=90.0,
                    help="seconds after the first arrival at which unfinished requests are reported as censored")
     return p.parse_args()
@@ -514,6 +516,42 @@ def udot_rel_err(d_mixed, d_64, b):
     return errs
 
 
+def run_sections(result, sections, limit_s, report):
+    """Runs the extra sections, each into result[name], and prints the JSON
+    line. The extra sections never keep it from being printed: one that raises
+    leaves its error; when they take longer than limit_s altogether (a kernel
+    that does not return holds the host in a native call), the line is printed
+    without the rest and the process ends."""
+    lock = threading.Lock()
+    running = [""]  # the section; None: the line has been printed
+
+    def give_up():
+        with lock:
+            if running[0] is None:
+                return
+            line = dict(result, sections_unfinished=running[0])
+            if report:
+                print(json.dumps(line), flush=True)
+            os._exit(0)
+
+    timer = threading.Timer(limit_s, give_up)
+    timer.daemon = True
+    timer.start()
+    for name, section in sections:
+        running[0] = name
+        try:
+            value = section()
+        except Exception as e:  # noqa: BLE001
+            value = {"error": repr(e)}
+        with lock:
+            result[name] = value
+    with lock:
+        timer.cancel()
+        running[0] = None
+        if report:
+            print(json.dumps(result), flush=True)
+
+
 def run_ours(args):
     import torch
 
@@ -609,33 +647,26 @@ def run_ours(args):
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         result["cpu_baseline"] = cpu_baseline(w, args.cpu_seconds, min(args.instances, 65536))
-    try:
-        result["tree_operators"] = tree_operators(bmx, w, y0, 5, 8192)
-    except Exception as e:  # noqa: BLE001
-        result["tree_operators"] = {"error": repr(e)}
-    b64.close()
-    bmx.close()
-    # the extra sections never keep the headline line from being printed
+
+    def operators():
+        try:
+            return tree_operators(bmx, w, y0, 5, 8192)
+        finally:
+            b64.close()
+            bmx.close()
+
+    sections = [("tree_operators", operators)]
     if not args.no_trajectories:
-        try:
-            result["trajectories"] = trajectories()
-        except Exception as e:  # noqa: BLE001
-            result["trajectories"] = {"error": repr(e)}
+        sections.append(("trajectories", trajectories))
     if args.serve_seconds > 0:
-        try:
-            result["serving"] = serving(args.serve_seconds, args.serve_chunk, args.serve_budget_gb, 2e6,
-                                        args.serve_deadline)
-        except Exception as e:  # noqa: BLE001
-            result["serving"] = {"error": repr(e)}
+        sections.append(("serving", lambda: serving(args.serve_seconds, args.serve_chunk, args.serve_budget_gb, 2e6,
+                                                    args.serve_deadline)))
         # the same stream at a rate the server sustains (every request
         # finishes, the queue stays short): latency at sustained throughput
-        try:
-            result["serving_sustained"] = serving(args.serve_seconds * 4, args.serve_chunk, args.serve_budget_gb, 0,
-                                                  args.serve_deadline, rate=args.serve_sustained_rate)
-        except Exception as e:  # noqa: BLE001
-            result["serving_sustained"] = {"error": repr(e)}
-    if rank == 0:
-        print(json.dumps(result))
+        sections.append(("serving_sustained",
+                         lambda: serving(args.serve_seconds * 4, args.serve_chunk, args.serve_budget_gb, 0,
+                                         args.serve_deadline, rate=args.serve_sustained_rate)))
+    run_sections(result, sections, args.section_seconds, rank == 0)
     if world > 1:
         import torch.distributed as dist
 
