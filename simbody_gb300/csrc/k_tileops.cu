@@ -132,6 +132,8 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps)
             case CL_FREE: opJoint<CL_FREE>(r, par, rec, src, x, j); break;
             default: opJoint<CL_GEN>(r, par, rec, src, x, j); break;
             }
+            // on Ground a position enters nothing; a state that is not finite is reported
+            finite &= finiteBits(j.p.x) & finiteBits(j.p.y) & finiteBits(j.p.z);
             const M3<double> C = ci ? ident3<double>() : get9(par, PR_C);
             const M3<double> RL = ci ? j.E : mul(C, j.E);  // parent's axes <- these
             const Vec l = get3(par, PR_D) + (ci ? j.p : mul(C, j.p));

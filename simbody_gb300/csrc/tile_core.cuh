@@ -176,7 +176,8 @@ TILE_FN D rsqrtD(D x) {
 }
 // Quaternion (normalised here) -> R_FM (RigidBodyNodeSpec_Ball.h:134-214).
 TILE_FN M3<D> quatMatrix(const D* q) {
-    const D oo = rsqrtD(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+    D oo = rsqrtD(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+    if (!nonzero(oo)) oo = D(NAN);  // |q|^2 overflows: no rotation, not the identity that 1 - 0 would make
     const D e0 = q[0] * oo, e1 = q[1] * oo, e2 = q[2] * oo, e3 = q[3] * oo;
     const D f1 = e1 + e1, f2 = e2 + e2, f3 = e3 + e3;
     const D p01 = e0 * f1, p02 = e0 * f2, p03 = e0 * f3;
@@ -274,7 +275,9 @@ template <class PA> TILE_FN D mobForce(const PA& par, int info, int j, D q, D u)
 
 // ------------------------------------------------------------------ pass 1
 // Base to tip: joint rotation, spin, velocity terms, own inertia and force,
-// mobility forces, qdot. MINV: rest, the forces given by the source.
+// mobility forces, qdot. MINV: rest, the forces given by the source. out also gets
+// the positions: on Ground they enter nothing here, and a state that is not
+// finite is still reported.
 struct Model {
     const D* kpar;     // contact parameters
     const D* bodyPar;  // kParamStride per body row (contacts only)
@@ -406,6 +409,7 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const PA& par, const RC& r
         }
     } else if (CL == CL_SLIDER) {
         const D q0 = src.q(r.qo), u0 = MINV ? D(0) : src.u(r.uo);
+        out.position(q0);
         if (ci) l.x = l.x + q0;
         else l = l + q0 * Vec{par[PR_C], par[PR_C + 3], par[PR_C + 6]};
         out.qdot(r.qo, u0);
@@ -448,6 +452,9 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const PA& par, const RC& r
         Vec pf = zero(), uv = zero();
         if (CL == CL_FREE) {
             pf = Vec{src.q(r.qo + 4), src.q(r.qo + 5), src.q(r.qo + 6)};
+            out.position(pf.x);
+            out.position(pf.y);
+            out.position(pf.z);
             l = l + (ci ? pf : mul(get9(par, PR_C), pf));
         }
         constexpr int n = CL == CL_FREE ? 6 : 3;
@@ -487,6 +494,9 @@ TILE_FN void pass1(const Model& md, const SlotRow& r, const PA& par, const RC& r
         GenJoint j;
         pass1Gen<MINV>(r, par, rec, src, out, j);
         E = j.E;
+        out.position(j.p.x);
+        out.position(j.p.y);
+        out.position(j.p.z);
 #pragma unroll
         for (int k = 0; k < 9; ++k) rec[RC_E + k] = E.a[k];
         l = l + (ci ? j.p : mul(get9(par, PR_C), j.p));

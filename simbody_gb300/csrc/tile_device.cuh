@@ -332,6 +332,7 @@ template <int YS> struct TileOut {
     double* f;
     bool finite = true;
     __device__ __forceinline__ TileOut(TileCol<YS> col, double* p) : c(col), f(p) {}
+    __device__ __forceinline__ void position(double v) { finite &= tile::finiteBits(v); }
     __device__ __forceinline__ void qdot(int k, double v) { f[c.at(k)] = v; finite &= tile::finiteBits(v); }
     __device__ __forceinline__ void udot(int k, double v) { f[c.atU(k)] = v; finite &= tile::finiteBits(v); }
 };
@@ -340,6 +341,7 @@ template <int YS> struct TileUOut {  // M^-1 f: u slots only
     double* f;
     bool finite = true;
     __device__ __forceinline__ TileUOut(TileCol<YS> col, double* p) : c(col), f(p) {}
+    __device__ __forceinline__ void position(double) {}
     __device__ __forceinline__ void qdot(int, double) {}
     __device__ __forceinline__ void udot(int k, double v) { f[c.atU(k)] = v; finite &= tile::finiteBits(v); }
 };
