@@ -276,10 +276,12 @@ int sbg_realize_acceleration(sbg_batch batch, double* ydot, int32_t* status);
  * State::getYDot in one call, from and to host buffers (y and ydot in the
  * batch packing; status may be NULL): the same results as
  * sbg_batch_set_state(batch, NULL, y) + sbg_realize_acceleration. For a
- * batch of one topology on the one-thread-per-instance driver, the upload,
- * realize and download run in chunks of instances on several streams so
- * that copies overlap compute (after the batch's first realize has tuned
- * it); page-locked y/ydot/status are copied directly. Synchronous. */
+ * large batch in instance order without wide trees or loop closures (one
+ * chain topology), the upload, realize and download run in chunks of
+ * instances on several streams so that copies overlap compute (in the FP32
+ * forms after the batch's first realize has tuned it). Host arrays are copied
+ * directly where they are page-locked or the GPU uses the host's page
+ * tables. Synchronous. */
 int sbg_realize_acceleration_host(sbg_batch batch, const double* y, double* ydot, int32_t* status);
 
 /* SimbodyMatterSubsystem::multiplyByMInv(state, f, MInvf)
@@ -399,7 +401,8 @@ int sbg_batch_sync(sbg_batch batch);
 int64_t sbg_batch_launch_count(sbg_batch batch);
 /* Occupancy variant the batch's tuner picked for its FP32 kernels (1 = two
  * 128-thread blocks per SM, 4 = four, 7 = seven 64-thread blocks per SM for
- * the one-thread-per-instance segment), 0 before the first realize or
+ * the one-thread-per-instance segment, 8 = 7 with staged records, 9 = tiles of
+ * branching trees), 1 for an FP64 batch, 0 before the first realize or
  * integration, -1 for a null batch. No counterpart in the reference. */
 int sbg_batch_kernel_variant(sbg_batch batch);
 /* Lanes-per-tree setting the tuner picked for the batch's level-parallel

@@ -19,9 +19,9 @@
 // trees) to the few-1e-6 level set by the FP32 kinematics, as long as M is
 // well conditioned. Where the correction exceeds 1e-4 of udot (an
 // ill-conditioned M, the FP32 factorisation too poor for the refinement to
-// converge) the instance is flagged SBG_INST_ILL_CONDITIONED and, in a
-// realize or the server's mixed lane, recomputed in FP64 on an FP64 mirror
-// of its records.
+// converge) the instance is flagged SBG_INST_ILL_CONDITIONED and recomputed in
+// FP64: in a realize on the FP64 tiles (tile_device.cuh), in the server's mixed
+// lane on an FP64 mirror of its records.
 //
 // Two mappings drive the same per-body code:
 //   chain driver  one thread per instance walks its rows in order; along a
@@ -1286,7 +1286,7 @@ __device__ __forceinline__ int rhs(const DevTables& T, const Slot& s, R* scratch
         double* rec0 = scratch + T.sbase[s.inst];
         // tree passes on the group's lanes; the multiplier solve and the
         // constraint sweeps (loop paths only) on its first lane, the
-        // Gram columns on its first three
+        // Gram columns on its first three, or on one each;
         // record-major rows (the first lane's serial loop work touches a
         // few records many times: they stay in L1)
         const ScrGen S{rec0, (int)T.sstride[s.inst], 1};

@@ -1,7 +1,7 @@
 // k_loops.cu -- kernels of the loop-closure segments (FP64) on the
 // level-parallel driver: the tree passes on the lanes of each instance's
-// group, the Gram columns on three of them, the multiplier solve and the
-// projections on its first. Blocks [loopGroupFirst, +nLoopGroupBlocks) of the
+// group, the Gram columns on as many of them (three where the records have no
+// fields for more), the multiplier solve and the projections on its first. Blocks [loopGroupFirst, +nLoopGroupBlocks) of the
 // block table; records record-major (width in T.sstride). The server's blocks
 // have 128 threads, a batch's one warp. 300 trees of 20 to 40 bodies, a fifth
 // with closures, two steps: 13.1 ms, of which the busiest warp's FP64

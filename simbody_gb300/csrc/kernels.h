@@ -45,7 +45,7 @@ constexpr int kMaxStepsPerCall = 1 << 30;
 struct BatchBufs {
     void* scratch;       // scratch of the chain and group segments (R)
     void* scratchLoop;   // FP64 scratch of the loop-closure segment
-    void* fbuf;          // RK stage derivatives (R), 4 planes of fplane elements
+    void* fbuf;          // RK stage derivatives (R), 4 planes of fplane elements; FP64: and the stage input
     void* fbufLoop;      // FP64 stage derivatives of the loop-closure segment, 4 planes
     int64_t fplane;
     const TileSet* tiles;  // FP64: the chain and group segments' tiles (mixed form: for its FP64 work)
@@ -119,7 +119,7 @@ inline Launch1D spread(int64_t n, int bs) {
     return Launch1D{(int)((n + bs - 1) / bs), bs};
 }
 
-// Error-controlled RK-Merson (k_rkadapt.cu): Integrator::setFinalTime(tFinal),
+// Error-controlled RK-Merson (k_tileadapt.cu): Integrator::setFinalTime(tFinal),
 // initialize, stepTo(tFinal) with the given initial, minimum and maximum step
 // sizes (<= 0: the reference's defaults: initial 0.01, no limits) and at most
 // maxSteps accepted steps per instance. stats: accepted and rejected steps per
@@ -130,8 +130,8 @@ struct AdaptCtl {
     long long* stats;
 };
 
-// Per-segment launchers (k_r64.cu, k_r32c.cu, k_r32g.cu, k_rk64.cu,
-// k_rk32c.cu, k_rk32g.cu).
+// Per-segment launchers (k_r32c.cu, k_r32g.cu, k_rk64.cu, k_rk32c.cu,
+// k_rk32g.cu, k_loops.cu, k_tile*.cu).
 struct KArgs {
     const DevTables* T;
     const LaunchPlan* P;

@@ -4,9 +4,9 @@
 //
 // The one-thread driver is bound by latency: a few warps per SM, each walking
 // its 32 trees' rows one after another through five passes of dependent loads
-// and FP32 chains, lanes apart on mobilizers. Here up to eight warps share the
+// and FP32 chains, lanes apart on mobilizers. Here up to four warps share the
 // 32 trees, a body of each a step, so a pass has as many steps as the trees are
-// deep or an eighth of their rows, whichever is more. Every routine and the
+// deep or a quarter of their rows, whichever is more. Every routine and the
 // order in which a parent's children add to it (falling rows, kept by the
 // schedule) are the chain driver's, so the results are the same bit for bit.
 #pragma once
