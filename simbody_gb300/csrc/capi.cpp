@@ -1236,10 +1236,23 @@ static int createBatch(const sbg_topology* topos, int32_t ntopo, const int32_t* 
     if (precision != SBG_PRECISION_FP64 && !lean && (rc = buildTiles32(b))) return bail(rc);
     if (b->variant == 9 && !b->tiles32.ntiles) b->variant = 7;
     if (precision == SBG_PRECISION_MIXED && (rc = buildTiles(b, lean ? kTilesLean : kTilesOnes, &b->ones))) return bail(rc);
-    if (precision == SBG_PRECISION_FP64 || (precision == SBG_PRECISION_MIXED && (lean || ninst > 2 * b->sms))) {
-        rc = lean ? buildTilesLean(b, &b->ones, &b->tiles) : buildTiles(b, kTilesWide, &b->tiles);
-        if (rc) return bail(rc);
+    const bool mixed = precision == SBG_PRECISION_MIXED;
+    bool fromOnes = lean && (mixed || precision == SBG_PRECISION_FP64);
+    if (!lean && (precision == SBG_PRECISION_FP64 || (mixed && ninst > 2 * b->sms))) {
+        AllocScope scope(b);
+        rc = buildTiles(b, kTilesWide, &b->tiles);
+        // a mixed batch's where they leave room for what later calls allocate
+        if (!rc && mixed && b->budget > 0 && b->devBytes + lazyBytes(b) > b->budget)
+            rc = fail(SBG_ERR_BUDGET, "device budget exceeded by wide tiles");
+        if (!rc) {
+            scope.keep();
+        } else {
+            b->tiles = TileSet{};
+            if (!mixed || !noRoom(rc)) return bail(rc);
+            fromOnes = true;
+        }
     }
+    if (fromOnes && (rc = buildTilesLean(b, &b->ones, &b->tiles))) return bail(rc);
     cudaError_t e = cudaMemsetAsync(b->time, 0, std::max<int64_t>(ninst, 1) * sizeof(double), b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->status, 0, std::max<int64_t>(ninst, 1) * sizeof(int32_t), b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

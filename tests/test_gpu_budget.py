@@ -131,3 +131,30 @@ def test_a_small_budget_costs_time_not_the_batch(engine, precision, config, n, a
                 np.testing.assert_allclose(a, want[k], rtol=0, atol=tol * np.abs(want[k]).max(), err_msg=k)
             else:
                 np.testing.assert_array_equal(a, want[k], err_msg=f"{k} within {budget} bytes")
+
+
+def test_a_mixed_batch_keeps_its_fp32_tiles_without_wide_fp64_ones(engine):
+    """Of a mixed batch the wide FP64 tiles go first: with room for all but
+    those, realize and steps stay on the FP32 tiles, operators work, and the
+    results agree with those of a batch with room (FP64 work: parity tolerances)."""
+    w = Workload(3, 700)
+    topo = [Topology(w.systems[k], keepalive=w) for k in range(w.nsys)]
+    fast = Batch(topo, w.instance_system, precision="mixed_fast")
+    fast.set_state(w.y0)
+    wide = -fast.device_bytes
+    fast.multiply_by_m(np.ones(fast.u_offsets[-1]))
+    wide += fast.device_bytes  # the wide FP64 tiles and the operators' operands
+    need = Batch(topo, w.instance_system, precision="mixed").device_bytes
+    out = []
+    for budget in (0, need, need - wide // 2):
+        b = Batch(topo, w.instance_system, precision="mixed", device_budget_bytes=budget)
+        b.set_state(w.y0)
+        d, st = b.realize_acceleration()
+        assert b.kernel_variant == 9 and (st == 0).all()
+        mv = b.multiply_by_m(np.ones(b.u_offsets[-1]))[0]
+        b.rk_merson_fixed(w.h, 2)
+        out.append((d, mv, b.get_state()[0]))
+        assert not budget or b.device_bytes <= budget
+    for o in out[1:]:
+        for a, c, tol in zip(o, out[0], (1e-12, 0, 1e-10)):
+            np.testing.assert_allclose(a, c, rtol=0, atol=tol * np.abs(c).max())
