@@ -216,7 +216,11 @@ typedef struct sbg_adaptive_opts {
 typedef struct sbg_batch_config {
     int32_t precision;            /* sbg_precision */
     int32_t device;               /* CUDA device ordinal */
-    int64_t device_budget_bytes;  /* 0 = no limit */
+    /* 0 = no limit. A batch whose tiles do not fit is created without them where
+     * one record per body fits, with the same results and at a lower speed; a
+     * call whose own buffers do not fit returns SBG_ERR_BUDGET and keeps
+     * nothing. */
+    int64_t device_budget_bytes;
 } sbg_batch_config;
 
 typedef struct sbg_topology_s* sbg_topology;
